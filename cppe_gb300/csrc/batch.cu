@@ -44,6 +44,7 @@ void Geometry::combine(const std::vector<const Geometry*>& parts, int copies, Ge
   out.damping   = parts[0]->damping;
   out.theta     = parts[0]->theta;
   out.ncopies   = copies;
+  for (auto* p : parts) out.grid = std::max(out.grid, p->grid);
   // cells: by (level, segment, cell)
   std::vector<std::vector<int>> cmap(nseg);
   for (int s = 0; s < nseg; ++s) cmap[s].assign(parts[part_of(s)]->layout.ncells, -1);
@@ -130,6 +131,8 @@ void Geometry::combine(const std::vector<const Geometry*>& parts, int copies, Ge
       out.h_pos64.push_back(p->h_pos64[k]);
       out.h_hi.push_back(p->h_hi[k]);
       out.h_lo.push_back(p->h_lo[k]);
+      out.h_mid.push_back(p->h_mid[k]);
+      out.h_low.push_back(p->h_low[k]);
     }
     if (out.h_cptr.empty()) out.h_cptr.push_back(0);
     for (int k = 0; k < p->n; ++k) {

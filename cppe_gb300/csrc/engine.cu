@@ -2,7 +2,7 @@
 // the FMM passes and the finishing pass.
 //
 // Reference counterparts (maxscheurer/cppe, src/core/fmm/):
-//   k_p2p, k_p2p32_m1, k_p2p_dd2
+//   k_p2p, k_p2p64 (near64.cuh), k_p2p32_m1, k_p2p_dd2
 //              evaluate_direct{,_damping} calculate.cc:262-300,
 //              evaluate_P2P_lazy + P2P_Cells{,_damping} calculate.cc:29-72,205-225
 //   k_p2m_tasks + k_msum
@@ -44,6 +44,8 @@ constexpr int M2M_TASK_LEAVES = 8;    // leaf multipoles shifted per upward-pass
 constexpr bool M2L_TABLE_FP64 = true;  // FP64 M2L from tabulated derivative tensors
 constexpr int PW = PMAX + 1;          // powers 0..PMAX of one coordinate
 constexpr int FINISH_BLOCK = 128;
+constexpr int NEAR64_ETAB  = 12 * 16 + 8;  // e^(-k/16) in FP64, v < 12 and a grid step
+constexpr int NEAR64_DDTAB = 26 * 16 + 2;  // the same as double-float pairs, v < 26
 
 // ---------------------------------------------------------------------------
 // Table uploads
@@ -97,6 +99,9 @@ TreeView Geometry::view() const {
 void Geometry::build(int n_, const double* xyz, const double* s_damp, const int* excl_ptr,
                      const int* excl_idx, bool fmm_, int ncrit_, double theta_,
                      cudaStream_t s) {
+  // small direct systems in chunks of 32 (999 sites: 1,024 work items instead of
+  // 256, evenly over the SMs)
+  direct_chunk = n_ < 4096 ? 32 : 64;
   prepare(n_, xyz, s_damp, excl_ptr, excl_idx, fmm_, ncrit_, theta_);
   upload(s);
 }
@@ -115,9 +120,9 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
     make_layout(t, n, L);
     level_start = L.level_start;
   } else {
-    // Direct summation: chunks of 64 sites in caller order act as "leaves",
+    // Direct summation: chunks of sites in caller order act as "leaves",
     // every chunk interacting with every chunk.
-    const int chunk = 64;
+    const int chunk = direct_chunk;
     L           = TreeLayout();
     L.n         = n;
     L.nleaves   = (n + chunk - 1) / chunk;
@@ -172,6 +177,10 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
     if (n) ext = std::max(ext, 0.5 * (hi_c[c] - lo_c[c]) * 1.0001);
   }
   const double quantum = std::ldexp(1.0, (int)std::ceil(std::log2(ext)) - 22);
+  const double fine    = std::ldexp(quantum, -22);  // grid of the remainders' leading parts
+  grid = quantum;
+  h_mid.assign(n, float4{});
+  h_low.assign(n, float4{});
   auto& p64 = h_pos64;
   auto& hi  = h_hi;
   auto& lo  = h_lo;
@@ -181,14 +190,22 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
     const double sd = s_damp ? s_damp[i] : 0.0;
     p64[k]         = make_double4_32a(x, y, z, sd);
     double r[3]    = {x - ctr[0], y - ctr[1], z - ctr[2]};
-    float h[3], l[3];
+    float h[3], l[3], m[3], e[3];
+    const double in[3] = {x, y, z};
     for (int c = 0; c < 3; ++c) {
       h[c] = (float)(std::nearbyint(r[c] / quantum) * quantum);
       l[c] = (float)(r[c] - (double)h[c]);
+      // three parts: the rounding of x - ctr (a two-sum) goes to the last one
+      const double rem = r[c] - (double)h[c], b = r[c] - in[c];
+      const double rerr = (in[c] - (r[c] - b)) + (-ctr[c] - b);
+      m[c] = (float)(std::nearbyint(rem / fine) * fine);
+      e[c] = (float)((rem - (double)m[c]) + rerr);
     }
     const float sh = (float)sd;
     hi[k]          = make_float4(h[0], h[1], h[2], sh);
     lo[k]          = make_float4(l[0], l[1], l[2], (float)(sd - (double)sh));
+    h_mid[k]       = make_float4(m[0], m[1], m[2], 0.f);
+    h_low[k]       = make_float4(e[0], e[1], e[2], (float)(sd - (double)sh));
   }
 
   // Exclusion corrections: pairs the reference skips but the near-field pass
@@ -277,6 +294,13 @@ bool m2l_vectors(const TreeLayout& L, std::vector<int>& vid, std::vector<double4
 void Geometry::make_vectors() {
   // off the grid: the M2L builds each tensor itself
   if (!fmm || !m2l_vectors(layout, h_m2l_vid, h_vec)) h_m2l_vid.clear(), h_vec.clear();
+}
+
+// Pairs per near-field work item: 32 items per SM, at least 8,192 pairs each
+// while that still gives every SM eight items, at least 1,024 below that.
+long default_item_pairs(long total) {
+  return std::max(total / (32L * 152),
+                  std::min(8192L, std::max(1024L, total / (8L * 152))));
 }
 
 // Cuts every target leaf's source list into pieces of about `W` pairs so that
@@ -391,7 +415,7 @@ void Geometry::make_schedules() {
       total += na * (L.leaf_start[b + 1] - L.leaf_start[b]);
     }
   }
-  const long W = item_pairs > 0 ? item_pairs : std::max<long>(8192, total / (32L * 152));
+  const long W = item_pairs > 0 ? item_pairs : default_item_pairs(total);
   struct It {
     long w;
     int4 v;
@@ -543,6 +567,30 @@ void Geometry::upload_schedules(cudaStream_t s) {
   cell_chunk_ptr.upload(h_cell_chunk_ptr, s);
 }
 
+// e^-v = hi + lo to about 100 bits, 0 <= v < 64: the Taylor series of e^(-v / 64)
+// in pairs of doubles (two-sum additions, FMA products), squared six times.
+static void exp_neg_pair(double v, double& hi, double& lo) {
+  auto add = [](double ah, double al, double bh, double bl, double& h, double& l) {
+    const double s = ah + bh, b = s - ah;
+    const double e = ((ah - (s - b)) + (bh - b)) + (al + bl);
+    h = s + e, l = e - (h - s);
+  };
+  auto mul = [](double ah, double al, double bh, double bl, double& h, double& l) {
+    const double p = ah * bh, e = std::fma(ah, bh, -p) + (ah * bl + al * bh);
+    h = p + e, l = e - (h - p);
+  };
+  const double t = -v / 64.0;  // exact
+  double sh = 1.0, sl = 0.0;
+  for (int k = 24; k >= 1; --k) {  // Horner: s = 1 + (t / k) s
+    const double qh = t / k, ql = -std::fma(qh, (double)k, -t) / k;
+    double ph, pl;
+    mul(sh, sl, qh, ql, ph, pl);
+    add(1.0, 0.0, ph, pl, sh, sl);
+  }
+  for (int k = 0; k < 6; ++k) mul(sh, sl, sh, sl, sh, sl);
+  hi = sh, lo = sl;
+}
+
 void Geometry::upload(cudaStream_t s) {
   {
     std::vector<float2> tab(DD_EXP_TAB);
@@ -551,6 +599,15 @@ void Geometry::upload(cudaStream_t s) {
       tab[k]         = make_float2((float)e, (float)(e - (double)(float)e));
     }
     dd_exp.upload(tab, s);
+    tab.resize(NEAR64_DDTAB);
+    std::vector<double> tab64(2 * NEAR64_ETAB);  // value and rest (a Taylor product below)
+    for (int k = 0; k < NEAR64_DDTAB; ++k) {
+      const double e = std::exp(-0.0625 * k);
+      tab[k]         = make_float2((float)e, (float)(e - (double)(float)e));
+      if (k < NEAR64_ETAB) exp_neg_pair(0.0625 * k, tab64[2 * k], tab64[2 * k + 1]);
+    }
+    near_exp.upload(tab, s);
+    near_exp64.upload(tab64, s);
   }
   items.upload(h_items, s);
   item_split.upload(h_item_split, s);
@@ -602,6 +659,8 @@ void Geometry::upload(cudaStream_t s) {
   pos64.upload(h_pos64, s);
   hi32.upload(h_hi, s);
   lo32.upload(h_lo, s);
+  mid32.upload(h_mid, s);
+  low32.upload(h_low, s);
   corr_ptr.upload(h_cptr, s);
   corr_idx.upload(h_cidx.empty() ? std::vector<int>{0} : h_cidx, s);
   CG_CUDA(cudaStreamSynchronize(s));
@@ -1729,6 +1788,10 @@ __global__ void __launch_bounds__(P2P_BLOCK)
   }
 }
 
+}  // namespace cg
+#include "near64.cuh"
+namespace cg {
+
 // ---------------------------------------------------------------------------
 // Double-float near field over a batch's right-hand sides together (the
 // residual counterpart of k_p2p32_m1_multi): the pair tensor G1 I + G2 r r^T
@@ -2348,9 +2411,16 @@ struct SegSkip {
   const int* skip     = nullptr;
 };
 
+// Excluded pairs that the near-field pass has left out itself (k_p2p64's near
+// ones): class by near64_class, when hi is set.
+struct NearSkip {
+  const float4* hi = nullptr;
+  float damping    = 0.f;
+};
+
 template <typename T, int M, int MODE, int P = 0>
 __global__ void __launch_bounds__(FINISH_BLOCK) k_finish(int n, const int* __restrict__ leaf_nslot, const T* __restrict__ Fnear,
-                         SymRows<T> sr, SegSkip sk,
+                         SymRows<T> sr, SegSkip sk, NearSkip ns,
                          int use_fmm,
                          TreeView tv, OpsView ov, const T* __restrict__ L, PosArgs<T> pa,
                          CellPos<T> cp, const T* __restrict__ src,
@@ -2407,6 +2477,9 @@ __global__ void __launch_bounds__(FINISH_BLOCK) k_finish(int n, const int* __res
       T cx = 0, cy = 0, cz = 0;
       for (int e = e0; e < e1; ++e) {
         const int j = corr_idx[e];
+        if (ns.hi && (damp ? near64_class<true>(ns.hi[i], ns.hi[j], ns.damping)
+                           : near64_class<false>(ns.hi[i], ns.hi[j], ns.damping)))
+          continue;
         if (damp)
           pair_field<T, M, true>(me, ai, pa.load(j), src + (size_t)j * NS, cx, cy, cz);
         else
@@ -2417,9 +2490,17 @@ __global__ void __launch_bounds__(FINISH_BLOCK) k_finish(int n, const int* __res
     if (MODE == FINISH_APPLY) {
       const T* a  = ainv6 + 6 * (size_t)i;
       const T* sv = src + 3 * (size_t)i;
-      const T o0  = f[0] + (a[0] * sv[0] + a[1] * sv[1] + a[2] * sv[2]);
-      const T o1  = f[1] + (a[1] * sv[0] + a[3] * sv[1] + a[4] * sv[2]);
-      const T o2  = f[2] + (a[2] * sv[0] + a[4] * sv[1] + a[5] * sv[2]);
+      T o0, o1, o2;
+      if constexpr (sizeof(T) == 8) {
+        // the largest product last and unrounded
+        o0 = fma(a[0], sv[0], fma(a[1], sv[1], fma(a[2], sv[2], f[0])));
+        o1 = fma(a[3], sv[1], fma(a[1], sv[0], fma(a[4], sv[2], f[1])));
+        o2 = fma(a[5], sv[2], fma(a[2], sv[0], fma(a[4], sv[1], f[2])));
+      } else {
+        o0 = f[0] + (a[0] * sv[0] + a[1] * sv[1] + a[2] * sv[2]);
+        o1 = f[1] + (a[1] * sv[0] + a[3] * sv[1] + a[4] * sv[2]);
+        o2 = f[2] + (a[2] * sv[0] + a[4] * sv[1] + a[5] * sv[2]);
+      }
       out[3 * (size_t)i]     = o0;
       out[3 * (size_t)i + 1] = o1;
       out[3 * (size_t)i + 2] = o2;
@@ -2597,6 +2678,24 @@ static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, doubl
   CG_LAUNCH();
 }
 
+static void launch_p2p64(const Geometry& g, bool damp, const double* src, double damping,
+                         double* Fnear, cudaStream_t s, const int* seg_done) {
+  const int grid  = (int)g.h_items.size();
+  const int* lseg = seg_done ? g.leaf_seg.p : nullptr;
+  if (seg_done && !lseg) fail(CPPE_GPU_INVALID_ARG, "segment mask without segments");
+  const Pos3 ps{g.hi32.p, g.mid32.p, g.low32.p};
+  auto run = [&](auto d) {
+    k_p2p64<decltype(d)::value><<<grid, P2P_BLOCK, 0, s>>>(
+          g.n, g.leaf_start.p, g.items.p, g.p2p_src.p, ps, g.pos64.p, src, g.near_exp.p,
+          g.near_exp64.p, damping, g.corr_ptr.p, g.corr_idx.p, Fnear, lseg, seg_done);
+  };
+  if (damp)
+    run(std::true_type{});
+  else
+    run(std::false_type{});
+  CG_LAUNCH();
+}
+
 template <typename T>
 void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m, const T* src,
                 bool damp, double damping, FinishMode mode, const T* ainv6, T* out,
@@ -2728,9 +2827,16 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
   const bool fast = near_mode != NEAR_FP64;
   bool done       = false;
   SymRows<T> sym_rows;  // set when the symmetric near field ran
+  NearSkip nskip;       // set when the near-field pass leaves excluded pairs out
   if constexpr (std::is_same<T, double>::value) {
     if (near_mode == NEAR_DD && m == 1) {
       launch_p2p_dd(g, damp, src, damping, w, s);
+      done = true;
+    } else if (m == 1 && g.grid <= NEAR64_GRID) {
+      // (k_p2p keeps systems of more than 2^18 bohr, whose coordinate grid is too
+      // coarse for the distance classes)
+      launch_p2p64(g, damp, src, damping, w.Fnear.p, s, seg_done);
+      nskip.hi = g.hi32.p, nskip.damping = (float)damping;
       done = true;
     }
   }
@@ -2768,7 +2874,7 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
   SegSkip sk;  // a batch's masked segments (site-value dots only: no grid sum)
   if (seg_done && (!dot || !dot->partials)) sk.leaf_seg = g.leaf_seg.p, sk.skip = seg_done;
 #define CG_FINISH(TT, MM, MODE, PP)                                                           \
-  k_finish<TT, MM, MODE, PP><<<nb, FB, 0, s>>>(n, g.leaf_nslot.p, w.Fnear.p, sym_rows, sk, g.fmm ? 1 : 0, tv, ov, Lp, \
+  k_finish<TT, MM, MODE, PP><<<nb, FB, 0, s>>>(n, g.leaf_nslot.p, w.Fnear.p, sym_rows, sk, nskip, g.fmm ? 1 : 0, tv, ov, Lp, \
                                            pos_args<TT>(g), cell_pos<TT>(g), src, damp ? 1 : 0, \
                                            dampT, g.corr_ptr.p, g.corr_idx.p, ainv6, out,    \
                                            out64, sign, rs)

@@ -80,12 +80,17 @@ __host__ __device__ constexpr int m_stride(int ms) { return (ms + 3) & ~3; }
 
 constexpr int M2L_CHUNK = 64;  // built-in sources of one target cell per M2L warp
 
+// Built-in size (target-source pairs) of the near-field work items for a
+// system with `total` pairs.
+long default_item_pairs(long total);
+
 // Geometry: the sites, their permutation and the interaction structure.
 struct Geometry {
   int n       = 0;
   bool fmm    = false;
   int ncrit   = 64;
   double theta = 0.5;
+  int direct_chunk = 64;  // sites per "leaf" of a direct-summation geometry
   TreeLayout layout;
   std::vector<int> level_start;
   DBuf<double> center;
@@ -94,6 +99,14 @@ struct Geometry {
   DBuf<int> perm, inv_perm;  // perm[k] = caller index of site k
   DBuf<double4_32a> pos64;
   DBuf<float4> hi32, lo32;
+  // the FP64 operator's three-part coordinates: hi32 plus the remainder on a
+  // finer grid (mid32) plus what is left (low32; w: s - float(s)), and the
+  // tables of e^-(k/16) of its Thole factors (near64.cuh)
+  std::vector<float4> h_mid, h_low;
+  DBuf<float4> mid32, low32;
+  DBuf<float2> near_exp;
+  DBuf<double> near_exp64;
+  double grid = 0.0;    // spacing of hi32's grid (bohr)
   DBuf<float2> dd_exp;  // e^-(k/16), k = 0..320, as double-float pairs
   // pairs the reference skips (exclusions) that the near-field pass computed
   DBuf<int> corr_ptr, corr_idx;

@@ -409,7 +409,7 @@ double autotune_schedule(Geometry& geo, SideStream& side, cudaStream_t stream, i
     for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q)
       total += (long)(L.leaf_start[a + 1] - L.leaf_start[a]) *
                (L.leaf_start[L.p2p_src[q] + 1] - L.leaf_start[L.p2p_src[q]]);
-  const long w0 = std::max<long>(8192, total / (32L * 152));
+  const long w0 = default_item_pairs(total);
   const long ws[3]  = {std::max<long>(4096, w0 / 2), w0, 2 * w0};
   const int chs[3]  = {32, 64, 128};
   const int nch     = geo.fmm ? 3 : 1;

@@ -1,0 +1,75 @@
+"""The FP64 dipole operator's near field (far pairs in double-float, near pairs
+in FP64) against the oracle, at the sizes and inputs where its split can go
+wrong: one chunk and its edges, the staged tile's edges (304 sources), leaves
+of more than 128 sites, every pair near, every pair far, excluded far pairs,
+moments at the ends of the FP64 range, and systems too large for the split.
+
+Tolerance: a sum of n terms in FP64 (the oracle's and the kernel's) rounds to
+about sqrt(n) 2^-53 of its largest terms; far terms carry 5e-14 of themselves
+at most and are below 2 / 24^3 = 1.5e-4 of a unit moment against
+alpha^-1 >= 0.17, i.e. 4e-17 of the result each.  4e-15 in norm covers n <=
+3,000 with a factor of two.
+"""
+import numpy as np
+import pytest
+
+import cabi
+
+pytestmark = pytest.mark.gpu
+DAMPING = 2.1304
+TOL = 4e-15
+
+
+def close(a, ref, tol=TOL):
+    assert np.linalg.norm(a - ref) < tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("damp", [False, True])
+@pytest.mark.parametrize("waters", [1, 10, 11, 22, 43, 101, 102, 333, 700])
+def test_direct_sizes(gpu, port, waters, damp):
+    from cppe_gb300 import synthetic
+    b = synthetic.water_box(waters, seed=waters)
+    s = cabi.System(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, damp=damp)
+    v = np.random.default_rng(1).normal(size=3 * b.n)
+    ref = port.bmatrix_apply(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, v, fmm=0,
+                             damping=DAMPING if damp else 0.0)
+    close(s.apply(v), ref)
+    # powers of two scale the result exactly
+    for e in (-900, 900):
+        assert np.array_equal(s.apply(v * 2.0 ** e), s.apply(v) * 2.0 ** e)
+    s.close()
+
+
+@pytest.mark.parametrize("ncrit", [16, 64, 300])
+def test_fmm_leaf_sizes(gpu, port, ncrit):
+    from cppe_gb300 import synthetic
+    b = synthetic.water_box(900, seed=5)
+    s = cabi.System(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, damp=True, summation=cabi.FMM,
+                    order=5, ncrit=ncrit)
+    v = np.random.default_rng(2).normal(size=3 * b.n)
+    ref = port.bmatrix_apply(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, v, fmm=1, ncrit=ncrit,
+                             order=5, theta=0.5, damping=DAMPING)
+    close(s.apply(v), ref)
+    s.close()
+
+
+@pytest.mark.parametrize("damp", [False, True])
+@pytest.mark.parametrize("spacing", [1.5, 24.0, 40.0, 3.0e4])
+def test_distance_classes(gpu, port, spacing, damp):
+    """A jittered lattice of 343 sites with random (near and far) exclusions:
+    all near, around the 24-bohr limit, all far, and 2^18 bohr across."""
+    rng = np.random.default_rng(7)
+    g = np.stack(np.meshgrid(*[np.arange(7.0)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    xyz = spacing * (g + rng.uniform(-0.1, 0.1, g.shape))
+    n = xyz.shape[0]
+    alpha6 = np.zeros((n, 6))
+    alpha6[:, [0, 3, 5]] = rng.uniform(1.0, 12.0, (n, 1))
+    excl = [sorted(rng.choice(n, rng.integers(0, 9), replace=False)) for _ in range(n)]
+    ptr = np.concatenate([[0], np.cumsum([len(e) for e in excl])]).astype(np.int32)
+    idx = np.array([j for e in excl for j in e], np.int32)
+    s = cabi.System(xyz, alpha6, ptr, idx, damp=damp)
+    v = rng.normal(size=3 * n)
+    v[: 3 * (n // 2)] *= 1e-30  # a range of moments within the tiles
+    ref = port.bmatrix_apply(xyz, alpha6, ptr, idx, v, fmm=0, damping=DAMPING if damp else 0.0)
+    close(s.apply(v), ref)
+    s.close()
