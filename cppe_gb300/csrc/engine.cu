@@ -41,7 +41,6 @@ constexpr int M2L_WARPS  = 4;
 constexpr int P2M_LEAF_SITES  = 128;  // sites staged per round of the leaf P2M
 constexpr int M2M_TASK_LEAVES = 8;    // leaf multipoles shifted per upward-pass task
 // M2L_CHUNK (engine.h): sources of one target cell per M2L warp
-constexpr bool M2L_TABLE_FP64 = true;  // FP64 M2L from tabulated derivative tensors
 constexpr int PW = PMAX + 1;          // powers 0..PMAX of one coordinate
 constexpr int FINISH_BLOCK = 128;
 constexpr int NEAR64_ETAB  = 12 * 16 + 8;  // e^(-k/16) in FP64, v < 12 and a grid step
@@ -2627,14 +2626,6 @@ void SideStream::destroy() {
   s = hi = lo = nullptr, fork = join = nullptr;
 }
 
-__global__ void k_split_dd_vec(long n, const double* __restrict__ in, float2* __restrict__ out) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double v = in[i];
-  const float h  = (float)v;
-  out[i]         = make_float2(h, (float)(v - (double)h));
-}
-
 __global__ void k_split_dd(long n, const double* __restrict__ in, float2* __restrict__ out) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -2766,30 +2757,27 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
       CG_LAUNCH();
     }
     mark(1);
-    w.Lpart.alloc((size_t)std::max<size_t>(1, g.h_m2l_chunks.size()) * ov.lsize);
     bool m2l_done = false;
     // tabulated tensors of the distinct M2L vectors (fixed orders): in FP64
     // and double-float, where the recurrence is the expensive part; the FP32
     // translation builds its tensor in registers faster than it loads one
-    const T* dtab_t = nullptr;
-    if constexpr (std::is_same<T, double>::value)
-      if (fixedP && M2L_TABLE_FP64)
-        dtab_t = static_cast<const T*>(m2l_dtab<T>(g, ov.m, ov.p, w, false, fs));
+    const int nchunks = (int)g.h_m2l_chunks.size();
     if constexpr (std::is_same<T, double>::value) {
-      if (near_mode == NEAR_DD) {
-        w.Mdd.alloc((size_t)std::max(1, tv.ncells) * mst);
-        const float2* dtdd =
-              static_cast<const float2*>(m2l_dtab<T>(g, ov.m, ov.p, w, true, fs));
-        m2l_done = launch_m2l_dd(tv, ov.m, ov.p, g.m2l_chunks.p, (int)g.h_m2l_chunks.size(),
-                                 g.cell_chunk_ptr.p, w.M.p, mst, w.Mdd.p, w.Lpart.p, w.L.p,
-                                 ov.lsize, fs, dtdd, dtdd ? g.m2l_vid.p : nullptr);
+      if (fixedP && near_mode == NEAR_DD) {
+        const void* dt = m2l_dtab<T>(g, ov.m, ov.p, w, true, fs);
+        m2l_done = launch_m2l_fixed<true>(tv, ov.m, ov.p, g.m2l_chunks.p, nchunks,
+                                          g.cell_chunk_ptr.p, w.M.p, w.Mdd, w.Lpart, w.L.p, fs,
+                                          nullptr, nullptr, dt, dt ? g.m2l_vid.p : nullptr);
       }
     }
-    if (m2l_done ||
-        launch_m2l_fixed<T>(tv, ov.m, ov.p, g.m2l_chunks.p, (int)g.h_m2l_chunks.size(),
-                            g.cell_chunk_ptr.p, w.M.p, w.Lpart.p, w.L.p, ov.lsize, fs, cseg,
-                            seg_done, dtab_t, dtab_t ? g.m2l_vid.p : nullptr)) {
-    } else {
+    if (fixedP && !m2l_done) {
+      const void* dt = nullptr;
+      if constexpr (std::is_same<T, double>::value) dt = m2l_dtab<T>(g, ov.m, ov.p, w, false, fs);
+      m2l_done = launch_m2l_fixed<false>(tv, ov.m, ov.p, g.m2l_chunks.p, nchunks,
+                                         g.cell_chunk_ptr.p, w.M.p, w.Mr, w.Lpart, w.L.p, fs, cseg,
+                                         seg_done, dt, dt ? g.m2l_vid.p : nullptr);
+    }
+    if (!m2l_done) {
       size_t smem = (size_t)(ov.nm2l_terms + 9 * ov.nt) * sizeof(int);
       smem        = (smem + 15) & ~(size_t)15;
       smem += (size_t)M2L_WARPS * (ov.nt + ov.msize + 32 * M2L_SLOTS) * sizeof(T);

@@ -243,7 +243,9 @@ struct FieldWork {
   DBuf<T> M, L, Fnear, Mpart, Lleaf, Lpart;
   DBuf<T> Fsym;  // rows of the symmetric near field (Geometry::sym_*)
   DBuf<float2> dd_src;  // double-float copy of the sources (double-float pass)
-  DBuf<float2> Mdd;     // double-float copy of the multipoles (double-float M2L)
+  // reduced multipoles of the fixed-order M2L, in T and in double-float
+  DBuf<T> Mr;
+  DBuf<float2> Mdd;
   // derivative tensors of the geometry's M2L vectors, in T and in
   // double-float (built on first use)
   DBuf<T> dtab;

@@ -26,6 +26,15 @@ mono(a, b, c) = px_a py_b pz_c,
     L2L  L_n += sum_{k >= n} mono(k - n) L'_k
     L2P  f_c -= sum_{n_c >= 1} mono(n - e_c) L_n
 
+Away from the source D is harmonic, D_{j + 2e_z} = -(D_{j + 2e_x} + D_{j + 2e_y}),
+so the translation needs only the coefficients with z-power 0 or 1 on both
+sides (emit_reduced): multipole coefficients with a higher z-power are folded
+into those first (fold_rows), once per cell, and the local coefficients with a
+higher z-power follow from the others afterwards (unfold_rows).  Same sums,
+another order: per translation 483 terms instead of 840 at order 6 (265
+instead of 406 at order 5), 48 instead of 83 multipole and 36 instead of 56
+local coefficients.
+
 This file is run by the build
 (cppe_gb300/_build.py) and its output is not edited by hand.
 """
@@ -170,6 +179,122 @@ def emit_tables(m, p):
     return "\n".join(lines), name, nt
 
 
+def reduced(o_lo, o_hi):
+    """The multi-indices of orders o_lo..o_hi with z-power 0 or 1."""
+    return [t for t in multi_indices(o_hi) if sum(t) >= o_lo and t[2] <= 1]
+
+
+def z_terms(t):
+    """L_t (or D_t) as [(coefficient, index with z-power 0 or 1)]: the harmonic
+    relation applied floor(t_z / 2) times."""
+    from math import comb
+    a, b, c = t
+    j = c // 2
+    return [((-1) ** j * comb(j, i), (a + 2 * i, b + 2 * (j - i), c - 2 * j)) for i in range(j + 1)]
+
+
+def fold_rows(m, p):
+    """Per reduced multipole coefficient, the [(full coefficient, factor)] it collects."""
+    mi, moff = multi_indices(p), nterms(m - 1)
+    rows = {t: [] for t in reduced(m, p)}
+    for k in range(moff, nterms(p)):
+        for f, t in z_terms(mi[k]):
+            rows[t].append((k - moff, f))
+    return [rows[t] for t in reduced(m, p)]
+
+
+def unfold_rows(m, p):
+    """Per local coefficient, its [(reduced coefficient, factor)]."""
+    red = {t: j for j, t in enumerate(reduced(0, p - m))}
+    return [[(red[t], f) for f, t in z_terms(n)] for n in multi_indices(p - m)]
+
+
+def reduced_terms(m, p):
+    """(Multipole, local, tensor) indices of the translation's terms: multipole and
+    local coefficients in reduced order, tensor entries with z-power 0, 1, 2."""
+    dix = {t: j for j, t in enumerate(t for t in multi_indices(p) if t[2] <= 2)}
+    out = []
+    for k, tk in enumerate(reduced(m, p)):
+        for n, tn in enumerate(reduced(0, p - sum(tk))):
+            out.append((k, n, dix[tuple(a + b for a, b in zip(tk, tn))]))
+    return out
+
+
+def emit_reduced(m, p):
+    """The translation between reduced coefficients: straight-line with the
+    tensor in registers, with a tabulated tensor, and the tensor alone."""
+    didx = [t for t in multi_indices(p) if t[2] <= 2]
+    dix = {t: j for j, t in enumerate(didx)}
+    nd, ms, ls = len(didx), len(reduced(m, p)), len(reduced(0, p - m))
+    name = f"m2l_m{m}_p{p}"
+    head = ["  const T r2 = x * x + y * y + z * z;", "  const T ir2 = T(1) / r2;",
+            "  const T D0 = rsqrt_t(r2);"]
+    rvar = ("x", "y", "z")
+    rec = []
+    for j, n in enumerate(didx):
+        o = sum(n)
+        if o == 0:
+            continue
+        if n[2] == 2:  # after its two terms: both come earlier in this order
+            a, b = dix[(n[0] + 2, n[1], 0)], dix[(n[0], n[1] + 2, 0)]
+            rec.append(f"  const T D{j} = -(D{a} + D{b});")
+            continue
+        t1, t2 = [], []
+        for i in range(3):
+            if n[i] >= 1:
+                q = list(n)
+                q[i] -= 1
+                t1.append((f"T({n[i]}) * " if n[i] != 1 else "") + f"{rvar[i]} * D{dix[tuple(q)]}")
+            if n[i] >= 2:
+                q = list(n)
+                q[i] -= 2
+                t2.append(f"T({n[i] * (n[i] - 1)}) * D{dix[tuple(q)]}")
+        expr = f"T({2 * o - 1}) * ({' + '.join(t1)})"
+        if t2 and o > 1:
+            expr += f" + T({o - 1}) * ({' + '.join(t2)})"
+        rec.append(f"  const T D{j} = -({expr}) * ir2 * cinv<T>({o});")
+    contr, last = [], -1
+    for k, n, w in reduced_terms(m, p):
+        if k != last:
+            if last >= 0:
+                contr.append("  }")
+            contr.append(f"  {{ const T mk = Mb[{k}];")
+            last = k
+        contr.append(f"    acc[{n}] = fma(D{w}, mk, acc[{n}]);")
+    contr.append("  }")
+    out = [f"// M2L between reduced coefficients, source order {m}, expansion order {p}: "
+           f"{ms} multipole, {ls} local, {nd} tensor entries, {len(reduced_terms(m, p))} terms",
+           "template <typename T>",
+           f"__device__ __forceinline__ void {name}(T x, T y, T z, const T* __restrict__ Mb, "
+           "T* __restrict__ acc) {"]
+    out += head + rec + contr + ["}", "template <typename T>",
+                                 f"__device__ __forceinline__ void dtensor_m{m}_p{p}(T x, T y, T z, "
+                                 "T* __restrict__ Dout) {"]
+    out += head + rec + [f"  Dout[{j}] = D{j};" for j in range(nd)] + ["}"]
+    out += ["template <typename T>",
+            f"__device__ __forceinline__ void {name}_pre(const T* __restrict__ Dt, "
+            "const T* __restrict__ Mb, T* __restrict__ acc) {"]
+    out += [f"  const T D{j} = Dt[{j}];" for j in range(nd)] + contr + ["}"]
+    # loop form: the tensor entry of every term in order
+    out.append(f"static __constant__ unsigned char m2l_w_m{m}_p{p}[{len(reduced_terms(m, p))}] = {{")
+    out.append("  " + ", ".join(str(w) for _, _, w in reduced_terms(m, p)) + "};")
+
+    # folding and unfolding rows: up to four (input, factor) each, 0 factors after
+    def rows(nm, rr, width):
+        # (indexed per thread: in global memory, constant memory would serialise)
+        o = [f"static __device__ const signed char {nm}[{len(rr)}][{width}][2] = {{"]
+        for r in rr:
+            assert len(r) <= width
+            r = r + [(0, 0)] * (width - len(r))
+            o.append("  {" + ", ".join(f"{{{i}, {f}}}" for i, f in r) + "},")
+        return o + ["};"]
+    fw = max(len(r) for r in fold_rows(m, p))
+    uw = max(len(r) for r in unfold_rows(m, p))
+    out += rows(f"m2l_fold_m{m}_p{p}", fold_rows(m, p), fw)
+    out += rows(f"m2l_unfold_m{m}_p{p}", unfold_rows(m, p), uw)
+    return "\n".join(out), f"m{m}_p{p}", nd, ls, ms, fw, uw
+
+
 def powers_lines(q):
     """Scaled powers px_a = x^a / a!, a = 1..q (px_0 = 1 is left out)."""
     out = []
@@ -287,33 +412,25 @@ def emit_shifts(m, p):
 
 def main(out_path):
     parts = ["// Generated by gen_m2l.py -- do not edit.", "#pragma once", ""]
-    table = []
+    red, shifts = [], []
     for m, p in ORDERS:
-        code, name, ls, ms = emit(m, p)
-        parts.append(code)
-        parts.append("")
-        table.append((m, p, name, ls, ms))
+        code, *r = emit_reduced(m, p)
+        parts += [code, ""]
+        red.append((m, p, *r))
     for m, p in ORDERS:
         code, ls, ms = emit_shifts(m, p)
-        parts.append(code)
-        parts.append("")
-    tabs = []
-    for m, p in ORDERS:
-        code, name, nt = emit_tables(m, p)
-        parts.append(code)
-        parts.append("")
-        tabs.append((m, p, name, nt))
-    parts.append("#define CPPE_M2L_GENERATED(X) \\")
-    parts.append(" \\\n".join(f"  X({m}, {p}, {name}, {ls}, {ms})" for m, p, name, ls, ms in table))
+        parts += [code, ""]
+        shifts.append((m, p, ls, ms))
+    # (m, p, name suffix, tensor entries, reduced Lsize, reduced Msize, widths of the
+    # folding and unfolding rows, Lsize, Msize)
+    parts.append("#define CPPE_M2L_REDUCED(X) \\")
+    parts.append(" \\\n".join(f"  X({m}, {p}, {nm}, {nd}, {ls}, {ms}, {fw}, {uw}, {sl}, {sm})"
+                              for (m, p, nm, nd, ls, ms, fw, uw), (_, _, sl, sm)
+                              in zip(red, shifts)))
     parts.append("")
     # (m, p, Lsize, Msize) of the straight-line shifts
     parts.append("#define CPPE_SHIFTS_GENERATED(X) \\")
-    parts.append(" \\\n".join(f"  X({m}, {p}, {ls}, {ms})" for m, p, name, ls, ms in table))
-    parts.append("")
-    # (m, p, name suffix of the tables, nterms(p), Lsize, Msize) of the loop form
-    parts.append("#define CPPE_M2L_TABLES(X) \\")
-    parts.append(" \\\n".join(f"  X({m}, {p}, {name}, {nt}, {ls}, {ms})"
-                              for (m, p, name, nt), (_, _, _, ls, ms) in zip(tabs, table)))
+    parts.append(" \\\n".join(f"  X({m}, {p}, {ls}, {ms})" for m, p, ls, ms in shifts))
     parts.append("")
     src = "\n".join(parts)
     if os.path.exists(out_path) and open(out_path).read() == src:

@@ -1,7 +1,7 @@
 // Generated by gen_m2l.py -- do not edit.
 #pragma once
 
-// M2L, source order 1, expansion order 5: Msize 55, Lsize 35
+// M2L between reduced coefficients, source order 1, expansion order 5: 35 multipole, 25 local, 46 tensor entries, 265 terms
 template <typename T>
 __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ Mb, T* __restrict__ acc) {
   const T r2 = x * x + y * y + z * z;
@@ -15,53 +15,43 @@ __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ M
   const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
   const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
   const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
-  const T D9 = -(T(3) * (T(2) * z * D3) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
+  const T D9 = -(D4 + D7);
   const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
   const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
   const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
   const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
   const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
-  const T D15 = -(T(5) * (x * D9 + T(2) * z * D6) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
+  const T D15 = -(D10 + D13);
   const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
   const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D18 = -(T(5) * (y * D9 + T(2) * z * D8) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D19 = -(T(5) * (T(3) * z * D9) + T(2) * (T(6) * D3)) * ir2 * cinv<T>(3);
-  const T D20 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D24 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
-  const T D25 = -(T(7) * (T(2) * x * D15 + T(2) * z * D12) + T(3) * (T(2) * D9 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D27 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
-  const T D28 = -(T(7) * (x * D18 + y * D15 + T(2) * z * D14) + T(3) * (T(2) * D5)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (x * D19 + T(3) * z * D15) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D30 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D31 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D32 = -(T(7) * (T(2) * y * D18 + T(2) * z * D17) + T(3) * (T(2) * D9 + T(2) * D7)) * ir2 * cinv<T>(4);
-  const T D33 = -(T(7) * (y * D19 + T(3) * z * D18) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D34 = -(T(7) * (T(4) * z * D19) + T(3) * (T(12) * D9)) * ir2 * cinv<T>(4);
-  const T D35 = -(T(9) * (T(5) * x * D20) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D36 = -(T(9) * (T(4) * x * D21 + y * D20) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D37 = -(T(9) * (T(4) * x * D22 + z * D20) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(3) * x * D23 + T(2) * y * D21) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D39 = -(T(9) * (T(3) * x * D24 + y * D22 + z * D21) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D40 = -(T(9) * (T(3) * x * D25 + T(2) * z * D22) + T(4) * (T(6) * D15 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (T(2) * x * D26 + T(3) * y * D23) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D42 = -(T(9) * (T(2) * x * D27 + T(2) * y * D24 + z * D23) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
-  const T D43 = -(T(9) * (T(2) * x * D28 + y * D25 + T(2) * z * D24) + T(4) * (T(2) * D18 + T(2) * D11)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(2) * x * D29 + T(3) * z * D25) + T(4) * (T(2) * D19 + T(6) * D12)) * ir2 * cinv<T>(5);
-  const T D45 = -(T(9) * (x * D30 + T(4) * y * D26) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D46 = -(T(9) * (x * D31 + T(3) * y * D27 + z * D26) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D47 = -(T(9) * (x * D32 + T(2) * y * D28 + T(2) * z * D27) + T(4) * (T(2) * D15 + T(2) * D13)) * ir2 * cinv<T>(5);
-  const T D48 = -(T(9) * (x * D33 + y * D29 + T(3) * z * D28) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D49 = -(T(9) * (x * D34 + T(4) * z * D29) + T(4) * (T(12) * D15)) * ir2 * cinv<T>(5);
-  const T D50 = -(T(9) * (T(5) * y * D30) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D51 = -(T(9) * (T(4) * y * D31 + z * D30) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
-  const T D52 = -(T(9) * (T(3) * y * D32 + T(2) * z * D31) + T(4) * (T(6) * D18 + T(2) * D16)) * ir2 * cinv<T>(5);
-  const T D53 = -(T(9) * (T(2) * y * D33 + T(3) * z * D32) + T(4) * (T(2) * D19 + T(6) * D17)) * ir2 * cinv<T>(5);
-  const T D54 = -(T(9) * (y * D34 + T(4) * z * D33) + T(4) * (T(12) * D18)) * ir2 * cinv<T>(5);
-  const T D55 = -(T(9) * (T(5) * z * D34) + T(4) * (T(20) * D19)) * ir2 * cinv<T>(5);
+  const T D18 = -(D11 + D16);
+  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
+  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
+  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
+  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T D24 = -(D19 + D22);
+  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T D27 = -(D20 + D25);
+  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
+  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T D30 = -(D22 + D28);
+  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
+  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
+  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
+  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
+  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D36 = -(D31 + D34);
+  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
+  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T D39 = -(D32 + D37);
+  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
+  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D42 = -(D34 + D40);
+  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
+  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T D45 = -(D37 + D43);
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
     acc[1] = fma(D4, mk, acc[1]);
@@ -72,32 +62,22 @@ __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D12, mk, acc[6]);
     acc[7] = fma(D13, mk, acc[7]);
     acc[8] = fma(D14, mk, acc[8]);
-    acc[9] = fma(D15, mk, acc[9]);
+    acc[9] = fma(D19, mk, acc[9]);
     acc[10] = fma(D20, mk, acc[10]);
     acc[11] = fma(D21, mk, acc[11]);
     acc[12] = fma(D22, mk, acc[12]);
     acc[13] = fma(D23, mk, acc[13]);
-    acc[14] = fma(D24, mk, acc[14]);
-    acc[15] = fma(D25, mk, acc[15]);
-    acc[16] = fma(D26, mk, acc[16]);
-    acc[17] = fma(D27, mk, acc[17]);
-    acc[18] = fma(D28, mk, acc[18]);
-    acc[19] = fma(D29, mk, acc[19]);
+    acc[14] = fma(D25, mk, acc[14]);
+    acc[15] = fma(D26, mk, acc[15]);
+    acc[16] = fma(D31, mk, acc[16]);
+    acc[17] = fma(D32, mk, acc[17]);
+    acc[18] = fma(D33, mk, acc[18]);
+    acc[19] = fma(D34, mk, acc[19]);
     acc[20] = fma(D35, mk, acc[20]);
-    acc[21] = fma(D36, mk, acc[21]);
-    acc[22] = fma(D37, mk, acc[22]);
-    acc[23] = fma(D38, mk, acc[23]);
-    acc[24] = fma(D39, mk, acc[24]);
-    acc[25] = fma(D40, mk, acc[25]);
-    acc[26] = fma(D41, mk, acc[26]);
-    acc[27] = fma(D42, mk, acc[27]);
-    acc[28] = fma(D43, mk, acc[28]);
-    acc[29] = fma(D44, mk, acc[29]);
-    acc[30] = fma(D45, mk, acc[30]);
-    acc[31] = fma(D46, mk, acc[31]);
-    acc[32] = fma(D47, mk, acc[32]);
-    acc[33] = fma(D48, mk, acc[33]);
-    acc[34] = fma(D49, mk, acc[34]);
+    acc[21] = fma(D37, mk, acc[21]);
+    acc[22] = fma(D38, mk, acc[22]);
+    acc[23] = fma(D40, mk, acc[23]);
+    acc[24] = fma(D41, mk, acc[24]);
   }
   { const T mk = Mb[1];
     acc[0] = fma(D2, mk, acc[0]);
@@ -109,32 +89,22 @@ __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D14, mk, acc[6]);
     acc[7] = fma(D16, mk, acc[7]);
     acc[8] = fma(D17, mk, acc[8]);
-    acc[9] = fma(D18, mk, acc[9]);
-    acc[10] = fma(D21, mk, acc[10]);
+    acc[9] = fma(D20, mk, acc[9]);
+    acc[10] = fma(D22, mk, acc[10]);
     acc[11] = fma(D23, mk, acc[11]);
-    acc[12] = fma(D24, mk, acc[12]);
+    acc[12] = fma(D25, mk, acc[12]);
     acc[13] = fma(D26, mk, acc[13]);
-    acc[14] = fma(D27, mk, acc[14]);
-    acc[15] = fma(D28, mk, acc[15]);
-    acc[16] = fma(D30, mk, acc[16]);
-    acc[17] = fma(D31, mk, acc[17]);
-    acc[18] = fma(D32, mk, acc[18]);
-    acc[19] = fma(D33, mk, acc[19]);
-    acc[20] = fma(D36, mk, acc[20]);
-    acc[21] = fma(D38, mk, acc[21]);
-    acc[22] = fma(D39, mk, acc[22]);
-    acc[23] = fma(D41, mk, acc[23]);
-    acc[24] = fma(D42, mk, acc[24]);
-    acc[25] = fma(D43, mk, acc[25]);
-    acc[26] = fma(D45, mk, acc[26]);
-    acc[27] = fma(D46, mk, acc[27]);
-    acc[28] = fma(D47, mk, acc[28]);
-    acc[29] = fma(D48, mk, acc[29]);
-    acc[30] = fma(D50, mk, acc[30]);
-    acc[31] = fma(D51, mk, acc[31]);
-    acc[32] = fma(D52, mk, acc[32]);
-    acc[33] = fma(D53, mk, acc[33]);
-    acc[34] = fma(D54, mk, acc[34]);
+    acc[14] = fma(D28, mk, acc[14]);
+    acc[15] = fma(D29, mk, acc[15]);
+    acc[16] = fma(D32, mk, acc[16]);
+    acc[17] = fma(D34, mk, acc[17]);
+    acc[18] = fma(D35, mk, acc[18]);
+    acc[19] = fma(D37, mk, acc[19]);
+    acc[20] = fma(D38, mk, acc[20]);
+    acc[21] = fma(D40, mk, acc[21]);
+    acc[22] = fma(D41, mk, acc[22]);
+    acc[23] = fma(D43, mk, acc[23]);
+    acc[24] = fma(D44, mk, acc[24]);
   }
   { const T mk = Mb[2];
     acc[0] = fma(D3, mk, acc[0]);
@@ -146,440 +116,278 @@ __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D15, mk, acc[6]);
     acc[7] = fma(D17, mk, acc[7]);
     acc[8] = fma(D18, mk, acc[8]);
-    acc[9] = fma(D19, mk, acc[9]);
-    acc[10] = fma(D22, mk, acc[10]);
+    acc[9] = fma(D21, mk, acc[9]);
+    acc[10] = fma(D23, mk, acc[10]);
     acc[11] = fma(D24, mk, acc[11]);
-    acc[12] = fma(D25, mk, acc[12]);
+    acc[12] = fma(D26, mk, acc[12]);
     acc[13] = fma(D27, mk, acc[13]);
-    acc[14] = fma(D28, mk, acc[14]);
-    acc[15] = fma(D29, mk, acc[15]);
-    acc[16] = fma(D31, mk, acc[16]);
-    acc[17] = fma(D32, mk, acc[17]);
-    acc[18] = fma(D33, mk, acc[18]);
-    acc[19] = fma(D34, mk, acc[19]);
-    acc[20] = fma(D37, mk, acc[20]);
-    acc[21] = fma(D39, mk, acc[21]);
-    acc[22] = fma(D40, mk, acc[22]);
-    acc[23] = fma(D42, mk, acc[23]);
-    acc[24] = fma(D43, mk, acc[24]);
-    acc[25] = fma(D44, mk, acc[25]);
-    acc[26] = fma(D46, mk, acc[26]);
-    acc[27] = fma(D47, mk, acc[27]);
-    acc[28] = fma(D48, mk, acc[28]);
-    acc[29] = fma(D49, mk, acc[29]);
-    acc[30] = fma(D51, mk, acc[30]);
-    acc[31] = fma(D52, mk, acc[31]);
-    acc[32] = fma(D53, mk, acc[32]);
-    acc[33] = fma(D54, mk, acc[33]);
-    acc[34] = fma(D55, mk, acc[34]);
+    acc[14] = fma(D29, mk, acc[14]);
+    acc[15] = fma(D30, mk, acc[15]);
+    acc[16] = fma(D33, mk, acc[16]);
+    acc[17] = fma(D35, mk, acc[17]);
+    acc[18] = fma(D36, mk, acc[18]);
+    acc[19] = fma(D38, mk, acc[19]);
+    acc[20] = fma(D39, mk, acc[20]);
+    acc[21] = fma(D41, mk, acc[21]);
+    acc[22] = fma(D42, mk, acc[22]);
+    acc[23] = fma(D44, mk, acc[23]);
+    acc[24] = fma(D45, mk, acc[24]);
   }
   { const T mk = Mb[3];
     acc[0] = fma(D4, mk, acc[0]);
     acc[1] = fma(D10, mk, acc[1]);
     acc[2] = fma(D11, mk, acc[2]);
     acc[3] = fma(D12, mk, acc[3]);
-    acc[4] = fma(D20, mk, acc[4]);
-    acc[5] = fma(D21, mk, acc[5]);
-    acc[6] = fma(D22, mk, acc[6]);
-    acc[7] = fma(D23, mk, acc[7]);
-    acc[8] = fma(D24, mk, acc[8]);
-    acc[9] = fma(D25, mk, acc[9]);
-    acc[10] = fma(D35, mk, acc[10]);
-    acc[11] = fma(D36, mk, acc[11]);
-    acc[12] = fma(D37, mk, acc[12]);
-    acc[13] = fma(D38, mk, acc[13]);
-    acc[14] = fma(D39, mk, acc[14]);
-    acc[15] = fma(D40, mk, acc[15]);
-    acc[16] = fma(D41, mk, acc[16]);
-    acc[17] = fma(D42, mk, acc[17]);
-    acc[18] = fma(D43, mk, acc[18]);
-    acc[19] = fma(D44, mk, acc[19]);
+    acc[4] = fma(D19, mk, acc[4]);
+    acc[5] = fma(D20, mk, acc[5]);
+    acc[6] = fma(D21, mk, acc[6]);
+    acc[7] = fma(D22, mk, acc[7]);
+    acc[8] = fma(D23, mk, acc[8]);
+    acc[9] = fma(D31, mk, acc[9]);
+    acc[10] = fma(D32, mk, acc[10]);
+    acc[11] = fma(D33, mk, acc[11]);
+    acc[12] = fma(D34, mk, acc[12]);
+    acc[13] = fma(D35, mk, acc[13]);
+    acc[14] = fma(D37, mk, acc[14]);
+    acc[15] = fma(D38, mk, acc[15]);
   }
   { const T mk = Mb[4];
     acc[0] = fma(D5, mk, acc[0]);
     acc[1] = fma(D11, mk, acc[1]);
     acc[2] = fma(D13, mk, acc[2]);
     acc[3] = fma(D14, mk, acc[3]);
-    acc[4] = fma(D21, mk, acc[4]);
-    acc[5] = fma(D23, mk, acc[5]);
-    acc[6] = fma(D24, mk, acc[6]);
-    acc[7] = fma(D26, mk, acc[7]);
-    acc[8] = fma(D27, mk, acc[8]);
-    acc[9] = fma(D28, mk, acc[9]);
-    acc[10] = fma(D36, mk, acc[10]);
-    acc[11] = fma(D38, mk, acc[11]);
-    acc[12] = fma(D39, mk, acc[12]);
-    acc[13] = fma(D41, mk, acc[13]);
-    acc[14] = fma(D42, mk, acc[14]);
-    acc[15] = fma(D43, mk, acc[15]);
-    acc[16] = fma(D45, mk, acc[16]);
-    acc[17] = fma(D46, mk, acc[17]);
-    acc[18] = fma(D47, mk, acc[18]);
-    acc[19] = fma(D48, mk, acc[19]);
+    acc[4] = fma(D20, mk, acc[4]);
+    acc[5] = fma(D22, mk, acc[5]);
+    acc[6] = fma(D23, mk, acc[6]);
+    acc[7] = fma(D25, mk, acc[7]);
+    acc[8] = fma(D26, mk, acc[8]);
+    acc[9] = fma(D32, mk, acc[9]);
+    acc[10] = fma(D34, mk, acc[10]);
+    acc[11] = fma(D35, mk, acc[11]);
+    acc[12] = fma(D37, mk, acc[12]);
+    acc[13] = fma(D38, mk, acc[13]);
+    acc[14] = fma(D40, mk, acc[14]);
+    acc[15] = fma(D41, mk, acc[15]);
   }
   { const T mk = Mb[5];
     acc[0] = fma(D6, mk, acc[0]);
     acc[1] = fma(D12, mk, acc[1]);
     acc[2] = fma(D14, mk, acc[2]);
     acc[3] = fma(D15, mk, acc[3]);
-    acc[4] = fma(D22, mk, acc[4]);
-    acc[5] = fma(D24, mk, acc[5]);
-    acc[6] = fma(D25, mk, acc[6]);
-    acc[7] = fma(D27, mk, acc[7]);
-    acc[8] = fma(D28, mk, acc[8]);
-    acc[9] = fma(D29, mk, acc[9]);
-    acc[10] = fma(D37, mk, acc[10]);
-    acc[11] = fma(D39, mk, acc[11]);
-    acc[12] = fma(D40, mk, acc[12]);
-    acc[13] = fma(D42, mk, acc[13]);
-    acc[14] = fma(D43, mk, acc[14]);
-    acc[15] = fma(D44, mk, acc[15]);
-    acc[16] = fma(D46, mk, acc[16]);
-    acc[17] = fma(D47, mk, acc[17]);
-    acc[18] = fma(D48, mk, acc[18]);
-    acc[19] = fma(D49, mk, acc[19]);
+    acc[4] = fma(D21, mk, acc[4]);
+    acc[5] = fma(D23, mk, acc[5]);
+    acc[6] = fma(D24, mk, acc[6]);
+    acc[7] = fma(D26, mk, acc[7]);
+    acc[8] = fma(D27, mk, acc[8]);
+    acc[9] = fma(D33, mk, acc[9]);
+    acc[10] = fma(D35, mk, acc[10]);
+    acc[11] = fma(D36, mk, acc[11]);
+    acc[12] = fma(D38, mk, acc[12]);
+    acc[13] = fma(D39, mk, acc[13]);
+    acc[14] = fma(D41, mk, acc[14]);
+    acc[15] = fma(D42, mk, acc[15]);
   }
   { const T mk = Mb[6];
     acc[0] = fma(D7, mk, acc[0]);
     acc[1] = fma(D13, mk, acc[1]);
     acc[2] = fma(D16, mk, acc[2]);
     acc[3] = fma(D17, mk, acc[3]);
-    acc[4] = fma(D23, mk, acc[4]);
-    acc[5] = fma(D26, mk, acc[5]);
-    acc[6] = fma(D27, mk, acc[6]);
-    acc[7] = fma(D30, mk, acc[7]);
-    acc[8] = fma(D31, mk, acc[8]);
-    acc[9] = fma(D32, mk, acc[9]);
-    acc[10] = fma(D38, mk, acc[10]);
-    acc[11] = fma(D41, mk, acc[11]);
-    acc[12] = fma(D42, mk, acc[12]);
-    acc[13] = fma(D45, mk, acc[13]);
-    acc[14] = fma(D46, mk, acc[14]);
-    acc[15] = fma(D47, mk, acc[15]);
-    acc[16] = fma(D50, mk, acc[16]);
-    acc[17] = fma(D51, mk, acc[17]);
-    acc[18] = fma(D52, mk, acc[18]);
-    acc[19] = fma(D53, mk, acc[19]);
+    acc[4] = fma(D22, mk, acc[4]);
+    acc[5] = fma(D25, mk, acc[5]);
+    acc[6] = fma(D26, mk, acc[6]);
+    acc[7] = fma(D28, mk, acc[7]);
+    acc[8] = fma(D29, mk, acc[8]);
+    acc[9] = fma(D34, mk, acc[9]);
+    acc[10] = fma(D37, mk, acc[10]);
+    acc[11] = fma(D38, mk, acc[11]);
+    acc[12] = fma(D40, mk, acc[12]);
+    acc[13] = fma(D41, mk, acc[13]);
+    acc[14] = fma(D43, mk, acc[14]);
+    acc[15] = fma(D44, mk, acc[15]);
   }
   { const T mk = Mb[7];
     acc[0] = fma(D8, mk, acc[0]);
     acc[1] = fma(D14, mk, acc[1]);
     acc[2] = fma(D17, mk, acc[2]);
     acc[3] = fma(D18, mk, acc[3]);
-    acc[4] = fma(D24, mk, acc[4]);
-    acc[5] = fma(D27, mk, acc[5]);
-    acc[6] = fma(D28, mk, acc[6]);
-    acc[7] = fma(D31, mk, acc[7]);
-    acc[8] = fma(D32, mk, acc[8]);
-    acc[9] = fma(D33, mk, acc[9]);
-    acc[10] = fma(D39, mk, acc[10]);
-    acc[11] = fma(D42, mk, acc[11]);
-    acc[12] = fma(D43, mk, acc[12]);
-    acc[13] = fma(D46, mk, acc[13]);
-    acc[14] = fma(D47, mk, acc[14]);
-    acc[15] = fma(D48, mk, acc[15]);
-    acc[16] = fma(D51, mk, acc[16]);
-    acc[17] = fma(D52, mk, acc[17]);
-    acc[18] = fma(D53, mk, acc[18]);
-    acc[19] = fma(D54, mk, acc[19]);
+    acc[4] = fma(D23, mk, acc[4]);
+    acc[5] = fma(D26, mk, acc[5]);
+    acc[6] = fma(D27, mk, acc[6]);
+    acc[7] = fma(D29, mk, acc[7]);
+    acc[8] = fma(D30, mk, acc[8]);
+    acc[9] = fma(D35, mk, acc[9]);
+    acc[10] = fma(D38, mk, acc[10]);
+    acc[11] = fma(D39, mk, acc[11]);
+    acc[12] = fma(D41, mk, acc[12]);
+    acc[13] = fma(D42, mk, acc[13]);
+    acc[14] = fma(D44, mk, acc[14]);
+    acc[15] = fma(D45, mk, acc[15]);
   }
   { const T mk = Mb[8];
-    acc[0] = fma(D9, mk, acc[0]);
-    acc[1] = fma(D15, mk, acc[1]);
-    acc[2] = fma(D18, mk, acc[2]);
-    acc[3] = fma(D19, mk, acc[3]);
-    acc[4] = fma(D25, mk, acc[4]);
-    acc[5] = fma(D28, mk, acc[5]);
-    acc[6] = fma(D29, mk, acc[6]);
-    acc[7] = fma(D32, mk, acc[7]);
-    acc[8] = fma(D33, mk, acc[8]);
-    acc[9] = fma(D34, mk, acc[9]);
-    acc[10] = fma(D40, mk, acc[10]);
-    acc[11] = fma(D43, mk, acc[11]);
-    acc[12] = fma(D44, mk, acc[12]);
-    acc[13] = fma(D47, mk, acc[13]);
-    acc[14] = fma(D48, mk, acc[14]);
-    acc[15] = fma(D49, mk, acc[15]);
-    acc[16] = fma(D52, mk, acc[16]);
-    acc[17] = fma(D53, mk, acc[17]);
-    acc[18] = fma(D54, mk, acc[18]);
-    acc[19] = fma(D55, mk, acc[19]);
+    acc[0] = fma(D10, mk, acc[0]);
+    acc[1] = fma(D19, mk, acc[1]);
+    acc[2] = fma(D20, mk, acc[2]);
+    acc[3] = fma(D21, mk, acc[3]);
+    acc[4] = fma(D31, mk, acc[4]);
+    acc[5] = fma(D32, mk, acc[5]);
+    acc[6] = fma(D33, mk, acc[6]);
+    acc[7] = fma(D34, mk, acc[7]);
+    acc[8] = fma(D35, mk, acc[8]);
   }
   { const T mk = Mb[9];
-    acc[0] = fma(D10, mk, acc[0]);
+    acc[0] = fma(D11, mk, acc[0]);
     acc[1] = fma(D20, mk, acc[1]);
-    acc[2] = fma(D21, mk, acc[2]);
-    acc[3] = fma(D22, mk, acc[3]);
-    acc[4] = fma(D35, mk, acc[4]);
-    acc[5] = fma(D36, mk, acc[5]);
-    acc[6] = fma(D37, mk, acc[6]);
-    acc[7] = fma(D38, mk, acc[7]);
-    acc[8] = fma(D39, mk, acc[8]);
-    acc[9] = fma(D40, mk, acc[9]);
+    acc[2] = fma(D22, mk, acc[2]);
+    acc[3] = fma(D23, mk, acc[3]);
+    acc[4] = fma(D32, mk, acc[4]);
+    acc[5] = fma(D34, mk, acc[5]);
+    acc[6] = fma(D35, mk, acc[6]);
+    acc[7] = fma(D37, mk, acc[7]);
+    acc[8] = fma(D38, mk, acc[8]);
   }
   { const T mk = Mb[10];
-    acc[0] = fma(D11, mk, acc[0]);
+    acc[0] = fma(D12, mk, acc[0]);
     acc[1] = fma(D21, mk, acc[1]);
     acc[2] = fma(D23, mk, acc[2]);
     acc[3] = fma(D24, mk, acc[3]);
-    acc[4] = fma(D36, mk, acc[4]);
+    acc[4] = fma(D33, mk, acc[4]);
+    acc[5] = fma(D35, mk, acc[5]);
+    acc[6] = fma(D36, mk, acc[6]);
+    acc[7] = fma(D38, mk, acc[7]);
+    acc[8] = fma(D39, mk, acc[8]);
+  }
+  { const T mk = Mb[11];
+    acc[0] = fma(D13, mk, acc[0]);
+    acc[1] = fma(D22, mk, acc[1]);
+    acc[2] = fma(D25, mk, acc[2]);
+    acc[3] = fma(D26, mk, acc[3]);
+    acc[4] = fma(D34, mk, acc[4]);
+    acc[5] = fma(D37, mk, acc[5]);
+    acc[6] = fma(D38, mk, acc[6]);
+    acc[7] = fma(D40, mk, acc[7]);
+    acc[8] = fma(D41, mk, acc[8]);
+  }
+  { const T mk = Mb[12];
+    acc[0] = fma(D14, mk, acc[0]);
+    acc[1] = fma(D23, mk, acc[1]);
+    acc[2] = fma(D26, mk, acc[2]);
+    acc[3] = fma(D27, mk, acc[3]);
+    acc[4] = fma(D35, mk, acc[4]);
     acc[5] = fma(D38, mk, acc[5]);
     acc[6] = fma(D39, mk, acc[6]);
     acc[7] = fma(D41, mk, acc[7]);
     acc[8] = fma(D42, mk, acc[8]);
-    acc[9] = fma(D43, mk, acc[9]);
-  }
-  { const T mk = Mb[11];
-    acc[0] = fma(D12, mk, acc[0]);
-    acc[1] = fma(D22, mk, acc[1]);
-    acc[2] = fma(D24, mk, acc[2]);
-    acc[3] = fma(D25, mk, acc[3]);
-    acc[4] = fma(D37, mk, acc[4]);
-    acc[5] = fma(D39, mk, acc[5]);
-    acc[6] = fma(D40, mk, acc[6]);
-    acc[7] = fma(D42, mk, acc[7]);
-    acc[8] = fma(D43, mk, acc[8]);
-    acc[9] = fma(D44, mk, acc[9]);
-  }
-  { const T mk = Mb[12];
-    acc[0] = fma(D13, mk, acc[0]);
-    acc[1] = fma(D23, mk, acc[1]);
-    acc[2] = fma(D26, mk, acc[2]);
-    acc[3] = fma(D27, mk, acc[3]);
-    acc[4] = fma(D38, mk, acc[4]);
-    acc[5] = fma(D41, mk, acc[5]);
-    acc[6] = fma(D42, mk, acc[6]);
-    acc[7] = fma(D45, mk, acc[7]);
-    acc[8] = fma(D46, mk, acc[8]);
-    acc[9] = fma(D47, mk, acc[9]);
   }
   { const T mk = Mb[13];
-    acc[0] = fma(D14, mk, acc[0]);
-    acc[1] = fma(D24, mk, acc[1]);
-    acc[2] = fma(D27, mk, acc[2]);
-    acc[3] = fma(D28, mk, acc[3]);
-    acc[4] = fma(D39, mk, acc[4]);
-    acc[5] = fma(D42, mk, acc[5]);
-    acc[6] = fma(D43, mk, acc[6]);
-    acc[7] = fma(D46, mk, acc[7]);
-    acc[8] = fma(D47, mk, acc[8]);
-    acc[9] = fma(D48, mk, acc[9]);
-  }
-  { const T mk = Mb[14];
-    acc[0] = fma(D15, mk, acc[0]);
+    acc[0] = fma(D16, mk, acc[0]);
     acc[1] = fma(D25, mk, acc[1]);
     acc[2] = fma(D28, mk, acc[2]);
     acc[3] = fma(D29, mk, acc[3]);
-    acc[4] = fma(D40, mk, acc[4]);
-    acc[5] = fma(D43, mk, acc[5]);
-    acc[6] = fma(D44, mk, acc[6]);
-    acc[7] = fma(D47, mk, acc[7]);
-    acc[8] = fma(D48, mk, acc[8]);
-    acc[9] = fma(D49, mk, acc[9]);
+    acc[4] = fma(D37, mk, acc[4]);
+    acc[5] = fma(D40, mk, acc[5]);
+    acc[6] = fma(D41, mk, acc[6]);
+    acc[7] = fma(D43, mk, acc[7]);
+    acc[8] = fma(D44, mk, acc[8]);
+  }
+  { const T mk = Mb[14];
+    acc[0] = fma(D17, mk, acc[0]);
+    acc[1] = fma(D26, mk, acc[1]);
+    acc[2] = fma(D29, mk, acc[2]);
+    acc[3] = fma(D30, mk, acc[3]);
+    acc[4] = fma(D38, mk, acc[4]);
+    acc[5] = fma(D41, mk, acc[5]);
+    acc[6] = fma(D42, mk, acc[6]);
+    acc[7] = fma(D44, mk, acc[7]);
+    acc[8] = fma(D45, mk, acc[8]);
   }
   { const T mk = Mb[15];
-    acc[0] = fma(D16, mk, acc[0]);
-    acc[1] = fma(D26, mk, acc[1]);
-    acc[2] = fma(D30, mk, acc[2]);
-    acc[3] = fma(D31, mk, acc[3]);
-    acc[4] = fma(D41, mk, acc[4]);
-    acc[5] = fma(D45, mk, acc[5]);
-    acc[6] = fma(D46, mk, acc[6]);
-    acc[7] = fma(D50, mk, acc[7]);
-    acc[8] = fma(D51, mk, acc[8]);
-    acc[9] = fma(D52, mk, acc[9]);
-  }
-  { const T mk = Mb[16];
-    acc[0] = fma(D17, mk, acc[0]);
-    acc[1] = fma(D27, mk, acc[1]);
-    acc[2] = fma(D31, mk, acc[2]);
-    acc[3] = fma(D32, mk, acc[3]);
-    acc[4] = fma(D42, mk, acc[4]);
-    acc[5] = fma(D46, mk, acc[5]);
-    acc[6] = fma(D47, mk, acc[6]);
-    acc[7] = fma(D51, mk, acc[7]);
-    acc[8] = fma(D52, mk, acc[8]);
-    acc[9] = fma(D53, mk, acc[9]);
-  }
-  { const T mk = Mb[17];
-    acc[0] = fma(D18, mk, acc[0]);
-    acc[1] = fma(D28, mk, acc[1]);
+    acc[0] = fma(D19, mk, acc[0]);
+    acc[1] = fma(D31, mk, acc[1]);
     acc[2] = fma(D32, mk, acc[2]);
     acc[3] = fma(D33, mk, acc[3]);
-    acc[4] = fma(D43, mk, acc[4]);
-    acc[5] = fma(D47, mk, acc[5]);
-    acc[6] = fma(D48, mk, acc[6]);
-    acc[7] = fma(D52, mk, acc[7]);
-    acc[8] = fma(D53, mk, acc[8]);
-    acc[9] = fma(D54, mk, acc[9]);
+  }
+  { const T mk = Mb[16];
+    acc[0] = fma(D20, mk, acc[0]);
+    acc[1] = fma(D32, mk, acc[1]);
+    acc[2] = fma(D34, mk, acc[2]);
+    acc[3] = fma(D35, mk, acc[3]);
+  }
+  { const T mk = Mb[17];
+    acc[0] = fma(D21, mk, acc[0]);
+    acc[1] = fma(D33, mk, acc[1]);
+    acc[2] = fma(D35, mk, acc[2]);
+    acc[3] = fma(D36, mk, acc[3]);
   }
   { const T mk = Mb[18];
-    acc[0] = fma(D19, mk, acc[0]);
-    acc[1] = fma(D29, mk, acc[1]);
-    acc[2] = fma(D33, mk, acc[2]);
-    acc[3] = fma(D34, mk, acc[3]);
-    acc[4] = fma(D44, mk, acc[4]);
-    acc[5] = fma(D48, mk, acc[5]);
-    acc[6] = fma(D49, mk, acc[6]);
-    acc[7] = fma(D53, mk, acc[7]);
-    acc[8] = fma(D54, mk, acc[8]);
-    acc[9] = fma(D55, mk, acc[9]);
+    acc[0] = fma(D22, mk, acc[0]);
+    acc[1] = fma(D34, mk, acc[1]);
+    acc[2] = fma(D37, mk, acc[2]);
+    acc[3] = fma(D38, mk, acc[3]);
   }
   { const T mk = Mb[19];
-    acc[0] = fma(D20, mk, acc[0]);
+    acc[0] = fma(D23, mk, acc[0]);
     acc[1] = fma(D35, mk, acc[1]);
-    acc[2] = fma(D36, mk, acc[2]);
-    acc[3] = fma(D37, mk, acc[3]);
-  }
-  { const T mk = Mb[20];
-    acc[0] = fma(D21, mk, acc[0]);
-    acc[1] = fma(D36, mk, acc[1]);
     acc[2] = fma(D38, mk, acc[2]);
     acc[3] = fma(D39, mk, acc[3]);
   }
-  { const T mk = Mb[21];
-    acc[0] = fma(D22, mk, acc[0]);
+  { const T mk = Mb[20];
+    acc[0] = fma(D25, mk, acc[0]);
     acc[1] = fma(D37, mk, acc[1]);
-    acc[2] = fma(D39, mk, acc[2]);
-    acc[3] = fma(D40, mk, acc[3]);
+    acc[2] = fma(D40, mk, acc[2]);
+    acc[3] = fma(D41, mk, acc[3]);
   }
-  { const T mk = Mb[22];
-    acc[0] = fma(D23, mk, acc[0]);
+  { const T mk = Mb[21];
+    acc[0] = fma(D26, mk, acc[0]);
     acc[1] = fma(D38, mk, acc[1]);
     acc[2] = fma(D41, mk, acc[2]);
     acc[3] = fma(D42, mk, acc[3]);
   }
-  { const T mk = Mb[23];
-    acc[0] = fma(D24, mk, acc[0]);
-    acc[1] = fma(D39, mk, acc[1]);
-    acc[2] = fma(D42, mk, acc[2]);
-    acc[3] = fma(D43, mk, acc[3]);
-  }
-  { const T mk = Mb[24];
-    acc[0] = fma(D25, mk, acc[0]);
+  { const T mk = Mb[22];
+    acc[0] = fma(D28, mk, acc[0]);
     acc[1] = fma(D40, mk, acc[1]);
     acc[2] = fma(D43, mk, acc[2]);
     acc[3] = fma(D44, mk, acc[3]);
   }
-  { const T mk = Mb[25];
-    acc[0] = fma(D26, mk, acc[0]);
+  { const T mk = Mb[23];
+    acc[0] = fma(D29, mk, acc[0]);
     acc[1] = fma(D41, mk, acc[1]);
-    acc[2] = fma(D45, mk, acc[2]);
-    acc[3] = fma(D46, mk, acc[3]);
+    acc[2] = fma(D44, mk, acc[2]);
+    acc[3] = fma(D45, mk, acc[3]);
+  }
+  { const T mk = Mb[24];
+    acc[0] = fma(D31, mk, acc[0]);
+  }
+  { const T mk = Mb[25];
+    acc[0] = fma(D32, mk, acc[0]);
   }
   { const T mk = Mb[26];
-    acc[0] = fma(D27, mk, acc[0]);
-    acc[1] = fma(D42, mk, acc[1]);
-    acc[2] = fma(D46, mk, acc[2]);
-    acc[3] = fma(D47, mk, acc[3]);
+    acc[0] = fma(D33, mk, acc[0]);
   }
   { const T mk = Mb[27];
-    acc[0] = fma(D28, mk, acc[0]);
-    acc[1] = fma(D43, mk, acc[1]);
-    acc[2] = fma(D47, mk, acc[2]);
-    acc[3] = fma(D48, mk, acc[3]);
+    acc[0] = fma(D34, mk, acc[0]);
   }
   { const T mk = Mb[28];
-    acc[0] = fma(D29, mk, acc[0]);
-    acc[1] = fma(D44, mk, acc[1]);
-    acc[2] = fma(D48, mk, acc[2]);
-    acc[3] = fma(D49, mk, acc[3]);
-  }
-  { const T mk = Mb[29];
-    acc[0] = fma(D30, mk, acc[0]);
-    acc[1] = fma(D45, mk, acc[1]);
-    acc[2] = fma(D50, mk, acc[2]);
-    acc[3] = fma(D51, mk, acc[3]);
-  }
-  { const T mk = Mb[30];
-    acc[0] = fma(D31, mk, acc[0]);
-    acc[1] = fma(D46, mk, acc[1]);
-    acc[2] = fma(D51, mk, acc[2]);
-    acc[3] = fma(D52, mk, acc[3]);
-  }
-  { const T mk = Mb[31];
-    acc[0] = fma(D32, mk, acc[0]);
-    acc[1] = fma(D47, mk, acc[1]);
-    acc[2] = fma(D52, mk, acc[2]);
-    acc[3] = fma(D53, mk, acc[3]);
-  }
-  { const T mk = Mb[32];
-    acc[0] = fma(D33, mk, acc[0]);
-    acc[1] = fma(D48, mk, acc[1]);
-    acc[2] = fma(D53, mk, acc[2]);
-    acc[3] = fma(D54, mk, acc[3]);
-  }
-  { const T mk = Mb[33];
-    acc[0] = fma(D34, mk, acc[0]);
-    acc[1] = fma(D49, mk, acc[1]);
-    acc[2] = fma(D54, mk, acc[2]);
-    acc[3] = fma(D55, mk, acc[3]);
-  }
-  { const T mk = Mb[34];
     acc[0] = fma(D35, mk, acc[0]);
   }
-  { const T mk = Mb[35];
-    acc[0] = fma(D36, mk, acc[0]);
-  }
-  { const T mk = Mb[36];
+  { const T mk = Mb[29];
     acc[0] = fma(D37, mk, acc[0]);
   }
-  { const T mk = Mb[37];
+  { const T mk = Mb[30];
     acc[0] = fma(D38, mk, acc[0]);
   }
-  { const T mk = Mb[38];
-    acc[0] = fma(D39, mk, acc[0]);
-  }
-  { const T mk = Mb[39];
+  { const T mk = Mb[31];
     acc[0] = fma(D40, mk, acc[0]);
   }
-  { const T mk = Mb[40];
+  { const T mk = Mb[32];
     acc[0] = fma(D41, mk, acc[0]);
   }
-  { const T mk = Mb[41];
-    acc[0] = fma(D42, mk, acc[0]);
-  }
-  { const T mk = Mb[42];
+  { const T mk = Mb[33];
     acc[0] = fma(D43, mk, acc[0]);
   }
-  { const T mk = Mb[43];
+  { const T mk = Mb[34];
     acc[0] = fma(D44, mk, acc[0]);
   }
-  { const T mk = Mb[44];
-    acc[0] = fma(D45, mk, acc[0]);
-  }
-  { const T mk = Mb[45];
-    acc[0] = fma(D46, mk, acc[0]);
-  }
-  { const T mk = Mb[46];
-    acc[0] = fma(D47, mk, acc[0]);
-  }
-  { const T mk = Mb[47];
-    acc[0] = fma(D48, mk, acc[0]);
-  }
-  { const T mk = Mb[48];
-    acc[0] = fma(D49, mk, acc[0]);
-  }
-  { const T mk = Mb[49];
-    acc[0] = fma(D50, mk, acc[0]);
-  }
-  { const T mk = Mb[50];
-    acc[0] = fma(D51, mk, acc[0]);
-  }
-  { const T mk = Mb[51];
-    acc[0] = fma(D52, mk, acc[0]);
-  }
-  { const T mk = Mb[52];
-    acc[0] = fma(D53, mk, acc[0]);
-  }
-  { const T mk = Mb[53];
-    acc[0] = fma(D54, mk, acc[0]);
-  }
-  { const T mk = Mb[54];
-    acc[0] = fma(D55, mk, acc[0]);
-  }
 }
-// derivative tensor D_j = d^j (1/R), j < 56, of M2L m1 p5
 template <typename T>
 __device__ __forceinline__ void dtensor_m1_p5(T x, T y, T z, T* __restrict__ Dout) {
   const T r2 = x * x + y * y + z * z;
@@ -593,53 +401,43 @@ __device__ __forceinline__ void dtensor_m1_p5(T x, T y, T z, T* __restrict__ Dou
   const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
   const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
   const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
-  const T D9 = -(T(3) * (T(2) * z * D3) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
+  const T D9 = -(D4 + D7);
   const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
   const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
   const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
   const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
   const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
-  const T D15 = -(T(5) * (x * D9 + T(2) * z * D6) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
+  const T D15 = -(D10 + D13);
   const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
   const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D18 = -(T(5) * (y * D9 + T(2) * z * D8) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D19 = -(T(5) * (T(3) * z * D9) + T(2) * (T(6) * D3)) * ir2 * cinv<T>(3);
-  const T D20 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D24 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
-  const T D25 = -(T(7) * (T(2) * x * D15 + T(2) * z * D12) + T(3) * (T(2) * D9 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D27 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
-  const T D28 = -(T(7) * (x * D18 + y * D15 + T(2) * z * D14) + T(3) * (T(2) * D5)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (x * D19 + T(3) * z * D15) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D30 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D31 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D32 = -(T(7) * (T(2) * y * D18 + T(2) * z * D17) + T(3) * (T(2) * D9 + T(2) * D7)) * ir2 * cinv<T>(4);
-  const T D33 = -(T(7) * (y * D19 + T(3) * z * D18) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D34 = -(T(7) * (T(4) * z * D19) + T(3) * (T(12) * D9)) * ir2 * cinv<T>(4);
-  const T D35 = -(T(9) * (T(5) * x * D20) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D36 = -(T(9) * (T(4) * x * D21 + y * D20) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D37 = -(T(9) * (T(4) * x * D22 + z * D20) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(3) * x * D23 + T(2) * y * D21) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D39 = -(T(9) * (T(3) * x * D24 + y * D22 + z * D21) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D40 = -(T(9) * (T(3) * x * D25 + T(2) * z * D22) + T(4) * (T(6) * D15 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (T(2) * x * D26 + T(3) * y * D23) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D42 = -(T(9) * (T(2) * x * D27 + T(2) * y * D24 + z * D23) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
-  const T D43 = -(T(9) * (T(2) * x * D28 + y * D25 + T(2) * z * D24) + T(4) * (T(2) * D18 + T(2) * D11)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(2) * x * D29 + T(3) * z * D25) + T(4) * (T(2) * D19 + T(6) * D12)) * ir2 * cinv<T>(5);
-  const T D45 = -(T(9) * (x * D30 + T(4) * y * D26) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D46 = -(T(9) * (x * D31 + T(3) * y * D27 + z * D26) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D47 = -(T(9) * (x * D32 + T(2) * y * D28 + T(2) * z * D27) + T(4) * (T(2) * D15 + T(2) * D13)) * ir2 * cinv<T>(5);
-  const T D48 = -(T(9) * (x * D33 + y * D29 + T(3) * z * D28) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D49 = -(T(9) * (x * D34 + T(4) * z * D29) + T(4) * (T(12) * D15)) * ir2 * cinv<T>(5);
-  const T D50 = -(T(9) * (T(5) * y * D30) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D51 = -(T(9) * (T(4) * y * D31 + z * D30) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
-  const T D52 = -(T(9) * (T(3) * y * D32 + T(2) * z * D31) + T(4) * (T(6) * D18 + T(2) * D16)) * ir2 * cinv<T>(5);
-  const T D53 = -(T(9) * (T(2) * y * D33 + T(3) * z * D32) + T(4) * (T(2) * D19 + T(6) * D17)) * ir2 * cinv<T>(5);
-  const T D54 = -(T(9) * (y * D34 + T(4) * z * D33) + T(4) * (T(12) * D18)) * ir2 * cinv<T>(5);
-  const T D55 = -(T(9) * (T(5) * z * D34) + T(4) * (T(20) * D19)) * ir2 * cinv<T>(5);
+  const T D18 = -(D11 + D16);
+  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
+  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
+  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
+  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T D24 = -(D19 + D22);
+  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T D27 = -(D20 + D25);
+  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
+  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T D30 = -(D22 + D28);
+  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
+  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
+  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
+  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
+  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D36 = -(D31 + D34);
+  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
+  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T D39 = -(D32 + D37);
+  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
+  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D42 = -(D34 + D40);
+  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
+  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T D45 = -(D37 + D43);
   Dout[0] = D0;
   Dout[1] = D1;
   Dout[2] = D2;
@@ -686,18 +484,7 @@ __device__ __forceinline__ void dtensor_m1_p5(T x, T y, T z, T* __restrict__ Dou
   Dout[43] = D43;
   Dout[44] = D44;
   Dout[45] = D45;
-  Dout[46] = D46;
-  Dout[47] = D47;
-  Dout[48] = D48;
-  Dout[49] = D49;
-  Dout[50] = D50;
-  Dout[51] = D51;
-  Dout[52] = D52;
-  Dout[53] = D53;
-  Dout[54] = D54;
-  Dout[55] = D55;
 }
-// M2L m1 p5 with the derivative tensor read from Dt
 template <typename T>
 __device__ __forceinline__ void m2l_m1_p5_pre(const T* __restrict__ Dt, const T* __restrict__ Mb, T* __restrict__ acc) {
   const T D0 = Dt[0];
@@ -746,16 +533,6 @@ __device__ __forceinline__ void m2l_m1_p5_pre(const T* __restrict__ Dt, const T*
   const T D43 = Dt[43];
   const T D44 = Dt[44];
   const T D45 = Dt[45];
-  const T D46 = Dt[46];
-  const T D47 = Dt[47];
-  const T D48 = Dt[48];
-  const T D49 = Dt[49];
-  const T D50 = Dt[50];
-  const T D51 = Dt[51];
-  const T D52 = Dt[52];
-  const T D53 = Dt[53];
-  const T D54 = Dt[54];
-  const T D55 = Dt[55];
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
     acc[1] = fma(D4, mk, acc[1]);
@@ -766,32 +543,22 @@ __device__ __forceinline__ void m2l_m1_p5_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D12, mk, acc[6]);
     acc[7] = fma(D13, mk, acc[7]);
     acc[8] = fma(D14, mk, acc[8]);
-    acc[9] = fma(D15, mk, acc[9]);
+    acc[9] = fma(D19, mk, acc[9]);
     acc[10] = fma(D20, mk, acc[10]);
     acc[11] = fma(D21, mk, acc[11]);
     acc[12] = fma(D22, mk, acc[12]);
     acc[13] = fma(D23, mk, acc[13]);
-    acc[14] = fma(D24, mk, acc[14]);
-    acc[15] = fma(D25, mk, acc[15]);
-    acc[16] = fma(D26, mk, acc[16]);
-    acc[17] = fma(D27, mk, acc[17]);
-    acc[18] = fma(D28, mk, acc[18]);
-    acc[19] = fma(D29, mk, acc[19]);
+    acc[14] = fma(D25, mk, acc[14]);
+    acc[15] = fma(D26, mk, acc[15]);
+    acc[16] = fma(D31, mk, acc[16]);
+    acc[17] = fma(D32, mk, acc[17]);
+    acc[18] = fma(D33, mk, acc[18]);
+    acc[19] = fma(D34, mk, acc[19]);
     acc[20] = fma(D35, mk, acc[20]);
-    acc[21] = fma(D36, mk, acc[21]);
-    acc[22] = fma(D37, mk, acc[22]);
-    acc[23] = fma(D38, mk, acc[23]);
-    acc[24] = fma(D39, mk, acc[24]);
-    acc[25] = fma(D40, mk, acc[25]);
-    acc[26] = fma(D41, mk, acc[26]);
-    acc[27] = fma(D42, mk, acc[27]);
-    acc[28] = fma(D43, mk, acc[28]);
-    acc[29] = fma(D44, mk, acc[29]);
-    acc[30] = fma(D45, mk, acc[30]);
-    acc[31] = fma(D46, mk, acc[31]);
-    acc[32] = fma(D47, mk, acc[32]);
-    acc[33] = fma(D48, mk, acc[33]);
-    acc[34] = fma(D49, mk, acc[34]);
+    acc[21] = fma(D37, mk, acc[21]);
+    acc[22] = fma(D38, mk, acc[22]);
+    acc[23] = fma(D40, mk, acc[23]);
+    acc[24] = fma(D41, mk, acc[24]);
   }
   { const T mk = Mb[1];
     acc[0] = fma(D2, mk, acc[0]);
@@ -803,32 +570,22 @@ __device__ __forceinline__ void m2l_m1_p5_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D14, mk, acc[6]);
     acc[7] = fma(D16, mk, acc[7]);
     acc[8] = fma(D17, mk, acc[8]);
-    acc[9] = fma(D18, mk, acc[9]);
-    acc[10] = fma(D21, mk, acc[10]);
+    acc[9] = fma(D20, mk, acc[9]);
+    acc[10] = fma(D22, mk, acc[10]);
     acc[11] = fma(D23, mk, acc[11]);
-    acc[12] = fma(D24, mk, acc[12]);
+    acc[12] = fma(D25, mk, acc[12]);
     acc[13] = fma(D26, mk, acc[13]);
-    acc[14] = fma(D27, mk, acc[14]);
-    acc[15] = fma(D28, mk, acc[15]);
-    acc[16] = fma(D30, mk, acc[16]);
-    acc[17] = fma(D31, mk, acc[17]);
-    acc[18] = fma(D32, mk, acc[18]);
-    acc[19] = fma(D33, mk, acc[19]);
-    acc[20] = fma(D36, mk, acc[20]);
-    acc[21] = fma(D38, mk, acc[21]);
-    acc[22] = fma(D39, mk, acc[22]);
-    acc[23] = fma(D41, mk, acc[23]);
-    acc[24] = fma(D42, mk, acc[24]);
-    acc[25] = fma(D43, mk, acc[25]);
-    acc[26] = fma(D45, mk, acc[26]);
-    acc[27] = fma(D46, mk, acc[27]);
-    acc[28] = fma(D47, mk, acc[28]);
-    acc[29] = fma(D48, mk, acc[29]);
-    acc[30] = fma(D50, mk, acc[30]);
-    acc[31] = fma(D51, mk, acc[31]);
-    acc[32] = fma(D52, mk, acc[32]);
-    acc[33] = fma(D53, mk, acc[33]);
-    acc[34] = fma(D54, mk, acc[34]);
+    acc[14] = fma(D28, mk, acc[14]);
+    acc[15] = fma(D29, mk, acc[15]);
+    acc[16] = fma(D32, mk, acc[16]);
+    acc[17] = fma(D34, mk, acc[17]);
+    acc[18] = fma(D35, mk, acc[18]);
+    acc[19] = fma(D37, mk, acc[19]);
+    acc[20] = fma(D38, mk, acc[20]);
+    acc[21] = fma(D40, mk, acc[21]);
+    acc[22] = fma(D41, mk, acc[22]);
+    acc[23] = fma(D43, mk, acc[23]);
+    acc[24] = fma(D44, mk, acc[24]);
   }
   { const T mk = Mb[2];
     acc[0] = fma(D3, mk, acc[0]);
@@ -840,441 +597,356 @@ __device__ __forceinline__ void m2l_m1_p5_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D15, mk, acc[6]);
     acc[7] = fma(D17, mk, acc[7]);
     acc[8] = fma(D18, mk, acc[8]);
-    acc[9] = fma(D19, mk, acc[9]);
-    acc[10] = fma(D22, mk, acc[10]);
+    acc[9] = fma(D21, mk, acc[9]);
+    acc[10] = fma(D23, mk, acc[10]);
     acc[11] = fma(D24, mk, acc[11]);
-    acc[12] = fma(D25, mk, acc[12]);
+    acc[12] = fma(D26, mk, acc[12]);
     acc[13] = fma(D27, mk, acc[13]);
-    acc[14] = fma(D28, mk, acc[14]);
-    acc[15] = fma(D29, mk, acc[15]);
-    acc[16] = fma(D31, mk, acc[16]);
-    acc[17] = fma(D32, mk, acc[17]);
-    acc[18] = fma(D33, mk, acc[18]);
-    acc[19] = fma(D34, mk, acc[19]);
-    acc[20] = fma(D37, mk, acc[20]);
-    acc[21] = fma(D39, mk, acc[21]);
-    acc[22] = fma(D40, mk, acc[22]);
-    acc[23] = fma(D42, mk, acc[23]);
-    acc[24] = fma(D43, mk, acc[24]);
-    acc[25] = fma(D44, mk, acc[25]);
-    acc[26] = fma(D46, mk, acc[26]);
-    acc[27] = fma(D47, mk, acc[27]);
-    acc[28] = fma(D48, mk, acc[28]);
-    acc[29] = fma(D49, mk, acc[29]);
-    acc[30] = fma(D51, mk, acc[30]);
-    acc[31] = fma(D52, mk, acc[31]);
-    acc[32] = fma(D53, mk, acc[32]);
-    acc[33] = fma(D54, mk, acc[33]);
-    acc[34] = fma(D55, mk, acc[34]);
+    acc[14] = fma(D29, mk, acc[14]);
+    acc[15] = fma(D30, mk, acc[15]);
+    acc[16] = fma(D33, mk, acc[16]);
+    acc[17] = fma(D35, mk, acc[17]);
+    acc[18] = fma(D36, mk, acc[18]);
+    acc[19] = fma(D38, mk, acc[19]);
+    acc[20] = fma(D39, mk, acc[20]);
+    acc[21] = fma(D41, mk, acc[21]);
+    acc[22] = fma(D42, mk, acc[22]);
+    acc[23] = fma(D44, mk, acc[23]);
+    acc[24] = fma(D45, mk, acc[24]);
   }
   { const T mk = Mb[3];
     acc[0] = fma(D4, mk, acc[0]);
     acc[1] = fma(D10, mk, acc[1]);
     acc[2] = fma(D11, mk, acc[2]);
     acc[3] = fma(D12, mk, acc[3]);
-    acc[4] = fma(D20, mk, acc[4]);
-    acc[5] = fma(D21, mk, acc[5]);
-    acc[6] = fma(D22, mk, acc[6]);
-    acc[7] = fma(D23, mk, acc[7]);
-    acc[8] = fma(D24, mk, acc[8]);
-    acc[9] = fma(D25, mk, acc[9]);
-    acc[10] = fma(D35, mk, acc[10]);
-    acc[11] = fma(D36, mk, acc[11]);
-    acc[12] = fma(D37, mk, acc[12]);
-    acc[13] = fma(D38, mk, acc[13]);
-    acc[14] = fma(D39, mk, acc[14]);
-    acc[15] = fma(D40, mk, acc[15]);
-    acc[16] = fma(D41, mk, acc[16]);
-    acc[17] = fma(D42, mk, acc[17]);
-    acc[18] = fma(D43, mk, acc[18]);
-    acc[19] = fma(D44, mk, acc[19]);
+    acc[4] = fma(D19, mk, acc[4]);
+    acc[5] = fma(D20, mk, acc[5]);
+    acc[6] = fma(D21, mk, acc[6]);
+    acc[7] = fma(D22, mk, acc[7]);
+    acc[8] = fma(D23, mk, acc[8]);
+    acc[9] = fma(D31, mk, acc[9]);
+    acc[10] = fma(D32, mk, acc[10]);
+    acc[11] = fma(D33, mk, acc[11]);
+    acc[12] = fma(D34, mk, acc[12]);
+    acc[13] = fma(D35, mk, acc[13]);
+    acc[14] = fma(D37, mk, acc[14]);
+    acc[15] = fma(D38, mk, acc[15]);
   }
   { const T mk = Mb[4];
     acc[0] = fma(D5, mk, acc[0]);
     acc[1] = fma(D11, mk, acc[1]);
     acc[2] = fma(D13, mk, acc[2]);
     acc[3] = fma(D14, mk, acc[3]);
-    acc[4] = fma(D21, mk, acc[4]);
-    acc[5] = fma(D23, mk, acc[5]);
-    acc[6] = fma(D24, mk, acc[6]);
-    acc[7] = fma(D26, mk, acc[7]);
-    acc[8] = fma(D27, mk, acc[8]);
-    acc[9] = fma(D28, mk, acc[9]);
-    acc[10] = fma(D36, mk, acc[10]);
-    acc[11] = fma(D38, mk, acc[11]);
-    acc[12] = fma(D39, mk, acc[12]);
-    acc[13] = fma(D41, mk, acc[13]);
-    acc[14] = fma(D42, mk, acc[14]);
-    acc[15] = fma(D43, mk, acc[15]);
-    acc[16] = fma(D45, mk, acc[16]);
-    acc[17] = fma(D46, mk, acc[17]);
-    acc[18] = fma(D47, mk, acc[18]);
-    acc[19] = fma(D48, mk, acc[19]);
+    acc[4] = fma(D20, mk, acc[4]);
+    acc[5] = fma(D22, mk, acc[5]);
+    acc[6] = fma(D23, mk, acc[6]);
+    acc[7] = fma(D25, mk, acc[7]);
+    acc[8] = fma(D26, mk, acc[8]);
+    acc[9] = fma(D32, mk, acc[9]);
+    acc[10] = fma(D34, mk, acc[10]);
+    acc[11] = fma(D35, mk, acc[11]);
+    acc[12] = fma(D37, mk, acc[12]);
+    acc[13] = fma(D38, mk, acc[13]);
+    acc[14] = fma(D40, mk, acc[14]);
+    acc[15] = fma(D41, mk, acc[15]);
   }
   { const T mk = Mb[5];
     acc[0] = fma(D6, mk, acc[0]);
     acc[1] = fma(D12, mk, acc[1]);
     acc[2] = fma(D14, mk, acc[2]);
     acc[3] = fma(D15, mk, acc[3]);
-    acc[4] = fma(D22, mk, acc[4]);
-    acc[5] = fma(D24, mk, acc[5]);
-    acc[6] = fma(D25, mk, acc[6]);
-    acc[7] = fma(D27, mk, acc[7]);
-    acc[8] = fma(D28, mk, acc[8]);
-    acc[9] = fma(D29, mk, acc[9]);
-    acc[10] = fma(D37, mk, acc[10]);
-    acc[11] = fma(D39, mk, acc[11]);
-    acc[12] = fma(D40, mk, acc[12]);
-    acc[13] = fma(D42, mk, acc[13]);
-    acc[14] = fma(D43, mk, acc[14]);
-    acc[15] = fma(D44, mk, acc[15]);
-    acc[16] = fma(D46, mk, acc[16]);
-    acc[17] = fma(D47, mk, acc[17]);
-    acc[18] = fma(D48, mk, acc[18]);
-    acc[19] = fma(D49, mk, acc[19]);
+    acc[4] = fma(D21, mk, acc[4]);
+    acc[5] = fma(D23, mk, acc[5]);
+    acc[6] = fma(D24, mk, acc[6]);
+    acc[7] = fma(D26, mk, acc[7]);
+    acc[8] = fma(D27, mk, acc[8]);
+    acc[9] = fma(D33, mk, acc[9]);
+    acc[10] = fma(D35, mk, acc[10]);
+    acc[11] = fma(D36, mk, acc[11]);
+    acc[12] = fma(D38, mk, acc[12]);
+    acc[13] = fma(D39, mk, acc[13]);
+    acc[14] = fma(D41, mk, acc[14]);
+    acc[15] = fma(D42, mk, acc[15]);
   }
   { const T mk = Mb[6];
     acc[0] = fma(D7, mk, acc[0]);
     acc[1] = fma(D13, mk, acc[1]);
     acc[2] = fma(D16, mk, acc[2]);
     acc[3] = fma(D17, mk, acc[3]);
-    acc[4] = fma(D23, mk, acc[4]);
-    acc[5] = fma(D26, mk, acc[5]);
-    acc[6] = fma(D27, mk, acc[6]);
-    acc[7] = fma(D30, mk, acc[7]);
-    acc[8] = fma(D31, mk, acc[8]);
-    acc[9] = fma(D32, mk, acc[9]);
-    acc[10] = fma(D38, mk, acc[10]);
-    acc[11] = fma(D41, mk, acc[11]);
-    acc[12] = fma(D42, mk, acc[12]);
-    acc[13] = fma(D45, mk, acc[13]);
-    acc[14] = fma(D46, mk, acc[14]);
-    acc[15] = fma(D47, mk, acc[15]);
-    acc[16] = fma(D50, mk, acc[16]);
-    acc[17] = fma(D51, mk, acc[17]);
-    acc[18] = fma(D52, mk, acc[18]);
-    acc[19] = fma(D53, mk, acc[19]);
+    acc[4] = fma(D22, mk, acc[4]);
+    acc[5] = fma(D25, mk, acc[5]);
+    acc[6] = fma(D26, mk, acc[6]);
+    acc[7] = fma(D28, mk, acc[7]);
+    acc[8] = fma(D29, mk, acc[8]);
+    acc[9] = fma(D34, mk, acc[9]);
+    acc[10] = fma(D37, mk, acc[10]);
+    acc[11] = fma(D38, mk, acc[11]);
+    acc[12] = fma(D40, mk, acc[12]);
+    acc[13] = fma(D41, mk, acc[13]);
+    acc[14] = fma(D43, mk, acc[14]);
+    acc[15] = fma(D44, mk, acc[15]);
   }
   { const T mk = Mb[7];
     acc[0] = fma(D8, mk, acc[0]);
     acc[1] = fma(D14, mk, acc[1]);
     acc[2] = fma(D17, mk, acc[2]);
     acc[3] = fma(D18, mk, acc[3]);
-    acc[4] = fma(D24, mk, acc[4]);
-    acc[5] = fma(D27, mk, acc[5]);
-    acc[6] = fma(D28, mk, acc[6]);
-    acc[7] = fma(D31, mk, acc[7]);
-    acc[8] = fma(D32, mk, acc[8]);
-    acc[9] = fma(D33, mk, acc[9]);
-    acc[10] = fma(D39, mk, acc[10]);
-    acc[11] = fma(D42, mk, acc[11]);
-    acc[12] = fma(D43, mk, acc[12]);
-    acc[13] = fma(D46, mk, acc[13]);
-    acc[14] = fma(D47, mk, acc[14]);
-    acc[15] = fma(D48, mk, acc[15]);
-    acc[16] = fma(D51, mk, acc[16]);
-    acc[17] = fma(D52, mk, acc[17]);
-    acc[18] = fma(D53, mk, acc[18]);
-    acc[19] = fma(D54, mk, acc[19]);
+    acc[4] = fma(D23, mk, acc[4]);
+    acc[5] = fma(D26, mk, acc[5]);
+    acc[6] = fma(D27, mk, acc[6]);
+    acc[7] = fma(D29, mk, acc[7]);
+    acc[8] = fma(D30, mk, acc[8]);
+    acc[9] = fma(D35, mk, acc[9]);
+    acc[10] = fma(D38, mk, acc[10]);
+    acc[11] = fma(D39, mk, acc[11]);
+    acc[12] = fma(D41, mk, acc[12]);
+    acc[13] = fma(D42, mk, acc[13]);
+    acc[14] = fma(D44, mk, acc[14]);
+    acc[15] = fma(D45, mk, acc[15]);
   }
   { const T mk = Mb[8];
-    acc[0] = fma(D9, mk, acc[0]);
-    acc[1] = fma(D15, mk, acc[1]);
-    acc[2] = fma(D18, mk, acc[2]);
-    acc[3] = fma(D19, mk, acc[3]);
-    acc[4] = fma(D25, mk, acc[4]);
-    acc[5] = fma(D28, mk, acc[5]);
-    acc[6] = fma(D29, mk, acc[6]);
-    acc[7] = fma(D32, mk, acc[7]);
-    acc[8] = fma(D33, mk, acc[8]);
-    acc[9] = fma(D34, mk, acc[9]);
-    acc[10] = fma(D40, mk, acc[10]);
-    acc[11] = fma(D43, mk, acc[11]);
-    acc[12] = fma(D44, mk, acc[12]);
-    acc[13] = fma(D47, mk, acc[13]);
-    acc[14] = fma(D48, mk, acc[14]);
-    acc[15] = fma(D49, mk, acc[15]);
-    acc[16] = fma(D52, mk, acc[16]);
-    acc[17] = fma(D53, mk, acc[17]);
-    acc[18] = fma(D54, mk, acc[18]);
-    acc[19] = fma(D55, mk, acc[19]);
+    acc[0] = fma(D10, mk, acc[0]);
+    acc[1] = fma(D19, mk, acc[1]);
+    acc[2] = fma(D20, mk, acc[2]);
+    acc[3] = fma(D21, mk, acc[3]);
+    acc[4] = fma(D31, mk, acc[4]);
+    acc[5] = fma(D32, mk, acc[5]);
+    acc[6] = fma(D33, mk, acc[6]);
+    acc[7] = fma(D34, mk, acc[7]);
+    acc[8] = fma(D35, mk, acc[8]);
   }
   { const T mk = Mb[9];
-    acc[0] = fma(D10, mk, acc[0]);
+    acc[0] = fma(D11, mk, acc[0]);
     acc[1] = fma(D20, mk, acc[1]);
-    acc[2] = fma(D21, mk, acc[2]);
-    acc[3] = fma(D22, mk, acc[3]);
-    acc[4] = fma(D35, mk, acc[4]);
-    acc[5] = fma(D36, mk, acc[5]);
-    acc[6] = fma(D37, mk, acc[6]);
-    acc[7] = fma(D38, mk, acc[7]);
-    acc[8] = fma(D39, mk, acc[8]);
-    acc[9] = fma(D40, mk, acc[9]);
+    acc[2] = fma(D22, mk, acc[2]);
+    acc[3] = fma(D23, mk, acc[3]);
+    acc[4] = fma(D32, mk, acc[4]);
+    acc[5] = fma(D34, mk, acc[5]);
+    acc[6] = fma(D35, mk, acc[6]);
+    acc[7] = fma(D37, mk, acc[7]);
+    acc[8] = fma(D38, mk, acc[8]);
   }
   { const T mk = Mb[10];
-    acc[0] = fma(D11, mk, acc[0]);
+    acc[0] = fma(D12, mk, acc[0]);
     acc[1] = fma(D21, mk, acc[1]);
     acc[2] = fma(D23, mk, acc[2]);
     acc[3] = fma(D24, mk, acc[3]);
-    acc[4] = fma(D36, mk, acc[4]);
+    acc[4] = fma(D33, mk, acc[4]);
+    acc[5] = fma(D35, mk, acc[5]);
+    acc[6] = fma(D36, mk, acc[6]);
+    acc[7] = fma(D38, mk, acc[7]);
+    acc[8] = fma(D39, mk, acc[8]);
+  }
+  { const T mk = Mb[11];
+    acc[0] = fma(D13, mk, acc[0]);
+    acc[1] = fma(D22, mk, acc[1]);
+    acc[2] = fma(D25, mk, acc[2]);
+    acc[3] = fma(D26, mk, acc[3]);
+    acc[4] = fma(D34, mk, acc[4]);
+    acc[5] = fma(D37, mk, acc[5]);
+    acc[6] = fma(D38, mk, acc[6]);
+    acc[7] = fma(D40, mk, acc[7]);
+    acc[8] = fma(D41, mk, acc[8]);
+  }
+  { const T mk = Mb[12];
+    acc[0] = fma(D14, mk, acc[0]);
+    acc[1] = fma(D23, mk, acc[1]);
+    acc[2] = fma(D26, mk, acc[2]);
+    acc[3] = fma(D27, mk, acc[3]);
+    acc[4] = fma(D35, mk, acc[4]);
     acc[5] = fma(D38, mk, acc[5]);
     acc[6] = fma(D39, mk, acc[6]);
     acc[7] = fma(D41, mk, acc[7]);
     acc[8] = fma(D42, mk, acc[8]);
-    acc[9] = fma(D43, mk, acc[9]);
-  }
-  { const T mk = Mb[11];
-    acc[0] = fma(D12, mk, acc[0]);
-    acc[1] = fma(D22, mk, acc[1]);
-    acc[2] = fma(D24, mk, acc[2]);
-    acc[3] = fma(D25, mk, acc[3]);
-    acc[4] = fma(D37, mk, acc[4]);
-    acc[5] = fma(D39, mk, acc[5]);
-    acc[6] = fma(D40, mk, acc[6]);
-    acc[7] = fma(D42, mk, acc[7]);
-    acc[8] = fma(D43, mk, acc[8]);
-    acc[9] = fma(D44, mk, acc[9]);
-  }
-  { const T mk = Mb[12];
-    acc[0] = fma(D13, mk, acc[0]);
-    acc[1] = fma(D23, mk, acc[1]);
-    acc[2] = fma(D26, mk, acc[2]);
-    acc[3] = fma(D27, mk, acc[3]);
-    acc[4] = fma(D38, mk, acc[4]);
-    acc[5] = fma(D41, mk, acc[5]);
-    acc[6] = fma(D42, mk, acc[6]);
-    acc[7] = fma(D45, mk, acc[7]);
-    acc[8] = fma(D46, mk, acc[8]);
-    acc[9] = fma(D47, mk, acc[9]);
   }
   { const T mk = Mb[13];
-    acc[0] = fma(D14, mk, acc[0]);
-    acc[1] = fma(D24, mk, acc[1]);
-    acc[2] = fma(D27, mk, acc[2]);
-    acc[3] = fma(D28, mk, acc[3]);
-    acc[4] = fma(D39, mk, acc[4]);
-    acc[5] = fma(D42, mk, acc[5]);
-    acc[6] = fma(D43, mk, acc[6]);
-    acc[7] = fma(D46, mk, acc[7]);
-    acc[8] = fma(D47, mk, acc[8]);
-    acc[9] = fma(D48, mk, acc[9]);
-  }
-  { const T mk = Mb[14];
-    acc[0] = fma(D15, mk, acc[0]);
+    acc[0] = fma(D16, mk, acc[0]);
     acc[1] = fma(D25, mk, acc[1]);
     acc[2] = fma(D28, mk, acc[2]);
     acc[3] = fma(D29, mk, acc[3]);
-    acc[4] = fma(D40, mk, acc[4]);
-    acc[5] = fma(D43, mk, acc[5]);
-    acc[6] = fma(D44, mk, acc[6]);
-    acc[7] = fma(D47, mk, acc[7]);
-    acc[8] = fma(D48, mk, acc[8]);
-    acc[9] = fma(D49, mk, acc[9]);
+    acc[4] = fma(D37, mk, acc[4]);
+    acc[5] = fma(D40, mk, acc[5]);
+    acc[6] = fma(D41, mk, acc[6]);
+    acc[7] = fma(D43, mk, acc[7]);
+    acc[8] = fma(D44, mk, acc[8]);
+  }
+  { const T mk = Mb[14];
+    acc[0] = fma(D17, mk, acc[0]);
+    acc[1] = fma(D26, mk, acc[1]);
+    acc[2] = fma(D29, mk, acc[2]);
+    acc[3] = fma(D30, mk, acc[3]);
+    acc[4] = fma(D38, mk, acc[4]);
+    acc[5] = fma(D41, mk, acc[5]);
+    acc[6] = fma(D42, mk, acc[6]);
+    acc[7] = fma(D44, mk, acc[7]);
+    acc[8] = fma(D45, mk, acc[8]);
   }
   { const T mk = Mb[15];
-    acc[0] = fma(D16, mk, acc[0]);
-    acc[1] = fma(D26, mk, acc[1]);
-    acc[2] = fma(D30, mk, acc[2]);
-    acc[3] = fma(D31, mk, acc[3]);
-    acc[4] = fma(D41, mk, acc[4]);
-    acc[5] = fma(D45, mk, acc[5]);
-    acc[6] = fma(D46, mk, acc[6]);
-    acc[7] = fma(D50, mk, acc[7]);
-    acc[8] = fma(D51, mk, acc[8]);
-    acc[9] = fma(D52, mk, acc[9]);
-  }
-  { const T mk = Mb[16];
-    acc[0] = fma(D17, mk, acc[0]);
-    acc[1] = fma(D27, mk, acc[1]);
-    acc[2] = fma(D31, mk, acc[2]);
-    acc[3] = fma(D32, mk, acc[3]);
-    acc[4] = fma(D42, mk, acc[4]);
-    acc[5] = fma(D46, mk, acc[5]);
-    acc[6] = fma(D47, mk, acc[6]);
-    acc[7] = fma(D51, mk, acc[7]);
-    acc[8] = fma(D52, mk, acc[8]);
-    acc[9] = fma(D53, mk, acc[9]);
-  }
-  { const T mk = Mb[17];
-    acc[0] = fma(D18, mk, acc[0]);
-    acc[1] = fma(D28, mk, acc[1]);
+    acc[0] = fma(D19, mk, acc[0]);
+    acc[1] = fma(D31, mk, acc[1]);
     acc[2] = fma(D32, mk, acc[2]);
     acc[3] = fma(D33, mk, acc[3]);
-    acc[4] = fma(D43, mk, acc[4]);
-    acc[5] = fma(D47, mk, acc[5]);
-    acc[6] = fma(D48, mk, acc[6]);
-    acc[7] = fma(D52, mk, acc[7]);
-    acc[8] = fma(D53, mk, acc[8]);
-    acc[9] = fma(D54, mk, acc[9]);
+  }
+  { const T mk = Mb[16];
+    acc[0] = fma(D20, mk, acc[0]);
+    acc[1] = fma(D32, mk, acc[1]);
+    acc[2] = fma(D34, mk, acc[2]);
+    acc[3] = fma(D35, mk, acc[3]);
+  }
+  { const T mk = Mb[17];
+    acc[0] = fma(D21, mk, acc[0]);
+    acc[1] = fma(D33, mk, acc[1]);
+    acc[2] = fma(D35, mk, acc[2]);
+    acc[3] = fma(D36, mk, acc[3]);
   }
   { const T mk = Mb[18];
-    acc[0] = fma(D19, mk, acc[0]);
-    acc[1] = fma(D29, mk, acc[1]);
-    acc[2] = fma(D33, mk, acc[2]);
-    acc[3] = fma(D34, mk, acc[3]);
-    acc[4] = fma(D44, mk, acc[4]);
-    acc[5] = fma(D48, mk, acc[5]);
-    acc[6] = fma(D49, mk, acc[6]);
-    acc[7] = fma(D53, mk, acc[7]);
-    acc[8] = fma(D54, mk, acc[8]);
-    acc[9] = fma(D55, mk, acc[9]);
+    acc[0] = fma(D22, mk, acc[0]);
+    acc[1] = fma(D34, mk, acc[1]);
+    acc[2] = fma(D37, mk, acc[2]);
+    acc[3] = fma(D38, mk, acc[3]);
   }
   { const T mk = Mb[19];
-    acc[0] = fma(D20, mk, acc[0]);
+    acc[0] = fma(D23, mk, acc[0]);
     acc[1] = fma(D35, mk, acc[1]);
-    acc[2] = fma(D36, mk, acc[2]);
-    acc[3] = fma(D37, mk, acc[3]);
-  }
-  { const T mk = Mb[20];
-    acc[0] = fma(D21, mk, acc[0]);
-    acc[1] = fma(D36, mk, acc[1]);
     acc[2] = fma(D38, mk, acc[2]);
     acc[3] = fma(D39, mk, acc[3]);
   }
-  { const T mk = Mb[21];
-    acc[0] = fma(D22, mk, acc[0]);
+  { const T mk = Mb[20];
+    acc[0] = fma(D25, mk, acc[0]);
     acc[1] = fma(D37, mk, acc[1]);
-    acc[2] = fma(D39, mk, acc[2]);
-    acc[3] = fma(D40, mk, acc[3]);
+    acc[2] = fma(D40, mk, acc[2]);
+    acc[3] = fma(D41, mk, acc[3]);
   }
-  { const T mk = Mb[22];
-    acc[0] = fma(D23, mk, acc[0]);
+  { const T mk = Mb[21];
+    acc[0] = fma(D26, mk, acc[0]);
     acc[1] = fma(D38, mk, acc[1]);
     acc[2] = fma(D41, mk, acc[2]);
     acc[3] = fma(D42, mk, acc[3]);
   }
-  { const T mk = Mb[23];
-    acc[0] = fma(D24, mk, acc[0]);
-    acc[1] = fma(D39, mk, acc[1]);
-    acc[2] = fma(D42, mk, acc[2]);
-    acc[3] = fma(D43, mk, acc[3]);
-  }
-  { const T mk = Mb[24];
-    acc[0] = fma(D25, mk, acc[0]);
+  { const T mk = Mb[22];
+    acc[0] = fma(D28, mk, acc[0]);
     acc[1] = fma(D40, mk, acc[1]);
     acc[2] = fma(D43, mk, acc[2]);
     acc[3] = fma(D44, mk, acc[3]);
   }
-  { const T mk = Mb[25];
-    acc[0] = fma(D26, mk, acc[0]);
+  { const T mk = Mb[23];
+    acc[0] = fma(D29, mk, acc[0]);
     acc[1] = fma(D41, mk, acc[1]);
-    acc[2] = fma(D45, mk, acc[2]);
-    acc[3] = fma(D46, mk, acc[3]);
+    acc[2] = fma(D44, mk, acc[2]);
+    acc[3] = fma(D45, mk, acc[3]);
+  }
+  { const T mk = Mb[24];
+    acc[0] = fma(D31, mk, acc[0]);
+  }
+  { const T mk = Mb[25];
+    acc[0] = fma(D32, mk, acc[0]);
   }
   { const T mk = Mb[26];
-    acc[0] = fma(D27, mk, acc[0]);
-    acc[1] = fma(D42, mk, acc[1]);
-    acc[2] = fma(D46, mk, acc[2]);
-    acc[3] = fma(D47, mk, acc[3]);
+    acc[0] = fma(D33, mk, acc[0]);
   }
   { const T mk = Mb[27];
-    acc[0] = fma(D28, mk, acc[0]);
-    acc[1] = fma(D43, mk, acc[1]);
-    acc[2] = fma(D47, mk, acc[2]);
-    acc[3] = fma(D48, mk, acc[3]);
+    acc[0] = fma(D34, mk, acc[0]);
   }
   { const T mk = Mb[28];
-    acc[0] = fma(D29, mk, acc[0]);
-    acc[1] = fma(D44, mk, acc[1]);
-    acc[2] = fma(D48, mk, acc[2]);
-    acc[3] = fma(D49, mk, acc[3]);
-  }
-  { const T mk = Mb[29];
-    acc[0] = fma(D30, mk, acc[0]);
-    acc[1] = fma(D45, mk, acc[1]);
-    acc[2] = fma(D50, mk, acc[2]);
-    acc[3] = fma(D51, mk, acc[3]);
-  }
-  { const T mk = Mb[30];
-    acc[0] = fma(D31, mk, acc[0]);
-    acc[1] = fma(D46, mk, acc[1]);
-    acc[2] = fma(D51, mk, acc[2]);
-    acc[3] = fma(D52, mk, acc[3]);
-  }
-  { const T mk = Mb[31];
-    acc[0] = fma(D32, mk, acc[0]);
-    acc[1] = fma(D47, mk, acc[1]);
-    acc[2] = fma(D52, mk, acc[2]);
-    acc[3] = fma(D53, mk, acc[3]);
-  }
-  { const T mk = Mb[32];
-    acc[0] = fma(D33, mk, acc[0]);
-    acc[1] = fma(D48, mk, acc[1]);
-    acc[2] = fma(D53, mk, acc[2]);
-    acc[3] = fma(D54, mk, acc[3]);
-  }
-  { const T mk = Mb[33];
-    acc[0] = fma(D34, mk, acc[0]);
-    acc[1] = fma(D49, mk, acc[1]);
-    acc[2] = fma(D54, mk, acc[2]);
-    acc[3] = fma(D55, mk, acc[3]);
-  }
-  { const T mk = Mb[34];
     acc[0] = fma(D35, mk, acc[0]);
   }
-  { const T mk = Mb[35];
-    acc[0] = fma(D36, mk, acc[0]);
-  }
-  { const T mk = Mb[36];
+  { const T mk = Mb[29];
     acc[0] = fma(D37, mk, acc[0]);
   }
-  { const T mk = Mb[37];
+  { const T mk = Mb[30];
     acc[0] = fma(D38, mk, acc[0]);
   }
-  { const T mk = Mb[38];
-    acc[0] = fma(D39, mk, acc[0]);
-  }
-  { const T mk = Mb[39];
+  { const T mk = Mb[31];
     acc[0] = fma(D40, mk, acc[0]);
   }
-  { const T mk = Mb[40];
+  { const T mk = Mb[32];
     acc[0] = fma(D41, mk, acc[0]);
   }
-  { const T mk = Mb[41];
-    acc[0] = fma(D42, mk, acc[0]);
-  }
-  { const T mk = Mb[42];
+  { const T mk = Mb[33];
     acc[0] = fma(D43, mk, acc[0]);
   }
-  { const T mk = Mb[43];
+  { const T mk = Mb[34];
     acc[0] = fma(D44, mk, acc[0]);
   }
-  { const T mk = Mb[44];
-    acc[0] = fma(D45, mk, acc[0]);
-  }
-  { const T mk = Mb[45];
-    acc[0] = fma(D46, mk, acc[0]);
-  }
-  { const T mk = Mb[46];
-    acc[0] = fma(D47, mk, acc[0]);
-  }
-  { const T mk = Mb[47];
-    acc[0] = fma(D48, mk, acc[0]);
-  }
-  { const T mk = Mb[48];
-    acc[0] = fma(D49, mk, acc[0]);
-  }
-  { const T mk = Mb[49];
-    acc[0] = fma(D50, mk, acc[0]);
-  }
-  { const T mk = Mb[50];
-    acc[0] = fma(D51, mk, acc[0]);
-  }
-  { const T mk = Mb[51];
-    acc[0] = fma(D52, mk, acc[0]);
-  }
-  { const T mk = Mb[52];
-    acc[0] = fma(D53, mk, acc[0]);
-  }
-  { const T mk = Mb[53];
-    acc[0] = fma(D54, mk, acc[0]);
-  }
-  { const T mk = Mb[54];
-    acc[0] = fma(D55, mk, acc[0]);
-  }
 }
+static __constant__ unsigned char m2l_w_m1_p5[265] = {
+  1, 4, 5, 6, 10, 11, 12, 13, 14, 19, 20, 21, 22, 23, 25, 26, 31, 32, 33, 34, 35, 37, 38, 40, 41, 2, 5, 7, 8, 11, 13, 14, 16, 17, 20, 22, 23, 25, 26, 28, 29, 32, 34, 35, 37, 38, 40, 41, 43, 44, 3, 6, 8, 9, 12, 14, 15, 17, 18, 21, 23, 24, 26, 27, 29, 30, 33, 35, 36, 38, 39, 41, 42, 44, 45, 4, 10, 11, 12, 19, 20, 21, 22, 23, 31, 32, 33, 34, 35, 37, 38, 5, 11, 13, 14, 20, 22, 23, 25, 26, 32, 34, 35, 37, 38, 40, 41, 6, 12, 14, 15, 21, 23, 24, 26, 27, 33, 35, 36, 38, 39, 41, 42, 7, 13, 16, 17, 22, 25, 26, 28, 29, 34, 37, 38, 40, 41, 43, 44, 8, 14, 17, 18, 23, 26, 27, 29, 30, 35, 38, 39, 41, 42, 44, 45, 10, 19, 20, 21, 31, 32, 33, 34, 35, 11, 20, 22, 23, 32, 34, 35, 37, 38, 12, 21, 23, 24, 33, 35, 36, 38, 39, 13, 22, 25, 26, 34, 37, 38, 40, 41, 14, 23, 26, 27, 35, 38, 39, 41, 42, 16, 25, 28, 29, 37, 40, 41, 43, 44, 17, 26, 29, 30, 38, 41, 42, 44, 45, 19, 31, 32, 33, 20, 32, 34, 35, 21, 33, 35, 36, 22, 34, 37, 38, 23, 35, 38, 39, 25, 37, 40, 41, 26, 38, 41, 42, 28, 40, 43, 44, 29, 41, 44, 45, 31, 32, 33, 34, 35, 37, 38, 40, 41, 43, 44};
+static __device__ const signed char m2l_fold_m1_p5[35][4][2] = {
+  {{0, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{1, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{2, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{3, 1}, {8, -1}, {0, 0}, {0, 0}},
+  {{4, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{5, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{6, 1}, {8, -1}, {0, 0}, {0, 0}},
+  {{7, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{9, 1}, {14, -1}, {0, 0}, {0, 0}},
+  {{10, 1}, {17, -1}, {0, 0}, {0, 0}},
+  {{11, 1}, {18, -1}, {0, 0}, {0, 0}},
+  {{12, 1}, {14, -1}, {0, 0}, {0, 0}},
+  {{13, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{15, 1}, {17, -1}, {0, 0}, {0, 0}},
+  {{16, 1}, {18, -1}, {0, 0}, {0, 0}},
+  {{19, 1}, {24, -1}, {33, 1}, {0, 0}},
+  {{20, 1}, {27, -1}, {0, 0}, {0, 0}},
+  {{21, 1}, {28, -1}, {0, 0}, {0, 0}},
+  {{22, 1}, {24, -1}, {31, -1}, {33, 2}},
+  {{23, 1}, {32, -1}, {0, 0}, {0, 0}},
+  {{25, 1}, {27, -1}, {0, 0}, {0, 0}},
+  {{26, 1}, {28, -1}, {0, 0}, {0, 0}},
+  {{29, 1}, {31, -1}, {33, 1}, {0, 0}},
+  {{30, 1}, {32, -1}, {0, 0}, {0, 0}},
+  {{34, 1}, {39, -1}, {48, 1}, {0, 0}},
+  {{35, 1}, {42, -1}, {53, 1}, {0, 0}},
+  {{36, 1}, {43, -1}, {54, 1}, {0, 0}},
+  {{37, 1}, {39, -1}, {46, -1}, {48, 2}},
+  {{38, 1}, {47, -1}, {0, 0}, {0, 0}},
+  {{40, 1}, {42, -1}, {51, -1}, {53, 2}},
+  {{41, 1}, {43, -1}, {52, -1}, {54, 2}},
+  {{44, 1}, {46, -1}, {48, 1}, {0, 0}},
+  {{45, 1}, {47, -1}, {0, 0}, {0, 0}},
+  {{49, 1}, {51, -1}, {53, 1}, {0, 0}},
+  {{50, 1}, {52, -1}, {54, 1}, {0, 0}},
+};
+static __device__ const signed char m2l_unfold_m1_p5[35][3][2] = {
+  {{0, 1}, {0, 0}, {0, 0}},
+  {{1, 1}, {0, 0}, {0, 0}},
+  {{2, 1}, {0, 0}, {0, 0}},
+  {{3, 1}, {0, 0}, {0, 0}},
+  {{4, 1}, {0, 0}, {0, 0}},
+  {{5, 1}, {0, 0}, {0, 0}},
+  {{6, 1}, {0, 0}, {0, 0}},
+  {{7, 1}, {0, 0}, {0, 0}},
+  {{8, 1}, {0, 0}, {0, 0}},
+  {{7, -1}, {4, -1}, {0, 0}},
+  {{9, 1}, {0, 0}, {0, 0}},
+  {{10, 1}, {0, 0}, {0, 0}},
+  {{11, 1}, {0, 0}, {0, 0}},
+  {{12, 1}, {0, 0}, {0, 0}},
+  {{13, 1}, {0, 0}, {0, 0}},
+  {{12, -1}, {9, -1}, {0, 0}},
+  {{14, 1}, {0, 0}, {0, 0}},
+  {{15, 1}, {0, 0}, {0, 0}},
+  {{14, -1}, {10, -1}, {0, 0}},
+  {{15, -1}, {11, -1}, {0, 0}},
+  {{16, 1}, {0, 0}, {0, 0}},
+  {{17, 1}, {0, 0}, {0, 0}},
+  {{18, 1}, {0, 0}, {0, 0}},
+  {{19, 1}, {0, 0}, {0, 0}},
+  {{20, 1}, {0, 0}, {0, 0}},
+  {{19, -1}, {16, -1}, {0, 0}},
+  {{21, 1}, {0, 0}, {0, 0}},
+  {{22, 1}, {0, 0}, {0, 0}},
+  {{21, -1}, {17, -1}, {0, 0}},
+  {{22, -1}, {18, -1}, {0, 0}},
+  {{23, 1}, {0, 0}, {0, 0}},
+  {{24, 1}, {0, 0}, {0, 0}},
+  {{23, -1}, {19, -1}, {0, 0}},
+  {{24, -1}, {20, -1}, {0, 0}},
+  {{23, 1}, {19, 2}, {16, 1}},
+};
 
-// M2L, source order 1, expansion order 6: Msize 83, Lsize 56
+// M2L between reduced coefficients, source order 1, expansion order 6: 48 multipole, 36 local, 64 tensor entries, 483 terms
 template <typename T>
 __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ Mb, T* __restrict__ acc) {
   const T r2 = x * x + y * y + z * z;
@@ -1288,81 +960,61 @@ __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ M
   const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
   const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
   const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
-  const T D9 = -(T(3) * (T(2) * z * D3) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
+  const T D9 = -(D4 + D7);
   const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
   const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
   const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
   const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
   const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
-  const T D15 = -(T(5) * (x * D9 + T(2) * z * D6) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
+  const T D15 = -(D10 + D13);
   const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
   const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D18 = -(T(5) * (y * D9 + T(2) * z * D8) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D19 = -(T(5) * (T(3) * z * D9) + T(2) * (T(6) * D3)) * ir2 * cinv<T>(3);
-  const T D20 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D24 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
-  const T D25 = -(T(7) * (T(2) * x * D15 + T(2) * z * D12) + T(3) * (T(2) * D9 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D27 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
-  const T D28 = -(T(7) * (x * D18 + y * D15 + T(2) * z * D14) + T(3) * (T(2) * D5)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (x * D19 + T(3) * z * D15) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D30 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D31 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D32 = -(T(7) * (T(2) * y * D18 + T(2) * z * D17) + T(3) * (T(2) * D9 + T(2) * D7)) * ir2 * cinv<T>(4);
-  const T D33 = -(T(7) * (y * D19 + T(3) * z * D18) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D34 = -(T(7) * (T(4) * z * D19) + T(3) * (T(12) * D9)) * ir2 * cinv<T>(4);
-  const T D35 = -(T(9) * (T(5) * x * D20) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D36 = -(T(9) * (T(4) * x * D21 + y * D20) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D37 = -(T(9) * (T(4) * x * D22 + z * D20) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(3) * x * D23 + T(2) * y * D21) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D39 = -(T(9) * (T(3) * x * D24 + y * D22 + z * D21) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D40 = -(T(9) * (T(3) * x * D25 + T(2) * z * D22) + T(4) * (T(6) * D15 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (T(2) * x * D26 + T(3) * y * D23) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D42 = -(T(9) * (T(2) * x * D27 + T(2) * y * D24 + z * D23) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
-  const T D43 = -(T(9) * (T(2) * x * D28 + y * D25 + T(2) * z * D24) + T(4) * (T(2) * D18 + T(2) * D11)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(2) * x * D29 + T(3) * z * D25) + T(4) * (T(2) * D19 + T(6) * D12)) * ir2 * cinv<T>(5);
-  const T D45 = -(T(9) * (x * D30 + T(4) * y * D26) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D46 = -(T(9) * (x * D31 + T(3) * y * D27 + z * D26) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D47 = -(T(9) * (x * D32 + T(2) * y * D28 + T(2) * z * D27) + T(4) * (T(2) * D15 + T(2) * D13)) * ir2 * cinv<T>(5);
-  const T D48 = -(T(9) * (x * D33 + y * D29 + T(3) * z * D28) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D49 = -(T(9) * (x * D34 + T(4) * z * D29) + T(4) * (T(12) * D15)) * ir2 * cinv<T>(5);
-  const T D50 = -(T(9) * (T(5) * y * D30) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D51 = -(T(9) * (T(4) * y * D31 + z * D30) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
-  const T D52 = -(T(9) * (T(3) * y * D32 + T(2) * z * D31) + T(4) * (T(6) * D18 + T(2) * D16)) * ir2 * cinv<T>(5);
-  const T D53 = -(T(9) * (T(2) * y * D33 + T(3) * z * D32) + T(4) * (T(2) * D19 + T(6) * D17)) * ir2 * cinv<T>(5);
-  const T D54 = -(T(9) * (y * D34 + T(4) * z * D33) + T(4) * (T(12) * D18)) * ir2 * cinv<T>(5);
-  const T D55 = -(T(9) * (T(5) * z * D34) + T(4) * (T(20) * D19)) * ir2 * cinv<T>(5);
-  const T D56 = -(T(11) * (T(6) * x * D35) + T(5) * (T(30) * D20)) * ir2 * cinv<T>(6);
-  const T D57 = -(T(11) * (T(5) * x * D36 + y * D35) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
-  const T D58 = -(T(11) * (T(5) * x * D37 + z * D35) + T(5) * (T(20) * D22)) * ir2 * cinv<T>(6);
-  const T D59 = -(T(11) * (T(4) * x * D38 + T(2) * y * D36) + T(5) * (T(12) * D23 + T(2) * D20)) * ir2 * cinv<T>(6);
-  const T D60 = -(T(11) * (T(4) * x * D39 + y * D37 + z * D36) + T(5) * (T(12) * D24)) * ir2 * cinv<T>(6);
-  const T D61 = -(T(11) * (T(4) * x * D40 + T(2) * z * D37) + T(5) * (T(12) * D25 + T(2) * D20)) * ir2 * cinv<T>(6);
-  const T D62 = -(T(11) * (T(3) * x * D41 + T(3) * y * D38) + T(5) * (T(6) * D26 + T(6) * D21)) * ir2 * cinv<T>(6);
-  const T D63 = -(T(11) * (T(3) * x * D42 + T(2) * y * D39 + z * D38) + T(5) * (T(6) * D27 + T(2) * D22)) * ir2 * cinv<T>(6);
-  const T D64 = -(T(11) * (T(3) * x * D43 + y * D40 + T(2) * z * D39) + T(5) * (T(6) * D28 + T(2) * D21)) * ir2 * cinv<T>(6);
-  const T D65 = -(T(11) * (T(3) * x * D44 + T(3) * z * D40) + T(5) * (T(6) * D29 + T(6) * D22)) * ir2 * cinv<T>(6);
-  const T D66 = -(T(11) * (T(2) * x * D45 + T(4) * y * D41) + T(5) * (T(2) * D30 + T(12) * D23)) * ir2 * cinv<T>(6);
-  const T D67 = -(T(11) * (T(2) * x * D46 + T(3) * y * D42 + z * D41) + T(5) * (T(2) * D31 + T(6) * D24)) * ir2 * cinv<T>(6);
-  const T D68 = -(T(11) * (T(2) * x * D47 + T(2) * y * D43 + T(2) * z * D42) + T(5) * (T(2) * D32 + T(2) * D25 + T(2) * D23)) * ir2 * cinv<T>(6);
-  const T D69 = -(T(11) * (T(2) * x * D48 + y * D44 + T(3) * z * D43) + T(5) * (T(2) * D33 + T(6) * D24)) * ir2 * cinv<T>(6);
-  const T D70 = -(T(11) * (T(2) * x * D49 + T(4) * z * D44) + T(5) * (T(2) * D34 + T(12) * D25)) * ir2 * cinv<T>(6);
-  const T D71 = -(T(11) * (x * D50 + T(5) * y * D45) + T(5) * (T(20) * D26)) * ir2 * cinv<T>(6);
-  const T D72 = -(T(11) * (x * D51 + T(4) * y * D46 + z * D45) + T(5) * (T(12) * D27)) * ir2 * cinv<T>(6);
-  const T D73 = -(T(11) * (x * D52 + T(3) * y * D47 + T(2) * z * D46) + T(5) * (T(6) * D28 + T(2) * D26)) * ir2 * cinv<T>(6);
-  const T D74 = -(T(11) * (x * D53 + T(2) * y * D48 + T(3) * z * D47) + T(5) * (T(2) * D29 + T(6) * D27)) * ir2 * cinv<T>(6);
-  const T D75 = -(T(11) * (x * D54 + y * D49 + T(4) * z * D48) + T(5) * (T(12) * D28)) * ir2 * cinv<T>(6);
-  const T D76 = -(T(11) * (x * D55 + T(5) * z * D49) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
-  const T D77 = -(T(11) * (T(6) * y * D50) + T(5) * (T(30) * D30)) * ir2 * cinv<T>(6);
-  const T D78 = -(T(11) * (T(5) * y * D51 + z * D50) + T(5) * (T(20) * D31)) * ir2 * cinv<T>(6);
-  const T D79 = -(T(11) * (T(4) * y * D52 + T(2) * z * D51) + T(5) * (T(12) * D32 + T(2) * D30)) * ir2 * cinv<T>(6);
-  const T D80 = -(T(11) * (T(3) * y * D53 + T(3) * z * D52) + T(5) * (T(6) * D33 + T(6) * D31)) * ir2 * cinv<T>(6);
-  const T D81 = -(T(11) * (T(2) * y * D54 + T(4) * z * D53) + T(5) * (T(2) * D34 + T(12) * D32)) * ir2 * cinv<T>(6);
-  const T D82 = -(T(11) * (y * D55 + T(5) * z * D54) + T(5) * (T(20) * D33)) * ir2 * cinv<T>(6);
-  const T D83 = -(T(11) * (T(6) * z * D55) + T(5) * (T(30) * D34)) * ir2 * cinv<T>(6);
+  const T D18 = -(D11 + D16);
+  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
+  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
+  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
+  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T D24 = -(D19 + D22);
+  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T D27 = -(D20 + D25);
+  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
+  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T D30 = -(D22 + D28);
+  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
+  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
+  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
+  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
+  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D36 = -(D31 + D34);
+  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
+  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T D39 = -(D32 + D37);
+  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
+  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D42 = -(D34 + D40);
+  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
+  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T D45 = -(D37 + D43);
+  const T D46 = -(T(11) * (T(6) * x * D31) + T(5) * (T(30) * D19)) * ir2 * cinv<T>(6);
+  const T D47 = -(T(11) * (T(5) * x * D32 + y * D31) + T(5) * (T(20) * D20)) * ir2 * cinv<T>(6);
+  const T D48 = -(T(11) * (T(5) * x * D33 + z * D31) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
+  const T D49 = -(T(11) * (T(4) * x * D34 + T(2) * y * D32) + T(5) * (T(12) * D22 + T(2) * D19)) * ir2 * cinv<T>(6);
+  const T D50 = -(T(11) * (T(4) * x * D35 + y * D33 + z * D32) + T(5) * (T(12) * D23)) * ir2 * cinv<T>(6);
+  const T D51 = -(D46 + D49);
+  const T D52 = -(T(11) * (T(3) * x * D37 + T(3) * y * D34) + T(5) * (T(6) * D25 + T(6) * D20)) * ir2 * cinv<T>(6);
+  const T D53 = -(T(11) * (T(3) * x * D38 + T(2) * y * D35 + z * D34) + T(5) * (T(6) * D26 + T(2) * D21)) * ir2 * cinv<T>(6);
+  const T D54 = -(D47 + D52);
+  const T D55 = -(T(11) * (T(2) * x * D40 + T(4) * y * D37) + T(5) * (T(2) * D28 + T(12) * D22)) * ir2 * cinv<T>(6);
+  const T D56 = -(T(11) * (T(2) * x * D41 + T(3) * y * D38 + z * D37) + T(5) * (T(2) * D29 + T(6) * D23)) * ir2 * cinv<T>(6);
+  const T D57 = -(D49 + D55);
+  const T D58 = -(T(11) * (x * D43 + T(5) * y * D40) + T(5) * (T(20) * D25)) * ir2 * cinv<T>(6);
+  const T D59 = -(T(11) * (x * D44 + T(4) * y * D41 + z * D40) + T(5) * (T(12) * D26)) * ir2 * cinv<T>(6);
+  const T D60 = -(D52 + D58);
+  const T D61 = -(T(11) * (T(6) * y * D43) + T(5) * (T(30) * D28)) * ir2 * cinv<T>(6);
+  const T D62 = -(T(11) * (T(5) * y * D44 + z * D43) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
+  const T D63 = -(D55 + D61);
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
     acc[1] = fma(D4, mk, acc[1]);
@@ -1373,53 +1025,33 @@ __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D12, mk, acc[6]);
     acc[7] = fma(D13, mk, acc[7]);
     acc[8] = fma(D14, mk, acc[8]);
-    acc[9] = fma(D15, mk, acc[9]);
+    acc[9] = fma(D19, mk, acc[9]);
     acc[10] = fma(D20, mk, acc[10]);
     acc[11] = fma(D21, mk, acc[11]);
     acc[12] = fma(D22, mk, acc[12]);
     acc[13] = fma(D23, mk, acc[13]);
-    acc[14] = fma(D24, mk, acc[14]);
-    acc[15] = fma(D25, mk, acc[15]);
-    acc[16] = fma(D26, mk, acc[16]);
-    acc[17] = fma(D27, mk, acc[17]);
-    acc[18] = fma(D28, mk, acc[18]);
-    acc[19] = fma(D29, mk, acc[19]);
+    acc[14] = fma(D25, mk, acc[14]);
+    acc[15] = fma(D26, mk, acc[15]);
+    acc[16] = fma(D31, mk, acc[16]);
+    acc[17] = fma(D32, mk, acc[17]);
+    acc[18] = fma(D33, mk, acc[18]);
+    acc[19] = fma(D34, mk, acc[19]);
     acc[20] = fma(D35, mk, acc[20]);
-    acc[21] = fma(D36, mk, acc[21]);
-    acc[22] = fma(D37, mk, acc[22]);
-    acc[23] = fma(D38, mk, acc[23]);
-    acc[24] = fma(D39, mk, acc[24]);
-    acc[25] = fma(D40, mk, acc[25]);
-    acc[26] = fma(D41, mk, acc[26]);
-    acc[27] = fma(D42, mk, acc[27]);
-    acc[28] = fma(D43, mk, acc[28]);
-    acc[29] = fma(D44, mk, acc[29]);
-    acc[30] = fma(D45, mk, acc[30]);
-    acc[31] = fma(D46, mk, acc[31]);
-    acc[32] = fma(D47, mk, acc[32]);
-    acc[33] = fma(D48, mk, acc[33]);
-    acc[34] = fma(D49, mk, acc[34]);
-    acc[35] = fma(D56, mk, acc[35]);
-    acc[36] = fma(D57, mk, acc[36]);
-    acc[37] = fma(D58, mk, acc[37]);
-    acc[38] = fma(D59, mk, acc[38]);
-    acc[39] = fma(D60, mk, acc[39]);
-    acc[40] = fma(D61, mk, acc[40]);
-    acc[41] = fma(D62, mk, acc[41]);
-    acc[42] = fma(D63, mk, acc[42]);
-    acc[43] = fma(D64, mk, acc[43]);
-    acc[44] = fma(D65, mk, acc[44]);
-    acc[45] = fma(D66, mk, acc[45]);
-    acc[46] = fma(D67, mk, acc[46]);
-    acc[47] = fma(D68, mk, acc[47]);
-    acc[48] = fma(D69, mk, acc[48]);
-    acc[49] = fma(D70, mk, acc[49]);
-    acc[50] = fma(D71, mk, acc[50]);
-    acc[51] = fma(D72, mk, acc[51]);
-    acc[52] = fma(D73, mk, acc[52]);
-    acc[53] = fma(D74, mk, acc[53]);
-    acc[54] = fma(D75, mk, acc[54]);
-    acc[55] = fma(D76, mk, acc[55]);
+    acc[21] = fma(D37, mk, acc[21]);
+    acc[22] = fma(D38, mk, acc[22]);
+    acc[23] = fma(D40, mk, acc[23]);
+    acc[24] = fma(D41, mk, acc[24]);
+    acc[25] = fma(D46, mk, acc[25]);
+    acc[26] = fma(D47, mk, acc[26]);
+    acc[27] = fma(D48, mk, acc[27]);
+    acc[28] = fma(D49, mk, acc[28]);
+    acc[29] = fma(D50, mk, acc[29]);
+    acc[30] = fma(D52, mk, acc[30]);
+    acc[31] = fma(D53, mk, acc[31]);
+    acc[32] = fma(D55, mk, acc[32]);
+    acc[33] = fma(D56, mk, acc[33]);
+    acc[34] = fma(D58, mk, acc[34]);
+    acc[35] = fma(D59, mk, acc[35]);
   }
   { const T mk = Mb[1];
     acc[0] = fma(D2, mk, acc[0]);
@@ -1431,53 +1063,33 @@ __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D14, mk, acc[6]);
     acc[7] = fma(D16, mk, acc[7]);
     acc[8] = fma(D17, mk, acc[8]);
-    acc[9] = fma(D18, mk, acc[9]);
-    acc[10] = fma(D21, mk, acc[10]);
+    acc[9] = fma(D20, mk, acc[9]);
+    acc[10] = fma(D22, mk, acc[10]);
     acc[11] = fma(D23, mk, acc[11]);
-    acc[12] = fma(D24, mk, acc[12]);
+    acc[12] = fma(D25, mk, acc[12]);
     acc[13] = fma(D26, mk, acc[13]);
-    acc[14] = fma(D27, mk, acc[14]);
-    acc[15] = fma(D28, mk, acc[15]);
-    acc[16] = fma(D30, mk, acc[16]);
-    acc[17] = fma(D31, mk, acc[17]);
-    acc[18] = fma(D32, mk, acc[18]);
-    acc[19] = fma(D33, mk, acc[19]);
-    acc[20] = fma(D36, mk, acc[20]);
-    acc[21] = fma(D38, mk, acc[21]);
-    acc[22] = fma(D39, mk, acc[22]);
-    acc[23] = fma(D41, mk, acc[23]);
-    acc[24] = fma(D42, mk, acc[24]);
-    acc[25] = fma(D43, mk, acc[25]);
-    acc[26] = fma(D45, mk, acc[26]);
-    acc[27] = fma(D46, mk, acc[27]);
-    acc[28] = fma(D47, mk, acc[28]);
-    acc[29] = fma(D48, mk, acc[29]);
-    acc[30] = fma(D50, mk, acc[30]);
-    acc[31] = fma(D51, mk, acc[31]);
-    acc[32] = fma(D52, mk, acc[32]);
-    acc[33] = fma(D53, mk, acc[33]);
-    acc[34] = fma(D54, mk, acc[34]);
-    acc[35] = fma(D57, mk, acc[35]);
-    acc[36] = fma(D59, mk, acc[36]);
-    acc[37] = fma(D60, mk, acc[37]);
-    acc[38] = fma(D62, mk, acc[38]);
-    acc[39] = fma(D63, mk, acc[39]);
-    acc[40] = fma(D64, mk, acc[40]);
-    acc[41] = fma(D66, mk, acc[41]);
-    acc[42] = fma(D67, mk, acc[42]);
-    acc[43] = fma(D68, mk, acc[43]);
-    acc[44] = fma(D69, mk, acc[44]);
-    acc[45] = fma(D71, mk, acc[45]);
-    acc[46] = fma(D72, mk, acc[46]);
-    acc[47] = fma(D73, mk, acc[47]);
-    acc[48] = fma(D74, mk, acc[48]);
-    acc[49] = fma(D75, mk, acc[49]);
-    acc[50] = fma(D77, mk, acc[50]);
-    acc[51] = fma(D78, mk, acc[51]);
-    acc[52] = fma(D79, mk, acc[52]);
-    acc[53] = fma(D80, mk, acc[53]);
-    acc[54] = fma(D81, mk, acc[54]);
-    acc[55] = fma(D82, mk, acc[55]);
+    acc[14] = fma(D28, mk, acc[14]);
+    acc[15] = fma(D29, mk, acc[15]);
+    acc[16] = fma(D32, mk, acc[16]);
+    acc[17] = fma(D34, mk, acc[17]);
+    acc[18] = fma(D35, mk, acc[18]);
+    acc[19] = fma(D37, mk, acc[19]);
+    acc[20] = fma(D38, mk, acc[20]);
+    acc[21] = fma(D40, mk, acc[21]);
+    acc[22] = fma(D41, mk, acc[22]);
+    acc[23] = fma(D43, mk, acc[23]);
+    acc[24] = fma(D44, mk, acc[24]);
+    acc[25] = fma(D47, mk, acc[25]);
+    acc[26] = fma(D49, mk, acc[26]);
+    acc[27] = fma(D50, mk, acc[27]);
+    acc[28] = fma(D52, mk, acc[28]);
+    acc[29] = fma(D53, mk, acc[29]);
+    acc[30] = fma(D55, mk, acc[30]);
+    acc[31] = fma(D56, mk, acc[31]);
+    acc[32] = fma(D58, mk, acc[32]);
+    acc[33] = fma(D59, mk, acc[33]);
+    acc[34] = fma(D61, mk, acc[34]);
+    acc[35] = fma(D62, mk, acc[35]);
   }
   { const T mk = Mb[2];
     acc[0] = fma(D3, mk, acc[0]);
@@ -1489,888 +1101,500 @@ __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ M
     acc[6] = fma(D15, mk, acc[6]);
     acc[7] = fma(D17, mk, acc[7]);
     acc[8] = fma(D18, mk, acc[8]);
-    acc[9] = fma(D19, mk, acc[9]);
-    acc[10] = fma(D22, mk, acc[10]);
+    acc[9] = fma(D21, mk, acc[9]);
+    acc[10] = fma(D23, mk, acc[10]);
     acc[11] = fma(D24, mk, acc[11]);
-    acc[12] = fma(D25, mk, acc[12]);
+    acc[12] = fma(D26, mk, acc[12]);
     acc[13] = fma(D27, mk, acc[13]);
-    acc[14] = fma(D28, mk, acc[14]);
-    acc[15] = fma(D29, mk, acc[15]);
-    acc[16] = fma(D31, mk, acc[16]);
-    acc[17] = fma(D32, mk, acc[17]);
-    acc[18] = fma(D33, mk, acc[18]);
-    acc[19] = fma(D34, mk, acc[19]);
-    acc[20] = fma(D37, mk, acc[20]);
-    acc[21] = fma(D39, mk, acc[21]);
-    acc[22] = fma(D40, mk, acc[22]);
-    acc[23] = fma(D42, mk, acc[23]);
-    acc[24] = fma(D43, mk, acc[24]);
-    acc[25] = fma(D44, mk, acc[25]);
-    acc[26] = fma(D46, mk, acc[26]);
-    acc[27] = fma(D47, mk, acc[27]);
-    acc[28] = fma(D48, mk, acc[28]);
-    acc[29] = fma(D49, mk, acc[29]);
-    acc[30] = fma(D51, mk, acc[30]);
-    acc[31] = fma(D52, mk, acc[31]);
-    acc[32] = fma(D53, mk, acc[32]);
-    acc[33] = fma(D54, mk, acc[33]);
-    acc[34] = fma(D55, mk, acc[34]);
-    acc[35] = fma(D58, mk, acc[35]);
-    acc[36] = fma(D60, mk, acc[36]);
-    acc[37] = fma(D61, mk, acc[37]);
-    acc[38] = fma(D63, mk, acc[38]);
-    acc[39] = fma(D64, mk, acc[39]);
-    acc[40] = fma(D65, mk, acc[40]);
-    acc[41] = fma(D67, mk, acc[41]);
-    acc[42] = fma(D68, mk, acc[42]);
-    acc[43] = fma(D69, mk, acc[43]);
-    acc[44] = fma(D70, mk, acc[44]);
-    acc[45] = fma(D72, mk, acc[45]);
-    acc[46] = fma(D73, mk, acc[46]);
-    acc[47] = fma(D74, mk, acc[47]);
-    acc[48] = fma(D75, mk, acc[48]);
-    acc[49] = fma(D76, mk, acc[49]);
-    acc[50] = fma(D78, mk, acc[50]);
-    acc[51] = fma(D79, mk, acc[51]);
-    acc[52] = fma(D80, mk, acc[52]);
-    acc[53] = fma(D81, mk, acc[53]);
-    acc[54] = fma(D82, mk, acc[54]);
-    acc[55] = fma(D83, mk, acc[55]);
+    acc[14] = fma(D29, mk, acc[14]);
+    acc[15] = fma(D30, mk, acc[15]);
+    acc[16] = fma(D33, mk, acc[16]);
+    acc[17] = fma(D35, mk, acc[17]);
+    acc[18] = fma(D36, mk, acc[18]);
+    acc[19] = fma(D38, mk, acc[19]);
+    acc[20] = fma(D39, mk, acc[20]);
+    acc[21] = fma(D41, mk, acc[21]);
+    acc[22] = fma(D42, mk, acc[22]);
+    acc[23] = fma(D44, mk, acc[23]);
+    acc[24] = fma(D45, mk, acc[24]);
+    acc[25] = fma(D48, mk, acc[25]);
+    acc[26] = fma(D50, mk, acc[26]);
+    acc[27] = fma(D51, mk, acc[27]);
+    acc[28] = fma(D53, mk, acc[28]);
+    acc[29] = fma(D54, mk, acc[29]);
+    acc[30] = fma(D56, mk, acc[30]);
+    acc[31] = fma(D57, mk, acc[31]);
+    acc[32] = fma(D59, mk, acc[32]);
+    acc[33] = fma(D60, mk, acc[33]);
+    acc[34] = fma(D62, mk, acc[34]);
+    acc[35] = fma(D63, mk, acc[35]);
   }
   { const T mk = Mb[3];
     acc[0] = fma(D4, mk, acc[0]);
     acc[1] = fma(D10, mk, acc[1]);
     acc[2] = fma(D11, mk, acc[2]);
     acc[3] = fma(D12, mk, acc[3]);
-    acc[4] = fma(D20, mk, acc[4]);
-    acc[5] = fma(D21, mk, acc[5]);
-    acc[6] = fma(D22, mk, acc[6]);
-    acc[7] = fma(D23, mk, acc[7]);
-    acc[8] = fma(D24, mk, acc[8]);
-    acc[9] = fma(D25, mk, acc[9]);
-    acc[10] = fma(D35, mk, acc[10]);
-    acc[11] = fma(D36, mk, acc[11]);
-    acc[12] = fma(D37, mk, acc[12]);
-    acc[13] = fma(D38, mk, acc[13]);
-    acc[14] = fma(D39, mk, acc[14]);
-    acc[15] = fma(D40, mk, acc[15]);
-    acc[16] = fma(D41, mk, acc[16]);
-    acc[17] = fma(D42, mk, acc[17]);
-    acc[18] = fma(D43, mk, acc[18]);
-    acc[19] = fma(D44, mk, acc[19]);
-    acc[20] = fma(D56, mk, acc[20]);
-    acc[21] = fma(D57, mk, acc[21]);
-    acc[22] = fma(D58, mk, acc[22]);
-    acc[23] = fma(D59, mk, acc[23]);
-    acc[24] = fma(D60, mk, acc[24]);
-    acc[25] = fma(D61, mk, acc[25]);
-    acc[26] = fma(D62, mk, acc[26]);
-    acc[27] = fma(D63, mk, acc[27]);
-    acc[28] = fma(D64, mk, acc[28]);
-    acc[29] = fma(D65, mk, acc[29]);
-    acc[30] = fma(D66, mk, acc[30]);
-    acc[31] = fma(D67, mk, acc[31]);
-    acc[32] = fma(D68, mk, acc[32]);
-    acc[33] = fma(D69, mk, acc[33]);
-    acc[34] = fma(D70, mk, acc[34]);
+    acc[4] = fma(D19, mk, acc[4]);
+    acc[5] = fma(D20, mk, acc[5]);
+    acc[6] = fma(D21, mk, acc[6]);
+    acc[7] = fma(D22, mk, acc[7]);
+    acc[8] = fma(D23, mk, acc[8]);
+    acc[9] = fma(D31, mk, acc[9]);
+    acc[10] = fma(D32, mk, acc[10]);
+    acc[11] = fma(D33, mk, acc[11]);
+    acc[12] = fma(D34, mk, acc[12]);
+    acc[13] = fma(D35, mk, acc[13]);
+    acc[14] = fma(D37, mk, acc[14]);
+    acc[15] = fma(D38, mk, acc[15]);
+    acc[16] = fma(D46, mk, acc[16]);
+    acc[17] = fma(D47, mk, acc[17]);
+    acc[18] = fma(D48, mk, acc[18]);
+    acc[19] = fma(D49, mk, acc[19]);
+    acc[20] = fma(D50, mk, acc[20]);
+    acc[21] = fma(D52, mk, acc[21]);
+    acc[22] = fma(D53, mk, acc[22]);
+    acc[23] = fma(D55, mk, acc[23]);
+    acc[24] = fma(D56, mk, acc[24]);
   }
   { const T mk = Mb[4];
     acc[0] = fma(D5, mk, acc[0]);
     acc[1] = fma(D11, mk, acc[1]);
     acc[2] = fma(D13, mk, acc[2]);
     acc[3] = fma(D14, mk, acc[3]);
-    acc[4] = fma(D21, mk, acc[4]);
-    acc[5] = fma(D23, mk, acc[5]);
-    acc[6] = fma(D24, mk, acc[6]);
-    acc[7] = fma(D26, mk, acc[7]);
-    acc[8] = fma(D27, mk, acc[8]);
-    acc[9] = fma(D28, mk, acc[9]);
-    acc[10] = fma(D36, mk, acc[10]);
-    acc[11] = fma(D38, mk, acc[11]);
-    acc[12] = fma(D39, mk, acc[12]);
-    acc[13] = fma(D41, mk, acc[13]);
-    acc[14] = fma(D42, mk, acc[14]);
-    acc[15] = fma(D43, mk, acc[15]);
-    acc[16] = fma(D45, mk, acc[16]);
-    acc[17] = fma(D46, mk, acc[17]);
-    acc[18] = fma(D47, mk, acc[18]);
-    acc[19] = fma(D48, mk, acc[19]);
-    acc[20] = fma(D57, mk, acc[20]);
-    acc[21] = fma(D59, mk, acc[21]);
-    acc[22] = fma(D60, mk, acc[22]);
-    acc[23] = fma(D62, mk, acc[23]);
-    acc[24] = fma(D63, mk, acc[24]);
-    acc[25] = fma(D64, mk, acc[25]);
-    acc[26] = fma(D66, mk, acc[26]);
-    acc[27] = fma(D67, mk, acc[27]);
-    acc[28] = fma(D68, mk, acc[28]);
-    acc[29] = fma(D69, mk, acc[29]);
-    acc[30] = fma(D71, mk, acc[30]);
-    acc[31] = fma(D72, mk, acc[31]);
-    acc[32] = fma(D73, mk, acc[32]);
-    acc[33] = fma(D74, mk, acc[33]);
-    acc[34] = fma(D75, mk, acc[34]);
+    acc[4] = fma(D20, mk, acc[4]);
+    acc[5] = fma(D22, mk, acc[5]);
+    acc[6] = fma(D23, mk, acc[6]);
+    acc[7] = fma(D25, mk, acc[7]);
+    acc[8] = fma(D26, mk, acc[8]);
+    acc[9] = fma(D32, mk, acc[9]);
+    acc[10] = fma(D34, mk, acc[10]);
+    acc[11] = fma(D35, mk, acc[11]);
+    acc[12] = fma(D37, mk, acc[12]);
+    acc[13] = fma(D38, mk, acc[13]);
+    acc[14] = fma(D40, mk, acc[14]);
+    acc[15] = fma(D41, mk, acc[15]);
+    acc[16] = fma(D47, mk, acc[16]);
+    acc[17] = fma(D49, mk, acc[17]);
+    acc[18] = fma(D50, mk, acc[18]);
+    acc[19] = fma(D52, mk, acc[19]);
+    acc[20] = fma(D53, mk, acc[20]);
+    acc[21] = fma(D55, mk, acc[21]);
+    acc[22] = fma(D56, mk, acc[22]);
+    acc[23] = fma(D58, mk, acc[23]);
+    acc[24] = fma(D59, mk, acc[24]);
   }
   { const T mk = Mb[5];
     acc[0] = fma(D6, mk, acc[0]);
     acc[1] = fma(D12, mk, acc[1]);
     acc[2] = fma(D14, mk, acc[2]);
     acc[3] = fma(D15, mk, acc[3]);
-    acc[4] = fma(D22, mk, acc[4]);
-    acc[5] = fma(D24, mk, acc[5]);
-    acc[6] = fma(D25, mk, acc[6]);
-    acc[7] = fma(D27, mk, acc[7]);
-    acc[8] = fma(D28, mk, acc[8]);
-    acc[9] = fma(D29, mk, acc[9]);
-    acc[10] = fma(D37, mk, acc[10]);
-    acc[11] = fma(D39, mk, acc[11]);
-    acc[12] = fma(D40, mk, acc[12]);
-    acc[13] = fma(D42, mk, acc[13]);
-    acc[14] = fma(D43, mk, acc[14]);
-    acc[15] = fma(D44, mk, acc[15]);
-    acc[16] = fma(D46, mk, acc[16]);
-    acc[17] = fma(D47, mk, acc[17]);
-    acc[18] = fma(D48, mk, acc[18]);
-    acc[19] = fma(D49, mk, acc[19]);
-    acc[20] = fma(D58, mk, acc[20]);
-    acc[21] = fma(D60, mk, acc[21]);
-    acc[22] = fma(D61, mk, acc[22]);
-    acc[23] = fma(D63, mk, acc[23]);
-    acc[24] = fma(D64, mk, acc[24]);
-    acc[25] = fma(D65, mk, acc[25]);
-    acc[26] = fma(D67, mk, acc[26]);
-    acc[27] = fma(D68, mk, acc[27]);
-    acc[28] = fma(D69, mk, acc[28]);
-    acc[29] = fma(D70, mk, acc[29]);
-    acc[30] = fma(D72, mk, acc[30]);
-    acc[31] = fma(D73, mk, acc[31]);
-    acc[32] = fma(D74, mk, acc[32]);
-    acc[33] = fma(D75, mk, acc[33]);
-    acc[34] = fma(D76, mk, acc[34]);
+    acc[4] = fma(D21, mk, acc[4]);
+    acc[5] = fma(D23, mk, acc[5]);
+    acc[6] = fma(D24, mk, acc[6]);
+    acc[7] = fma(D26, mk, acc[7]);
+    acc[8] = fma(D27, mk, acc[8]);
+    acc[9] = fma(D33, mk, acc[9]);
+    acc[10] = fma(D35, mk, acc[10]);
+    acc[11] = fma(D36, mk, acc[11]);
+    acc[12] = fma(D38, mk, acc[12]);
+    acc[13] = fma(D39, mk, acc[13]);
+    acc[14] = fma(D41, mk, acc[14]);
+    acc[15] = fma(D42, mk, acc[15]);
+    acc[16] = fma(D48, mk, acc[16]);
+    acc[17] = fma(D50, mk, acc[17]);
+    acc[18] = fma(D51, mk, acc[18]);
+    acc[19] = fma(D53, mk, acc[19]);
+    acc[20] = fma(D54, mk, acc[20]);
+    acc[21] = fma(D56, mk, acc[21]);
+    acc[22] = fma(D57, mk, acc[22]);
+    acc[23] = fma(D59, mk, acc[23]);
+    acc[24] = fma(D60, mk, acc[24]);
   }
   { const T mk = Mb[6];
     acc[0] = fma(D7, mk, acc[0]);
     acc[1] = fma(D13, mk, acc[1]);
     acc[2] = fma(D16, mk, acc[2]);
     acc[3] = fma(D17, mk, acc[3]);
-    acc[4] = fma(D23, mk, acc[4]);
-    acc[5] = fma(D26, mk, acc[5]);
-    acc[6] = fma(D27, mk, acc[6]);
-    acc[7] = fma(D30, mk, acc[7]);
-    acc[8] = fma(D31, mk, acc[8]);
-    acc[9] = fma(D32, mk, acc[9]);
-    acc[10] = fma(D38, mk, acc[10]);
-    acc[11] = fma(D41, mk, acc[11]);
-    acc[12] = fma(D42, mk, acc[12]);
-    acc[13] = fma(D45, mk, acc[13]);
-    acc[14] = fma(D46, mk, acc[14]);
-    acc[15] = fma(D47, mk, acc[15]);
-    acc[16] = fma(D50, mk, acc[16]);
-    acc[17] = fma(D51, mk, acc[17]);
-    acc[18] = fma(D52, mk, acc[18]);
-    acc[19] = fma(D53, mk, acc[19]);
-    acc[20] = fma(D59, mk, acc[20]);
-    acc[21] = fma(D62, mk, acc[21]);
-    acc[22] = fma(D63, mk, acc[22]);
-    acc[23] = fma(D66, mk, acc[23]);
-    acc[24] = fma(D67, mk, acc[24]);
-    acc[25] = fma(D68, mk, acc[25]);
-    acc[26] = fma(D71, mk, acc[26]);
-    acc[27] = fma(D72, mk, acc[27]);
-    acc[28] = fma(D73, mk, acc[28]);
-    acc[29] = fma(D74, mk, acc[29]);
-    acc[30] = fma(D77, mk, acc[30]);
-    acc[31] = fma(D78, mk, acc[31]);
-    acc[32] = fma(D79, mk, acc[32]);
-    acc[33] = fma(D80, mk, acc[33]);
-    acc[34] = fma(D81, mk, acc[34]);
+    acc[4] = fma(D22, mk, acc[4]);
+    acc[5] = fma(D25, mk, acc[5]);
+    acc[6] = fma(D26, mk, acc[6]);
+    acc[7] = fma(D28, mk, acc[7]);
+    acc[8] = fma(D29, mk, acc[8]);
+    acc[9] = fma(D34, mk, acc[9]);
+    acc[10] = fma(D37, mk, acc[10]);
+    acc[11] = fma(D38, mk, acc[11]);
+    acc[12] = fma(D40, mk, acc[12]);
+    acc[13] = fma(D41, mk, acc[13]);
+    acc[14] = fma(D43, mk, acc[14]);
+    acc[15] = fma(D44, mk, acc[15]);
+    acc[16] = fma(D49, mk, acc[16]);
+    acc[17] = fma(D52, mk, acc[17]);
+    acc[18] = fma(D53, mk, acc[18]);
+    acc[19] = fma(D55, mk, acc[19]);
+    acc[20] = fma(D56, mk, acc[20]);
+    acc[21] = fma(D58, mk, acc[21]);
+    acc[22] = fma(D59, mk, acc[22]);
+    acc[23] = fma(D61, mk, acc[23]);
+    acc[24] = fma(D62, mk, acc[24]);
   }
   { const T mk = Mb[7];
     acc[0] = fma(D8, mk, acc[0]);
     acc[1] = fma(D14, mk, acc[1]);
     acc[2] = fma(D17, mk, acc[2]);
     acc[3] = fma(D18, mk, acc[3]);
-    acc[4] = fma(D24, mk, acc[4]);
-    acc[5] = fma(D27, mk, acc[5]);
-    acc[6] = fma(D28, mk, acc[6]);
-    acc[7] = fma(D31, mk, acc[7]);
-    acc[8] = fma(D32, mk, acc[8]);
-    acc[9] = fma(D33, mk, acc[9]);
-    acc[10] = fma(D39, mk, acc[10]);
-    acc[11] = fma(D42, mk, acc[11]);
-    acc[12] = fma(D43, mk, acc[12]);
-    acc[13] = fma(D46, mk, acc[13]);
-    acc[14] = fma(D47, mk, acc[14]);
-    acc[15] = fma(D48, mk, acc[15]);
-    acc[16] = fma(D51, mk, acc[16]);
-    acc[17] = fma(D52, mk, acc[17]);
-    acc[18] = fma(D53, mk, acc[18]);
-    acc[19] = fma(D54, mk, acc[19]);
-    acc[20] = fma(D60, mk, acc[20]);
-    acc[21] = fma(D63, mk, acc[21]);
-    acc[22] = fma(D64, mk, acc[22]);
-    acc[23] = fma(D67, mk, acc[23]);
-    acc[24] = fma(D68, mk, acc[24]);
-    acc[25] = fma(D69, mk, acc[25]);
-    acc[26] = fma(D72, mk, acc[26]);
-    acc[27] = fma(D73, mk, acc[27]);
-    acc[28] = fma(D74, mk, acc[28]);
-    acc[29] = fma(D75, mk, acc[29]);
-    acc[30] = fma(D78, mk, acc[30]);
-    acc[31] = fma(D79, mk, acc[31]);
-    acc[32] = fma(D80, mk, acc[32]);
-    acc[33] = fma(D81, mk, acc[33]);
-    acc[34] = fma(D82, mk, acc[34]);
-  }
-  { const T mk = Mb[8];
-    acc[0] = fma(D9, mk, acc[0]);
-    acc[1] = fma(D15, mk, acc[1]);
-    acc[2] = fma(D18, mk, acc[2]);
-    acc[3] = fma(D19, mk, acc[3]);
-    acc[4] = fma(D25, mk, acc[4]);
-    acc[5] = fma(D28, mk, acc[5]);
-    acc[6] = fma(D29, mk, acc[6]);
-    acc[7] = fma(D32, mk, acc[7]);
-    acc[8] = fma(D33, mk, acc[8]);
-    acc[9] = fma(D34, mk, acc[9]);
-    acc[10] = fma(D40, mk, acc[10]);
-    acc[11] = fma(D43, mk, acc[11]);
-    acc[12] = fma(D44, mk, acc[12]);
-    acc[13] = fma(D47, mk, acc[13]);
-    acc[14] = fma(D48, mk, acc[14]);
-    acc[15] = fma(D49, mk, acc[15]);
-    acc[16] = fma(D52, mk, acc[16]);
+    acc[4] = fma(D23, mk, acc[4]);
+    acc[5] = fma(D26, mk, acc[5]);
+    acc[6] = fma(D27, mk, acc[6]);
+    acc[7] = fma(D29, mk, acc[7]);
+    acc[8] = fma(D30, mk, acc[8]);
+    acc[9] = fma(D35, mk, acc[9]);
+    acc[10] = fma(D38, mk, acc[10]);
+    acc[11] = fma(D39, mk, acc[11]);
+    acc[12] = fma(D41, mk, acc[12]);
+    acc[13] = fma(D42, mk, acc[13]);
+    acc[14] = fma(D44, mk, acc[14]);
+    acc[15] = fma(D45, mk, acc[15]);
+    acc[16] = fma(D50, mk, acc[16]);
     acc[17] = fma(D53, mk, acc[17]);
     acc[18] = fma(D54, mk, acc[18]);
-    acc[19] = fma(D55, mk, acc[19]);
-    acc[20] = fma(D61, mk, acc[20]);
-    acc[21] = fma(D64, mk, acc[21]);
-    acc[22] = fma(D65, mk, acc[22]);
-    acc[23] = fma(D68, mk, acc[23]);
-    acc[24] = fma(D69, mk, acc[24]);
-    acc[25] = fma(D70, mk, acc[25]);
-    acc[26] = fma(D73, mk, acc[26]);
-    acc[27] = fma(D74, mk, acc[27]);
-    acc[28] = fma(D75, mk, acc[28]);
-    acc[29] = fma(D76, mk, acc[29]);
-    acc[30] = fma(D79, mk, acc[30]);
-    acc[31] = fma(D80, mk, acc[31]);
-    acc[32] = fma(D81, mk, acc[32]);
-    acc[33] = fma(D82, mk, acc[33]);
-    acc[34] = fma(D83, mk, acc[34]);
+    acc[19] = fma(D56, mk, acc[19]);
+    acc[20] = fma(D57, mk, acc[20]);
+    acc[21] = fma(D59, mk, acc[21]);
+    acc[22] = fma(D60, mk, acc[22]);
+    acc[23] = fma(D62, mk, acc[23]);
+    acc[24] = fma(D63, mk, acc[24]);
+  }
+  { const T mk = Mb[8];
+    acc[0] = fma(D10, mk, acc[0]);
+    acc[1] = fma(D19, mk, acc[1]);
+    acc[2] = fma(D20, mk, acc[2]);
+    acc[3] = fma(D21, mk, acc[3]);
+    acc[4] = fma(D31, mk, acc[4]);
+    acc[5] = fma(D32, mk, acc[5]);
+    acc[6] = fma(D33, mk, acc[6]);
+    acc[7] = fma(D34, mk, acc[7]);
+    acc[8] = fma(D35, mk, acc[8]);
+    acc[9] = fma(D46, mk, acc[9]);
+    acc[10] = fma(D47, mk, acc[10]);
+    acc[11] = fma(D48, mk, acc[11]);
+    acc[12] = fma(D49, mk, acc[12]);
+    acc[13] = fma(D50, mk, acc[13]);
+    acc[14] = fma(D52, mk, acc[14]);
+    acc[15] = fma(D53, mk, acc[15]);
   }
   { const T mk = Mb[9];
-    acc[0] = fma(D10, mk, acc[0]);
+    acc[0] = fma(D11, mk, acc[0]);
     acc[1] = fma(D20, mk, acc[1]);
-    acc[2] = fma(D21, mk, acc[2]);
-    acc[3] = fma(D22, mk, acc[3]);
-    acc[4] = fma(D35, mk, acc[4]);
-    acc[5] = fma(D36, mk, acc[5]);
-    acc[6] = fma(D37, mk, acc[6]);
-    acc[7] = fma(D38, mk, acc[7]);
-    acc[8] = fma(D39, mk, acc[8]);
-    acc[9] = fma(D40, mk, acc[9]);
-    acc[10] = fma(D56, mk, acc[10]);
-    acc[11] = fma(D57, mk, acc[11]);
-    acc[12] = fma(D58, mk, acc[12]);
-    acc[13] = fma(D59, mk, acc[13]);
-    acc[14] = fma(D60, mk, acc[14]);
-    acc[15] = fma(D61, mk, acc[15]);
-    acc[16] = fma(D62, mk, acc[16]);
-    acc[17] = fma(D63, mk, acc[17]);
-    acc[18] = fma(D64, mk, acc[18]);
-    acc[19] = fma(D65, mk, acc[19]);
+    acc[2] = fma(D22, mk, acc[2]);
+    acc[3] = fma(D23, mk, acc[3]);
+    acc[4] = fma(D32, mk, acc[4]);
+    acc[5] = fma(D34, mk, acc[5]);
+    acc[6] = fma(D35, mk, acc[6]);
+    acc[7] = fma(D37, mk, acc[7]);
+    acc[8] = fma(D38, mk, acc[8]);
+    acc[9] = fma(D47, mk, acc[9]);
+    acc[10] = fma(D49, mk, acc[10]);
+    acc[11] = fma(D50, mk, acc[11]);
+    acc[12] = fma(D52, mk, acc[12]);
+    acc[13] = fma(D53, mk, acc[13]);
+    acc[14] = fma(D55, mk, acc[14]);
+    acc[15] = fma(D56, mk, acc[15]);
   }
   { const T mk = Mb[10];
-    acc[0] = fma(D11, mk, acc[0]);
+    acc[0] = fma(D12, mk, acc[0]);
     acc[1] = fma(D21, mk, acc[1]);
     acc[2] = fma(D23, mk, acc[2]);
     acc[3] = fma(D24, mk, acc[3]);
-    acc[4] = fma(D36, mk, acc[4]);
+    acc[4] = fma(D33, mk, acc[4]);
+    acc[5] = fma(D35, mk, acc[5]);
+    acc[6] = fma(D36, mk, acc[6]);
+    acc[7] = fma(D38, mk, acc[7]);
+    acc[8] = fma(D39, mk, acc[8]);
+    acc[9] = fma(D48, mk, acc[9]);
+    acc[10] = fma(D50, mk, acc[10]);
+    acc[11] = fma(D51, mk, acc[11]);
+    acc[12] = fma(D53, mk, acc[12]);
+    acc[13] = fma(D54, mk, acc[13]);
+    acc[14] = fma(D56, mk, acc[14]);
+    acc[15] = fma(D57, mk, acc[15]);
+  }
+  { const T mk = Mb[11];
+    acc[0] = fma(D13, mk, acc[0]);
+    acc[1] = fma(D22, mk, acc[1]);
+    acc[2] = fma(D25, mk, acc[2]);
+    acc[3] = fma(D26, mk, acc[3]);
+    acc[4] = fma(D34, mk, acc[4]);
+    acc[5] = fma(D37, mk, acc[5]);
+    acc[6] = fma(D38, mk, acc[6]);
+    acc[7] = fma(D40, mk, acc[7]);
+    acc[8] = fma(D41, mk, acc[8]);
+    acc[9] = fma(D49, mk, acc[9]);
+    acc[10] = fma(D52, mk, acc[10]);
+    acc[11] = fma(D53, mk, acc[11]);
+    acc[12] = fma(D55, mk, acc[12]);
+    acc[13] = fma(D56, mk, acc[13]);
+    acc[14] = fma(D58, mk, acc[14]);
+    acc[15] = fma(D59, mk, acc[15]);
+  }
+  { const T mk = Mb[12];
+    acc[0] = fma(D14, mk, acc[0]);
+    acc[1] = fma(D23, mk, acc[1]);
+    acc[2] = fma(D26, mk, acc[2]);
+    acc[3] = fma(D27, mk, acc[3]);
+    acc[4] = fma(D35, mk, acc[4]);
     acc[5] = fma(D38, mk, acc[5]);
     acc[6] = fma(D39, mk, acc[6]);
     acc[7] = fma(D41, mk, acc[7]);
     acc[8] = fma(D42, mk, acc[8]);
-    acc[9] = fma(D43, mk, acc[9]);
-    acc[10] = fma(D57, mk, acc[10]);
-    acc[11] = fma(D59, mk, acc[11]);
-    acc[12] = fma(D60, mk, acc[12]);
-    acc[13] = fma(D62, mk, acc[13]);
-    acc[14] = fma(D63, mk, acc[14]);
-    acc[15] = fma(D64, mk, acc[15]);
-    acc[16] = fma(D66, mk, acc[16]);
-    acc[17] = fma(D67, mk, acc[17]);
-    acc[18] = fma(D68, mk, acc[18]);
-    acc[19] = fma(D69, mk, acc[19]);
-  }
-  { const T mk = Mb[11];
-    acc[0] = fma(D12, mk, acc[0]);
-    acc[1] = fma(D22, mk, acc[1]);
-    acc[2] = fma(D24, mk, acc[2]);
-    acc[3] = fma(D25, mk, acc[3]);
-    acc[4] = fma(D37, mk, acc[4]);
-    acc[5] = fma(D39, mk, acc[5]);
-    acc[6] = fma(D40, mk, acc[6]);
-    acc[7] = fma(D42, mk, acc[7]);
-    acc[8] = fma(D43, mk, acc[8]);
-    acc[9] = fma(D44, mk, acc[9]);
-    acc[10] = fma(D58, mk, acc[10]);
-    acc[11] = fma(D60, mk, acc[11]);
-    acc[12] = fma(D61, mk, acc[12]);
-    acc[13] = fma(D63, mk, acc[13]);
-    acc[14] = fma(D64, mk, acc[14]);
-    acc[15] = fma(D65, mk, acc[15]);
-    acc[16] = fma(D67, mk, acc[16]);
-    acc[17] = fma(D68, mk, acc[17]);
-    acc[18] = fma(D69, mk, acc[18]);
-    acc[19] = fma(D70, mk, acc[19]);
-  }
-  { const T mk = Mb[12];
-    acc[0] = fma(D13, mk, acc[0]);
-    acc[1] = fma(D23, mk, acc[1]);
-    acc[2] = fma(D26, mk, acc[2]);
-    acc[3] = fma(D27, mk, acc[3]);
-    acc[4] = fma(D38, mk, acc[4]);
-    acc[5] = fma(D41, mk, acc[5]);
-    acc[6] = fma(D42, mk, acc[6]);
-    acc[7] = fma(D45, mk, acc[7]);
-    acc[8] = fma(D46, mk, acc[8]);
-    acc[9] = fma(D47, mk, acc[9]);
-    acc[10] = fma(D59, mk, acc[10]);
-    acc[11] = fma(D62, mk, acc[11]);
-    acc[12] = fma(D63, mk, acc[12]);
-    acc[13] = fma(D66, mk, acc[13]);
-    acc[14] = fma(D67, mk, acc[14]);
-    acc[15] = fma(D68, mk, acc[15]);
-    acc[16] = fma(D71, mk, acc[16]);
-    acc[17] = fma(D72, mk, acc[17]);
-    acc[18] = fma(D73, mk, acc[18]);
-    acc[19] = fma(D74, mk, acc[19]);
+    acc[9] = fma(D50, mk, acc[9]);
+    acc[10] = fma(D53, mk, acc[10]);
+    acc[11] = fma(D54, mk, acc[11]);
+    acc[12] = fma(D56, mk, acc[12]);
+    acc[13] = fma(D57, mk, acc[13]);
+    acc[14] = fma(D59, mk, acc[14]);
+    acc[15] = fma(D60, mk, acc[15]);
   }
   { const T mk = Mb[13];
-    acc[0] = fma(D14, mk, acc[0]);
-    acc[1] = fma(D24, mk, acc[1]);
-    acc[2] = fma(D27, mk, acc[2]);
-    acc[3] = fma(D28, mk, acc[3]);
-    acc[4] = fma(D39, mk, acc[4]);
-    acc[5] = fma(D42, mk, acc[5]);
-    acc[6] = fma(D43, mk, acc[6]);
-    acc[7] = fma(D46, mk, acc[7]);
-    acc[8] = fma(D47, mk, acc[8]);
-    acc[9] = fma(D48, mk, acc[9]);
-    acc[10] = fma(D60, mk, acc[10]);
-    acc[11] = fma(D63, mk, acc[11]);
-    acc[12] = fma(D64, mk, acc[12]);
-    acc[13] = fma(D67, mk, acc[13]);
-    acc[14] = fma(D68, mk, acc[14]);
-    acc[15] = fma(D69, mk, acc[15]);
-    acc[16] = fma(D72, mk, acc[16]);
-    acc[17] = fma(D73, mk, acc[17]);
-    acc[18] = fma(D74, mk, acc[18]);
-    acc[19] = fma(D75, mk, acc[19]);
-  }
-  { const T mk = Mb[14];
-    acc[0] = fma(D15, mk, acc[0]);
+    acc[0] = fma(D16, mk, acc[0]);
     acc[1] = fma(D25, mk, acc[1]);
     acc[2] = fma(D28, mk, acc[2]);
     acc[3] = fma(D29, mk, acc[3]);
-    acc[4] = fma(D40, mk, acc[4]);
-    acc[5] = fma(D43, mk, acc[5]);
-    acc[6] = fma(D44, mk, acc[6]);
-    acc[7] = fma(D47, mk, acc[7]);
-    acc[8] = fma(D48, mk, acc[8]);
-    acc[9] = fma(D49, mk, acc[9]);
-    acc[10] = fma(D61, mk, acc[10]);
-    acc[11] = fma(D64, mk, acc[11]);
-    acc[12] = fma(D65, mk, acc[12]);
-    acc[13] = fma(D68, mk, acc[13]);
-    acc[14] = fma(D69, mk, acc[14]);
-    acc[15] = fma(D70, mk, acc[15]);
-    acc[16] = fma(D73, mk, acc[16]);
-    acc[17] = fma(D74, mk, acc[17]);
-    acc[18] = fma(D75, mk, acc[18]);
-    acc[19] = fma(D76, mk, acc[19]);
+    acc[4] = fma(D37, mk, acc[4]);
+    acc[5] = fma(D40, mk, acc[5]);
+    acc[6] = fma(D41, mk, acc[6]);
+    acc[7] = fma(D43, mk, acc[7]);
+    acc[8] = fma(D44, mk, acc[8]);
+    acc[9] = fma(D52, mk, acc[9]);
+    acc[10] = fma(D55, mk, acc[10]);
+    acc[11] = fma(D56, mk, acc[11]);
+    acc[12] = fma(D58, mk, acc[12]);
+    acc[13] = fma(D59, mk, acc[13]);
+    acc[14] = fma(D61, mk, acc[14]);
+    acc[15] = fma(D62, mk, acc[15]);
+  }
+  { const T mk = Mb[14];
+    acc[0] = fma(D17, mk, acc[0]);
+    acc[1] = fma(D26, mk, acc[1]);
+    acc[2] = fma(D29, mk, acc[2]);
+    acc[3] = fma(D30, mk, acc[3]);
+    acc[4] = fma(D38, mk, acc[4]);
+    acc[5] = fma(D41, mk, acc[5]);
+    acc[6] = fma(D42, mk, acc[6]);
+    acc[7] = fma(D44, mk, acc[7]);
+    acc[8] = fma(D45, mk, acc[8]);
+    acc[9] = fma(D53, mk, acc[9]);
+    acc[10] = fma(D56, mk, acc[10]);
+    acc[11] = fma(D57, mk, acc[11]);
+    acc[12] = fma(D59, mk, acc[12]);
+    acc[13] = fma(D60, mk, acc[13]);
+    acc[14] = fma(D62, mk, acc[14]);
+    acc[15] = fma(D63, mk, acc[15]);
   }
   { const T mk = Mb[15];
-    acc[0] = fma(D16, mk, acc[0]);
-    acc[1] = fma(D26, mk, acc[1]);
-    acc[2] = fma(D30, mk, acc[2]);
-    acc[3] = fma(D31, mk, acc[3]);
-    acc[4] = fma(D41, mk, acc[4]);
-    acc[5] = fma(D45, mk, acc[5]);
-    acc[6] = fma(D46, mk, acc[6]);
-    acc[7] = fma(D50, mk, acc[7]);
-    acc[8] = fma(D51, mk, acc[8]);
-    acc[9] = fma(D52, mk, acc[9]);
-    acc[10] = fma(D62, mk, acc[10]);
-    acc[11] = fma(D66, mk, acc[11]);
-    acc[12] = fma(D67, mk, acc[12]);
-    acc[13] = fma(D71, mk, acc[13]);
-    acc[14] = fma(D72, mk, acc[14]);
-    acc[15] = fma(D73, mk, acc[15]);
-    acc[16] = fma(D77, mk, acc[16]);
-    acc[17] = fma(D78, mk, acc[17]);
-    acc[18] = fma(D79, mk, acc[18]);
-    acc[19] = fma(D80, mk, acc[19]);
-  }
-  { const T mk = Mb[16];
-    acc[0] = fma(D17, mk, acc[0]);
-    acc[1] = fma(D27, mk, acc[1]);
-    acc[2] = fma(D31, mk, acc[2]);
-    acc[3] = fma(D32, mk, acc[3]);
-    acc[4] = fma(D42, mk, acc[4]);
-    acc[5] = fma(D46, mk, acc[5]);
-    acc[6] = fma(D47, mk, acc[6]);
-    acc[7] = fma(D51, mk, acc[7]);
-    acc[8] = fma(D52, mk, acc[8]);
-    acc[9] = fma(D53, mk, acc[9]);
-    acc[10] = fma(D63, mk, acc[10]);
-    acc[11] = fma(D67, mk, acc[11]);
-    acc[12] = fma(D68, mk, acc[12]);
-    acc[13] = fma(D72, mk, acc[13]);
-    acc[14] = fma(D73, mk, acc[14]);
-    acc[15] = fma(D74, mk, acc[15]);
-    acc[16] = fma(D78, mk, acc[16]);
-    acc[17] = fma(D79, mk, acc[17]);
-    acc[18] = fma(D80, mk, acc[18]);
-    acc[19] = fma(D81, mk, acc[19]);
-  }
-  { const T mk = Mb[17];
-    acc[0] = fma(D18, mk, acc[0]);
-    acc[1] = fma(D28, mk, acc[1]);
+    acc[0] = fma(D19, mk, acc[0]);
+    acc[1] = fma(D31, mk, acc[1]);
     acc[2] = fma(D32, mk, acc[2]);
     acc[3] = fma(D33, mk, acc[3]);
-    acc[4] = fma(D43, mk, acc[4]);
+    acc[4] = fma(D46, mk, acc[4]);
     acc[5] = fma(D47, mk, acc[5]);
     acc[6] = fma(D48, mk, acc[6]);
+    acc[7] = fma(D49, mk, acc[7]);
+    acc[8] = fma(D50, mk, acc[8]);
+  }
+  { const T mk = Mb[16];
+    acc[0] = fma(D20, mk, acc[0]);
+    acc[1] = fma(D32, mk, acc[1]);
+    acc[2] = fma(D34, mk, acc[2]);
+    acc[3] = fma(D35, mk, acc[3]);
+    acc[4] = fma(D47, mk, acc[4]);
+    acc[5] = fma(D49, mk, acc[5]);
+    acc[6] = fma(D50, mk, acc[6]);
     acc[7] = fma(D52, mk, acc[7]);
     acc[8] = fma(D53, mk, acc[8]);
-    acc[9] = fma(D54, mk, acc[9]);
-    acc[10] = fma(D64, mk, acc[10]);
-    acc[11] = fma(D68, mk, acc[11]);
-    acc[12] = fma(D69, mk, acc[12]);
-    acc[13] = fma(D73, mk, acc[13]);
-    acc[14] = fma(D74, mk, acc[14]);
-    acc[15] = fma(D75, mk, acc[15]);
-    acc[16] = fma(D79, mk, acc[16]);
-    acc[17] = fma(D80, mk, acc[17]);
-    acc[18] = fma(D81, mk, acc[18]);
-    acc[19] = fma(D82, mk, acc[19]);
   }
-  { const T mk = Mb[18];
-    acc[0] = fma(D19, mk, acc[0]);
-    acc[1] = fma(D29, mk, acc[1]);
-    acc[2] = fma(D33, mk, acc[2]);
-    acc[3] = fma(D34, mk, acc[3]);
-    acc[4] = fma(D44, mk, acc[4]);
-    acc[5] = fma(D48, mk, acc[5]);
-    acc[6] = fma(D49, mk, acc[6]);
+  { const T mk = Mb[17];
+    acc[0] = fma(D21, mk, acc[0]);
+    acc[1] = fma(D33, mk, acc[1]);
+    acc[2] = fma(D35, mk, acc[2]);
+    acc[3] = fma(D36, mk, acc[3]);
+    acc[4] = fma(D48, mk, acc[4]);
+    acc[5] = fma(D50, mk, acc[5]);
+    acc[6] = fma(D51, mk, acc[6]);
     acc[7] = fma(D53, mk, acc[7]);
     acc[8] = fma(D54, mk, acc[8]);
-    acc[9] = fma(D55, mk, acc[9]);
-    acc[10] = fma(D65, mk, acc[10]);
-    acc[11] = fma(D69, mk, acc[11]);
-    acc[12] = fma(D70, mk, acc[12]);
-    acc[13] = fma(D74, mk, acc[13]);
-    acc[14] = fma(D75, mk, acc[14]);
-    acc[15] = fma(D76, mk, acc[15]);
-    acc[16] = fma(D80, mk, acc[16]);
-    acc[17] = fma(D81, mk, acc[17]);
-    acc[18] = fma(D82, mk, acc[18]);
-    acc[19] = fma(D83, mk, acc[19]);
+  }
+  { const T mk = Mb[18];
+    acc[0] = fma(D22, mk, acc[0]);
+    acc[1] = fma(D34, mk, acc[1]);
+    acc[2] = fma(D37, mk, acc[2]);
+    acc[3] = fma(D38, mk, acc[3]);
+    acc[4] = fma(D49, mk, acc[4]);
+    acc[5] = fma(D52, mk, acc[5]);
+    acc[6] = fma(D53, mk, acc[6]);
+    acc[7] = fma(D55, mk, acc[7]);
+    acc[8] = fma(D56, mk, acc[8]);
   }
   { const T mk = Mb[19];
-    acc[0] = fma(D20, mk, acc[0]);
+    acc[0] = fma(D23, mk, acc[0]);
     acc[1] = fma(D35, mk, acc[1]);
-    acc[2] = fma(D36, mk, acc[2]);
-    acc[3] = fma(D37, mk, acc[3]);
-    acc[4] = fma(D56, mk, acc[4]);
-    acc[5] = fma(D57, mk, acc[5]);
-    acc[6] = fma(D58, mk, acc[6]);
-    acc[7] = fma(D59, mk, acc[7]);
-    acc[8] = fma(D60, mk, acc[8]);
-    acc[9] = fma(D61, mk, acc[9]);
-  }
-  { const T mk = Mb[20];
-    acc[0] = fma(D21, mk, acc[0]);
-    acc[1] = fma(D36, mk, acc[1]);
     acc[2] = fma(D38, mk, acc[2]);
     acc[3] = fma(D39, mk, acc[3]);
-    acc[4] = fma(D57, mk, acc[4]);
+    acc[4] = fma(D50, mk, acc[4]);
+    acc[5] = fma(D53, mk, acc[5]);
+    acc[6] = fma(D54, mk, acc[6]);
+    acc[7] = fma(D56, mk, acc[7]);
+    acc[8] = fma(D57, mk, acc[8]);
+  }
+  { const T mk = Mb[20];
+    acc[0] = fma(D25, mk, acc[0]);
+    acc[1] = fma(D37, mk, acc[1]);
+    acc[2] = fma(D40, mk, acc[2]);
+    acc[3] = fma(D41, mk, acc[3]);
+    acc[4] = fma(D52, mk, acc[4]);
+    acc[5] = fma(D55, mk, acc[5]);
+    acc[6] = fma(D56, mk, acc[6]);
+    acc[7] = fma(D58, mk, acc[7]);
+    acc[8] = fma(D59, mk, acc[8]);
+  }
+  { const T mk = Mb[21];
+    acc[0] = fma(D26, mk, acc[0]);
+    acc[1] = fma(D38, mk, acc[1]);
+    acc[2] = fma(D41, mk, acc[2]);
+    acc[3] = fma(D42, mk, acc[3]);
+    acc[4] = fma(D53, mk, acc[4]);
+    acc[5] = fma(D56, mk, acc[5]);
+    acc[6] = fma(D57, mk, acc[6]);
+    acc[7] = fma(D59, mk, acc[7]);
+    acc[8] = fma(D60, mk, acc[8]);
+  }
+  { const T mk = Mb[22];
+    acc[0] = fma(D28, mk, acc[0]);
+    acc[1] = fma(D40, mk, acc[1]);
+    acc[2] = fma(D43, mk, acc[2]);
+    acc[3] = fma(D44, mk, acc[3]);
+    acc[4] = fma(D55, mk, acc[4]);
+    acc[5] = fma(D58, mk, acc[5]);
+    acc[6] = fma(D59, mk, acc[6]);
+    acc[7] = fma(D61, mk, acc[7]);
+    acc[8] = fma(D62, mk, acc[8]);
+  }
+  { const T mk = Mb[23];
+    acc[0] = fma(D29, mk, acc[0]);
+    acc[1] = fma(D41, mk, acc[1]);
+    acc[2] = fma(D44, mk, acc[2]);
+    acc[3] = fma(D45, mk, acc[3]);
+    acc[4] = fma(D56, mk, acc[4]);
     acc[5] = fma(D59, mk, acc[5]);
     acc[6] = fma(D60, mk, acc[6]);
     acc[7] = fma(D62, mk, acc[7]);
     acc[8] = fma(D63, mk, acc[8]);
-    acc[9] = fma(D64, mk, acc[9]);
-  }
-  { const T mk = Mb[21];
-    acc[0] = fma(D22, mk, acc[0]);
-    acc[1] = fma(D37, mk, acc[1]);
-    acc[2] = fma(D39, mk, acc[2]);
-    acc[3] = fma(D40, mk, acc[3]);
-    acc[4] = fma(D58, mk, acc[4]);
-    acc[5] = fma(D60, mk, acc[5]);
-    acc[6] = fma(D61, mk, acc[6]);
-    acc[7] = fma(D63, mk, acc[7]);
-    acc[8] = fma(D64, mk, acc[8]);
-    acc[9] = fma(D65, mk, acc[9]);
-  }
-  { const T mk = Mb[22];
-    acc[0] = fma(D23, mk, acc[0]);
-    acc[1] = fma(D38, mk, acc[1]);
-    acc[2] = fma(D41, mk, acc[2]);
-    acc[3] = fma(D42, mk, acc[3]);
-    acc[4] = fma(D59, mk, acc[4]);
-    acc[5] = fma(D62, mk, acc[5]);
-    acc[6] = fma(D63, mk, acc[6]);
-    acc[7] = fma(D66, mk, acc[7]);
-    acc[8] = fma(D67, mk, acc[8]);
-    acc[9] = fma(D68, mk, acc[9]);
-  }
-  { const T mk = Mb[23];
-    acc[0] = fma(D24, mk, acc[0]);
-    acc[1] = fma(D39, mk, acc[1]);
-    acc[2] = fma(D42, mk, acc[2]);
-    acc[3] = fma(D43, mk, acc[3]);
-    acc[4] = fma(D60, mk, acc[4]);
-    acc[5] = fma(D63, mk, acc[5]);
-    acc[6] = fma(D64, mk, acc[6]);
-    acc[7] = fma(D67, mk, acc[7]);
-    acc[8] = fma(D68, mk, acc[8]);
-    acc[9] = fma(D69, mk, acc[9]);
   }
   { const T mk = Mb[24];
-    acc[0] = fma(D25, mk, acc[0]);
-    acc[1] = fma(D40, mk, acc[1]);
-    acc[2] = fma(D43, mk, acc[2]);
-    acc[3] = fma(D44, mk, acc[3]);
-    acc[4] = fma(D61, mk, acc[4]);
-    acc[5] = fma(D64, mk, acc[5]);
-    acc[6] = fma(D65, mk, acc[6]);
-    acc[7] = fma(D68, mk, acc[7]);
-    acc[8] = fma(D69, mk, acc[8]);
-    acc[9] = fma(D70, mk, acc[9]);
-  }
-  { const T mk = Mb[25];
-    acc[0] = fma(D26, mk, acc[0]);
-    acc[1] = fma(D41, mk, acc[1]);
-    acc[2] = fma(D45, mk, acc[2]);
-    acc[3] = fma(D46, mk, acc[3]);
-    acc[4] = fma(D62, mk, acc[4]);
-    acc[5] = fma(D66, mk, acc[5]);
-    acc[6] = fma(D67, mk, acc[6]);
-    acc[7] = fma(D71, mk, acc[7]);
-    acc[8] = fma(D72, mk, acc[8]);
-    acc[9] = fma(D73, mk, acc[9]);
-  }
-  { const T mk = Mb[26];
-    acc[0] = fma(D27, mk, acc[0]);
-    acc[1] = fma(D42, mk, acc[1]);
-    acc[2] = fma(D46, mk, acc[2]);
-    acc[3] = fma(D47, mk, acc[3]);
-    acc[4] = fma(D63, mk, acc[4]);
-    acc[5] = fma(D67, mk, acc[5]);
-    acc[6] = fma(D68, mk, acc[6]);
-    acc[7] = fma(D72, mk, acc[7]);
-    acc[8] = fma(D73, mk, acc[8]);
-    acc[9] = fma(D74, mk, acc[9]);
-  }
-  { const T mk = Mb[27];
-    acc[0] = fma(D28, mk, acc[0]);
-    acc[1] = fma(D43, mk, acc[1]);
-    acc[2] = fma(D47, mk, acc[2]);
-    acc[3] = fma(D48, mk, acc[3]);
-    acc[4] = fma(D64, mk, acc[4]);
-    acc[5] = fma(D68, mk, acc[5]);
-    acc[6] = fma(D69, mk, acc[6]);
-    acc[7] = fma(D73, mk, acc[7]);
-    acc[8] = fma(D74, mk, acc[8]);
-    acc[9] = fma(D75, mk, acc[9]);
-  }
-  { const T mk = Mb[28];
-    acc[0] = fma(D29, mk, acc[0]);
-    acc[1] = fma(D44, mk, acc[1]);
-    acc[2] = fma(D48, mk, acc[2]);
-    acc[3] = fma(D49, mk, acc[3]);
-    acc[4] = fma(D65, mk, acc[4]);
-    acc[5] = fma(D69, mk, acc[5]);
-    acc[6] = fma(D70, mk, acc[6]);
-    acc[7] = fma(D74, mk, acc[7]);
-    acc[8] = fma(D75, mk, acc[8]);
-    acc[9] = fma(D76, mk, acc[9]);
-  }
-  { const T mk = Mb[29];
-    acc[0] = fma(D30, mk, acc[0]);
-    acc[1] = fma(D45, mk, acc[1]);
-    acc[2] = fma(D50, mk, acc[2]);
-    acc[3] = fma(D51, mk, acc[3]);
-    acc[4] = fma(D66, mk, acc[4]);
-    acc[5] = fma(D71, mk, acc[5]);
-    acc[6] = fma(D72, mk, acc[6]);
-    acc[7] = fma(D77, mk, acc[7]);
-    acc[8] = fma(D78, mk, acc[8]);
-    acc[9] = fma(D79, mk, acc[9]);
-  }
-  { const T mk = Mb[30];
     acc[0] = fma(D31, mk, acc[0]);
     acc[1] = fma(D46, mk, acc[1]);
-    acc[2] = fma(D51, mk, acc[2]);
-    acc[3] = fma(D52, mk, acc[3]);
-    acc[4] = fma(D67, mk, acc[4]);
-    acc[5] = fma(D72, mk, acc[5]);
-    acc[6] = fma(D73, mk, acc[6]);
-    acc[7] = fma(D78, mk, acc[7]);
-    acc[8] = fma(D79, mk, acc[8]);
-    acc[9] = fma(D80, mk, acc[9]);
+    acc[2] = fma(D47, mk, acc[2]);
+    acc[3] = fma(D48, mk, acc[3]);
   }
-  { const T mk = Mb[31];
+  { const T mk = Mb[25];
     acc[0] = fma(D32, mk, acc[0]);
     acc[1] = fma(D47, mk, acc[1]);
-    acc[2] = fma(D52, mk, acc[2]);
-    acc[3] = fma(D53, mk, acc[3]);
-    acc[4] = fma(D68, mk, acc[4]);
-    acc[5] = fma(D73, mk, acc[5]);
-    acc[6] = fma(D74, mk, acc[6]);
-    acc[7] = fma(D79, mk, acc[7]);
-    acc[8] = fma(D80, mk, acc[8]);
-    acc[9] = fma(D81, mk, acc[9]);
+    acc[2] = fma(D49, mk, acc[2]);
+    acc[3] = fma(D50, mk, acc[3]);
   }
-  { const T mk = Mb[32];
+  { const T mk = Mb[26];
     acc[0] = fma(D33, mk, acc[0]);
     acc[1] = fma(D48, mk, acc[1]);
-    acc[2] = fma(D53, mk, acc[2]);
-    acc[3] = fma(D54, mk, acc[3]);
-    acc[4] = fma(D69, mk, acc[4]);
-    acc[5] = fma(D74, mk, acc[5]);
-    acc[6] = fma(D75, mk, acc[6]);
-    acc[7] = fma(D80, mk, acc[7]);
-    acc[8] = fma(D81, mk, acc[8]);
-    acc[9] = fma(D82, mk, acc[9]);
+    acc[2] = fma(D50, mk, acc[2]);
+    acc[3] = fma(D51, mk, acc[3]);
   }
-  { const T mk = Mb[33];
+  { const T mk = Mb[27];
     acc[0] = fma(D34, mk, acc[0]);
     acc[1] = fma(D49, mk, acc[1]);
-    acc[2] = fma(D54, mk, acc[2]);
-    acc[3] = fma(D55, mk, acc[3]);
-    acc[4] = fma(D70, mk, acc[4]);
-    acc[5] = fma(D75, mk, acc[5]);
-    acc[6] = fma(D76, mk, acc[6]);
-    acc[7] = fma(D81, mk, acc[7]);
-    acc[8] = fma(D82, mk, acc[8]);
-    acc[9] = fma(D83, mk, acc[9]);
+    acc[2] = fma(D52, mk, acc[2]);
+    acc[3] = fma(D53, mk, acc[3]);
   }
-  { const T mk = Mb[34];
+  { const T mk = Mb[28];
     acc[0] = fma(D35, mk, acc[0]);
-    acc[1] = fma(D56, mk, acc[1]);
-    acc[2] = fma(D57, mk, acc[2]);
-    acc[3] = fma(D58, mk, acc[3]);
+    acc[1] = fma(D50, mk, acc[1]);
+    acc[2] = fma(D53, mk, acc[2]);
+    acc[3] = fma(D54, mk, acc[3]);
   }
-  { const T mk = Mb[35];
-    acc[0] = fma(D36, mk, acc[0]);
-    acc[1] = fma(D57, mk, acc[1]);
+  { const T mk = Mb[29];
+    acc[0] = fma(D37, mk, acc[0]);
+    acc[1] = fma(D52, mk, acc[1]);
+    acc[2] = fma(D55, mk, acc[2]);
+    acc[3] = fma(D56, mk, acc[3]);
+  }
+  { const T mk = Mb[30];
+    acc[0] = fma(D38, mk, acc[0]);
+    acc[1] = fma(D53, mk, acc[1]);
+    acc[2] = fma(D56, mk, acc[2]);
+    acc[3] = fma(D57, mk, acc[3]);
+  }
+  { const T mk = Mb[31];
+    acc[0] = fma(D40, mk, acc[0]);
+    acc[1] = fma(D55, mk, acc[1]);
+    acc[2] = fma(D58, mk, acc[2]);
+    acc[3] = fma(D59, mk, acc[3]);
+  }
+  { const T mk = Mb[32];
+    acc[0] = fma(D41, mk, acc[0]);
+    acc[1] = fma(D56, mk, acc[1]);
     acc[2] = fma(D59, mk, acc[2]);
     acc[3] = fma(D60, mk, acc[3]);
   }
-  { const T mk = Mb[36];
-    acc[0] = fma(D37, mk, acc[0]);
+  { const T mk = Mb[33];
+    acc[0] = fma(D43, mk, acc[0]);
     acc[1] = fma(D58, mk, acc[1]);
-    acc[2] = fma(D60, mk, acc[2]);
-    acc[3] = fma(D61, mk, acc[3]);
+    acc[2] = fma(D61, mk, acc[2]);
+    acc[3] = fma(D62, mk, acc[3]);
   }
-  { const T mk = Mb[37];
-    acc[0] = fma(D38, mk, acc[0]);
+  { const T mk = Mb[34];
+    acc[0] = fma(D44, mk, acc[0]);
     acc[1] = fma(D59, mk, acc[1]);
     acc[2] = fma(D62, mk, acc[2]);
     acc[3] = fma(D63, mk, acc[3]);
   }
+  { const T mk = Mb[35];
+    acc[0] = fma(D46, mk, acc[0]);
+  }
+  { const T mk = Mb[36];
+    acc[0] = fma(D47, mk, acc[0]);
+  }
+  { const T mk = Mb[37];
+    acc[0] = fma(D48, mk, acc[0]);
+  }
   { const T mk = Mb[38];
-    acc[0] = fma(D39, mk, acc[0]);
-    acc[1] = fma(D60, mk, acc[1]);
-    acc[2] = fma(D63, mk, acc[2]);
-    acc[3] = fma(D64, mk, acc[3]);
+    acc[0] = fma(D49, mk, acc[0]);
   }
   { const T mk = Mb[39];
-    acc[0] = fma(D40, mk, acc[0]);
-    acc[1] = fma(D61, mk, acc[1]);
-    acc[2] = fma(D64, mk, acc[2]);
-    acc[3] = fma(D65, mk, acc[3]);
+    acc[0] = fma(D50, mk, acc[0]);
   }
   { const T mk = Mb[40];
-    acc[0] = fma(D41, mk, acc[0]);
-    acc[1] = fma(D62, mk, acc[1]);
-    acc[2] = fma(D66, mk, acc[2]);
-    acc[3] = fma(D67, mk, acc[3]);
+    acc[0] = fma(D52, mk, acc[0]);
   }
   { const T mk = Mb[41];
-    acc[0] = fma(D42, mk, acc[0]);
-    acc[1] = fma(D63, mk, acc[1]);
-    acc[2] = fma(D67, mk, acc[2]);
-    acc[3] = fma(D68, mk, acc[3]);
+    acc[0] = fma(D53, mk, acc[0]);
   }
   { const T mk = Mb[42];
-    acc[0] = fma(D43, mk, acc[0]);
-    acc[1] = fma(D64, mk, acc[1]);
-    acc[2] = fma(D68, mk, acc[2]);
-    acc[3] = fma(D69, mk, acc[3]);
+    acc[0] = fma(D55, mk, acc[0]);
   }
   { const T mk = Mb[43];
-    acc[0] = fma(D44, mk, acc[0]);
-    acc[1] = fma(D65, mk, acc[1]);
-    acc[2] = fma(D69, mk, acc[2]);
-    acc[3] = fma(D70, mk, acc[3]);
-  }
-  { const T mk = Mb[44];
-    acc[0] = fma(D45, mk, acc[0]);
-    acc[1] = fma(D66, mk, acc[1]);
-    acc[2] = fma(D71, mk, acc[2]);
-    acc[3] = fma(D72, mk, acc[3]);
-  }
-  { const T mk = Mb[45];
-    acc[0] = fma(D46, mk, acc[0]);
-    acc[1] = fma(D67, mk, acc[1]);
-    acc[2] = fma(D72, mk, acc[2]);
-    acc[3] = fma(D73, mk, acc[3]);
-  }
-  { const T mk = Mb[46];
-    acc[0] = fma(D47, mk, acc[0]);
-    acc[1] = fma(D68, mk, acc[1]);
-    acc[2] = fma(D73, mk, acc[2]);
-    acc[3] = fma(D74, mk, acc[3]);
-  }
-  { const T mk = Mb[47];
-    acc[0] = fma(D48, mk, acc[0]);
-    acc[1] = fma(D69, mk, acc[1]);
-    acc[2] = fma(D74, mk, acc[2]);
-    acc[3] = fma(D75, mk, acc[3]);
-  }
-  { const T mk = Mb[48];
-    acc[0] = fma(D49, mk, acc[0]);
-    acc[1] = fma(D70, mk, acc[1]);
-    acc[2] = fma(D75, mk, acc[2]);
-    acc[3] = fma(D76, mk, acc[3]);
-  }
-  { const T mk = Mb[49];
-    acc[0] = fma(D50, mk, acc[0]);
-    acc[1] = fma(D71, mk, acc[1]);
-    acc[2] = fma(D77, mk, acc[2]);
-    acc[3] = fma(D78, mk, acc[3]);
-  }
-  { const T mk = Mb[50];
-    acc[0] = fma(D51, mk, acc[0]);
-    acc[1] = fma(D72, mk, acc[1]);
-    acc[2] = fma(D78, mk, acc[2]);
-    acc[3] = fma(D79, mk, acc[3]);
-  }
-  { const T mk = Mb[51];
-    acc[0] = fma(D52, mk, acc[0]);
-    acc[1] = fma(D73, mk, acc[1]);
-    acc[2] = fma(D79, mk, acc[2]);
-    acc[3] = fma(D80, mk, acc[3]);
-  }
-  { const T mk = Mb[52];
-    acc[0] = fma(D53, mk, acc[0]);
-    acc[1] = fma(D74, mk, acc[1]);
-    acc[2] = fma(D80, mk, acc[2]);
-    acc[3] = fma(D81, mk, acc[3]);
-  }
-  { const T mk = Mb[53];
-    acc[0] = fma(D54, mk, acc[0]);
-    acc[1] = fma(D75, mk, acc[1]);
-    acc[2] = fma(D81, mk, acc[2]);
-    acc[3] = fma(D82, mk, acc[3]);
-  }
-  { const T mk = Mb[54];
-    acc[0] = fma(D55, mk, acc[0]);
-    acc[1] = fma(D76, mk, acc[1]);
-    acc[2] = fma(D82, mk, acc[2]);
-    acc[3] = fma(D83, mk, acc[3]);
-  }
-  { const T mk = Mb[55];
     acc[0] = fma(D56, mk, acc[0]);
   }
-  { const T mk = Mb[56];
-    acc[0] = fma(D57, mk, acc[0]);
-  }
-  { const T mk = Mb[57];
+  { const T mk = Mb[44];
     acc[0] = fma(D58, mk, acc[0]);
   }
-  { const T mk = Mb[58];
+  { const T mk = Mb[45];
     acc[0] = fma(D59, mk, acc[0]);
   }
-  { const T mk = Mb[59];
-    acc[0] = fma(D60, mk, acc[0]);
-  }
-  { const T mk = Mb[60];
+  { const T mk = Mb[46];
     acc[0] = fma(D61, mk, acc[0]);
   }
-  { const T mk = Mb[61];
+  { const T mk = Mb[47];
     acc[0] = fma(D62, mk, acc[0]);
   }
-  { const T mk = Mb[62];
-    acc[0] = fma(D63, mk, acc[0]);
-  }
-  { const T mk = Mb[63];
-    acc[0] = fma(D64, mk, acc[0]);
-  }
-  { const T mk = Mb[64];
-    acc[0] = fma(D65, mk, acc[0]);
-  }
-  { const T mk = Mb[65];
-    acc[0] = fma(D66, mk, acc[0]);
-  }
-  { const T mk = Mb[66];
-    acc[0] = fma(D67, mk, acc[0]);
-  }
-  { const T mk = Mb[67];
-    acc[0] = fma(D68, mk, acc[0]);
-  }
-  { const T mk = Mb[68];
-    acc[0] = fma(D69, mk, acc[0]);
-  }
-  { const T mk = Mb[69];
-    acc[0] = fma(D70, mk, acc[0]);
-  }
-  { const T mk = Mb[70];
-    acc[0] = fma(D71, mk, acc[0]);
-  }
-  { const T mk = Mb[71];
-    acc[0] = fma(D72, mk, acc[0]);
-  }
-  { const T mk = Mb[72];
-    acc[0] = fma(D73, mk, acc[0]);
-  }
-  { const T mk = Mb[73];
-    acc[0] = fma(D74, mk, acc[0]);
-  }
-  { const T mk = Mb[74];
-    acc[0] = fma(D75, mk, acc[0]);
-  }
-  { const T mk = Mb[75];
-    acc[0] = fma(D76, mk, acc[0]);
-  }
-  { const T mk = Mb[76];
-    acc[0] = fma(D77, mk, acc[0]);
-  }
-  { const T mk = Mb[77];
-    acc[0] = fma(D78, mk, acc[0]);
-  }
-  { const T mk = Mb[78];
-    acc[0] = fma(D79, mk, acc[0]);
-  }
-  { const T mk = Mb[79];
-    acc[0] = fma(D80, mk, acc[0]);
-  }
-  { const T mk = Mb[80];
-    acc[0] = fma(D81, mk, acc[0]);
-  }
-  { const T mk = Mb[81];
-    acc[0] = fma(D82, mk, acc[0]);
-  }
-  { const T mk = Mb[82];
-    acc[0] = fma(D83, mk, acc[0]);
-  }
 }
-// derivative tensor D_j = d^j (1/R), j < 84, of M2L m1 p6
 template <typename T>
 __device__ __forceinline__ void dtensor_m1_p6(T x, T y, T z, T* __restrict__ Dout) {
   const T r2 = x * x + y * y + z * z;
@@ -2384,81 +1608,61 @@ __device__ __forceinline__ void dtensor_m1_p6(T x, T y, T z, T* __restrict__ Dou
   const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
   const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
   const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
-  const T D9 = -(T(3) * (T(2) * z * D3) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
+  const T D9 = -(D4 + D7);
   const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
   const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
   const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
   const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
   const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
-  const T D15 = -(T(5) * (x * D9 + T(2) * z * D6) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
+  const T D15 = -(D10 + D13);
   const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
   const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D18 = -(T(5) * (y * D9 + T(2) * z * D8) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D19 = -(T(5) * (T(3) * z * D9) + T(2) * (T(6) * D3)) * ir2 * cinv<T>(3);
-  const T D20 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D24 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
-  const T D25 = -(T(7) * (T(2) * x * D15 + T(2) * z * D12) + T(3) * (T(2) * D9 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D27 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
-  const T D28 = -(T(7) * (x * D18 + y * D15 + T(2) * z * D14) + T(3) * (T(2) * D5)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (x * D19 + T(3) * z * D15) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D30 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D31 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D32 = -(T(7) * (T(2) * y * D18 + T(2) * z * D17) + T(3) * (T(2) * D9 + T(2) * D7)) * ir2 * cinv<T>(4);
-  const T D33 = -(T(7) * (y * D19 + T(3) * z * D18) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
-  const T D34 = -(T(7) * (T(4) * z * D19) + T(3) * (T(12) * D9)) * ir2 * cinv<T>(4);
-  const T D35 = -(T(9) * (T(5) * x * D20) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D36 = -(T(9) * (T(4) * x * D21 + y * D20) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D37 = -(T(9) * (T(4) * x * D22 + z * D20) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(3) * x * D23 + T(2) * y * D21) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D39 = -(T(9) * (T(3) * x * D24 + y * D22 + z * D21) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D40 = -(T(9) * (T(3) * x * D25 + T(2) * z * D22) + T(4) * (T(6) * D15 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (T(2) * x * D26 + T(3) * y * D23) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D42 = -(T(9) * (T(2) * x * D27 + T(2) * y * D24 + z * D23) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
-  const T D43 = -(T(9) * (T(2) * x * D28 + y * D25 + T(2) * z * D24) + T(4) * (T(2) * D18 + T(2) * D11)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(2) * x * D29 + T(3) * z * D25) + T(4) * (T(2) * D19 + T(6) * D12)) * ir2 * cinv<T>(5);
-  const T D45 = -(T(9) * (x * D30 + T(4) * y * D26) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D46 = -(T(9) * (x * D31 + T(3) * y * D27 + z * D26) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D47 = -(T(9) * (x * D32 + T(2) * y * D28 + T(2) * z * D27) + T(4) * (T(2) * D15 + T(2) * D13)) * ir2 * cinv<T>(5);
-  const T D48 = -(T(9) * (x * D33 + y * D29 + T(3) * z * D28) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
-  const T D49 = -(T(9) * (x * D34 + T(4) * z * D29) + T(4) * (T(12) * D15)) * ir2 * cinv<T>(5);
-  const T D50 = -(T(9) * (T(5) * y * D30) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D51 = -(T(9) * (T(4) * y * D31 + z * D30) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
-  const T D52 = -(T(9) * (T(3) * y * D32 + T(2) * z * D31) + T(4) * (T(6) * D18 + T(2) * D16)) * ir2 * cinv<T>(5);
-  const T D53 = -(T(9) * (T(2) * y * D33 + T(3) * z * D32) + T(4) * (T(2) * D19 + T(6) * D17)) * ir2 * cinv<T>(5);
-  const T D54 = -(T(9) * (y * D34 + T(4) * z * D33) + T(4) * (T(12) * D18)) * ir2 * cinv<T>(5);
-  const T D55 = -(T(9) * (T(5) * z * D34) + T(4) * (T(20) * D19)) * ir2 * cinv<T>(5);
-  const T D56 = -(T(11) * (T(6) * x * D35) + T(5) * (T(30) * D20)) * ir2 * cinv<T>(6);
-  const T D57 = -(T(11) * (T(5) * x * D36 + y * D35) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
-  const T D58 = -(T(11) * (T(5) * x * D37 + z * D35) + T(5) * (T(20) * D22)) * ir2 * cinv<T>(6);
-  const T D59 = -(T(11) * (T(4) * x * D38 + T(2) * y * D36) + T(5) * (T(12) * D23 + T(2) * D20)) * ir2 * cinv<T>(6);
-  const T D60 = -(T(11) * (T(4) * x * D39 + y * D37 + z * D36) + T(5) * (T(12) * D24)) * ir2 * cinv<T>(6);
-  const T D61 = -(T(11) * (T(4) * x * D40 + T(2) * z * D37) + T(5) * (T(12) * D25 + T(2) * D20)) * ir2 * cinv<T>(6);
-  const T D62 = -(T(11) * (T(3) * x * D41 + T(3) * y * D38) + T(5) * (T(6) * D26 + T(6) * D21)) * ir2 * cinv<T>(6);
-  const T D63 = -(T(11) * (T(3) * x * D42 + T(2) * y * D39 + z * D38) + T(5) * (T(6) * D27 + T(2) * D22)) * ir2 * cinv<T>(6);
-  const T D64 = -(T(11) * (T(3) * x * D43 + y * D40 + T(2) * z * D39) + T(5) * (T(6) * D28 + T(2) * D21)) * ir2 * cinv<T>(6);
-  const T D65 = -(T(11) * (T(3) * x * D44 + T(3) * z * D40) + T(5) * (T(6) * D29 + T(6) * D22)) * ir2 * cinv<T>(6);
-  const T D66 = -(T(11) * (T(2) * x * D45 + T(4) * y * D41) + T(5) * (T(2) * D30 + T(12) * D23)) * ir2 * cinv<T>(6);
-  const T D67 = -(T(11) * (T(2) * x * D46 + T(3) * y * D42 + z * D41) + T(5) * (T(2) * D31 + T(6) * D24)) * ir2 * cinv<T>(6);
-  const T D68 = -(T(11) * (T(2) * x * D47 + T(2) * y * D43 + T(2) * z * D42) + T(5) * (T(2) * D32 + T(2) * D25 + T(2) * D23)) * ir2 * cinv<T>(6);
-  const T D69 = -(T(11) * (T(2) * x * D48 + y * D44 + T(3) * z * D43) + T(5) * (T(2) * D33 + T(6) * D24)) * ir2 * cinv<T>(6);
-  const T D70 = -(T(11) * (T(2) * x * D49 + T(4) * z * D44) + T(5) * (T(2) * D34 + T(12) * D25)) * ir2 * cinv<T>(6);
-  const T D71 = -(T(11) * (x * D50 + T(5) * y * D45) + T(5) * (T(20) * D26)) * ir2 * cinv<T>(6);
-  const T D72 = -(T(11) * (x * D51 + T(4) * y * D46 + z * D45) + T(5) * (T(12) * D27)) * ir2 * cinv<T>(6);
-  const T D73 = -(T(11) * (x * D52 + T(3) * y * D47 + T(2) * z * D46) + T(5) * (T(6) * D28 + T(2) * D26)) * ir2 * cinv<T>(6);
-  const T D74 = -(T(11) * (x * D53 + T(2) * y * D48 + T(3) * z * D47) + T(5) * (T(2) * D29 + T(6) * D27)) * ir2 * cinv<T>(6);
-  const T D75 = -(T(11) * (x * D54 + y * D49 + T(4) * z * D48) + T(5) * (T(12) * D28)) * ir2 * cinv<T>(6);
-  const T D76 = -(T(11) * (x * D55 + T(5) * z * D49) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
-  const T D77 = -(T(11) * (T(6) * y * D50) + T(5) * (T(30) * D30)) * ir2 * cinv<T>(6);
-  const T D78 = -(T(11) * (T(5) * y * D51 + z * D50) + T(5) * (T(20) * D31)) * ir2 * cinv<T>(6);
-  const T D79 = -(T(11) * (T(4) * y * D52 + T(2) * z * D51) + T(5) * (T(12) * D32 + T(2) * D30)) * ir2 * cinv<T>(6);
-  const T D80 = -(T(11) * (T(3) * y * D53 + T(3) * z * D52) + T(5) * (T(6) * D33 + T(6) * D31)) * ir2 * cinv<T>(6);
-  const T D81 = -(T(11) * (T(2) * y * D54 + T(4) * z * D53) + T(5) * (T(2) * D34 + T(12) * D32)) * ir2 * cinv<T>(6);
-  const T D82 = -(T(11) * (y * D55 + T(5) * z * D54) + T(5) * (T(20) * D33)) * ir2 * cinv<T>(6);
-  const T D83 = -(T(11) * (T(6) * z * D55) + T(5) * (T(30) * D34)) * ir2 * cinv<T>(6);
+  const T D18 = -(D11 + D16);
+  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
+  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
+  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
+  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T D24 = -(D19 + D22);
+  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
+  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T D27 = -(D20 + D25);
+  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
+  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T D30 = -(D22 + D28);
+  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
+  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
+  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
+  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
+  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D36 = -(D31 + D34);
+  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
+  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T D39 = -(D32 + D37);
+  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
+  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T D42 = -(D34 + D40);
+  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
+  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T D45 = -(D37 + D43);
+  const T D46 = -(T(11) * (T(6) * x * D31) + T(5) * (T(30) * D19)) * ir2 * cinv<T>(6);
+  const T D47 = -(T(11) * (T(5) * x * D32 + y * D31) + T(5) * (T(20) * D20)) * ir2 * cinv<T>(6);
+  const T D48 = -(T(11) * (T(5) * x * D33 + z * D31) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
+  const T D49 = -(T(11) * (T(4) * x * D34 + T(2) * y * D32) + T(5) * (T(12) * D22 + T(2) * D19)) * ir2 * cinv<T>(6);
+  const T D50 = -(T(11) * (T(4) * x * D35 + y * D33 + z * D32) + T(5) * (T(12) * D23)) * ir2 * cinv<T>(6);
+  const T D51 = -(D46 + D49);
+  const T D52 = -(T(11) * (T(3) * x * D37 + T(3) * y * D34) + T(5) * (T(6) * D25 + T(6) * D20)) * ir2 * cinv<T>(6);
+  const T D53 = -(T(11) * (T(3) * x * D38 + T(2) * y * D35 + z * D34) + T(5) * (T(6) * D26 + T(2) * D21)) * ir2 * cinv<T>(6);
+  const T D54 = -(D47 + D52);
+  const T D55 = -(T(11) * (T(2) * x * D40 + T(4) * y * D37) + T(5) * (T(2) * D28 + T(12) * D22)) * ir2 * cinv<T>(6);
+  const T D56 = -(T(11) * (T(2) * x * D41 + T(3) * y * D38 + z * D37) + T(5) * (T(2) * D29 + T(6) * D23)) * ir2 * cinv<T>(6);
+  const T D57 = -(D49 + D55);
+  const T D58 = -(T(11) * (x * D43 + T(5) * y * D40) + T(5) * (T(20) * D25)) * ir2 * cinv<T>(6);
+  const T D59 = -(T(11) * (x * D44 + T(4) * y * D41 + z * D40) + T(5) * (T(12) * D26)) * ir2 * cinv<T>(6);
+  const T D60 = -(D52 + D58);
+  const T D61 = -(T(11) * (T(6) * y * D43) + T(5) * (T(30) * D28)) * ir2 * cinv<T>(6);
+  const T D62 = -(T(11) * (T(5) * y * D44 + z * D43) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
+  const T D63 = -(D55 + D61);
   Dout[0] = D0;
   Dout[1] = D1;
   Dout[2] = D2;
@@ -2523,28 +1727,7 @@ __device__ __forceinline__ void dtensor_m1_p6(T x, T y, T z, T* __restrict__ Dou
   Dout[61] = D61;
   Dout[62] = D62;
   Dout[63] = D63;
-  Dout[64] = D64;
-  Dout[65] = D65;
-  Dout[66] = D66;
-  Dout[67] = D67;
-  Dout[68] = D68;
-  Dout[69] = D69;
-  Dout[70] = D70;
-  Dout[71] = D71;
-  Dout[72] = D72;
-  Dout[73] = D73;
-  Dout[74] = D74;
-  Dout[75] = D75;
-  Dout[76] = D76;
-  Dout[77] = D77;
-  Dout[78] = D78;
-  Dout[79] = D79;
-  Dout[80] = D80;
-  Dout[81] = D81;
-  Dout[82] = D82;
-  Dout[83] = D83;
 }
-// M2L m1 p6 with the derivative tensor read from Dt
 template <typename T>
 __device__ __forceinline__ void m2l_m1_p6_pre(const T* __restrict__ Dt, const T* __restrict__ Mb, T* __restrict__ acc) {
   const T D0 = Dt[0];
@@ -2611,26 +1794,6 @@ __device__ __forceinline__ void m2l_m1_p6_pre(const T* __restrict__ Dt, const T*
   const T D61 = Dt[61];
   const T D62 = Dt[62];
   const T D63 = Dt[63];
-  const T D64 = Dt[64];
-  const T D65 = Dt[65];
-  const T D66 = Dt[66];
-  const T D67 = Dt[67];
-  const T D68 = Dt[68];
-  const T D69 = Dt[69];
-  const T D70 = Dt[70];
-  const T D71 = Dt[71];
-  const T D72 = Dt[72];
-  const T D73 = Dt[73];
-  const T D74 = Dt[74];
-  const T D75 = Dt[75];
-  const T D76 = Dt[76];
-  const T D77 = Dt[77];
-  const T D78 = Dt[78];
-  const T D79 = Dt[79];
-  const T D80 = Dt[80];
-  const T D81 = Dt[81];
-  const T D82 = Dt[82];
-  const T D83 = Dt[83];
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
     acc[1] = fma(D4, mk, acc[1]);
@@ -2641,53 +1804,33 @@ __device__ __forceinline__ void m2l_m1_p6_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D12, mk, acc[6]);
     acc[7] = fma(D13, mk, acc[7]);
     acc[8] = fma(D14, mk, acc[8]);
-    acc[9] = fma(D15, mk, acc[9]);
+    acc[9] = fma(D19, mk, acc[9]);
     acc[10] = fma(D20, mk, acc[10]);
     acc[11] = fma(D21, mk, acc[11]);
     acc[12] = fma(D22, mk, acc[12]);
     acc[13] = fma(D23, mk, acc[13]);
-    acc[14] = fma(D24, mk, acc[14]);
-    acc[15] = fma(D25, mk, acc[15]);
-    acc[16] = fma(D26, mk, acc[16]);
-    acc[17] = fma(D27, mk, acc[17]);
-    acc[18] = fma(D28, mk, acc[18]);
-    acc[19] = fma(D29, mk, acc[19]);
+    acc[14] = fma(D25, mk, acc[14]);
+    acc[15] = fma(D26, mk, acc[15]);
+    acc[16] = fma(D31, mk, acc[16]);
+    acc[17] = fma(D32, mk, acc[17]);
+    acc[18] = fma(D33, mk, acc[18]);
+    acc[19] = fma(D34, mk, acc[19]);
     acc[20] = fma(D35, mk, acc[20]);
-    acc[21] = fma(D36, mk, acc[21]);
-    acc[22] = fma(D37, mk, acc[22]);
-    acc[23] = fma(D38, mk, acc[23]);
-    acc[24] = fma(D39, mk, acc[24]);
-    acc[25] = fma(D40, mk, acc[25]);
-    acc[26] = fma(D41, mk, acc[26]);
-    acc[27] = fma(D42, mk, acc[27]);
-    acc[28] = fma(D43, mk, acc[28]);
-    acc[29] = fma(D44, mk, acc[29]);
-    acc[30] = fma(D45, mk, acc[30]);
-    acc[31] = fma(D46, mk, acc[31]);
-    acc[32] = fma(D47, mk, acc[32]);
-    acc[33] = fma(D48, mk, acc[33]);
-    acc[34] = fma(D49, mk, acc[34]);
-    acc[35] = fma(D56, mk, acc[35]);
-    acc[36] = fma(D57, mk, acc[36]);
-    acc[37] = fma(D58, mk, acc[37]);
-    acc[38] = fma(D59, mk, acc[38]);
-    acc[39] = fma(D60, mk, acc[39]);
-    acc[40] = fma(D61, mk, acc[40]);
-    acc[41] = fma(D62, mk, acc[41]);
-    acc[42] = fma(D63, mk, acc[42]);
-    acc[43] = fma(D64, mk, acc[43]);
-    acc[44] = fma(D65, mk, acc[44]);
-    acc[45] = fma(D66, mk, acc[45]);
-    acc[46] = fma(D67, mk, acc[46]);
-    acc[47] = fma(D68, mk, acc[47]);
-    acc[48] = fma(D69, mk, acc[48]);
-    acc[49] = fma(D70, mk, acc[49]);
-    acc[50] = fma(D71, mk, acc[50]);
-    acc[51] = fma(D72, mk, acc[51]);
-    acc[52] = fma(D73, mk, acc[52]);
-    acc[53] = fma(D74, mk, acc[53]);
-    acc[54] = fma(D75, mk, acc[54]);
-    acc[55] = fma(D76, mk, acc[55]);
+    acc[21] = fma(D37, mk, acc[21]);
+    acc[22] = fma(D38, mk, acc[22]);
+    acc[23] = fma(D40, mk, acc[23]);
+    acc[24] = fma(D41, mk, acc[24]);
+    acc[25] = fma(D46, mk, acc[25]);
+    acc[26] = fma(D47, mk, acc[26]);
+    acc[27] = fma(D48, mk, acc[27]);
+    acc[28] = fma(D49, mk, acc[28]);
+    acc[29] = fma(D50, mk, acc[29]);
+    acc[30] = fma(D52, mk, acc[30]);
+    acc[31] = fma(D53, mk, acc[31]);
+    acc[32] = fma(D55, mk, acc[32]);
+    acc[33] = fma(D56, mk, acc[33]);
+    acc[34] = fma(D58, mk, acc[34]);
+    acc[35] = fma(D59, mk, acc[35]);
   }
   { const T mk = Mb[1];
     acc[0] = fma(D2, mk, acc[0]);
@@ -2699,53 +1842,33 @@ __device__ __forceinline__ void m2l_m1_p6_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D14, mk, acc[6]);
     acc[7] = fma(D16, mk, acc[7]);
     acc[8] = fma(D17, mk, acc[8]);
-    acc[9] = fma(D18, mk, acc[9]);
-    acc[10] = fma(D21, mk, acc[10]);
+    acc[9] = fma(D20, mk, acc[9]);
+    acc[10] = fma(D22, mk, acc[10]);
     acc[11] = fma(D23, mk, acc[11]);
-    acc[12] = fma(D24, mk, acc[12]);
+    acc[12] = fma(D25, mk, acc[12]);
     acc[13] = fma(D26, mk, acc[13]);
-    acc[14] = fma(D27, mk, acc[14]);
-    acc[15] = fma(D28, mk, acc[15]);
-    acc[16] = fma(D30, mk, acc[16]);
-    acc[17] = fma(D31, mk, acc[17]);
-    acc[18] = fma(D32, mk, acc[18]);
-    acc[19] = fma(D33, mk, acc[19]);
-    acc[20] = fma(D36, mk, acc[20]);
-    acc[21] = fma(D38, mk, acc[21]);
-    acc[22] = fma(D39, mk, acc[22]);
-    acc[23] = fma(D41, mk, acc[23]);
-    acc[24] = fma(D42, mk, acc[24]);
-    acc[25] = fma(D43, mk, acc[25]);
-    acc[26] = fma(D45, mk, acc[26]);
-    acc[27] = fma(D46, mk, acc[27]);
-    acc[28] = fma(D47, mk, acc[28]);
-    acc[29] = fma(D48, mk, acc[29]);
-    acc[30] = fma(D50, mk, acc[30]);
-    acc[31] = fma(D51, mk, acc[31]);
-    acc[32] = fma(D52, mk, acc[32]);
-    acc[33] = fma(D53, mk, acc[33]);
-    acc[34] = fma(D54, mk, acc[34]);
-    acc[35] = fma(D57, mk, acc[35]);
-    acc[36] = fma(D59, mk, acc[36]);
-    acc[37] = fma(D60, mk, acc[37]);
-    acc[38] = fma(D62, mk, acc[38]);
-    acc[39] = fma(D63, mk, acc[39]);
-    acc[40] = fma(D64, mk, acc[40]);
-    acc[41] = fma(D66, mk, acc[41]);
-    acc[42] = fma(D67, mk, acc[42]);
-    acc[43] = fma(D68, mk, acc[43]);
-    acc[44] = fma(D69, mk, acc[44]);
-    acc[45] = fma(D71, mk, acc[45]);
-    acc[46] = fma(D72, mk, acc[46]);
-    acc[47] = fma(D73, mk, acc[47]);
-    acc[48] = fma(D74, mk, acc[48]);
-    acc[49] = fma(D75, mk, acc[49]);
-    acc[50] = fma(D77, mk, acc[50]);
-    acc[51] = fma(D78, mk, acc[51]);
-    acc[52] = fma(D79, mk, acc[52]);
-    acc[53] = fma(D80, mk, acc[53]);
-    acc[54] = fma(D81, mk, acc[54]);
-    acc[55] = fma(D82, mk, acc[55]);
+    acc[14] = fma(D28, mk, acc[14]);
+    acc[15] = fma(D29, mk, acc[15]);
+    acc[16] = fma(D32, mk, acc[16]);
+    acc[17] = fma(D34, mk, acc[17]);
+    acc[18] = fma(D35, mk, acc[18]);
+    acc[19] = fma(D37, mk, acc[19]);
+    acc[20] = fma(D38, mk, acc[20]);
+    acc[21] = fma(D40, mk, acc[21]);
+    acc[22] = fma(D41, mk, acc[22]);
+    acc[23] = fma(D43, mk, acc[23]);
+    acc[24] = fma(D44, mk, acc[24]);
+    acc[25] = fma(D47, mk, acc[25]);
+    acc[26] = fma(D49, mk, acc[26]);
+    acc[27] = fma(D50, mk, acc[27]);
+    acc[28] = fma(D52, mk, acc[28]);
+    acc[29] = fma(D53, mk, acc[29]);
+    acc[30] = fma(D55, mk, acc[30]);
+    acc[31] = fma(D56, mk, acc[31]);
+    acc[32] = fma(D58, mk, acc[32]);
+    acc[33] = fma(D59, mk, acc[33]);
+    acc[34] = fma(D61, mk, acc[34]);
+    acc[35] = fma(D62, mk, acc[35]);
   }
   { const T mk = Mb[2];
     acc[0] = fma(D3, mk, acc[0]);
@@ -2757,887 +1880,610 @@ __device__ __forceinline__ void m2l_m1_p6_pre(const T* __restrict__ Dt, const T*
     acc[6] = fma(D15, mk, acc[6]);
     acc[7] = fma(D17, mk, acc[7]);
     acc[8] = fma(D18, mk, acc[8]);
-    acc[9] = fma(D19, mk, acc[9]);
-    acc[10] = fma(D22, mk, acc[10]);
+    acc[9] = fma(D21, mk, acc[9]);
+    acc[10] = fma(D23, mk, acc[10]);
     acc[11] = fma(D24, mk, acc[11]);
-    acc[12] = fma(D25, mk, acc[12]);
+    acc[12] = fma(D26, mk, acc[12]);
     acc[13] = fma(D27, mk, acc[13]);
-    acc[14] = fma(D28, mk, acc[14]);
-    acc[15] = fma(D29, mk, acc[15]);
-    acc[16] = fma(D31, mk, acc[16]);
-    acc[17] = fma(D32, mk, acc[17]);
-    acc[18] = fma(D33, mk, acc[18]);
-    acc[19] = fma(D34, mk, acc[19]);
-    acc[20] = fma(D37, mk, acc[20]);
-    acc[21] = fma(D39, mk, acc[21]);
-    acc[22] = fma(D40, mk, acc[22]);
-    acc[23] = fma(D42, mk, acc[23]);
-    acc[24] = fma(D43, mk, acc[24]);
-    acc[25] = fma(D44, mk, acc[25]);
-    acc[26] = fma(D46, mk, acc[26]);
-    acc[27] = fma(D47, mk, acc[27]);
-    acc[28] = fma(D48, mk, acc[28]);
-    acc[29] = fma(D49, mk, acc[29]);
-    acc[30] = fma(D51, mk, acc[30]);
-    acc[31] = fma(D52, mk, acc[31]);
-    acc[32] = fma(D53, mk, acc[32]);
-    acc[33] = fma(D54, mk, acc[33]);
-    acc[34] = fma(D55, mk, acc[34]);
-    acc[35] = fma(D58, mk, acc[35]);
-    acc[36] = fma(D60, mk, acc[36]);
-    acc[37] = fma(D61, mk, acc[37]);
-    acc[38] = fma(D63, mk, acc[38]);
-    acc[39] = fma(D64, mk, acc[39]);
-    acc[40] = fma(D65, mk, acc[40]);
-    acc[41] = fma(D67, mk, acc[41]);
-    acc[42] = fma(D68, mk, acc[42]);
-    acc[43] = fma(D69, mk, acc[43]);
-    acc[44] = fma(D70, mk, acc[44]);
-    acc[45] = fma(D72, mk, acc[45]);
-    acc[46] = fma(D73, mk, acc[46]);
-    acc[47] = fma(D74, mk, acc[47]);
-    acc[48] = fma(D75, mk, acc[48]);
-    acc[49] = fma(D76, mk, acc[49]);
-    acc[50] = fma(D78, mk, acc[50]);
-    acc[51] = fma(D79, mk, acc[51]);
-    acc[52] = fma(D80, mk, acc[52]);
-    acc[53] = fma(D81, mk, acc[53]);
-    acc[54] = fma(D82, mk, acc[54]);
-    acc[55] = fma(D83, mk, acc[55]);
+    acc[14] = fma(D29, mk, acc[14]);
+    acc[15] = fma(D30, mk, acc[15]);
+    acc[16] = fma(D33, mk, acc[16]);
+    acc[17] = fma(D35, mk, acc[17]);
+    acc[18] = fma(D36, mk, acc[18]);
+    acc[19] = fma(D38, mk, acc[19]);
+    acc[20] = fma(D39, mk, acc[20]);
+    acc[21] = fma(D41, mk, acc[21]);
+    acc[22] = fma(D42, mk, acc[22]);
+    acc[23] = fma(D44, mk, acc[23]);
+    acc[24] = fma(D45, mk, acc[24]);
+    acc[25] = fma(D48, mk, acc[25]);
+    acc[26] = fma(D50, mk, acc[26]);
+    acc[27] = fma(D51, mk, acc[27]);
+    acc[28] = fma(D53, mk, acc[28]);
+    acc[29] = fma(D54, mk, acc[29]);
+    acc[30] = fma(D56, mk, acc[30]);
+    acc[31] = fma(D57, mk, acc[31]);
+    acc[32] = fma(D59, mk, acc[32]);
+    acc[33] = fma(D60, mk, acc[33]);
+    acc[34] = fma(D62, mk, acc[34]);
+    acc[35] = fma(D63, mk, acc[35]);
   }
   { const T mk = Mb[3];
     acc[0] = fma(D4, mk, acc[0]);
     acc[1] = fma(D10, mk, acc[1]);
     acc[2] = fma(D11, mk, acc[2]);
     acc[3] = fma(D12, mk, acc[3]);
-    acc[4] = fma(D20, mk, acc[4]);
-    acc[5] = fma(D21, mk, acc[5]);
-    acc[6] = fma(D22, mk, acc[6]);
-    acc[7] = fma(D23, mk, acc[7]);
-    acc[8] = fma(D24, mk, acc[8]);
-    acc[9] = fma(D25, mk, acc[9]);
-    acc[10] = fma(D35, mk, acc[10]);
-    acc[11] = fma(D36, mk, acc[11]);
-    acc[12] = fma(D37, mk, acc[12]);
-    acc[13] = fma(D38, mk, acc[13]);
-    acc[14] = fma(D39, mk, acc[14]);
-    acc[15] = fma(D40, mk, acc[15]);
-    acc[16] = fma(D41, mk, acc[16]);
-    acc[17] = fma(D42, mk, acc[17]);
-    acc[18] = fma(D43, mk, acc[18]);
-    acc[19] = fma(D44, mk, acc[19]);
-    acc[20] = fma(D56, mk, acc[20]);
-    acc[21] = fma(D57, mk, acc[21]);
-    acc[22] = fma(D58, mk, acc[22]);
-    acc[23] = fma(D59, mk, acc[23]);
-    acc[24] = fma(D60, mk, acc[24]);
-    acc[25] = fma(D61, mk, acc[25]);
-    acc[26] = fma(D62, mk, acc[26]);
-    acc[27] = fma(D63, mk, acc[27]);
-    acc[28] = fma(D64, mk, acc[28]);
-    acc[29] = fma(D65, mk, acc[29]);
-    acc[30] = fma(D66, mk, acc[30]);
-    acc[31] = fma(D67, mk, acc[31]);
-    acc[32] = fma(D68, mk, acc[32]);
-    acc[33] = fma(D69, mk, acc[33]);
-    acc[34] = fma(D70, mk, acc[34]);
+    acc[4] = fma(D19, mk, acc[4]);
+    acc[5] = fma(D20, mk, acc[5]);
+    acc[6] = fma(D21, mk, acc[6]);
+    acc[7] = fma(D22, mk, acc[7]);
+    acc[8] = fma(D23, mk, acc[8]);
+    acc[9] = fma(D31, mk, acc[9]);
+    acc[10] = fma(D32, mk, acc[10]);
+    acc[11] = fma(D33, mk, acc[11]);
+    acc[12] = fma(D34, mk, acc[12]);
+    acc[13] = fma(D35, mk, acc[13]);
+    acc[14] = fma(D37, mk, acc[14]);
+    acc[15] = fma(D38, mk, acc[15]);
+    acc[16] = fma(D46, mk, acc[16]);
+    acc[17] = fma(D47, mk, acc[17]);
+    acc[18] = fma(D48, mk, acc[18]);
+    acc[19] = fma(D49, mk, acc[19]);
+    acc[20] = fma(D50, mk, acc[20]);
+    acc[21] = fma(D52, mk, acc[21]);
+    acc[22] = fma(D53, mk, acc[22]);
+    acc[23] = fma(D55, mk, acc[23]);
+    acc[24] = fma(D56, mk, acc[24]);
   }
   { const T mk = Mb[4];
     acc[0] = fma(D5, mk, acc[0]);
     acc[1] = fma(D11, mk, acc[1]);
     acc[2] = fma(D13, mk, acc[2]);
     acc[3] = fma(D14, mk, acc[3]);
-    acc[4] = fma(D21, mk, acc[4]);
-    acc[5] = fma(D23, mk, acc[5]);
-    acc[6] = fma(D24, mk, acc[6]);
-    acc[7] = fma(D26, mk, acc[7]);
-    acc[8] = fma(D27, mk, acc[8]);
-    acc[9] = fma(D28, mk, acc[9]);
-    acc[10] = fma(D36, mk, acc[10]);
-    acc[11] = fma(D38, mk, acc[11]);
-    acc[12] = fma(D39, mk, acc[12]);
-    acc[13] = fma(D41, mk, acc[13]);
-    acc[14] = fma(D42, mk, acc[14]);
-    acc[15] = fma(D43, mk, acc[15]);
-    acc[16] = fma(D45, mk, acc[16]);
-    acc[17] = fma(D46, mk, acc[17]);
-    acc[18] = fma(D47, mk, acc[18]);
-    acc[19] = fma(D48, mk, acc[19]);
-    acc[20] = fma(D57, mk, acc[20]);
-    acc[21] = fma(D59, mk, acc[21]);
-    acc[22] = fma(D60, mk, acc[22]);
-    acc[23] = fma(D62, mk, acc[23]);
-    acc[24] = fma(D63, mk, acc[24]);
-    acc[25] = fma(D64, mk, acc[25]);
-    acc[26] = fma(D66, mk, acc[26]);
-    acc[27] = fma(D67, mk, acc[27]);
-    acc[28] = fma(D68, mk, acc[28]);
-    acc[29] = fma(D69, mk, acc[29]);
-    acc[30] = fma(D71, mk, acc[30]);
-    acc[31] = fma(D72, mk, acc[31]);
-    acc[32] = fma(D73, mk, acc[32]);
-    acc[33] = fma(D74, mk, acc[33]);
-    acc[34] = fma(D75, mk, acc[34]);
+    acc[4] = fma(D20, mk, acc[4]);
+    acc[5] = fma(D22, mk, acc[5]);
+    acc[6] = fma(D23, mk, acc[6]);
+    acc[7] = fma(D25, mk, acc[7]);
+    acc[8] = fma(D26, mk, acc[8]);
+    acc[9] = fma(D32, mk, acc[9]);
+    acc[10] = fma(D34, mk, acc[10]);
+    acc[11] = fma(D35, mk, acc[11]);
+    acc[12] = fma(D37, mk, acc[12]);
+    acc[13] = fma(D38, mk, acc[13]);
+    acc[14] = fma(D40, mk, acc[14]);
+    acc[15] = fma(D41, mk, acc[15]);
+    acc[16] = fma(D47, mk, acc[16]);
+    acc[17] = fma(D49, mk, acc[17]);
+    acc[18] = fma(D50, mk, acc[18]);
+    acc[19] = fma(D52, mk, acc[19]);
+    acc[20] = fma(D53, mk, acc[20]);
+    acc[21] = fma(D55, mk, acc[21]);
+    acc[22] = fma(D56, mk, acc[22]);
+    acc[23] = fma(D58, mk, acc[23]);
+    acc[24] = fma(D59, mk, acc[24]);
   }
   { const T mk = Mb[5];
     acc[0] = fma(D6, mk, acc[0]);
     acc[1] = fma(D12, mk, acc[1]);
     acc[2] = fma(D14, mk, acc[2]);
     acc[3] = fma(D15, mk, acc[3]);
-    acc[4] = fma(D22, mk, acc[4]);
-    acc[5] = fma(D24, mk, acc[5]);
-    acc[6] = fma(D25, mk, acc[6]);
-    acc[7] = fma(D27, mk, acc[7]);
-    acc[8] = fma(D28, mk, acc[8]);
-    acc[9] = fma(D29, mk, acc[9]);
-    acc[10] = fma(D37, mk, acc[10]);
-    acc[11] = fma(D39, mk, acc[11]);
-    acc[12] = fma(D40, mk, acc[12]);
-    acc[13] = fma(D42, mk, acc[13]);
-    acc[14] = fma(D43, mk, acc[14]);
-    acc[15] = fma(D44, mk, acc[15]);
-    acc[16] = fma(D46, mk, acc[16]);
-    acc[17] = fma(D47, mk, acc[17]);
-    acc[18] = fma(D48, mk, acc[18]);
-    acc[19] = fma(D49, mk, acc[19]);
-    acc[20] = fma(D58, mk, acc[20]);
-    acc[21] = fma(D60, mk, acc[21]);
-    acc[22] = fma(D61, mk, acc[22]);
-    acc[23] = fma(D63, mk, acc[23]);
-    acc[24] = fma(D64, mk, acc[24]);
-    acc[25] = fma(D65, mk, acc[25]);
-    acc[26] = fma(D67, mk, acc[26]);
-    acc[27] = fma(D68, mk, acc[27]);
-    acc[28] = fma(D69, mk, acc[28]);
-    acc[29] = fma(D70, mk, acc[29]);
-    acc[30] = fma(D72, mk, acc[30]);
-    acc[31] = fma(D73, mk, acc[31]);
-    acc[32] = fma(D74, mk, acc[32]);
-    acc[33] = fma(D75, mk, acc[33]);
-    acc[34] = fma(D76, mk, acc[34]);
+    acc[4] = fma(D21, mk, acc[4]);
+    acc[5] = fma(D23, mk, acc[5]);
+    acc[6] = fma(D24, mk, acc[6]);
+    acc[7] = fma(D26, mk, acc[7]);
+    acc[8] = fma(D27, mk, acc[8]);
+    acc[9] = fma(D33, mk, acc[9]);
+    acc[10] = fma(D35, mk, acc[10]);
+    acc[11] = fma(D36, mk, acc[11]);
+    acc[12] = fma(D38, mk, acc[12]);
+    acc[13] = fma(D39, mk, acc[13]);
+    acc[14] = fma(D41, mk, acc[14]);
+    acc[15] = fma(D42, mk, acc[15]);
+    acc[16] = fma(D48, mk, acc[16]);
+    acc[17] = fma(D50, mk, acc[17]);
+    acc[18] = fma(D51, mk, acc[18]);
+    acc[19] = fma(D53, mk, acc[19]);
+    acc[20] = fma(D54, mk, acc[20]);
+    acc[21] = fma(D56, mk, acc[21]);
+    acc[22] = fma(D57, mk, acc[22]);
+    acc[23] = fma(D59, mk, acc[23]);
+    acc[24] = fma(D60, mk, acc[24]);
   }
   { const T mk = Mb[6];
     acc[0] = fma(D7, mk, acc[0]);
     acc[1] = fma(D13, mk, acc[1]);
     acc[2] = fma(D16, mk, acc[2]);
     acc[3] = fma(D17, mk, acc[3]);
-    acc[4] = fma(D23, mk, acc[4]);
-    acc[5] = fma(D26, mk, acc[5]);
-    acc[6] = fma(D27, mk, acc[6]);
-    acc[7] = fma(D30, mk, acc[7]);
-    acc[8] = fma(D31, mk, acc[8]);
-    acc[9] = fma(D32, mk, acc[9]);
-    acc[10] = fma(D38, mk, acc[10]);
-    acc[11] = fma(D41, mk, acc[11]);
-    acc[12] = fma(D42, mk, acc[12]);
-    acc[13] = fma(D45, mk, acc[13]);
-    acc[14] = fma(D46, mk, acc[14]);
-    acc[15] = fma(D47, mk, acc[15]);
-    acc[16] = fma(D50, mk, acc[16]);
-    acc[17] = fma(D51, mk, acc[17]);
-    acc[18] = fma(D52, mk, acc[18]);
-    acc[19] = fma(D53, mk, acc[19]);
-    acc[20] = fma(D59, mk, acc[20]);
-    acc[21] = fma(D62, mk, acc[21]);
-    acc[22] = fma(D63, mk, acc[22]);
-    acc[23] = fma(D66, mk, acc[23]);
-    acc[24] = fma(D67, mk, acc[24]);
-    acc[25] = fma(D68, mk, acc[25]);
-    acc[26] = fma(D71, mk, acc[26]);
-    acc[27] = fma(D72, mk, acc[27]);
-    acc[28] = fma(D73, mk, acc[28]);
-    acc[29] = fma(D74, mk, acc[29]);
-    acc[30] = fma(D77, mk, acc[30]);
-    acc[31] = fma(D78, mk, acc[31]);
-    acc[32] = fma(D79, mk, acc[32]);
-    acc[33] = fma(D80, mk, acc[33]);
-    acc[34] = fma(D81, mk, acc[34]);
+    acc[4] = fma(D22, mk, acc[4]);
+    acc[5] = fma(D25, mk, acc[5]);
+    acc[6] = fma(D26, mk, acc[6]);
+    acc[7] = fma(D28, mk, acc[7]);
+    acc[8] = fma(D29, mk, acc[8]);
+    acc[9] = fma(D34, mk, acc[9]);
+    acc[10] = fma(D37, mk, acc[10]);
+    acc[11] = fma(D38, mk, acc[11]);
+    acc[12] = fma(D40, mk, acc[12]);
+    acc[13] = fma(D41, mk, acc[13]);
+    acc[14] = fma(D43, mk, acc[14]);
+    acc[15] = fma(D44, mk, acc[15]);
+    acc[16] = fma(D49, mk, acc[16]);
+    acc[17] = fma(D52, mk, acc[17]);
+    acc[18] = fma(D53, mk, acc[18]);
+    acc[19] = fma(D55, mk, acc[19]);
+    acc[20] = fma(D56, mk, acc[20]);
+    acc[21] = fma(D58, mk, acc[21]);
+    acc[22] = fma(D59, mk, acc[22]);
+    acc[23] = fma(D61, mk, acc[23]);
+    acc[24] = fma(D62, mk, acc[24]);
   }
   { const T mk = Mb[7];
     acc[0] = fma(D8, mk, acc[0]);
     acc[1] = fma(D14, mk, acc[1]);
     acc[2] = fma(D17, mk, acc[2]);
     acc[3] = fma(D18, mk, acc[3]);
-    acc[4] = fma(D24, mk, acc[4]);
-    acc[5] = fma(D27, mk, acc[5]);
-    acc[6] = fma(D28, mk, acc[6]);
-    acc[7] = fma(D31, mk, acc[7]);
-    acc[8] = fma(D32, mk, acc[8]);
-    acc[9] = fma(D33, mk, acc[9]);
-    acc[10] = fma(D39, mk, acc[10]);
-    acc[11] = fma(D42, mk, acc[11]);
-    acc[12] = fma(D43, mk, acc[12]);
-    acc[13] = fma(D46, mk, acc[13]);
-    acc[14] = fma(D47, mk, acc[14]);
-    acc[15] = fma(D48, mk, acc[15]);
-    acc[16] = fma(D51, mk, acc[16]);
-    acc[17] = fma(D52, mk, acc[17]);
-    acc[18] = fma(D53, mk, acc[18]);
-    acc[19] = fma(D54, mk, acc[19]);
-    acc[20] = fma(D60, mk, acc[20]);
-    acc[21] = fma(D63, mk, acc[21]);
-    acc[22] = fma(D64, mk, acc[22]);
-    acc[23] = fma(D67, mk, acc[23]);
-    acc[24] = fma(D68, mk, acc[24]);
-    acc[25] = fma(D69, mk, acc[25]);
-    acc[26] = fma(D72, mk, acc[26]);
-    acc[27] = fma(D73, mk, acc[27]);
-    acc[28] = fma(D74, mk, acc[28]);
-    acc[29] = fma(D75, mk, acc[29]);
-    acc[30] = fma(D78, mk, acc[30]);
-    acc[31] = fma(D79, mk, acc[31]);
-    acc[32] = fma(D80, mk, acc[32]);
-    acc[33] = fma(D81, mk, acc[33]);
-    acc[34] = fma(D82, mk, acc[34]);
-  }
-  { const T mk = Mb[8];
-    acc[0] = fma(D9, mk, acc[0]);
-    acc[1] = fma(D15, mk, acc[1]);
-    acc[2] = fma(D18, mk, acc[2]);
-    acc[3] = fma(D19, mk, acc[3]);
-    acc[4] = fma(D25, mk, acc[4]);
-    acc[5] = fma(D28, mk, acc[5]);
-    acc[6] = fma(D29, mk, acc[6]);
-    acc[7] = fma(D32, mk, acc[7]);
-    acc[8] = fma(D33, mk, acc[8]);
-    acc[9] = fma(D34, mk, acc[9]);
-    acc[10] = fma(D40, mk, acc[10]);
-    acc[11] = fma(D43, mk, acc[11]);
-    acc[12] = fma(D44, mk, acc[12]);
-    acc[13] = fma(D47, mk, acc[13]);
-    acc[14] = fma(D48, mk, acc[14]);
-    acc[15] = fma(D49, mk, acc[15]);
-    acc[16] = fma(D52, mk, acc[16]);
+    acc[4] = fma(D23, mk, acc[4]);
+    acc[5] = fma(D26, mk, acc[5]);
+    acc[6] = fma(D27, mk, acc[6]);
+    acc[7] = fma(D29, mk, acc[7]);
+    acc[8] = fma(D30, mk, acc[8]);
+    acc[9] = fma(D35, mk, acc[9]);
+    acc[10] = fma(D38, mk, acc[10]);
+    acc[11] = fma(D39, mk, acc[11]);
+    acc[12] = fma(D41, mk, acc[12]);
+    acc[13] = fma(D42, mk, acc[13]);
+    acc[14] = fma(D44, mk, acc[14]);
+    acc[15] = fma(D45, mk, acc[15]);
+    acc[16] = fma(D50, mk, acc[16]);
     acc[17] = fma(D53, mk, acc[17]);
     acc[18] = fma(D54, mk, acc[18]);
-    acc[19] = fma(D55, mk, acc[19]);
-    acc[20] = fma(D61, mk, acc[20]);
-    acc[21] = fma(D64, mk, acc[21]);
-    acc[22] = fma(D65, mk, acc[22]);
-    acc[23] = fma(D68, mk, acc[23]);
-    acc[24] = fma(D69, mk, acc[24]);
-    acc[25] = fma(D70, mk, acc[25]);
-    acc[26] = fma(D73, mk, acc[26]);
-    acc[27] = fma(D74, mk, acc[27]);
-    acc[28] = fma(D75, mk, acc[28]);
-    acc[29] = fma(D76, mk, acc[29]);
-    acc[30] = fma(D79, mk, acc[30]);
-    acc[31] = fma(D80, mk, acc[31]);
-    acc[32] = fma(D81, mk, acc[32]);
-    acc[33] = fma(D82, mk, acc[33]);
-    acc[34] = fma(D83, mk, acc[34]);
+    acc[19] = fma(D56, mk, acc[19]);
+    acc[20] = fma(D57, mk, acc[20]);
+    acc[21] = fma(D59, mk, acc[21]);
+    acc[22] = fma(D60, mk, acc[22]);
+    acc[23] = fma(D62, mk, acc[23]);
+    acc[24] = fma(D63, mk, acc[24]);
+  }
+  { const T mk = Mb[8];
+    acc[0] = fma(D10, mk, acc[0]);
+    acc[1] = fma(D19, mk, acc[1]);
+    acc[2] = fma(D20, mk, acc[2]);
+    acc[3] = fma(D21, mk, acc[3]);
+    acc[4] = fma(D31, mk, acc[4]);
+    acc[5] = fma(D32, mk, acc[5]);
+    acc[6] = fma(D33, mk, acc[6]);
+    acc[7] = fma(D34, mk, acc[7]);
+    acc[8] = fma(D35, mk, acc[8]);
+    acc[9] = fma(D46, mk, acc[9]);
+    acc[10] = fma(D47, mk, acc[10]);
+    acc[11] = fma(D48, mk, acc[11]);
+    acc[12] = fma(D49, mk, acc[12]);
+    acc[13] = fma(D50, mk, acc[13]);
+    acc[14] = fma(D52, mk, acc[14]);
+    acc[15] = fma(D53, mk, acc[15]);
   }
   { const T mk = Mb[9];
-    acc[0] = fma(D10, mk, acc[0]);
+    acc[0] = fma(D11, mk, acc[0]);
     acc[1] = fma(D20, mk, acc[1]);
-    acc[2] = fma(D21, mk, acc[2]);
-    acc[3] = fma(D22, mk, acc[3]);
-    acc[4] = fma(D35, mk, acc[4]);
-    acc[5] = fma(D36, mk, acc[5]);
-    acc[6] = fma(D37, mk, acc[6]);
-    acc[7] = fma(D38, mk, acc[7]);
-    acc[8] = fma(D39, mk, acc[8]);
-    acc[9] = fma(D40, mk, acc[9]);
-    acc[10] = fma(D56, mk, acc[10]);
-    acc[11] = fma(D57, mk, acc[11]);
-    acc[12] = fma(D58, mk, acc[12]);
-    acc[13] = fma(D59, mk, acc[13]);
-    acc[14] = fma(D60, mk, acc[14]);
-    acc[15] = fma(D61, mk, acc[15]);
-    acc[16] = fma(D62, mk, acc[16]);
-    acc[17] = fma(D63, mk, acc[17]);
-    acc[18] = fma(D64, mk, acc[18]);
-    acc[19] = fma(D65, mk, acc[19]);
+    acc[2] = fma(D22, mk, acc[2]);
+    acc[3] = fma(D23, mk, acc[3]);
+    acc[4] = fma(D32, mk, acc[4]);
+    acc[5] = fma(D34, mk, acc[5]);
+    acc[6] = fma(D35, mk, acc[6]);
+    acc[7] = fma(D37, mk, acc[7]);
+    acc[8] = fma(D38, mk, acc[8]);
+    acc[9] = fma(D47, mk, acc[9]);
+    acc[10] = fma(D49, mk, acc[10]);
+    acc[11] = fma(D50, mk, acc[11]);
+    acc[12] = fma(D52, mk, acc[12]);
+    acc[13] = fma(D53, mk, acc[13]);
+    acc[14] = fma(D55, mk, acc[14]);
+    acc[15] = fma(D56, mk, acc[15]);
   }
   { const T mk = Mb[10];
-    acc[0] = fma(D11, mk, acc[0]);
+    acc[0] = fma(D12, mk, acc[0]);
     acc[1] = fma(D21, mk, acc[1]);
     acc[2] = fma(D23, mk, acc[2]);
     acc[3] = fma(D24, mk, acc[3]);
-    acc[4] = fma(D36, mk, acc[4]);
+    acc[4] = fma(D33, mk, acc[4]);
+    acc[5] = fma(D35, mk, acc[5]);
+    acc[6] = fma(D36, mk, acc[6]);
+    acc[7] = fma(D38, mk, acc[7]);
+    acc[8] = fma(D39, mk, acc[8]);
+    acc[9] = fma(D48, mk, acc[9]);
+    acc[10] = fma(D50, mk, acc[10]);
+    acc[11] = fma(D51, mk, acc[11]);
+    acc[12] = fma(D53, mk, acc[12]);
+    acc[13] = fma(D54, mk, acc[13]);
+    acc[14] = fma(D56, mk, acc[14]);
+    acc[15] = fma(D57, mk, acc[15]);
+  }
+  { const T mk = Mb[11];
+    acc[0] = fma(D13, mk, acc[0]);
+    acc[1] = fma(D22, mk, acc[1]);
+    acc[2] = fma(D25, mk, acc[2]);
+    acc[3] = fma(D26, mk, acc[3]);
+    acc[4] = fma(D34, mk, acc[4]);
+    acc[5] = fma(D37, mk, acc[5]);
+    acc[6] = fma(D38, mk, acc[6]);
+    acc[7] = fma(D40, mk, acc[7]);
+    acc[8] = fma(D41, mk, acc[8]);
+    acc[9] = fma(D49, mk, acc[9]);
+    acc[10] = fma(D52, mk, acc[10]);
+    acc[11] = fma(D53, mk, acc[11]);
+    acc[12] = fma(D55, mk, acc[12]);
+    acc[13] = fma(D56, mk, acc[13]);
+    acc[14] = fma(D58, mk, acc[14]);
+    acc[15] = fma(D59, mk, acc[15]);
+  }
+  { const T mk = Mb[12];
+    acc[0] = fma(D14, mk, acc[0]);
+    acc[1] = fma(D23, mk, acc[1]);
+    acc[2] = fma(D26, mk, acc[2]);
+    acc[3] = fma(D27, mk, acc[3]);
+    acc[4] = fma(D35, mk, acc[4]);
     acc[5] = fma(D38, mk, acc[5]);
     acc[6] = fma(D39, mk, acc[6]);
     acc[7] = fma(D41, mk, acc[7]);
     acc[8] = fma(D42, mk, acc[8]);
-    acc[9] = fma(D43, mk, acc[9]);
-    acc[10] = fma(D57, mk, acc[10]);
-    acc[11] = fma(D59, mk, acc[11]);
-    acc[12] = fma(D60, mk, acc[12]);
-    acc[13] = fma(D62, mk, acc[13]);
-    acc[14] = fma(D63, mk, acc[14]);
-    acc[15] = fma(D64, mk, acc[15]);
-    acc[16] = fma(D66, mk, acc[16]);
-    acc[17] = fma(D67, mk, acc[17]);
-    acc[18] = fma(D68, mk, acc[18]);
-    acc[19] = fma(D69, mk, acc[19]);
-  }
-  { const T mk = Mb[11];
-    acc[0] = fma(D12, mk, acc[0]);
-    acc[1] = fma(D22, mk, acc[1]);
-    acc[2] = fma(D24, mk, acc[2]);
-    acc[3] = fma(D25, mk, acc[3]);
-    acc[4] = fma(D37, mk, acc[4]);
-    acc[5] = fma(D39, mk, acc[5]);
-    acc[6] = fma(D40, mk, acc[6]);
-    acc[7] = fma(D42, mk, acc[7]);
-    acc[8] = fma(D43, mk, acc[8]);
-    acc[9] = fma(D44, mk, acc[9]);
-    acc[10] = fma(D58, mk, acc[10]);
-    acc[11] = fma(D60, mk, acc[11]);
-    acc[12] = fma(D61, mk, acc[12]);
-    acc[13] = fma(D63, mk, acc[13]);
-    acc[14] = fma(D64, mk, acc[14]);
-    acc[15] = fma(D65, mk, acc[15]);
-    acc[16] = fma(D67, mk, acc[16]);
-    acc[17] = fma(D68, mk, acc[17]);
-    acc[18] = fma(D69, mk, acc[18]);
-    acc[19] = fma(D70, mk, acc[19]);
-  }
-  { const T mk = Mb[12];
-    acc[0] = fma(D13, mk, acc[0]);
-    acc[1] = fma(D23, mk, acc[1]);
-    acc[2] = fma(D26, mk, acc[2]);
-    acc[3] = fma(D27, mk, acc[3]);
-    acc[4] = fma(D38, mk, acc[4]);
-    acc[5] = fma(D41, mk, acc[5]);
-    acc[6] = fma(D42, mk, acc[6]);
-    acc[7] = fma(D45, mk, acc[7]);
-    acc[8] = fma(D46, mk, acc[8]);
-    acc[9] = fma(D47, mk, acc[9]);
-    acc[10] = fma(D59, mk, acc[10]);
-    acc[11] = fma(D62, mk, acc[11]);
-    acc[12] = fma(D63, mk, acc[12]);
-    acc[13] = fma(D66, mk, acc[13]);
-    acc[14] = fma(D67, mk, acc[14]);
-    acc[15] = fma(D68, mk, acc[15]);
-    acc[16] = fma(D71, mk, acc[16]);
-    acc[17] = fma(D72, mk, acc[17]);
-    acc[18] = fma(D73, mk, acc[18]);
-    acc[19] = fma(D74, mk, acc[19]);
+    acc[9] = fma(D50, mk, acc[9]);
+    acc[10] = fma(D53, mk, acc[10]);
+    acc[11] = fma(D54, mk, acc[11]);
+    acc[12] = fma(D56, mk, acc[12]);
+    acc[13] = fma(D57, mk, acc[13]);
+    acc[14] = fma(D59, mk, acc[14]);
+    acc[15] = fma(D60, mk, acc[15]);
   }
   { const T mk = Mb[13];
-    acc[0] = fma(D14, mk, acc[0]);
-    acc[1] = fma(D24, mk, acc[1]);
-    acc[2] = fma(D27, mk, acc[2]);
-    acc[3] = fma(D28, mk, acc[3]);
-    acc[4] = fma(D39, mk, acc[4]);
-    acc[5] = fma(D42, mk, acc[5]);
-    acc[6] = fma(D43, mk, acc[6]);
-    acc[7] = fma(D46, mk, acc[7]);
-    acc[8] = fma(D47, mk, acc[8]);
-    acc[9] = fma(D48, mk, acc[9]);
-    acc[10] = fma(D60, mk, acc[10]);
-    acc[11] = fma(D63, mk, acc[11]);
-    acc[12] = fma(D64, mk, acc[12]);
-    acc[13] = fma(D67, mk, acc[13]);
-    acc[14] = fma(D68, mk, acc[14]);
-    acc[15] = fma(D69, mk, acc[15]);
-    acc[16] = fma(D72, mk, acc[16]);
-    acc[17] = fma(D73, mk, acc[17]);
-    acc[18] = fma(D74, mk, acc[18]);
-    acc[19] = fma(D75, mk, acc[19]);
-  }
-  { const T mk = Mb[14];
-    acc[0] = fma(D15, mk, acc[0]);
+    acc[0] = fma(D16, mk, acc[0]);
     acc[1] = fma(D25, mk, acc[1]);
     acc[2] = fma(D28, mk, acc[2]);
     acc[3] = fma(D29, mk, acc[3]);
-    acc[4] = fma(D40, mk, acc[4]);
-    acc[5] = fma(D43, mk, acc[5]);
-    acc[6] = fma(D44, mk, acc[6]);
-    acc[7] = fma(D47, mk, acc[7]);
-    acc[8] = fma(D48, mk, acc[8]);
-    acc[9] = fma(D49, mk, acc[9]);
-    acc[10] = fma(D61, mk, acc[10]);
-    acc[11] = fma(D64, mk, acc[11]);
-    acc[12] = fma(D65, mk, acc[12]);
-    acc[13] = fma(D68, mk, acc[13]);
-    acc[14] = fma(D69, mk, acc[14]);
-    acc[15] = fma(D70, mk, acc[15]);
-    acc[16] = fma(D73, mk, acc[16]);
-    acc[17] = fma(D74, mk, acc[17]);
-    acc[18] = fma(D75, mk, acc[18]);
-    acc[19] = fma(D76, mk, acc[19]);
+    acc[4] = fma(D37, mk, acc[4]);
+    acc[5] = fma(D40, mk, acc[5]);
+    acc[6] = fma(D41, mk, acc[6]);
+    acc[7] = fma(D43, mk, acc[7]);
+    acc[8] = fma(D44, mk, acc[8]);
+    acc[9] = fma(D52, mk, acc[9]);
+    acc[10] = fma(D55, mk, acc[10]);
+    acc[11] = fma(D56, mk, acc[11]);
+    acc[12] = fma(D58, mk, acc[12]);
+    acc[13] = fma(D59, mk, acc[13]);
+    acc[14] = fma(D61, mk, acc[14]);
+    acc[15] = fma(D62, mk, acc[15]);
+  }
+  { const T mk = Mb[14];
+    acc[0] = fma(D17, mk, acc[0]);
+    acc[1] = fma(D26, mk, acc[1]);
+    acc[2] = fma(D29, mk, acc[2]);
+    acc[3] = fma(D30, mk, acc[3]);
+    acc[4] = fma(D38, mk, acc[4]);
+    acc[5] = fma(D41, mk, acc[5]);
+    acc[6] = fma(D42, mk, acc[6]);
+    acc[7] = fma(D44, mk, acc[7]);
+    acc[8] = fma(D45, mk, acc[8]);
+    acc[9] = fma(D53, mk, acc[9]);
+    acc[10] = fma(D56, mk, acc[10]);
+    acc[11] = fma(D57, mk, acc[11]);
+    acc[12] = fma(D59, mk, acc[12]);
+    acc[13] = fma(D60, mk, acc[13]);
+    acc[14] = fma(D62, mk, acc[14]);
+    acc[15] = fma(D63, mk, acc[15]);
   }
   { const T mk = Mb[15];
-    acc[0] = fma(D16, mk, acc[0]);
-    acc[1] = fma(D26, mk, acc[1]);
-    acc[2] = fma(D30, mk, acc[2]);
-    acc[3] = fma(D31, mk, acc[3]);
-    acc[4] = fma(D41, mk, acc[4]);
-    acc[5] = fma(D45, mk, acc[5]);
-    acc[6] = fma(D46, mk, acc[6]);
-    acc[7] = fma(D50, mk, acc[7]);
-    acc[8] = fma(D51, mk, acc[8]);
-    acc[9] = fma(D52, mk, acc[9]);
-    acc[10] = fma(D62, mk, acc[10]);
-    acc[11] = fma(D66, mk, acc[11]);
-    acc[12] = fma(D67, mk, acc[12]);
-    acc[13] = fma(D71, mk, acc[13]);
-    acc[14] = fma(D72, mk, acc[14]);
-    acc[15] = fma(D73, mk, acc[15]);
-    acc[16] = fma(D77, mk, acc[16]);
-    acc[17] = fma(D78, mk, acc[17]);
-    acc[18] = fma(D79, mk, acc[18]);
-    acc[19] = fma(D80, mk, acc[19]);
-  }
-  { const T mk = Mb[16];
-    acc[0] = fma(D17, mk, acc[0]);
-    acc[1] = fma(D27, mk, acc[1]);
-    acc[2] = fma(D31, mk, acc[2]);
-    acc[3] = fma(D32, mk, acc[3]);
-    acc[4] = fma(D42, mk, acc[4]);
-    acc[5] = fma(D46, mk, acc[5]);
-    acc[6] = fma(D47, mk, acc[6]);
-    acc[7] = fma(D51, mk, acc[7]);
-    acc[8] = fma(D52, mk, acc[8]);
-    acc[9] = fma(D53, mk, acc[9]);
-    acc[10] = fma(D63, mk, acc[10]);
-    acc[11] = fma(D67, mk, acc[11]);
-    acc[12] = fma(D68, mk, acc[12]);
-    acc[13] = fma(D72, mk, acc[13]);
-    acc[14] = fma(D73, mk, acc[14]);
-    acc[15] = fma(D74, mk, acc[15]);
-    acc[16] = fma(D78, mk, acc[16]);
-    acc[17] = fma(D79, mk, acc[17]);
-    acc[18] = fma(D80, mk, acc[18]);
-    acc[19] = fma(D81, mk, acc[19]);
-  }
-  { const T mk = Mb[17];
-    acc[0] = fma(D18, mk, acc[0]);
-    acc[1] = fma(D28, mk, acc[1]);
+    acc[0] = fma(D19, mk, acc[0]);
+    acc[1] = fma(D31, mk, acc[1]);
     acc[2] = fma(D32, mk, acc[2]);
     acc[3] = fma(D33, mk, acc[3]);
-    acc[4] = fma(D43, mk, acc[4]);
+    acc[4] = fma(D46, mk, acc[4]);
     acc[5] = fma(D47, mk, acc[5]);
     acc[6] = fma(D48, mk, acc[6]);
+    acc[7] = fma(D49, mk, acc[7]);
+    acc[8] = fma(D50, mk, acc[8]);
+  }
+  { const T mk = Mb[16];
+    acc[0] = fma(D20, mk, acc[0]);
+    acc[1] = fma(D32, mk, acc[1]);
+    acc[2] = fma(D34, mk, acc[2]);
+    acc[3] = fma(D35, mk, acc[3]);
+    acc[4] = fma(D47, mk, acc[4]);
+    acc[5] = fma(D49, mk, acc[5]);
+    acc[6] = fma(D50, mk, acc[6]);
     acc[7] = fma(D52, mk, acc[7]);
     acc[8] = fma(D53, mk, acc[8]);
-    acc[9] = fma(D54, mk, acc[9]);
-    acc[10] = fma(D64, mk, acc[10]);
-    acc[11] = fma(D68, mk, acc[11]);
-    acc[12] = fma(D69, mk, acc[12]);
-    acc[13] = fma(D73, mk, acc[13]);
-    acc[14] = fma(D74, mk, acc[14]);
-    acc[15] = fma(D75, mk, acc[15]);
-    acc[16] = fma(D79, mk, acc[16]);
-    acc[17] = fma(D80, mk, acc[17]);
-    acc[18] = fma(D81, mk, acc[18]);
-    acc[19] = fma(D82, mk, acc[19]);
   }
-  { const T mk = Mb[18];
-    acc[0] = fma(D19, mk, acc[0]);
-    acc[1] = fma(D29, mk, acc[1]);
-    acc[2] = fma(D33, mk, acc[2]);
-    acc[3] = fma(D34, mk, acc[3]);
-    acc[4] = fma(D44, mk, acc[4]);
-    acc[5] = fma(D48, mk, acc[5]);
-    acc[6] = fma(D49, mk, acc[6]);
+  { const T mk = Mb[17];
+    acc[0] = fma(D21, mk, acc[0]);
+    acc[1] = fma(D33, mk, acc[1]);
+    acc[2] = fma(D35, mk, acc[2]);
+    acc[3] = fma(D36, mk, acc[3]);
+    acc[4] = fma(D48, mk, acc[4]);
+    acc[5] = fma(D50, mk, acc[5]);
+    acc[6] = fma(D51, mk, acc[6]);
     acc[7] = fma(D53, mk, acc[7]);
     acc[8] = fma(D54, mk, acc[8]);
-    acc[9] = fma(D55, mk, acc[9]);
-    acc[10] = fma(D65, mk, acc[10]);
-    acc[11] = fma(D69, mk, acc[11]);
-    acc[12] = fma(D70, mk, acc[12]);
-    acc[13] = fma(D74, mk, acc[13]);
-    acc[14] = fma(D75, mk, acc[14]);
-    acc[15] = fma(D76, mk, acc[15]);
-    acc[16] = fma(D80, mk, acc[16]);
-    acc[17] = fma(D81, mk, acc[17]);
-    acc[18] = fma(D82, mk, acc[18]);
-    acc[19] = fma(D83, mk, acc[19]);
+  }
+  { const T mk = Mb[18];
+    acc[0] = fma(D22, mk, acc[0]);
+    acc[1] = fma(D34, mk, acc[1]);
+    acc[2] = fma(D37, mk, acc[2]);
+    acc[3] = fma(D38, mk, acc[3]);
+    acc[4] = fma(D49, mk, acc[4]);
+    acc[5] = fma(D52, mk, acc[5]);
+    acc[6] = fma(D53, mk, acc[6]);
+    acc[7] = fma(D55, mk, acc[7]);
+    acc[8] = fma(D56, mk, acc[8]);
   }
   { const T mk = Mb[19];
-    acc[0] = fma(D20, mk, acc[0]);
+    acc[0] = fma(D23, mk, acc[0]);
     acc[1] = fma(D35, mk, acc[1]);
-    acc[2] = fma(D36, mk, acc[2]);
-    acc[3] = fma(D37, mk, acc[3]);
-    acc[4] = fma(D56, mk, acc[4]);
-    acc[5] = fma(D57, mk, acc[5]);
-    acc[6] = fma(D58, mk, acc[6]);
-    acc[7] = fma(D59, mk, acc[7]);
-    acc[8] = fma(D60, mk, acc[8]);
-    acc[9] = fma(D61, mk, acc[9]);
-  }
-  { const T mk = Mb[20];
-    acc[0] = fma(D21, mk, acc[0]);
-    acc[1] = fma(D36, mk, acc[1]);
     acc[2] = fma(D38, mk, acc[2]);
     acc[3] = fma(D39, mk, acc[3]);
-    acc[4] = fma(D57, mk, acc[4]);
+    acc[4] = fma(D50, mk, acc[4]);
+    acc[5] = fma(D53, mk, acc[5]);
+    acc[6] = fma(D54, mk, acc[6]);
+    acc[7] = fma(D56, mk, acc[7]);
+    acc[8] = fma(D57, mk, acc[8]);
+  }
+  { const T mk = Mb[20];
+    acc[0] = fma(D25, mk, acc[0]);
+    acc[1] = fma(D37, mk, acc[1]);
+    acc[2] = fma(D40, mk, acc[2]);
+    acc[3] = fma(D41, mk, acc[3]);
+    acc[4] = fma(D52, mk, acc[4]);
+    acc[5] = fma(D55, mk, acc[5]);
+    acc[6] = fma(D56, mk, acc[6]);
+    acc[7] = fma(D58, mk, acc[7]);
+    acc[8] = fma(D59, mk, acc[8]);
+  }
+  { const T mk = Mb[21];
+    acc[0] = fma(D26, mk, acc[0]);
+    acc[1] = fma(D38, mk, acc[1]);
+    acc[2] = fma(D41, mk, acc[2]);
+    acc[3] = fma(D42, mk, acc[3]);
+    acc[4] = fma(D53, mk, acc[4]);
+    acc[5] = fma(D56, mk, acc[5]);
+    acc[6] = fma(D57, mk, acc[6]);
+    acc[7] = fma(D59, mk, acc[7]);
+    acc[8] = fma(D60, mk, acc[8]);
+  }
+  { const T mk = Mb[22];
+    acc[0] = fma(D28, mk, acc[0]);
+    acc[1] = fma(D40, mk, acc[1]);
+    acc[2] = fma(D43, mk, acc[2]);
+    acc[3] = fma(D44, mk, acc[3]);
+    acc[4] = fma(D55, mk, acc[4]);
+    acc[5] = fma(D58, mk, acc[5]);
+    acc[6] = fma(D59, mk, acc[6]);
+    acc[7] = fma(D61, mk, acc[7]);
+    acc[8] = fma(D62, mk, acc[8]);
+  }
+  { const T mk = Mb[23];
+    acc[0] = fma(D29, mk, acc[0]);
+    acc[1] = fma(D41, mk, acc[1]);
+    acc[2] = fma(D44, mk, acc[2]);
+    acc[3] = fma(D45, mk, acc[3]);
+    acc[4] = fma(D56, mk, acc[4]);
     acc[5] = fma(D59, mk, acc[5]);
     acc[6] = fma(D60, mk, acc[6]);
     acc[7] = fma(D62, mk, acc[7]);
     acc[8] = fma(D63, mk, acc[8]);
-    acc[9] = fma(D64, mk, acc[9]);
-  }
-  { const T mk = Mb[21];
-    acc[0] = fma(D22, mk, acc[0]);
-    acc[1] = fma(D37, mk, acc[1]);
-    acc[2] = fma(D39, mk, acc[2]);
-    acc[3] = fma(D40, mk, acc[3]);
-    acc[4] = fma(D58, mk, acc[4]);
-    acc[5] = fma(D60, mk, acc[5]);
-    acc[6] = fma(D61, mk, acc[6]);
-    acc[7] = fma(D63, mk, acc[7]);
-    acc[8] = fma(D64, mk, acc[8]);
-    acc[9] = fma(D65, mk, acc[9]);
-  }
-  { const T mk = Mb[22];
-    acc[0] = fma(D23, mk, acc[0]);
-    acc[1] = fma(D38, mk, acc[1]);
-    acc[2] = fma(D41, mk, acc[2]);
-    acc[3] = fma(D42, mk, acc[3]);
-    acc[4] = fma(D59, mk, acc[4]);
-    acc[5] = fma(D62, mk, acc[5]);
-    acc[6] = fma(D63, mk, acc[6]);
-    acc[7] = fma(D66, mk, acc[7]);
-    acc[8] = fma(D67, mk, acc[8]);
-    acc[9] = fma(D68, mk, acc[9]);
-  }
-  { const T mk = Mb[23];
-    acc[0] = fma(D24, mk, acc[0]);
-    acc[1] = fma(D39, mk, acc[1]);
-    acc[2] = fma(D42, mk, acc[2]);
-    acc[3] = fma(D43, mk, acc[3]);
-    acc[4] = fma(D60, mk, acc[4]);
-    acc[5] = fma(D63, mk, acc[5]);
-    acc[6] = fma(D64, mk, acc[6]);
-    acc[7] = fma(D67, mk, acc[7]);
-    acc[8] = fma(D68, mk, acc[8]);
-    acc[9] = fma(D69, mk, acc[9]);
   }
   { const T mk = Mb[24];
-    acc[0] = fma(D25, mk, acc[0]);
-    acc[1] = fma(D40, mk, acc[1]);
-    acc[2] = fma(D43, mk, acc[2]);
-    acc[3] = fma(D44, mk, acc[3]);
-    acc[4] = fma(D61, mk, acc[4]);
-    acc[5] = fma(D64, mk, acc[5]);
-    acc[6] = fma(D65, mk, acc[6]);
-    acc[7] = fma(D68, mk, acc[7]);
-    acc[8] = fma(D69, mk, acc[8]);
-    acc[9] = fma(D70, mk, acc[9]);
-  }
-  { const T mk = Mb[25];
-    acc[0] = fma(D26, mk, acc[0]);
-    acc[1] = fma(D41, mk, acc[1]);
-    acc[2] = fma(D45, mk, acc[2]);
-    acc[3] = fma(D46, mk, acc[3]);
-    acc[4] = fma(D62, mk, acc[4]);
-    acc[5] = fma(D66, mk, acc[5]);
-    acc[6] = fma(D67, mk, acc[6]);
-    acc[7] = fma(D71, mk, acc[7]);
-    acc[8] = fma(D72, mk, acc[8]);
-    acc[9] = fma(D73, mk, acc[9]);
-  }
-  { const T mk = Mb[26];
-    acc[0] = fma(D27, mk, acc[0]);
-    acc[1] = fma(D42, mk, acc[1]);
-    acc[2] = fma(D46, mk, acc[2]);
-    acc[3] = fma(D47, mk, acc[3]);
-    acc[4] = fma(D63, mk, acc[4]);
-    acc[5] = fma(D67, mk, acc[5]);
-    acc[6] = fma(D68, mk, acc[6]);
-    acc[7] = fma(D72, mk, acc[7]);
-    acc[8] = fma(D73, mk, acc[8]);
-    acc[9] = fma(D74, mk, acc[9]);
-  }
-  { const T mk = Mb[27];
-    acc[0] = fma(D28, mk, acc[0]);
-    acc[1] = fma(D43, mk, acc[1]);
-    acc[2] = fma(D47, mk, acc[2]);
-    acc[3] = fma(D48, mk, acc[3]);
-    acc[4] = fma(D64, mk, acc[4]);
-    acc[5] = fma(D68, mk, acc[5]);
-    acc[6] = fma(D69, mk, acc[6]);
-    acc[7] = fma(D73, mk, acc[7]);
-    acc[8] = fma(D74, mk, acc[8]);
-    acc[9] = fma(D75, mk, acc[9]);
-  }
-  { const T mk = Mb[28];
-    acc[0] = fma(D29, mk, acc[0]);
-    acc[1] = fma(D44, mk, acc[1]);
-    acc[2] = fma(D48, mk, acc[2]);
-    acc[3] = fma(D49, mk, acc[3]);
-    acc[4] = fma(D65, mk, acc[4]);
-    acc[5] = fma(D69, mk, acc[5]);
-    acc[6] = fma(D70, mk, acc[6]);
-    acc[7] = fma(D74, mk, acc[7]);
-    acc[8] = fma(D75, mk, acc[8]);
-    acc[9] = fma(D76, mk, acc[9]);
-  }
-  { const T mk = Mb[29];
-    acc[0] = fma(D30, mk, acc[0]);
-    acc[1] = fma(D45, mk, acc[1]);
-    acc[2] = fma(D50, mk, acc[2]);
-    acc[3] = fma(D51, mk, acc[3]);
-    acc[4] = fma(D66, mk, acc[4]);
-    acc[5] = fma(D71, mk, acc[5]);
-    acc[6] = fma(D72, mk, acc[6]);
-    acc[7] = fma(D77, mk, acc[7]);
-    acc[8] = fma(D78, mk, acc[8]);
-    acc[9] = fma(D79, mk, acc[9]);
-  }
-  { const T mk = Mb[30];
     acc[0] = fma(D31, mk, acc[0]);
     acc[1] = fma(D46, mk, acc[1]);
-    acc[2] = fma(D51, mk, acc[2]);
-    acc[3] = fma(D52, mk, acc[3]);
-    acc[4] = fma(D67, mk, acc[4]);
-    acc[5] = fma(D72, mk, acc[5]);
-    acc[6] = fma(D73, mk, acc[6]);
-    acc[7] = fma(D78, mk, acc[7]);
-    acc[8] = fma(D79, mk, acc[8]);
-    acc[9] = fma(D80, mk, acc[9]);
+    acc[2] = fma(D47, mk, acc[2]);
+    acc[3] = fma(D48, mk, acc[3]);
   }
-  { const T mk = Mb[31];
+  { const T mk = Mb[25];
     acc[0] = fma(D32, mk, acc[0]);
     acc[1] = fma(D47, mk, acc[1]);
-    acc[2] = fma(D52, mk, acc[2]);
-    acc[3] = fma(D53, mk, acc[3]);
-    acc[4] = fma(D68, mk, acc[4]);
-    acc[5] = fma(D73, mk, acc[5]);
-    acc[6] = fma(D74, mk, acc[6]);
-    acc[7] = fma(D79, mk, acc[7]);
-    acc[8] = fma(D80, mk, acc[8]);
-    acc[9] = fma(D81, mk, acc[9]);
+    acc[2] = fma(D49, mk, acc[2]);
+    acc[3] = fma(D50, mk, acc[3]);
   }
-  { const T mk = Mb[32];
+  { const T mk = Mb[26];
     acc[0] = fma(D33, mk, acc[0]);
     acc[1] = fma(D48, mk, acc[1]);
-    acc[2] = fma(D53, mk, acc[2]);
-    acc[3] = fma(D54, mk, acc[3]);
-    acc[4] = fma(D69, mk, acc[4]);
-    acc[5] = fma(D74, mk, acc[5]);
-    acc[6] = fma(D75, mk, acc[6]);
-    acc[7] = fma(D80, mk, acc[7]);
-    acc[8] = fma(D81, mk, acc[8]);
-    acc[9] = fma(D82, mk, acc[9]);
+    acc[2] = fma(D50, mk, acc[2]);
+    acc[3] = fma(D51, mk, acc[3]);
   }
-  { const T mk = Mb[33];
+  { const T mk = Mb[27];
     acc[0] = fma(D34, mk, acc[0]);
     acc[1] = fma(D49, mk, acc[1]);
-    acc[2] = fma(D54, mk, acc[2]);
-    acc[3] = fma(D55, mk, acc[3]);
-    acc[4] = fma(D70, mk, acc[4]);
-    acc[5] = fma(D75, mk, acc[5]);
-    acc[6] = fma(D76, mk, acc[6]);
-    acc[7] = fma(D81, mk, acc[7]);
-    acc[8] = fma(D82, mk, acc[8]);
-    acc[9] = fma(D83, mk, acc[9]);
+    acc[2] = fma(D52, mk, acc[2]);
+    acc[3] = fma(D53, mk, acc[3]);
   }
-  { const T mk = Mb[34];
+  { const T mk = Mb[28];
     acc[0] = fma(D35, mk, acc[0]);
-    acc[1] = fma(D56, mk, acc[1]);
-    acc[2] = fma(D57, mk, acc[2]);
-    acc[3] = fma(D58, mk, acc[3]);
+    acc[1] = fma(D50, mk, acc[1]);
+    acc[2] = fma(D53, mk, acc[2]);
+    acc[3] = fma(D54, mk, acc[3]);
   }
-  { const T mk = Mb[35];
-    acc[0] = fma(D36, mk, acc[0]);
-    acc[1] = fma(D57, mk, acc[1]);
+  { const T mk = Mb[29];
+    acc[0] = fma(D37, mk, acc[0]);
+    acc[1] = fma(D52, mk, acc[1]);
+    acc[2] = fma(D55, mk, acc[2]);
+    acc[3] = fma(D56, mk, acc[3]);
+  }
+  { const T mk = Mb[30];
+    acc[0] = fma(D38, mk, acc[0]);
+    acc[1] = fma(D53, mk, acc[1]);
+    acc[2] = fma(D56, mk, acc[2]);
+    acc[3] = fma(D57, mk, acc[3]);
+  }
+  { const T mk = Mb[31];
+    acc[0] = fma(D40, mk, acc[0]);
+    acc[1] = fma(D55, mk, acc[1]);
+    acc[2] = fma(D58, mk, acc[2]);
+    acc[3] = fma(D59, mk, acc[3]);
+  }
+  { const T mk = Mb[32];
+    acc[0] = fma(D41, mk, acc[0]);
+    acc[1] = fma(D56, mk, acc[1]);
     acc[2] = fma(D59, mk, acc[2]);
     acc[3] = fma(D60, mk, acc[3]);
   }
-  { const T mk = Mb[36];
-    acc[0] = fma(D37, mk, acc[0]);
+  { const T mk = Mb[33];
+    acc[0] = fma(D43, mk, acc[0]);
     acc[1] = fma(D58, mk, acc[1]);
-    acc[2] = fma(D60, mk, acc[2]);
-    acc[3] = fma(D61, mk, acc[3]);
+    acc[2] = fma(D61, mk, acc[2]);
+    acc[3] = fma(D62, mk, acc[3]);
   }
-  { const T mk = Mb[37];
-    acc[0] = fma(D38, mk, acc[0]);
+  { const T mk = Mb[34];
+    acc[0] = fma(D44, mk, acc[0]);
     acc[1] = fma(D59, mk, acc[1]);
     acc[2] = fma(D62, mk, acc[2]);
     acc[3] = fma(D63, mk, acc[3]);
   }
+  { const T mk = Mb[35];
+    acc[0] = fma(D46, mk, acc[0]);
+  }
+  { const T mk = Mb[36];
+    acc[0] = fma(D47, mk, acc[0]);
+  }
+  { const T mk = Mb[37];
+    acc[0] = fma(D48, mk, acc[0]);
+  }
   { const T mk = Mb[38];
-    acc[0] = fma(D39, mk, acc[0]);
-    acc[1] = fma(D60, mk, acc[1]);
-    acc[2] = fma(D63, mk, acc[2]);
-    acc[3] = fma(D64, mk, acc[3]);
+    acc[0] = fma(D49, mk, acc[0]);
   }
   { const T mk = Mb[39];
-    acc[0] = fma(D40, mk, acc[0]);
-    acc[1] = fma(D61, mk, acc[1]);
-    acc[2] = fma(D64, mk, acc[2]);
-    acc[3] = fma(D65, mk, acc[3]);
+    acc[0] = fma(D50, mk, acc[0]);
   }
   { const T mk = Mb[40];
-    acc[0] = fma(D41, mk, acc[0]);
-    acc[1] = fma(D62, mk, acc[1]);
-    acc[2] = fma(D66, mk, acc[2]);
-    acc[3] = fma(D67, mk, acc[3]);
+    acc[0] = fma(D52, mk, acc[0]);
   }
   { const T mk = Mb[41];
-    acc[0] = fma(D42, mk, acc[0]);
-    acc[1] = fma(D63, mk, acc[1]);
-    acc[2] = fma(D67, mk, acc[2]);
-    acc[3] = fma(D68, mk, acc[3]);
+    acc[0] = fma(D53, mk, acc[0]);
   }
   { const T mk = Mb[42];
-    acc[0] = fma(D43, mk, acc[0]);
-    acc[1] = fma(D64, mk, acc[1]);
-    acc[2] = fma(D68, mk, acc[2]);
-    acc[3] = fma(D69, mk, acc[3]);
+    acc[0] = fma(D55, mk, acc[0]);
   }
   { const T mk = Mb[43];
-    acc[0] = fma(D44, mk, acc[0]);
-    acc[1] = fma(D65, mk, acc[1]);
-    acc[2] = fma(D69, mk, acc[2]);
-    acc[3] = fma(D70, mk, acc[3]);
-  }
-  { const T mk = Mb[44];
-    acc[0] = fma(D45, mk, acc[0]);
-    acc[1] = fma(D66, mk, acc[1]);
-    acc[2] = fma(D71, mk, acc[2]);
-    acc[3] = fma(D72, mk, acc[3]);
-  }
-  { const T mk = Mb[45];
-    acc[0] = fma(D46, mk, acc[0]);
-    acc[1] = fma(D67, mk, acc[1]);
-    acc[2] = fma(D72, mk, acc[2]);
-    acc[3] = fma(D73, mk, acc[3]);
-  }
-  { const T mk = Mb[46];
-    acc[0] = fma(D47, mk, acc[0]);
-    acc[1] = fma(D68, mk, acc[1]);
-    acc[2] = fma(D73, mk, acc[2]);
-    acc[3] = fma(D74, mk, acc[3]);
-  }
-  { const T mk = Mb[47];
-    acc[0] = fma(D48, mk, acc[0]);
-    acc[1] = fma(D69, mk, acc[1]);
-    acc[2] = fma(D74, mk, acc[2]);
-    acc[3] = fma(D75, mk, acc[3]);
-  }
-  { const T mk = Mb[48];
-    acc[0] = fma(D49, mk, acc[0]);
-    acc[1] = fma(D70, mk, acc[1]);
-    acc[2] = fma(D75, mk, acc[2]);
-    acc[3] = fma(D76, mk, acc[3]);
-  }
-  { const T mk = Mb[49];
-    acc[0] = fma(D50, mk, acc[0]);
-    acc[1] = fma(D71, mk, acc[1]);
-    acc[2] = fma(D77, mk, acc[2]);
-    acc[3] = fma(D78, mk, acc[3]);
-  }
-  { const T mk = Mb[50];
-    acc[0] = fma(D51, mk, acc[0]);
-    acc[1] = fma(D72, mk, acc[1]);
-    acc[2] = fma(D78, mk, acc[2]);
-    acc[3] = fma(D79, mk, acc[3]);
-  }
-  { const T mk = Mb[51];
-    acc[0] = fma(D52, mk, acc[0]);
-    acc[1] = fma(D73, mk, acc[1]);
-    acc[2] = fma(D79, mk, acc[2]);
-    acc[3] = fma(D80, mk, acc[3]);
-  }
-  { const T mk = Mb[52];
-    acc[0] = fma(D53, mk, acc[0]);
-    acc[1] = fma(D74, mk, acc[1]);
-    acc[2] = fma(D80, mk, acc[2]);
-    acc[3] = fma(D81, mk, acc[3]);
-  }
-  { const T mk = Mb[53];
-    acc[0] = fma(D54, mk, acc[0]);
-    acc[1] = fma(D75, mk, acc[1]);
-    acc[2] = fma(D81, mk, acc[2]);
-    acc[3] = fma(D82, mk, acc[3]);
-  }
-  { const T mk = Mb[54];
-    acc[0] = fma(D55, mk, acc[0]);
-    acc[1] = fma(D76, mk, acc[1]);
-    acc[2] = fma(D82, mk, acc[2]);
-    acc[3] = fma(D83, mk, acc[3]);
-  }
-  { const T mk = Mb[55];
     acc[0] = fma(D56, mk, acc[0]);
   }
-  { const T mk = Mb[56];
-    acc[0] = fma(D57, mk, acc[0]);
-  }
-  { const T mk = Mb[57];
+  { const T mk = Mb[44];
     acc[0] = fma(D58, mk, acc[0]);
   }
-  { const T mk = Mb[58];
+  { const T mk = Mb[45];
     acc[0] = fma(D59, mk, acc[0]);
   }
-  { const T mk = Mb[59];
-    acc[0] = fma(D60, mk, acc[0]);
-  }
-  { const T mk = Mb[60];
+  { const T mk = Mb[46];
     acc[0] = fma(D61, mk, acc[0]);
   }
-  { const T mk = Mb[61];
+  { const T mk = Mb[47];
     acc[0] = fma(D62, mk, acc[0]);
   }
-  { const T mk = Mb[62];
-    acc[0] = fma(D63, mk, acc[0]);
-  }
-  { const T mk = Mb[63];
-    acc[0] = fma(D64, mk, acc[0]);
-  }
-  { const T mk = Mb[64];
-    acc[0] = fma(D65, mk, acc[0]);
-  }
-  { const T mk = Mb[65];
-    acc[0] = fma(D66, mk, acc[0]);
-  }
-  { const T mk = Mb[66];
-    acc[0] = fma(D67, mk, acc[0]);
-  }
-  { const T mk = Mb[67];
-    acc[0] = fma(D68, mk, acc[0]);
-  }
-  { const T mk = Mb[68];
-    acc[0] = fma(D69, mk, acc[0]);
-  }
-  { const T mk = Mb[69];
-    acc[0] = fma(D70, mk, acc[0]);
-  }
-  { const T mk = Mb[70];
-    acc[0] = fma(D71, mk, acc[0]);
-  }
-  { const T mk = Mb[71];
-    acc[0] = fma(D72, mk, acc[0]);
-  }
-  { const T mk = Mb[72];
-    acc[0] = fma(D73, mk, acc[0]);
-  }
-  { const T mk = Mb[73];
-    acc[0] = fma(D74, mk, acc[0]);
-  }
-  { const T mk = Mb[74];
-    acc[0] = fma(D75, mk, acc[0]);
-  }
-  { const T mk = Mb[75];
-    acc[0] = fma(D76, mk, acc[0]);
-  }
-  { const T mk = Mb[76];
-    acc[0] = fma(D77, mk, acc[0]);
-  }
-  { const T mk = Mb[77];
-    acc[0] = fma(D78, mk, acc[0]);
-  }
-  { const T mk = Mb[78];
-    acc[0] = fma(D79, mk, acc[0]);
-  }
-  { const T mk = Mb[79];
-    acc[0] = fma(D80, mk, acc[0]);
-  }
-  { const T mk = Mb[80];
-    acc[0] = fma(D81, mk, acc[0]);
-  }
-  { const T mk = Mb[81];
-    acc[0] = fma(D82, mk, acc[0]);
-  }
-  { const T mk = Mb[82];
-    acc[0] = fma(D83, mk, acc[0]);
-  }
 }
+static __constant__ unsigned char m2l_w_m1_p6[483] = {
+  1, 4, 5, 6, 10, 11, 12, 13, 14, 19, 20, 21, 22, 23, 25, 26, 31, 32, 33, 34, 35, 37, 38, 40, 41, 46, 47, 48, 49, 50, 52, 53, 55, 56, 58, 59, 2, 5, 7, 8, 11, 13, 14, 16, 17, 20, 22, 23, 25, 26, 28, 29, 32, 34, 35, 37, 38, 40, 41, 43, 44, 47, 49, 50, 52, 53, 55, 56, 58, 59, 61, 62, 3, 6, 8, 9, 12, 14, 15, 17, 18, 21, 23, 24, 26, 27, 29, 30, 33, 35, 36, 38, 39, 41, 42, 44, 45, 48, 50, 51, 53, 54, 56, 57, 59, 60, 62, 63, 4, 10, 11, 12, 19, 20, 21, 22, 23, 31, 32, 33, 34, 35, 37, 38, 46, 47, 48, 49, 50, 52, 53, 55, 56, 5, 11, 13, 14, 20, 22, 23, 25, 26, 32, 34, 35, 37, 38, 40, 41, 47, 49, 50, 52, 53, 55, 56, 58, 59, 6, 12, 14, 15, 21, 23, 24, 26, 27, 33, 35, 36, 38, 39, 41, 42, 48, 50, 51, 53, 54, 56, 57, 59, 60, 7, 13, 16, 17, 22, 25, 26, 28, 29, 34, 37, 38, 40, 41, 43, 44, 49, 52, 53, 55, 56, 58, 59, 61, 62, 8, 14, 17, 18, 23, 26, 27, 29, 30, 35, 38, 39, 41, 42, 44, 45, 50, 53, 54, 56, 57, 59, 60, 62, 63, 10, 19, 20, 21, 31, 32, 33, 34, 35, 46, 47, 48, 49, 50, 52, 53, 11, 20, 22, 23, 32, 34, 35, 37, 38, 47, 49, 50, 52, 53, 55, 56, 12, 21, 23, 24, 33, 35, 36, 38, 39, 48, 50, 51, 53, 54, 56, 57, 13, 22, 25, 26, 34, 37, 38, 40, 41, 49, 52, 53, 55, 56, 58, 59, 14, 23, 26, 27, 35, 38, 39, 41, 42, 50, 53, 54, 56, 57, 59, 60, 16, 25, 28, 29, 37, 40, 41, 43, 44, 52, 55, 56, 58, 59, 61, 62, 17, 26, 29, 30, 38, 41, 42, 44, 45, 53, 56, 57, 59, 60, 62, 63, 19, 31, 32, 33, 46, 47, 48, 49, 50, 20, 32, 34, 35, 47, 49, 50, 52, 53, 21, 33, 35, 36, 48, 50, 51, 53, 54, 22, 34, 37, 38, 49, 52, 53, 55, 56, 23, 35, 38, 39, 50, 53, 54, 56, 57, 25, 37, 40, 41, 52, 55, 56, 58, 59, 26, 38, 41, 42, 53, 56, 57, 59, 60, 28, 40, 43, 44, 55, 58, 59, 61, 62, 29, 41, 44, 45, 56, 59, 60, 62, 63, 31, 46, 47, 48, 32, 47, 49, 50, 33, 48, 50, 51, 34, 49, 52, 53, 35, 50, 53, 54, 37, 52, 55, 56, 38, 53, 56, 57, 40, 55, 58, 59, 41, 56, 59, 60, 43, 58, 61, 62, 44, 59, 62, 63, 46, 47, 48, 49, 50, 52, 53, 55, 56, 58, 59, 61, 62};
+static __device__ const signed char m2l_fold_m1_p6[48][6][2] = {
+  {{0, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{1, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{2, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{3, 1}, {8, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{4, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{5, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{6, 1}, {8, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{7, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{9, 1}, {14, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{10, 1}, {17, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{11, 1}, {18, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{12, 1}, {14, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{13, 1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{15, 1}, {17, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{16, 1}, {18, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{19, 1}, {24, -1}, {33, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{20, 1}, {27, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{21, 1}, {28, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{22, 1}, {24, -1}, {31, -1}, {33, 2}, {0, 0}, {0, 0}},
+  {{23, 1}, {32, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{25, 1}, {27, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{26, 1}, {28, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{29, 1}, {31, -1}, {33, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{30, 1}, {32, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{34, 1}, {39, -1}, {48, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{35, 1}, {42, -1}, {53, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{36, 1}, {43, -1}, {54, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{37, 1}, {39, -1}, {46, -1}, {48, 2}, {0, 0}, {0, 0}},
+  {{38, 1}, {47, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{40, 1}, {42, -1}, {51, -1}, {53, 2}, {0, 0}, {0, 0}},
+  {{41, 1}, {43, -1}, {52, -1}, {54, 2}, {0, 0}, {0, 0}},
+  {{44, 1}, {46, -1}, {48, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{45, 1}, {47, -1}, {0, 0}, {0, 0}, {0, 0}, {0, 0}},
+  {{49, 1}, {51, -1}, {53, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{50, 1}, {52, -1}, {54, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{55, 1}, {60, -1}, {69, 1}, {82, -1}, {0, 0}, {0, 0}},
+  {{56, 1}, {63, -1}, {74, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{57, 1}, {64, -1}, {75, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{58, 1}, {60, -1}, {67, -1}, {69, 2}, {80, 1}, {82, -3}},
+  {{59, 1}, {68, -1}, {81, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{61, 1}, {63, -1}, {72, -1}, {74, 2}, {0, 0}, {0, 0}},
+  {{62, 1}, {64, -1}, {73, -1}, {75, 2}, {0, 0}, {0, 0}},
+  {{65, 1}, {67, -1}, {69, 1}, {78, -1}, {80, 2}, {82, -3}},
+  {{66, 1}, {68, -1}, {79, -1}, {81, 2}, {0, 0}, {0, 0}},
+  {{70, 1}, {72, -1}, {74, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{71, 1}, {73, -1}, {75, 1}, {0, 0}, {0, 0}, {0, 0}},
+  {{76, 1}, {78, -1}, {80, 1}, {82, -1}, {0, 0}, {0, 0}},
+  {{77, 1}, {79, -1}, {81, 1}, {0, 0}, {0, 0}, {0, 0}},
+};
+static __device__ const signed char m2l_unfold_m1_p6[56][3][2] = {
+  {{0, 1}, {0, 0}, {0, 0}},
+  {{1, 1}, {0, 0}, {0, 0}},
+  {{2, 1}, {0, 0}, {0, 0}},
+  {{3, 1}, {0, 0}, {0, 0}},
+  {{4, 1}, {0, 0}, {0, 0}},
+  {{5, 1}, {0, 0}, {0, 0}},
+  {{6, 1}, {0, 0}, {0, 0}},
+  {{7, 1}, {0, 0}, {0, 0}},
+  {{8, 1}, {0, 0}, {0, 0}},
+  {{7, -1}, {4, -1}, {0, 0}},
+  {{9, 1}, {0, 0}, {0, 0}},
+  {{10, 1}, {0, 0}, {0, 0}},
+  {{11, 1}, {0, 0}, {0, 0}},
+  {{12, 1}, {0, 0}, {0, 0}},
+  {{13, 1}, {0, 0}, {0, 0}},
+  {{12, -1}, {9, -1}, {0, 0}},
+  {{14, 1}, {0, 0}, {0, 0}},
+  {{15, 1}, {0, 0}, {0, 0}},
+  {{14, -1}, {10, -1}, {0, 0}},
+  {{15, -1}, {11, -1}, {0, 0}},
+  {{16, 1}, {0, 0}, {0, 0}},
+  {{17, 1}, {0, 0}, {0, 0}},
+  {{18, 1}, {0, 0}, {0, 0}},
+  {{19, 1}, {0, 0}, {0, 0}},
+  {{20, 1}, {0, 0}, {0, 0}},
+  {{19, -1}, {16, -1}, {0, 0}},
+  {{21, 1}, {0, 0}, {0, 0}},
+  {{22, 1}, {0, 0}, {0, 0}},
+  {{21, -1}, {17, -1}, {0, 0}},
+  {{22, -1}, {18, -1}, {0, 0}},
+  {{23, 1}, {0, 0}, {0, 0}},
+  {{24, 1}, {0, 0}, {0, 0}},
+  {{23, -1}, {19, -1}, {0, 0}},
+  {{24, -1}, {20, -1}, {0, 0}},
+  {{23, 1}, {19, 2}, {16, 1}},
+  {{25, 1}, {0, 0}, {0, 0}},
+  {{26, 1}, {0, 0}, {0, 0}},
+  {{27, 1}, {0, 0}, {0, 0}},
+  {{28, 1}, {0, 0}, {0, 0}},
+  {{29, 1}, {0, 0}, {0, 0}},
+  {{28, -1}, {25, -1}, {0, 0}},
+  {{30, 1}, {0, 0}, {0, 0}},
+  {{31, 1}, {0, 0}, {0, 0}},
+  {{30, -1}, {26, -1}, {0, 0}},
+  {{31, -1}, {27, -1}, {0, 0}},
+  {{32, 1}, {0, 0}, {0, 0}},
+  {{33, 1}, {0, 0}, {0, 0}},
+  {{32, -1}, {28, -1}, {0, 0}},
+  {{33, -1}, {29, -1}, {0, 0}},
+  {{32, 1}, {28, 2}, {25, 1}},
+  {{34, 1}, {0, 0}, {0, 0}},
+  {{35, 1}, {0, 0}, {0, 0}},
+  {{34, -1}, {30, -1}, {0, 0}},
+  {{35, -1}, {31, -1}, {0, 0}},
+  {{34, 1}, {30, 2}, {26, 1}},
+  {{35, 1}, {31, 2}, {27, 1}},
+};
 
 // P2M of a dipole (s0, s1, s2) at offset (x, y, z) = centre - site, order 5
 template <typename T>
@@ -6997,30 +5843,10 @@ __device__ __forceinline__ void l2p_m1_p6(T x, T y, T z, const T* __restrict__ L
   }
 }
 
-// loop-form tables of M2L, source order 1, expansion order 5
-static __constant__ short m2l_rec_m1_p5[448] = {
-  -1, -1, -1, -1, -1, -1, 0, 0, 0, -1, -1, -1, -1, -1, 1, 0, -1, 0, -1, -1, -1, -1, 1, 0, -1, -1, 0, -1, -1, -1, 1, 0, 1, -1, -1, 0, -1, -1, 2, 0, 2, 1, -1, -1, -1, -1, 2, 0, 3, -1, 1, -1, -1, -1, 2, 0, -1, 2, -1, -1, 0, -1, 2, 0, -1, 3, 2, -1, -1, -1, 2, 0, -1, -1, 3, -1, -1, 0, 2, 0, 4, -1, -1, 1, -1, -1, 3, 0, 5, 4, -1, 2, -1, -1, 3, 0, 6, -1, 4, 3, -1, -1, 3, 0, 7, 5, -1, -1, 1, -1, 3, 0, 8, 6, 5, -1, -1, -1, 3, 0, 9, -1, 6, -1, -1, 1, 3, 0, -1, 7, -1, -1, 2, -1, 3, 0, -1, 8, 7, -1, 3, -1, 3, 0, -1, 9, 8, -1, -1, 2, 3, 0, -1, -1, 9, -1, -1, 3, 3, 0, 10, -1, -1, 4, -1, -1, 4, 0, 11, 10, -1, 5, -1, -1, 4, 0, 12, -1, 10, 6, -1, -1, 4, 0, 13, 11, -1, 7, 4, -1, 4, 0, 14, 12, 11, 8, -1, -1, 4, 0, 15, -1, 12, 9, -1, 4, 4, 0, 16, 13, -1, -1, 5, -1, 4, 0, 17, 14, 13, -1, 6, -1, 4, 0, 18, 15, 14, -1, -1, 5, 4, 0, 19, -1, 15, -1, -1, 6, 4, 0, -1, 16, -1, -1, 7, -1, 4, 0, -1, 17, 16, -1, 8, -1, 4, 0, -1, 18, 17, -1, 9, 7, 4, 0, -1, 19, 18, -1, -1, 8, 4, 0, -1, -1, 19, -1, -1, 9, 4, 0, 20, -1, -1, 10, -1, -1, 5, 0, 21, 20, -1, 11, -1, -1, 5, 0, 22, -1, 20, 12, -1, -1, 5, 0, 23, 21, -1, 13, 10, -1, 5, 0, 24, 22, 21, 14, -1, -1, 5, 0, 25, -1, 22, 15, -1, 10, 5, 0, 26, 23, -1, 16, 11, -1, 5, 0, 27, 24, 23, 17, 12, -1, 5, 0, 28, 25, 24, 18, -1, 11, 5, 0, 29, -1, 25, 19, -1, 12, 5, 0, 30, 26, -1, -1, 13, -1, 5, 0, 31, 27, 26, -1, 14, -1, 5, 0, 32, 28, 27, -1, 15, 13, 5, 0, 33, 29, 28, -1, -1, 14, 5, 0, 34, -1, 29, -1, -1, 15, 5, 0, -1, 30, -1, -1, 16, -1, 5, 0, -1, 31, 30, -1, 17, -1, 5, 0, -1, 32, 31, -1, 18, 16, 5, 0, -1, 33, 32, -1, 19, 17, 5, 0, -1, 34, 33, -1, -1, 18, 5, 0, -1, -1, 34, -1, -1, 19, 5, 0};
-static __constant__ float m2l_coef_m1_p5[448] = {
-  0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.0f, 0.0f, 0.5f, 0.0f, 3.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 3.0f, 0.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.0f, 0.5f, 0.0f, 0.0f, 3.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 0.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.5f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 10.0f, 5.0f, 0.0f, 4.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 10.0f, 0.0f, 5.0f, 4.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 5.0f, 5.0f, 0.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 0.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 10.0f, 5.0f, 0.0f, 4.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 5.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.3333333432674408f, -9.934107758624577e-09f, 28.0f, 0.0f, 0.0f, 36.0f, 0.0f, 0.0f, 0.25f, 0.0f, 21.0f, 7.0f, 0.0f, 18.0f, 0.0f, 0.0f, 0.25f, 0.0f, 21.0f, 0.0f, 7.0f, 18.0f, 0.0f, 0.0f, 0.25f, 0.0f, 14.0f, 14.0f, 0.0f, 6.0f, 6.0f, 0.0f, 0.25f, 0.0f, 14.0f, 7.0f, 7.0f, 6.0f, 0.0f, 0.0f, 0.25f, 0.0f, 14.0f, 0.0f, 14.0f, 6.0f, 0.0f, 6.0f, 0.25f, 0.0f, 7.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.0f, 0.25f, 0.0f, 7.0f, 14.0f, 7.0f, 0.0f, 6.0f, 0.0f, 0.25f, 0.0f, 7.0f, 7.0f, 14.0f, 0.0f, 0.0f, 6.0f, 0.25f, 0.0f, 7.0f, 0.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.25f, 0.0f, 0.0f, 28.0f, 0.0f, 0.0f, 36.0f, 0.0f, 0.25f, 0.0f, 0.0f, 21.0f, 7.0f, 0.0f, 18.0f, 0.0f, 0.25f, 0.0f, 0.0f, 14.0f, 14.0f, 0.0f, 6.0f, 6.0f, 0.25f, 0.0f, 0.0f, 7.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.25f, 0.0f, 0.0f, 0.0f, 28.0f, 0.0f, 0.0f, 36.0f, 0.25f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 36.0f, 9.0f, 0.0f, 48.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 36.0f, 0.0f, 9.0f, 48.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 18.0f, 0.0f, 24.0f, 8.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 9.0f, 9.0f, 24.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 0.0f, 18.0f, 24.0f, 0.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 27.0f, 0.0f, 8.0f, 24.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 18.0f, 9.0f, 8.0f, 8.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 9.0f, 18.0f, 8.0f, 0.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 0.0f, 27.0f, 8.0f, 0.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 27.0f, 9.0f, 0.0f, 24.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 18.0f, 18.0f, 0.0f, 8.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 9.0f, 27.0f, 0.0f, 0.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 0.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 36.0f, 9.0f, 0.0f, 48.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 27.0f, 18.0f, 0.0f, 24.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 18.0f, 27.0f, 0.0f, 8.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 9.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.20000000298023224f, -2.9802322831784522e-09f};
-static __constant__ unsigned char m2l_w_m1_p5[406] = {
-  1, 4, 5, 6, 10, 11, 12, 13, 14, 15, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 2, 5, 7, 8, 11, 13, 14, 16, 17, 18, 21, 23, 24, 26, 27, 28, 30, 31, 32, 33, 36, 38, 39, 41, 42, 43, 45, 46, 47, 48, 50, 51, 52, 53, 54, 3, 6, 8, 9, 12, 14, 15, 17, 18, 19, 22, 24, 25, 27, 28, 29, 31, 32, 33, 34, 37, 39, 40, 42, 43, 44, 46, 47, 48, 49, 51, 52, 53, 54, 55, 4, 10, 11, 12, 20, 21, 22, 23, 24, 25, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 5, 11, 13, 14, 21, 23, 24, 26, 27, 28, 36, 38, 39, 41, 42, 43, 45, 46, 47, 48, 6, 12, 14, 15, 22, 24, 25, 27, 28, 29, 37, 39, 40, 42, 43, 44, 46, 47, 48, 49, 7, 13, 16, 17, 23, 26, 27, 30, 31, 32, 38, 41, 42, 45, 46, 47, 50, 51, 52, 53, 8, 14, 17, 18, 24, 27, 28, 31, 32, 33, 39, 42, 43, 46, 47, 48, 51, 52, 53, 54, 9, 15, 18, 19, 25, 28, 29, 32, 33, 34, 40, 43, 44, 47, 48, 49, 52, 53, 54, 55, 10, 20, 21, 22, 35, 36, 37, 38, 39, 40, 11, 21, 23, 24, 36, 38, 39, 41, 42, 43, 12, 22, 24, 25, 37, 39, 40, 42, 43, 44, 13, 23, 26, 27, 38, 41, 42, 45, 46, 47, 14, 24, 27, 28, 39, 42, 43, 46, 47, 48, 15, 25, 28, 29, 40, 43, 44, 47, 48, 49, 16, 26, 30, 31, 41, 45, 46, 50, 51, 52, 17, 27, 31, 32, 42, 46, 47, 51, 52, 53, 18, 28, 32, 33, 43, 47, 48, 52, 53, 54, 19, 29, 33, 34, 44, 48, 49, 53, 54, 55, 20, 35, 36, 37, 21, 36, 38, 39, 22, 37, 39, 40, 23, 38, 41, 42, 24, 39, 42, 43, 25, 40, 43, 44, 26, 41, 45, 46, 27, 42, 46, 47, 28, 43, 47, 48, 29, 44, 48, 49, 30, 45, 50, 51, 31, 46, 51, 52, 32, 47, 52, 53, 33, 48, 53, 54, 34, 49, 54, 55, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 50, 51, 52, 53, 54, 55};
-
-// loop-form tables of M2L, source order 1, expansion order 6
-static __constant__ short m2l_rec_m1_p6[672] = {
-  -1, -1, -1, -1, -1, -1, 0, 0, 0, -1, -1, -1, -1, -1, 1, 0, -1, 0, -1, -1, -1, -1, 1, 0, -1, -1, 0, -1, -1, -1, 1, 0, 1, -1, -1, 0, -1, -1, 2, 0, 2, 1, -1, -1, -1, -1, 2, 0, 3, -1, 1, -1, -1, -1, 2, 0, -1, 2, -1, -1, 0, -1, 2, 0, -1, 3, 2, -1, -1, -1, 2, 0, -1, -1, 3, -1, -1, 0, 2, 0, 4, -1, -1, 1, -1, -1, 3, 0, 5, 4, -1, 2, -1, -1, 3, 0, 6, -1, 4, 3, -1, -1, 3, 0, 7, 5, -1, -1, 1, -1, 3, 0, 8, 6, 5, -1, -1, -1, 3, 0, 9, -1, 6, -1, -1, 1, 3, 0, -1, 7, -1, -1, 2, -1, 3, 0, -1, 8, 7, -1, 3, -1, 3, 0, -1, 9, 8, -1, -1, 2, 3, 0, -1, -1, 9, -1, -1, 3, 3, 0, 10, -1, -1, 4, -1, -1, 4, 0, 11, 10, -1, 5, -1, -1, 4, 0, 12, -1, 10, 6, -1, -1, 4, 0, 13, 11, -1, 7, 4, -1, 4, 0, 14, 12, 11, 8, -1, -1, 4, 0, 15, -1, 12, 9, -1, 4, 4, 0, 16, 13, -1, -1, 5, -1, 4, 0, 17, 14, 13, -1, 6, -1, 4, 0, 18, 15, 14, -1, -1, 5, 4, 0, 19, -1, 15, -1, -1, 6, 4, 0, -1, 16, -1, -1, 7, -1, 4, 0, -1, 17, 16, -1, 8, -1, 4, 0, -1, 18, 17, -1, 9, 7, 4, 0, -1, 19, 18, -1, -1, 8, 4, 0, -1, -1, 19, -1, -1, 9, 4, 0, 20, -1, -1, 10, -1, -1, 5, 0, 21, 20, -1, 11, -1, -1, 5, 0, 22, -1, 20, 12, -1, -1, 5, 0, 23, 21, -1, 13, 10, -1, 5, 0, 24, 22, 21, 14, -1, -1, 5, 0, 25, -1, 22, 15, -1, 10, 5, 0, 26, 23, -1, 16, 11, -1, 5, 0, 27, 24, 23, 17, 12, -1, 5, 0, 28, 25, 24, 18, -1, 11, 5, 0, 29, -1, 25, 19, -1, 12, 5, 0, 30, 26, -1, -1, 13, -1, 5, 0, 31, 27, 26, -1, 14, -1, 5, 0, 32, 28, 27, -1, 15, 13, 5, 0, 33, 29, 28, -1, -1, 14, 5, 0, 34, -1, 29, -1, -1, 15, 5, 0, -1, 30, -1, -1, 16, -1, 5, 0, -1, 31, 30, -1, 17, -1, 5, 0, -1, 32, 31, -1, 18, 16, 5, 0, -1, 33, 32, -1, 19, 17, 5, 0, -1, 34, 33, -1, -1, 18, 5, 0, -1, -1, 34, -1, -1, 19, 5, 0, 35, -1, -1, 20, -1, -1, 6, 0, 36, 35, -1, 21, -1, -1, 6, 0, 37, -1, 35, 22, -1, -1, 6, 0, 38, 36, -1, 23, 20, -1, 6, 0, 39, 37, 36, 24, -1, -1, 6, 0, 40, -1, 37, 25, -1, 20, 6, 0, 41, 38, -1, 26, 21, -1, 6, 0, 42, 39, 38, 27, 22, -1, 6, 0, 43, 40, 39, 28, -1, 21, 6, 0, 44, -1, 40, 29, -1, 22, 6, 0, 45, 41, -1, 30, 23, -1, 6, 0, 46, 42, 41, 31, 24, -1, 6, 0, 47, 43, 42, 32, 25, 23, 6, 0, 48, 44, 43, 33, -1, 24, 6, 0, 49, -1, 44, 34, -1, 25, 6, 0, 50, 45, -1, -1, 26, -1, 6, 0, 51, 46, 45, -1, 27, -1, 6, 0, 52, 47, 46, -1, 28, 26, 6, 0, 53, 48, 47, -1, 29, 27, 6, 0, 54, 49, 48, -1, -1, 28, 6, 0, 55, -1, 49, -1, -1, 29, 6, 0, -1, 50, -1, -1, 30, -1, 6, 0, -1, 51, 50, -1, 31, -1, 6, 0, -1, 52, 51, -1, 32, 30, 6, 0, -1, 53, 52, -1, 33, 31, 6, 0, -1, 54, 53, -1, 34, 32, 6, 0, -1, 55, 54, -1, -1, 33, 6, 0, -1, -1, 55, -1, -1, 34, 6, 0};
-static __constant__ float m2l_coef_m1_p6[672] = {
-  0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.0f, 0.0f, 0.5f, 0.0f, 3.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 3.0f, 0.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.0f, 0.5f, 0.0f, 0.0f, 3.0f, 3.0f, 0.0f, 0.0f, 0.0f, 0.5f, 0.0f, 0.0f, 0.0f, 6.0f, 0.0f, 0.0f, 2.0f, 0.5f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 10.0f, 5.0f, 0.0f, 4.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 10.0f, 0.0f, 5.0f, 4.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 5.0f, 5.0f, 0.0f, 0.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 5.0f, 0.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 10.0f, 5.0f, 0.0f, 4.0f, 0.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 5.0f, 10.0f, 0.0f, 0.0f, 4.0f, 0.3333333432674408f, -9.934107758624577e-09f, 0.0f, 0.0f, 15.0f, 0.0f, 0.0f, 12.0f, 0.3333333432674408f, -9.934107758624577e-09f, 28.0f, 0.0f, 0.0f, 36.0f, 0.0f, 0.0f, 0.25f, 0.0f, 21.0f, 7.0f, 0.0f, 18.0f, 0.0f, 0.0f, 0.25f, 0.0f, 21.0f, 0.0f, 7.0f, 18.0f, 0.0f, 0.0f, 0.25f, 0.0f, 14.0f, 14.0f, 0.0f, 6.0f, 6.0f, 0.0f, 0.25f, 0.0f, 14.0f, 7.0f, 7.0f, 6.0f, 0.0f, 0.0f, 0.25f, 0.0f, 14.0f, 0.0f, 14.0f, 6.0f, 0.0f, 6.0f, 0.25f, 0.0f, 7.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.0f, 0.25f, 0.0f, 7.0f, 14.0f, 7.0f, 0.0f, 6.0f, 0.0f, 0.25f, 0.0f, 7.0f, 7.0f, 14.0f, 0.0f, 0.0f, 6.0f, 0.25f, 0.0f, 7.0f, 0.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.25f, 0.0f, 0.0f, 28.0f, 0.0f, 0.0f, 36.0f, 0.0f, 0.25f, 0.0f, 0.0f, 21.0f, 7.0f, 0.0f, 18.0f, 0.0f, 0.25f, 0.0f, 0.0f, 14.0f, 14.0f, 0.0f, 6.0f, 6.0f, 0.25f, 0.0f, 0.0f, 7.0f, 21.0f, 0.0f, 0.0f, 18.0f, 0.25f, 0.0f, 0.0f, 0.0f, 28.0f, 0.0f, 0.0f, 36.0f, 0.25f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 36.0f, 9.0f, 0.0f, 48.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 36.0f, 0.0f, 9.0f, 48.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 18.0f, 0.0f, 24.0f, 8.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 9.0f, 9.0f, 24.0f, 0.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 27.0f, 0.0f, 18.0f, 24.0f, 0.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 27.0f, 0.0f, 8.0f, 24.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 18.0f, 9.0f, 8.0f, 8.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 9.0f, 18.0f, 8.0f, 0.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 18.0f, 0.0f, 27.0f, 8.0f, 0.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 27.0f, 9.0f, 0.0f, 24.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 18.0f, 18.0f, 0.0f, 8.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 9.0f, 27.0f, 0.0f, 0.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 9.0f, 0.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 36.0f, 9.0f, 0.0f, 48.0f, 0.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 27.0f, 18.0f, 0.0f, 24.0f, 8.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 18.0f, 27.0f, 0.0f, 8.0f, 24.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 9.0f, 36.0f, 0.0f, 0.0f, 48.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 0.0f, 0.0f, 45.0f, 0.0f, 0.0f, 80.0f, 0.20000000298023224f, -2.9802322831784522e-09f, 66.0f, 0.0f, 0.0f, 150.0f, 0.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 55.0f, 11.0f, 0.0f, 100.0f, 0.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 55.0f, 0.0f, 11.0f, 100.0f, 0.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 44.0f, 22.0f, 0.0f, 60.0f, 10.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 44.0f, 11.0f, 11.0f, 60.0f, 0.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 44.0f, 0.0f, 22.0f, 60.0f, 0.0f, 10.0f, 0.1666666716337204f, -4.967053879312289e-09f, 33.0f, 33.0f, 0.0f, 30.0f, 30.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 33.0f, 22.0f, 11.0f, 30.0f, 10.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 33.0f, 11.0f, 22.0f, 30.0f, 0.0f, 10.0f, 0.1666666716337204f, -4.967053879312289e-09f, 33.0f, 0.0f, 33.0f, 30.0f, 0.0f, 30.0f, 0.1666666716337204f, -4.967053879312289e-09f, 22.0f, 44.0f, 0.0f, 10.0f, 60.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 22.0f, 33.0f, 11.0f, 10.0f, 30.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 22.0f, 22.0f, 22.0f, 10.0f, 10.0f, 10.0f, 0.1666666716337204f, -4.967053879312289e-09f, 22.0f, 11.0f, 33.0f, 10.0f, 0.0f, 30.0f, 0.1666666716337204f, -4.967053879312289e-09f, 22.0f, 0.0f, 44.0f, 10.0f, 0.0f, 60.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 55.0f, 0.0f, 0.0f, 100.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 44.0f, 11.0f, 0.0f, 60.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 33.0f, 22.0f, 0.0f, 30.0f, 10.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 22.0f, 33.0f, 0.0f, 10.0f, 30.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 11.0f, 44.0f, 0.0f, 0.0f, 60.0f, 0.1666666716337204f, -4.967053879312289e-09f, 11.0f, 0.0f, 55.0f, 0.0f, 0.0f, 100.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 66.0f, 0.0f, 0.0f, 150.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 55.0f, 11.0f, 0.0f, 100.0f, 0.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 44.0f, 22.0f, 0.0f, 60.0f, 10.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 33.0f, 33.0f, 0.0f, 30.0f, 30.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 22.0f, 44.0f, 0.0f, 10.0f, 60.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 11.0f, 55.0f, 0.0f, 0.0f, 100.0f, 0.1666666716337204f, -4.967053879312289e-09f, 0.0f, 0.0f, 66.0f, 0.0f, 0.0f, 150.0f, 0.1666666716337204f, -4.967053879312289e-09f};
-static __constant__ unsigned char m2l_w_m1_p6[840] = {
-  1, 4, 5, 6, 10, 11, 12, 13, 14, 15, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 56, 57, 58, 59, 60, 61, 62, 63, 64, 65, 66, 67, 68, 69, 70, 71, 72, 73, 74, 75, 76, 2, 5, 7, 8, 11, 13, 14, 16, 17, 18, 21, 23, 24, 26, 27, 28, 30, 31, 32, 33, 36, 38, 39, 41, 42, 43, 45, 46, 47, 48, 50, 51, 52, 53, 54, 57, 59, 60, 62, 63, 64, 66, 67, 68, 69, 71, 72, 73, 74, 75, 77, 78, 79, 80, 81, 82, 3, 6, 8, 9, 12, 14, 15, 17, 18, 19, 22, 24, 25, 27, 28, 29, 31, 32, 33, 34, 37, 39, 40, 42, 43, 44, 46, 47, 48, 49, 51, 52, 53, 54, 55, 58, 60, 61, 63, 64, 65, 67, 68, 69, 70, 72, 73, 74, 75, 76, 78, 79, 80, 81, 82, 83, 4, 10, 11, 12, 20, 21, 22, 23, 24, 25, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 56, 57, 58, 59, 60, 61, 62, 63, 64, 65, 66, 67, 68, 69, 70, 5, 11, 13, 14, 21, 23, 24, 26, 27, 28, 36, 38, 39, 41, 42, 43, 45, 46, 47, 48, 57, 59, 60, 62, 63, 64, 66, 67, 68, 69, 71, 72, 73, 74, 75, 6, 12, 14, 15, 22, 24, 25, 27, 28, 29, 37, 39, 40, 42, 43, 44, 46, 47, 48, 49, 58, 60, 61, 63, 64, 65, 67, 68, 69, 70, 72, 73, 74, 75, 76, 7, 13, 16, 17, 23, 26, 27, 30, 31, 32, 38, 41, 42, 45, 46, 47, 50, 51, 52, 53, 59, 62, 63, 66, 67, 68, 71, 72, 73, 74, 77, 78, 79, 80, 81, 8, 14, 17, 18, 24, 27, 28, 31, 32, 33, 39, 42, 43, 46, 47, 48, 51, 52, 53, 54, 60, 63, 64, 67, 68, 69, 72, 73, 74, 75, 78, 79, 80, 81, 82, 9, 15, 18, 19, 25, 28, 29, 32, 33, 34, 40, 43, 44, 47, 48, 49, 52, 53, 54, 55, 61, 64, 65, 68, 69, 70, 73, 74, 75, 76, 79, 80, 81, 82, 83, 10, 20, 21, 22, 35, 36, 37, 38, 39, 40, 56, 57, 58, 59, 60, 61, 62, 63, 64, 65, 11, 21, 23, 24, 36, 38, 39, 41, 42, 43, 57, 59, 60, 62, 63, 64, 66, 67, 68, 69, 12, 22, 24, 25, 37, 39, 40, 42, 43, 44, 58, 60, 61, 63, 64, 65, 67, 68, 69, 70, 13, 23, 26, 27, 38, 41, 42, 45, 46, 47, 59, 62, 63, 66, 67, 68, 71, 72, 73, 74, 14, 24, 27, 28, 39, 42, 43, 46, 47, 48, 60, 63, 64, 67, 68, 69, 72, 73, 74, 75, 15, 25, 28, 29, 40, 43, 44, 47, 48, 49, 61, 64, 65, 68, 69, 70, 73, 74, 75, 76, 16, 26, 30, 31, 41, 45, 46, 50, 51, 52, 62, 66, 67, 71, 72, 73, 77, 78, 79, 80, 17, 27, 31, 32, 42, 46, 47, 51, 52, 53, 63, 67, 68, 72, 73, 74, 78, 79, 80, 81, 18, 28, 32, 33, 43, 47, 48, 52, 53, 54, 64, 68, 69, 73, 74, 75, 79, 80, 81, 82, 19, 29, 33, 34, 44, 48, 49, 53, 54, 55, 65, 69, 70, 74, 75, 76, 80, 81, 82, 83, 20, 35, 36, 37, 56, 57, 58, 59, 60, 61, 21, 36, 38, 39, 57, 59, 60, 62, 63, 64, 22, 37, 39, 40, 58, 60, 61, 63, 64, 65, 23, 38, 41, 42, 59, 62, 63, 66, 67, 68, 24, 39, 42, 43, 60, 63, 64, 67, 68, 69, 25, 40, 43, 44, 61, 64, 65, 68, 69, 70, 26, 41, 45, 46, 62, 66, 67, 71, 72, 73, 27, 42, 46, 47, 63, 67, 68, 72, 73, 74, 28, 43, 47, 48, 64, 68, 69, 73, 74, 75, 29, 44, 48, 49, 65, 69, 70, 74, 75, 76, 30, 45, 50, 51, 66, 71, 72, 77, 78, 79, 31, 46, 51, 52, 67, 72, 73, 78, 79, 80, 32, 47, 52, 53, 68, 73, 74, 79, 80, 81, 33, 48, 53, 54, 69, 74, 75, 80, 81, 82, 34, 49, 54, 55, 70, 75, 76, 81, 82, 83, 35, 56, 57, 58, 36, 57, 59, 60, 37, 58, 60, 61, 38, 59, 62, 63, 39, 60, 63, 64, 40, 61, 64, 65, 41, 62, 66, 67, 42, 63, 67, 68, 43, 64, 68, 69, 44, 65, 69, 70, 45, 66, 71, 72, 46, 67, 72, 73, 47, 68, 73, 74, 48, 69, 74, 75, 49, 70, 75, 76, 50, 71, 77, 78, 51, 72, 78, 79, 52, 73, 79, 80, 53, 74, 80, 81, 54, 75, 81, 82, 55, 76, 82, 83, 56, 57, 58, 59, 60, 61, 62, 63, 64, 65, 66, 67, 68, 69, 70, 71, 72, 73, 74, 75, 76, 77, 78, 79, 80, 81, 82, 83};
-
-#define CPPE_M2L_GENERATED(X) \
-  X(1, 5, m2l_m1_p5, 35, 55) \
-  X(1, 6, m2l_m1_p6, 56, 83)
+#define CPPE_M2L_REDUCED(X) \
+  X(1, 5, m1_p5, 46, 25, 35, 4, 3, 35, 55) \
+  X(1, 6, m1_p6, 64, 36, 48, 6, 3, 56, 83)
 
 #define CPPE_SHIFTS_GENERATED(X) \
   X(1, 5, 35, 55) \
   X(1, 6, 56, 83)
-
-#define CPPE_M2L_TABLES(X) \
-  X(1, 5, m1_p5, 56, 35, 55) \
-  X(1, 6, m1_p6, 84, 56, 83)
