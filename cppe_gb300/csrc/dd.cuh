@@ -256,4 +256,16 @@ __device__ __forceinline__ ddv cinv<ddv>(int o) {
   return ddv(hh, (float)(v - (double)hh));
 }
 
+// n/d for small integers in the precision of T (constant-folded)
+template <typename T>
+__device__ __forceinline__ T crat(int n, int d) {
+  return T(n) / T(d);
+}
+template <>
+__device__ __forceinline__ ddv crat<ddv>(int n, int d) {
+  const double v = (double)n / (double)d;
+  const float hh = (float)v;
+  return ddv(hh, (float)(v - (double)hh));
+}
+
 }  // namespace cg

@@ -229,8 +229,24 @@ def emit_reduced(m, p):
     name = f"m2l_m{m}_p{p}"
     head = ["  const T r2 = x * x + y * y + z * z;", "  const T ir2 = T(1) / r2;",
             "  const T D0 = rsqrt_t(r2);"]
-    rvar = ("x", "y", "z")
-    rec = []
+    # the recurrence with its factors taken out per order o:
+    #   D_n = sum_i n_i (x_i)_o D_{n-e_i} + sum_i n_i (n_i - 1) w_o D_{n-2e_i},
+    #   (x_i)_o = -(2o-1)/o x_i / R^2,  w_o = -(o-1)/o / R^2
+    head += [f"  const T {v}r = {v} * ir2;" for v in "xyz"]
+    rec, have = [], set()
+
+    def scaled(v, o, a):
+        nm = f"{v}{o}_{a}"
+        if nm not in have:
+            have.add(nm)
+            if v == "w":
+                rec.append(f"  const T {nm} = crat<T>({-(o - 1) * a * (a - 1)}, {o}) * ir2;")
+            elif a == 1:
+                rec.append(f"  const T {nm} = crat<T>({-(2 * o - 1)}, {o}) * {v}r;")
+            else:
+                rec.append(f"  const T {nm} = T({a}) * {scaled(v, o, 1)};")
+        return nm
+
     for j, n in enumerate(didx):
         o = sum(n)
         if o == 0:
@@ -239,20 +255,17 @@ def emit_reduced(m, p):
             a, b = dix[(n[0] + 2, n[1], 0)], dix[(n[0], n[1] + 2, 0)]
             rec.append(f"  const T D{j} = -(D{a} + D{b});")
             continue
-        t1, t2 = [], []
+        expr = ""
+        down = lambda i, k: dix[tuple(c - (k if i == q else 0) for q, c in enumerate(n))]
+        for i in range(3):
+            if n[i] >= 2:
+                f = (scaled("w", o, n[i]), f"D{down(i, 2)}")
+                expr = f"{f[0]} * {f[1]}" if not expr else f"fma({f[0]}, {f[1]}, {expr})"
         for i in range(3):
             if n[i] >= 1:
-                q = list(n)
-                q[i] -= 1
-                t1.append((f"T({n[i]}) * " if n[i] != 1 else "") + f"{rvar[i]} * D{dix[tuple(q)]}")
-            if n[i] >= 2:
-                q = list(n)
-                q[i] -= 2
-                t2.append(f"T({n[i] * (n[i] - 1)}) * D{dix[tuple(q)]}")
-        expr = f"T({2 * o - 1}) * ({' + '.join(t1)})"
-        if t2 and o > 1:
-            expr += f" + T({o - 1}) * ({' + '.join(t2)})"
-        rec.append(f"  const T D{j} = -({expr}) * ir2 * cinv<T>({o});")
+                f = (scaled("xyz"[i], o, n[i]), f"D{down(i, 1)}")
+                expr = f"{f[0]} * {f[1]}" if not expr else f"fma({f[0]}, {f[1]}, {expr})"
+        rec.append(f"  const T D{j} = {expr};")
     contr, last = [], -1
     for k, n, w in reduced_terms(m, p):
         if k != last:

@@ -6,14 +6,19 @@
 // takes its own source cell of the target's interaction list, evaluates the
 // straight-line translation generated by gen_m2l.py (derivative tensor and
 // partial local expansion in registers, the source multipole streamed one
-// coefficient at a time), and the lanes' partial expansions are added with
-// warp shuffles in a fixed order at the end.
+// coefficient at a time), and the lanes' partial expansions are added over the
+// warp in a fixed order at the end (m2l_scatter).
 //
 // The translation works between harmonic-reduced coefficients (z-power 0 or 1,
 // see gen_m2l.py): k_m2l_fold turns each cell's multipole into its reduced row
 // before, k_lsum gives back the full local expansion after.  Measured (M2L
 // phase with folding and per-cell sums, 300,000 sites order 6, 14.6 M
-// translations, full coefficients against reduced): MEASURED_M2L
+// translations; full coefficients -> reduced -> with the lanes' sums scattered
+// and the recurrence's factors taken out):
+//   FP32         1.54 -> 0.83 -> 0.61 ms
+//   double-float 13.8 -> 7.8 -> 5.0 ms (also: source rows loaded an order ahead
+//                two coefficients at a time, tensors copied row by row)
+//   FP64         24.9 -> 14.9 -> 12.6 ms (bound by the FP64 pipe)
 #pragma once
 
 #include "dd.cuh"
@@ -93,29 +98,95 @@ __device__ __forceinline__ void m2l_store(float2& o, double v) {
   const float h = (float)v;
   o             = make_float2(h, (float)(v - (double)h));
 }
+// Double-float rows: every order starts on a 16-byte boundary (2 o + 2 pairs
+// for order o), so that the translation loads two coefficients at a time.
+constexpr int m2l_dd_off(int m, int o) {
+  int b = 0;
+  for (int q = m; q < o; ++q) b += 2 * q + 2;
+  return b;
+}
+template <typename O>
+struct FoldRow {  // plain rows: stride and reduced coefficient of a position
+  static constexpr int stride(int, int, int ms) { return m_stride(ms); }
+  __device__ static int coef(int, int, int ms, int r) { return r < ms ? r : -1; }
+};
+template <>
+struct FoldRow<float2> {
+  static constexpr int stride(int m, int p, int) { return m2l_dd_off(m, p + 1); }
+  __device__ static int coef(int m, int, int, int r) {
+    int o = m, k = 0;
+    while (r >= 2 * o + 2) r -= 2 * o + 2, k += 2 * o + 1, ++o;
+    return r < 2 * o + 1 ? k + r : -1;
+  }
+};
 #define CPPE_DEF_FOLD(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                            \
   template <typename T, typename O>                                                          \
   __global__ void k_m2l_fold_##NAME(int ncells, const T* __restrict__ M, O* __restrict__ Mr, \
                                     const int* __restrict__ cell_seg,                        \
                                     const int* __restrict__ seg_done) {                      \
-    constexpr int RS = m_stride(MS);                                                         \
+    constexpr int RS = FoldRow<O>::stride(MM, PP, MS);                                       \
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;                            \
-    const int cell = (int)(gid / RS), row = (int)(gid % RS);                                 \
+    const int cell = (int)(gid / RS), pos = (int)(gid % RS);                                 \
     if (cell >= ncells) return;                                                              \
     if (seg_done && seg_done[cell_seg[cell]]) return; /* a batch's masked segment */         \
     T v = T(0);                                                                              \
-    if (row < (MS)) {                                                                        \
+    const int row = FoldRow<O>::coef(MM, PP, MS, pos);                                       \
+    if (row >= 0) {                                                                          \
       const T* m = M + (size_t)cell * m_stride(FMS);                                         \
       _Pragma("unroll") for (int i = 0; i < (FW); ++i) {                                     \
         const int f = m2l_fold_##NAME[row][i][1];                                            \
         if (f != 0) v = fma(T(f), m[m2l_fold_##NAME[row][i][0]], v);                         \
       }                                                                                      \
     }                                                                                        \
-    m2l_store(Mr[(size_t)cell * RS + row], v);                                               \
+    m2l_store(Mr[(size_t)cell * RS + pos], v);                                               \
   }
 CPPE_M2L_REDUCED(CPPE_DEF_FOLD)
 #undef CPPE_DEF_FOLD
 
+// Sums of N per-lane values over the warp, scattered: every step halves the
+// values a lane still holds (the lanes with the bit set keep the second half), so
+// 36 values take 37 exchanges instead of 180.  Afterwards v[0..cnt) of a lane are
+// the sums of values base, base + 1, ...; the order of the additions is fixed.
+__device__ __forceinline__ float m2l_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double m2l_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ dd m2l_xor(dd v, int o) { return {m2l_xor(v.h, o), m2l_xor(v.l, o)}; }
+__device__ __forceinline__ float m2l_add(float a, float b) { return a + b; }
+__device__ __forceinline__ double m2l_add(double a, double b) { return a + b; }
+__device__ __forceinline__ dd m2l_add(dd a, dd b) { return dd_add(a, b); }
+template <int N, int OFF, typename V>
+__device__ __forceinline__ void m2l_scatter(V* v, int lane, int& base, int& cnt) {
+  constexpr int h = (N + 1) / 2;
+  const bool up   = lane & OFF;
+#pragma unroll
+  for (int i = 0; i < h; ++i) {
+    V keep = v[i], send = v[i];
+    if (h + i < N) {
+      keep = up ? v[h + i] : v[i];
+      send = up ? v[i] : v[h + i];
+    }
+    // (an unpaired value goes to the lower lanes only)
+    const V got = m2l_xor(send, OFF);
+    v[i]        = m2l_add(keep, got);
+  }
+  base += up ? h : 0;
+  cnt = up ? max(cnt - h, 0) : min(cnt, h);
+  if constexpr (OFF > 1) m2l_scatter<h, OFF / 2>(v, lane, base, cnt);
+}
+
+// Asynchronous copy of 8 bytes to shared memory.
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src));
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// (The FP32 kernel's source rows read directly: copied to shared memory by the
+// whole warp with cp.async, the L1 wavefronts fell by two thirds and the time
+// rose from 0.61 to 0.71 ms at 300,000 sites, the copies' instructions costing
+// more than the scattered loads.)
 #define CPPE_DEF_M2L_KERNEL(M, P, NAME, NT, LS, MS, FW, UW, FLS, FMS)                      \
   template <typename T, bool PRE>                                                          \
   __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : ((P) == 5 ? 2 : 1))          \
@@ -145,14 +216,10 @@ CPPE_M2L_REDUCED(CPPE_DEF_FOLD)
         m2l_##NAME<T>((T)(cA.x - cB.x), (T)(cA.y - cB.y), (T)(cA.z - cB.z), Mb, acc);      \
       }                                                                                    \
     }                                                                                      \
-    _Pragma("unroll") for (int q = 0; q < LS; ++q) {                                       \
-      T v = acc[q];                                                                        \
-      _Pragma("unroll") for (int off = 16; off > 0; off >>= 1) v +=                        \
-            __shfl_xor_sync(0xffffffffu, v, off);                                          \
-      acc[q] = v;                                                                          \
-    }                                                                                      \
-    T* LA = Lpart + (size_t)w * (LS);                                                      \
-    _Pragma("unroll") for (int q = 0; q < LS; ++q) if ((q & 31) == lane) LA[q] = acc[q];   \
+    int first = 0, cnt = LS;                                                               \
+    m2l_scatter<LS, 16>(acc, lane, first, cnt);                                            \
+    T* LA = Lpart + (size_t)w * (LS) + first;                                              \
+    _Pragma("unroll") for (int q = 0; q < (LS + 31) / 32; ++q) if (q < cnt) LA[q] = acc[q]; \
   }
 
 CPPE_M2L_REDUCED(CPPE_DEF_M2L_KERNEL)
@@ -172,29 +239,55 @@ constexpr int m2l_wbase(int m, int p, int ko) {
   for (int o = m; o < ko; ++o) b += (nred(o) - nred(o - 1)) * nred(p - o);
   return b;
 }
+// The multipole coefficients of order KO of a lane's source, all loads in
+// flight at once.
+template <int M, int KO>
+__device__ __forceinline__ void m2l_load_dd(const float2* __restrict__ Mb, float2* mv) {
+  const float4* q = reinterpret_cast<const float4*>(Mb + m2l_dd_off(M, KO));
+#pragma unroll
+  for (int i = 0; i < KO + 1; ++i) {
+    const float4 t = q[i];
+    mv[2 * i] = make_float2(t.x, t.y), mv[2 * i + 1] = make_float2(t.z, t.w);
+  }
+}
+// mv: the coefficients of order KO, loaded while the previous order was
+// contracted (one exposed load latency per translation instead of one per
+// coefficient).  A loop over k that picks mv[k] by selects: unrolled code is
+// longer than the instruction cache holds.
 template <int M, int P, int KO, typename WT>
 __device__ __forceinline__ void m2l_contract_dd(const float2* __restrict__ D,
-                                                const float2* __restrict__ Mb, WT wtab,
-                                                dd* acc) {
-  constexpr int R = nred(P - KO), k0 = nred(KO - 1), k1 = nred(KO);
-  constexpr int base = m2l_wbase(M, P, KO), moff = nred(M - 1);
-#pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const float2 mv = Mb[k - moff];
-    const int wr    = base + (k - k0) * R;
+                                                const float2* __restrict__ Mb,
+                                                const float2* mv, WT wtab, dd* acc) {
+  constexpr int R = nred(P - KO), K = nred(KO) - nred(KO - 1);
+  constexpr int base = m2l_wbase(M, P, KO);
+  float2 nx[KO < P ? 2 * KO + 4 : 1];
+  if constexpr (KO < P) m2l_load_dd<M, KO + 1>(Mb, nx);
+  if constexpr (R == 1) {
 #pragma unroll
-    for (int n = 0; n < R; ++n) {
-      const float2 d = D[wtab(wr + n)];
-      acc[n]         = dd_fma_lazy(dd{d.x, d.y}, dd{mv.x, mv.y}, acc[n]);
+    for (int k = 0; k < K; ++k) {
+      const float2 d = D[wtab(base + k)];
+      acc[0]         = dd_fma_lazy(dd{d.x, d.y}, dd{mv[k].x, mv[k].y}, acc[0]);
+    }
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+      float2 m = mv[0];
+#pragma unroll
+      for (int i = 1; i < K; ++i) m = k == i ? mv[i] : m;
+#pragma unroll
+      for (int n = 0; n < R; ++n) {
+        const float2 d = D[wtab(base + k * R + n)];
+        acc[n]         = dd_fma_lazy(dd{d.x, d.y}, dd{m.x, m.y}, acc[n]);
+      }
     }
   }
-  if constexpr (KO < P) m2l_contract_dd<M, P, KO + 1>(D, Mb, wtab, acc);
+  if constexpr (KO < P) m2l_contract_dd<M, P, KO + 1>(D, Mb, nx, wtab, acc);
 }
 
 // TAB: tensors read from the table; else (vectors off the grid) built per entry.
 #define CPPE_DEF_M2L_DD_KERNEL(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                  \
   template <bool TAB>                                                                       \
-  __global__ void __launch_bounds__(64)                                                     \
+  __global__ void __launch_bounds__(64, TAB ? ((PP) == 5 ? 8 : 6) : 1)                      \
         k_m2l_##NAME##_dd(TreeView tv, const int4* __restrict__ chunks, int nchunks,        \
                           const float2* __restrict__ Mdd, double* __restrict__ Lpart,       \
                           const float2* __restrict__ Dtab, const int* __restrict__ vid) {   \
@@ -209,18 +302,25 @@ __device__ __forceinline__ void m2l_contract_dd(const float2* __restrict__ D,
     _Pragma("unroll") for (int q = 0; q < LS; ++q) acc[q] = dd{0.f, 0.f};                   \
     const double4_32a cA = tv.center[ch.x];                                                 \
     auto wtab = [](int i) { return (int)m2l_w_##NAME[i]; };                                 \
-    for (int idx = ch.y + lane; idx < ch.z; idx += 32) {                                    \
-      const int B = tv.m2l_src[idx];                                                        \
-      const float2* Mb = static_cast<const float2*>(                                        \
-            __builtin_assume_aligned(Mdd + (size_t)B * m_stride(MS), 16));                  \
+    for (int base = ch.y; base < ch.z; base += 32) {                                        \
+      const int cnt = min(32, ch.z - base), idx = base + min(lane, cnt - 1);                \
+      const int B   = tv.m2l_src[idx];                                                      \
+      const float2* Mb = static_cast<const float2*>(__builtin_assume_aligned(               \
+            Mdd + (size_t)B * FoldRow<float2>::stride(MM, PP, MS), 16));                    \
+      float2 mv[2 * (MM) + 2];                                                              \
+      m2l_load_dd<MM, MM>(Mb, mv);                                                          \
       if constexpr (TAB) {                                                                  \
-        /* the tabulated tensor of this entry's vector into the lane's row */               \
-        const float4* Dv = reinterpret_cast<const float4*>(Dtab + (size_t)vid[idx] * (NT)); \
-        _Pragma("unroll 8") for (int i = 0; i < (NT) / 2; ++i) {                            \
-          const float4 t = Dv[i];                                                           \
-          D[2 * i]       = make_float2(t.x, t.y);                                           \
-          D[2 * i + 1]   = make_float2(t.z, t.w);                                           \
+        /* the tabulated tensors of the round's vectors, row by row by the whole warp */    \
+        const int v = vid[idx];                                                             \
+        __syncwarp();                                                                       \
+        _Pragma("unroll 4") for (int r = 0; r < cnt; ++r) {                                 \
+          const float2* Dv = Dtab + (size_t)__shfl_sync(0xffffffffu, v, r) * (NT);          \
+          float2* o        = D - (lane - r) * DS;                                           \
+          _Pragma("unroll") for (int i = 0; i < (NT); i += 32) if (i + lane < (NT))         \
+                cp_async8(o + i + lane, Dv + i + lane);                                     \
         }                                                                                   \
+        cp_async_wait();                                                                    \
+        __syncwarp();                                                                       \
       } else {                                                                              \
         /* off the grid of tabulated vectors: the tensor built here */                      \
         const double4_32a cB = tv.center[B];                                                \
@@ -229,18 +329,13 @@ __device__ __forceinline__ void m2l_contract_dd(const float2* __restrict__ D,
                             ddv(dd_from(cA.z - cB.z)), t);                                  \
         _Pragma("unroll") for (int j = 0; j < (NT); ++j) D[j] = make_float2(t[j].h, t[j].l); \
       }                                                                                     \
-      m2l_contract_dd<MM, PP, MM>(D, Mb, wtab, acc);                                        \
+      if (lane < cnt) m2l_contract_dd<MM, PP, MM>(D, Mb, mv, wtab, acc);                    \
     }                                                                                       \
-    double* LA = Lpart + (size_t)w * (LS);                                                  \
-    _Pragma("unroll") for (int q = 0; q < LS; ++q) {                                        \
-      dd v = acc[q];                                                                        \
-      _Pragma("unroll") for (int off = 16; off > 0; off >>= 1) {                            \
-        const dd o{__shfl_xor_sync(0xffffffffu, v.h, off),                                  \
-                   __shfl_xor_sync(0xffffffffu, v.l, off)};                                 \
-        v = dd_add(v, o);                                                                   \
-      }                                                                                     \
-      if ((q & 31) == lane) LA[q] = dd_to(v);                                               \
-    }                                                                                       \
+    int first = 0, cnt = LS;                                                                \
+    m2l_scatter<LS, 16>(acc, lane, first, cnt);                                             \
+    double* LA = Lpart + (size_t)w * (LS) + first;                                          \
+    _Pragma("unroll") for (int q = 0; q < (LS + 31) / 32; ++q) if (q < cnt)                 \
+          LA[q] = dd_to(acc[q]);                                                            \
   }
 
 CPPE_M2L_REDUCED(CPPE_DEF_M2L_DD_KERNEL)
@@ -287,10 +382,11 @@ bool launch_m2l_fixed(const TreeView& tv, int m, int p, const int4* chunks, int 
 #define CPPE_LAUNCH_M2L(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                            \
   if (!ok && m == MM && p == PP) {                                                             \
     ok = true;                                                                                 \
-    Mr.alloc((size_t)std::max(1, tv.ncells) * m_stride(MS));                                   \
+    constexpr int RS = FoldRow<O>::stride(MM, PP, MS);                                         \
+    Mr.alloc((size_t)std::max(1, tv.ncells) * RS);                                             \
     Lpart.alloc((size_t)std::max(1, nchunks) * (LS));                                          \
     if (nchunks > 0) {                                                                         \
-      k_m2l_fold_##NAME<T, O><<<grid((long)tv.ncells * m_stride(MS), 256), 256, 0, s>>>(       \
+      k_m2l_fold_##NAME<T, O><<<grid((long)tv.ncells * RS, 256), 256, 0, s>>>(                 \
             tv.ncells, M, Mr.p, cell_seg, seg_done);                                           \
       CG_LAUNCH();                                                                             \
       if constexpr (DD) {                                                                      \

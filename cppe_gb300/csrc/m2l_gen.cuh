@@ -7,50 +7,98 @@ __device__ __forceinline__ void m2l_m1_p5(T x, T y, T z, const T* __restrict__ M
   const T r2 = x * x + y * y + z * z;
   const T ir2 = T(1) / r2;
   const T D0 = rsqrt_t(r2);
-  const T D1 = -(T(1) * (x * D0)) * ir2 * cinv<T>(1);
-  const T D2 = -(T(1) * (y * D0)) * ir2 * cinv<T>(1);
-  const T D3 = -(T(1) * (z * D0)) * ir2 * cinv<T>(1);
-  const T D4 = -(T(3) * (T(2) * x * D1) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D5 = -(T(3) * (x * D2 + y * D1)) * ir2 * cinv<T>(2);
-  const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
-  const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
+  const T xr = x * ir2;
+  const T yr = y * ir2;
+  const T zr = z * ir2;
+  const T x1_1 = crat<T>(-1, 1) * xr;
+  const T D1 = x1_1 * D0;
+  const T y1_1 = crat<T>(-1, 1) * yr;
+  const T D2 = y1_1 * D0;
+  const T z1_1 = crat<T>(-1, 1) * zr;
+  const T D3 = z1_1 * D0;
+  const T w2_2 = crat<T>(-2, 2) * ir2;
+  const T x2_1 = crat<T>(-3, 2) * xr;
+  const T x2_2 = T(2) * x2_1;
+  const T D4 = fma(x2_2, D1, w2_2 * D0);
+  const T y2_1 = crat<T>(-3, 2) * yr;
+  const T D5 = fma(y2_1, D1, x2_1 * D2);
+  const T z2_1 = crat<T>(-3, 2) * zr;
+  const T D6 = fma(z2_1, D1, x2_1 * D3);
+  const T y2_2 = T(2) * y2_1;
+  const T D7 = fma(y2_2, D2, w2_2 * D0);
+  const T D8 = fma(z2_1, D2, y2_1 * D3);
   const T D9 = -(D4 + D7);
-  const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
-  const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
-  const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
+  const T w3_3 = crat<T>(-12, 3) * ir2;
+  const T x3_1 = crat<T>(-5, 3) * xr;
+  const T x3_3 = T(3) * x3_1;
+  const T D10 = fma(x3_3, D4, w3_3 * D1);
+  const T w3_2 = crat<T>(-4, 3) * ir2;
+  const T x3_2 = T(2) * x3_1;
+  const T y3_1 = crat<T>(-5, 3) * yr;
+  const T D11 = fma(y3_1, D4, fma(x3_2, D5, w3_2 * D2));
+  const T z3_1 = crat<T>(-5, 3) * zr;
+  const T D12 = fma(z3_1, D4, fma(x3_2, D6, w3_2 * D3));
+  const T y3_2 = T(2) * y3_1;
+  const T D13 = fma(y3_2, D5, fma(x3_1, D7, w3_2 * D1));
+  const T D14 = fma(z3_1, D5, fma(y3_1, D6, x3_1 * D8));
   const T D15 = -(D10 + D13);
-  const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
-  const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
+  const T y3_3 = T(3) * y3_1;
+  const T D16 = fma(y3_3, D7, w3_3 * D2);
+  const T D17 = fma(z3_1, D7, fma(y3_2, D8, w3_2 * D3));
   const T D18 = -(D11 + D16);
-  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T w4_4 = crat<T>(-36, 4) * ir2;
+  const T x4_1 = crat<T>(-7, 4) * xr;
+  const T x4_4 = T(4) * x4_1;
+  const T D19 = fma(x4_4, D10, w4_4 * D4);
+  const T w4_3 = crat<T>(-18, 4) * ir2;
+  const T x4_3 = T(3) * x4_1;
+  const T y4_1 = crat<T>(-7, 4) * yr;
+  const T D20 = fma(y4_1, D10, fma(x4_3, D11, w4_3 * D5));
+  const T z4_1 = crat<T>(-7, 4) * zr;
+  const T D21 = fma(z4_1, D10, fma(x4_3, D12, w4_3 * D6));
+  const T w4_2 = crat<T>(-6, 4) * ir2;
+  const T x4_2 = T(2) * x4_1;
+  const T y4_2 = T(2) * y4_1;
+  const T D22 = fma(y4_2, D11, fma(x4_2, D13, fma(w4_2, D4, w4_2 * D7)));
+  const T D23 = fma(z4_1, D11, fma(y4_1, D12, fma(x4_2, D14, w4_2 * D8)));
   const T D24 = -(D19 + D22);
-  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T y4_3 = T(3) * y4_1;
+  const T D25 = fma(y4_3, D13, fma(x4_1, D16, w4_3 * D5));
+  const T D26 = fma(z4_1, D13, fma(y4_2, D14, fma(x4_1, D17, w4_2 * D6)));
   const T D27 = -(D20 + D25);
-  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T y4_4 = T(4) * y4_1;
+  const T D28 = fma(y4_4, D16, w4_4 * D7);
+  const T D29 = fma(z4_1, D16, fma(y4_3, D17, w4_3 * D8));
   const T D30 = -(D22 + D28);
-  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T w5_5 = crat<T>(-80, 5) * ir2;
+  const T x5_1 = crat<T>(-9, 5) * xr;
+  const T x5_5 = T(5) * x5_1;
+  const T D31 = fma(x5_5, D19, w5_5 * D10);
+  const T w5_4 = crat<T>(-48, 5) * ir2;
+  const T x5_4 = T(4) * x5_1;
+  const T y5_1 = crat<T>(-9, 5) * yr;
+  const T D32 = fma(y5_1, D19, fma(x5_4, D20, w5_4 * D11));
+  const T z5_1 = crat<T>(-9, 5) * zr;
+  const T D33 = fma(z5_1, D19, fma(x5_4, D21, w5_4 * D12));
+  const T w5_3 = crat<T>(-24, 5) * ir2;
+  const T w5_2 = crat<T>(-8, 5) * ir2;
+  const T x5_3 = T(3) * x5_1;
+  const T y5_2 = T(2) * y5_1;
+  const T D34 = fma(y5_2, D20, fma(x5_3, D22, fma(w5_2, D10, w5_3 * D13)));
+  const T D35 = fma(z5_1, D20, fma(y5_1, D21, fma(x5_3, D23, w5_3 * D14)));
   const T D36 = -(D31 + D34);
-  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T x5_2 = T(2) * x5_1;
+  const T y5_3 = T(3) * y5_1;
+  const T D37 = fma(y5_3, D22, fma(x5_2, D25, fma(w5_3, D11, w5_2 * D16)));
+  const T D38 = fma(z5_1, D22, fma(y5_2, D23, fma(x5_2, D26, fma(w5_2, D12, w5_2 * D17))));
   const T D39 = -(D32 + D37);
-  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T y5_4 = T(4) * y5_1;
+  const T D40 = fma(y5_4, D25, fma(x5_1, D28, w5_4 * D13));
+  const T D41 = fma(z5_1, D25, fma(y5_3, D26, fma(x5_1, D29, w5_3 * D14)));
   const T D42 = -(D34 + D40);
-  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T y5_5 = T(5) * y5_1;
+  const T D43 = fma(y5_5, D28, w5_5 * D16);
+  const T D44 = fma(z5_1, D28, fma(y5_4, D29, w5_4 * D17));
   const T D45 = -(D37 + D43);
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
@@ -393,50 +441,98 @@ __device__ __forceinline__ void dtensor_m1_p5(T x, T y, T z, T* __restrict__ Dou
   const T r2 = x * x + y * y + z * z;
   const T ir2 = T(1) / r2;
   const T D0 = rsqrt_t(r2);
-  const T D1 = -(T(1) * (x * D0)) * ir2 * cinv<T>(1);
-  const T D2 = -(T(1) * (y * D0)) * ir2 * cinv<T>(1);
-  const T D3 = -(T(1) * (z * D0)) * ir2 * cinv<T>(1);
-  const T D4 = -(T(3) * (T(2) * x * D1) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D5 = -(T(3) * (x * D2 + y * D1)) * ir2 * cinv<T>(2);
-  const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
-  const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
+  const T xr = x * ir2;
+  const T yr = y * ir2;
+  const T zr = z * ir2;
+  const T x1_1 = crat<T>(-1, 1) * xr;
+  const T D1 = x1_1 * D0;
+  const T y1_1 = crat<T>(-1, 1) * yr;
+  const T D2 = y1_1 * D0;
+  const T z1_1 = crat<T>(-1, 1) * zr;
+  const T D3 = z1_1 * D0;
+  const T w2_2 = crat<T>(-2, 2) * ir2;
+  const T x2_1 = crat<T>(-3, 2) * xr;
+  const T x2_2 = T(2) * x2_1;
+  const T D4 = fma(x2_2, D1, w2_2 * D0);
+  const T y2_1 = crat<T>(-3, 2) * yr;
+  const T D5 = fma(y2_1, D1, x2_1 * D2);
+  const T z2_1 = crat<T>(-3, 2) * zr;
+  const T D6 = fma(z2_1, D1, x2_1 * D3);
+  const T y2_2 = T(2) * y2_1;
+  const T D7 = fma(y2_2, D2, w2_2 * D0);
+  const T D8 = fma(z2_1, D2, y2_1 * D3);
   const T D9 = -(D4 + D7);
-  const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
-  const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
-  const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
+  const T w3_3 = crat<T>(-12, 3) * ir2;
+  const T x3_1 = crat<T>(-5, 3) * xr;
+  const T x3_3 = T(3) * x3_1;
+  const T D10 = fma(x3_3, D4, w3_3 * D1);
+  const T w3_2 = crat<T>(-4, 3) * ir2;
+  const T x3_2 = T(2) * x3_1;
+  const T y3_1 = crat<T>(-5, 3) * yr;
+  const T D11 = fma(y3_1, D4, fma(x3_2, D5, w3_2 * D2));
+  const T z3_1 = crat<T>(-5, 3) * zr;
+  const T D12 = fma(z3_1, D4, fma(x3_2, D6, w3_2 * D3));
+  const T y3_2 = T(2) * y3_1;
+  const T D13 = fma(y3_2, D5, fma(x3_1, D7, w3_2 * D1));
+  const T D14 = fma(z3_1, D5, fma(y3_1, D6, x3_1 * D8));
   const T D15 = -(D10 + D13);
-  const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
-  const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
+  const T y3_3 = T(3) * y3_1;
+  const T D16 = fma(y3_3, D7, w3_3 * D2);
+  const T D17 = fma(z3_1, D7, fma(y3_2, D8, w3_2 * D3));
   const T D18 = -(D11 + D16);
-  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T w4_4 = crat<T>(-36, 4) * ir2;
+  const T x4_1 = crat<T>(-7, 4) * xr;
+  const T x4_4 = T(4) * x4_1;
+  const T D19 = fma(x4_4, D10, w4_4 * D4);
+  const T w4_3 = crat<T>(-18, 4) * ir2;
+  const T x4_3 = T(3) * x4_1;
+  const T y4_1 = crat<T>(-7, 4) * yr;
+  const T D20 = fma(y4_1, D10, fma(x4_3, D11, w4_3 * D5));
+  const T z4_1 = crat<T>(-7, 4) * zr;
+  const T D21 = fma(z4_1, D10, fma(x4_3, D12, w4_3 * D6));
+  const T w4_2 = crat<T>(-6, 4) * ir2;
+  const T x4_2 = T(2) * x4_1;
+  const T y4_2 = T(2) * y4_1;
+  const T D22 = fma(y4_2, D11, fma(x4_2, D13, fma(w4_2, D4, w4_2 * D7)));
+  const T D23 = fma(z4_1, D11, fma(y4_1, D12, fma(x4_2, D14, w4_2 * D8)));
   const T D24 = -(D19 + D22);
-  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T y4_3 = T(3) * y4_1;
+  const T D25 = fma(y4_3, D13, fma(x4_1, D16, w4_3 * D5));
+  const T D26 = fma(z4_1, D13, fma(y4_2, D14, fma(x4_1, D17, w4_2 * D6)));
   const T D27 = -(D20 + D25);
-  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T y4_4 = T(4) * y4_1;
+  const T D28 = fma(y4_4, D16, w4_4 * D7);
+  const T D29 = fma(z4_1, D16, fma(y4_3, D17, w4_3 * D8));
   const T D30 = -(D22 + D28);
-  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T w5_5 = crat<T>(-80, 5) * ir2;
+  const T x5_1 = crat<T>(-9, 5) * xr;
+  const T x5_5 = T(5) * x5_1;
+  const T D31 = fma(x5_5, D19, w5_5 * D10);
+  const T w5_4 = crat<T>(-48, 5) * ir2;
+  const T x5_4 = T(4) * x5_1;
+  const T y5_1 = crat<T>(-9, 5) * yr;
+  const T D32 = fma(y5_1, D19, fma(x5_4, D20, w5_4 * D11));
+  const T z5_1 = crat<T>(-9, 5) * zr;
+  const T D33 = fma(z5_1, D19, fma(x5_4, D21, w5_4 * D12));
+  const T w5_3 = crat<T>(-24, 5) * ir2;
+  const T w5_2 = crat<T>(-8, 5) * ir2;
+  const T x5_3 = T(3) * x5_1;
+  const T y5_2 = T(2) * y5_1;
+  const T D34 = fma(y5_2, D20, fma(x5_3, D22, fma(w5_2, D10, w5_3 * D13)));
+  const T D35 = fma(z5_1, D20, fma(y5_1, D21, fma(x5_3, D23, w5_3 * D14)));
   const T D36 = -(D31 + D34);
-  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T x5_2 = T(2) * x5_1;
+  const T y5_3 = T(3) * y5_1;
+  const T D37 = fma(y5_3, D22, fma(x5_2, D25, fma(w5_3, D11, w5_2 * D16)));
+  const T D38 = fma(z5_1, D22, fma(y5_2, D23, fma(x5_2, D26, fma(w5_2, D12, w5_2 * D17))));
   const T D39 = -(D32 + D37);
-  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T y5_4 = T(4) * y5_1;
+  const T D40 = fma(y5_4, D25, fma(x5_1, D28, w5_4 * D13));
+  const T D41 = fma(z5_1, D25, fma(y5_3, D26, fma(x5_1, D29, w5_3 * D14)));
   const T D42 = -(D34 + D40);
-  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T y5_5 = T(5) * y5_1;
+  const T D43 = fma(y5_5, D28, w5_5 * D16);
+  const T D44 = fma(z5_1, D28, fma(y5_4, D29, w5_4 * D17));
   const T D45 = -(D37 + D43);
   Dout[0] = D0;
   Dout[1] = D1;
@@ -952,68 +1048,134 @@ __device__ __forceinline__ void m2l_m1_p6(T x, T y, T z, const T* __restrict__ M
   const T r2 = x * x + y * y + z * z;
   const T ir2 = T(1) / r2;
   const T D0 = rsqrt_t(r2);
-  const T D1 = -(T(1) * (x * D0)) * ir2 * cinv<T>(1);
-  const T D2 = -(T(1) * (y * D0)) * ir2 * cinv<T>(1);
-  const T D3 = -(T(1) * (z * D0)) * ir2 * cinv<T>(1);
-  const T D4 = -(T(3) * (T(2) * x * D1) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D5 = -(T(3) * (x * D2 + y * D1)) * ir2 * cinv<T>(2);
-  const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
-  const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
+  const T xr = x * ir2;
+  const T yr = y * ir2;
+  const T zr = z * ir2;
+  const T x1_1 = crat<T>(-1, 1) * xr;
+  const T D1 = x1_1 * D0;
+  const T y1_1 = crat<T>(-1, 1) * yr;
+  const T D2 = y1_1 * D0;
+  const T z1_1 = crat<T>(-1, 1) * zr;
+  const T D3 = z1_1 * D0;
+  const T w2_2 = crat<T>(-2, 2) * ir2;
+  const T x2_1 = crat<T>(-3, 2) * xr;
+  const T x2_2 = T(2) * x2_1;
+  const T D4 = fma(x2_2, D1, w2_2 * D0);
+  const T y2_1 = crat<T>(-3, 2) * yr;
+  const T D5 = fma(y2_1, D1, x2_1 * D2);
+  const T z2_1 = crat<T>(-3, 2) * zr;
+  const T D6 = fma(z2_1, D1, x2_1 * D3);
+  const T y2_2 = T(2) * y2_1;
+  const T D7 = fma(y2_2, D2, w2_2 * D0);
+  const T D8 = fma(z2_1, D2, y2_1 * D3);
   const T D9 = -(D4 + D7);
-  const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
-  const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
-  const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
+  const T w3_3 = crat<T>(-12, 3) * ir2;
+  const T x3_1 = crat<T>(-5, 3) * xr;
+  const T x3_3 = T(3) * x3_1;
+  const T D10 = fma(x3_3, D4, w3_3 * D1);
+  const T w3_2 = crat<T>(-4, 3) * ir2;
+  const T x3_2 = T(2) * x3_1;
+  const T y3_1 = crat<T>(-5, 3) * yr;
+  const T D11 = fma(y3_1, D4, fma(x3_2, D5, w3_2 * D2));
+  const T z3_1 = crat<T>(-5, 3) * zr;
+  const T D12 = fma(z3_1, D4, fma(x3_2, D6, w3_2 * D3));
+  const T y3_2 = T(2) * y3_1;
+  const T D13 = fma(y3_2, D5, fma(x3_1, D7, w3_2 * D1));
+  const T D14 = fma(z3_1, D5, fma(y3_1, D6, x3_1 * D8));
   const T D15 = -(D10 + D13);
-  const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
-  const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
+  const T y3_3 = T(3) * y3_1;
+  const T D16 = fma(y3_3, D7, w3_3 * D2);
+  const T D17 = fma(z3_1, D7, fma(y3_2, D8, w3_2 * D3));
   const T D18 = -(D11 + D16);
-  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T w4_4 = crat<T>(-36, 4) * ir2;
+  const T x4_1 = crat<T>(-7, 4) * xr;
+  const T x4_4 = T(4) * x4_1;
+  const T D19 = fma(x4_4, D10, w4_4 * D4);
+  const T w4_3 = crat<T>(-18, 4) * ir2;
+  const T x4_3 = T(3) * x4_1;
+  const T y4_1 = crat<T>(-7, 4) * yr;
+  const T D20 = fma(y4_1, D10, fma(x4_3, D11, w4_3 * D5));
+  const T z4_1 = crat<T>(-7, 4) * zr;
+  const T D21 = fma(z4_1, D10, fma(x4_3, D12, w4_3 * D6));
+  const T w4_2 = crat<T>(-6, 4) * ir2;
+  const T x4_2 = T(2) * x4_1;
+  const T y4_2 = T(2) * y4_1;
+  const T D22 = fma(y4_2, D11, fma(x4_2, D13, fma(w4_2, D4, w4_2 * D7)));
+  const T D23 = fma(z4_1, D11, fma(y4_1, D12, fma(x4_2, D14, w4_2 * D8)));
   const T D24 = -(D19 + D22);
-  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T y4_3 = T(3) * y4_1;
+  const T D25 = fma(y4_3, D13, fma(x4_1, D16, w4_3 * D5));
+  const T D26 = fma(z4_1, D13, fma(y4_2, D14, fma(x4_1, D17, w4_2 * D6)));
   const T D27 = -(D20 + D25);
-  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T y4_4 = T(4) * y4_1;
+  const T D28 = fma(y4_4, D16, w4_4 * D7);
+  const T D29 = fma(z4_1, D16, fma(y4_3, D17, w4_3 * D8));
   const T D30 = -(D22 + D28);
-  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T w5_5 = crat<T>(-80, 5) * ir2;
+  const T x5_1 = crat<T>(-9, 5) * xr;
+  const T x5_5 = T(5) * x5_1;
+  const T D31 = fma(x5_5, D19, w5_5 * D10);
+  const T w5_4 = crat<T>(-48, 5) * ir2;
+  const T x5_4 = T(4) * x5_1;
+  const T y5_1 = crat<T>(-9, 5) * yr;
+  const T D32 = fma(y5_1, D19, fma(x5_4, D20, w5_4 * D11));
+  const T z5_1 = crat<T>(-9, 5) * zr;
+  const T D33 = fma(z5_1, D19, fma(x5_4, D21, w5_4 * D12));
+  const T w5_3 = crat<T>(-24, 5) * ir2;
+  const T w5_2 = crat<T>(-8, 5) * ir2;
+  const T x5_3 = T(3) * x5_1;
+  const T y5_2 = T(2) * y5_1;
+  const T D34 = fma(y5_2, D20, fma(x5_3, D22, fma(w5_2, D10, w5_3 * D13)));
+  const T D35 = fma(z5_1, D20, fma(y5_1, D21, fma(x5_3, D23, w5_3 * D14)));
   const T D36 = -(D31 + D34);
-  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T x5_2 = T(2) * x5_1;
+  const T y5_3 = T(3) * y5_1;
+  const T D37 = fma(y5_3, D22, fma(x5_2, D25, fma(w5_3, D11, w5_2 * D16)));
+  const T D38 = fma(z5_1, D22, fma(y5_2, D23, fma(x5_2, D26, fma(w5_2, D12, w5_2 * D17))));
   const T D39 = -(D32 + D37);
-  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T y5_4 = T(4) * y5_1;
+  const T D40 = fma(y5_4, D25, fma(x5_1, D28, w5_4 * D13));
+  const T D41 = fma(z5_1, D25, fma(y5_3, D26, fma(x5_1, D29, w5_3 * D14)));
   const T D42 = -(D34 + D40);
-  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T y5_5 = T(5) * y5_1;
+  const T D43 = fma(y5_5, D28, w5_5 * D16);
+  const T D44 = fma(z5_1, D28, fma(y5_4, D29, w5_4 * D17));
   const T D45 = -(D37 + D43);
-  const T D46 = -(T(11) * (T(6) * x * D31) + T(5) * (T(30) * D19)) * ir2 * cinv<T>(6);
-  const T D47 = -(T(11) * (T(5) * x * D32 + y * D31) + T(5) * (T(20) * D20)) * ir2 * cinv<T>(6);
-  const T D48 = -(T(11) * (T(5) * x * D33 + z * D31) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
-  const T D49 = -(T(11) * (T(4) * x * D34 + T(2) * y * D32) + T(5) * (T(12) * D22 + T(2) * D19)) * ir2 * cinv<T>(6);
-  const T D50 = -(T(11) * (T(4) * x * D35 + y * D33 + z * D32) + T(5) * (T(12) * D23)) * ir2 * cinv<T>(6);
+  const T w6_6 = crat<T>(-150, 6) * ir2;
+  const T x6_1 = crat<T>(-11, 6) * xr;
+  const T x6_6 = T(6) * x6_1;
+  const T D46 = fma(x6_6, D31, w6_6 * D19);
+  const T w6_5 = crat<T>(-100, 6) * ir2;
+  const T x6_5 = T(5) * x6_1;
+  const T y6_1 = crat<T>(-11, 6) * yr;
+  const T D47 = fma(y6_1, D31, fma(x6_5, D32, w6_5 * D20));
+  const T z6_1 = crat<T>(-11, 6) * zr;
+  const T D48 = fma(z6_1, D31, fma(x6_5, D33, w6_5 * D21));
+  const T w6_4 = crat<T>(-60, 6) * ir2;
+  const T w6_2 = crat<T>(-10, 6) * ir2;
+  const T x6_4 = T(4) * x6_1;
+  const T y6_2 = T(2) * y6_1;
+  const T D49 = fma(y6_2, D32, fma(x6_4, D34, fma(w6_2, D19, w6_4 * D22)));
+  const T D50 = fma(z6_1, D32, fma(y6_1, D33, fma(x6_4, D35, w6_4 * D23)));
   const T D51 = -(D46 + D49);
-  const T D52 = -(T(11) * (T(3) * x * D37 + T(3) * y * D34) + T(5) * (T(6) * D25 + T(6) * D20)) * ir2 * cinv<T>(6);
-  const T D53 = -(T(11) * (T(3) * x * D38 + T(2) * y * D35 + z * D34) + T(5) * (T(6) * D26 + T(2) * D21)) * ir2 * cinv<T>(6);
+  const T w6_3 = crat<T>(-30, 6) * ir2;
+  const T x6_3 = T(3) * x6_1;
+  const T y6_3 = T(3) * y6_1;
+  const T D52 = fma(y6_3, D34, fma(x6_3, D37, fma(w6_3, D20, w6_3 * D25)));
+  const T D53 = fma(z6_1, D34, fma(y6_2, D35, fma(x6_3, D38, fma(w6_2, D21, w6_3 * D26))));
   const T D54 = -(D47 + D52);
-  const T D55 = -(T(11) * (T(2) * x * D40 + T(4) * y * D37) + T(5) * (T(2) * D28 + T(12) * D22)) * ir2 * cinv<T>(6);
-  const T D56 = -(T(11) * (T(2) * x * D41 + T(3) * y * D38 + z * D37) + T(5) * (T(2) * D29 + T(6) * D23)) * ir2 * cinv<T>(6);
+  const T x6_2 = T(2) * x6_1;
+  const T y6_4 = T(4) * y6_1;
+  const T D55 = fma(y6_4, D37, fma(x6_2, D40, fma(w6_4, D22, w6_2 * D28)));
+  const T D56 = fma(z6_1, D37, fma(y6_3, D38, fma(x6_2, D41, fma(w6_3, D23, w6_2 * D29))));
   const T D57 = -(D49 + D55);
-  const T D58 = -(T(11) * (x * D43 + T(5) * y * D40) + T(5) * (T(20) * D25)) * ir2 * cinv<T>(6);
-  const T D59 = -(T(11) * (x * D44 + T(4) * y * D41 + z * D40) + T(5) * (T(12) * D26)) * ir2 * cinv<T>(6);
+  const T y6_5 = T(5) * y6_1;
+  const T D58 = fma(y6_5, D40, fma(x6_1, D43, w6_5 * D25));
+  const T D59 = fma(z6_1, D40, fma(y6_4, D41, fma(x6_1, D44, w6_4 * D26)));
   const T D60 = -(D52 + D58);
-  const T D61 = -(T(11) * (T(6) * y * D43) + T(5) * (T(30) * D28)) * ir2 * cinv<T>(6);
-  const T D62 = -(T(11) * (T(5) * y * D44 + z * D43) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
+  const T y6_6 = T(6) * y6_1;
+  const T D61 = fma(y6_6, D43, w6_6 * D28);
+  const T D62 = fma(z6_1, D43, fma(y6_5, D44, w6_5 * D29));
   const T D63 = -(D55 + D61);
   { const T mk = Mb[0];
     acc[0] = fma(D1, mk, acc[0]);
@@ -1600,68 +1762,134 @@ __device__ __forceinline__ void dtensor_m1_p6(T x, T y, T z, T* __restrict__ Dou
   const T r2 = x * x + y * y + z * z;
   const T ir2 = T(1) / r2;
   const T D0 = rsqrt_t(r2);
-  const T D1 = -(T(1) * (x * D0)) * ir2 * cinv<T>(1);
-  const T D2 = -(T(1) * (y * D0)) * ir2 * cinv<T>(1);
-  const T D3 = -(T(1) * (z * D0)) * ir2 * cinv<T>(1);
-  const T D4 = -(T(3) * (T(2) * x * D1) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D5 = -(T(3) * (x * D2 + y * D1)) * ir2 * cinv<T>(2);
-  const T D6 = -(T(3) * (x * D3 + z * D1)) * ir2 * cinv<T>(2);
-  const T D7 = -(T(3) * (T(2) * y * D2) + T(1) * (T(2) * D0)) * ir2 * cinv<T>(2);
-  const T D8 = -(T(3) * (y * D3 + z * D2)) * ir2 * cinv<T>(2);
+  const T xr = x * ir2;
+  const T yr = y * ir2;
+  const T zr = z * ir2;
+  const T x1_1 = crat<T>(-1, 1) * xr;
+  const T D1 = x1_1 * D0;
+  const T y1_1 = crat<T>(-1, 1) * yr;
+  const T D2 = y1_1 * D0;
+  const T z1_1 = crat<T>(-1, 1) * zr;
+  const T D3 = z1_1 * D0;
+  const T w2_2 = crat<T>(-2, 2) * ir2;
+  const T x2_1 = crat<T>(-3, 2) * xr;
+  const T x2_2 = T(2) * x2_1;
+  const T D4 = fma(x2_2, D1, w2_2 * D0);
+  const T y2_1 = crat<T>(-3, 2) * yr;
+  const T D5 = fma(y2_1, D1, x2_1 * D2);
+  const T z2_1 = crat<T>(-3, 2) * zr;
+  const T D6 = fma(z2_1, D1, x2_1 * D3);
+  const T y2_2 = T(2) * y2_1;
+  const T D7 = fma(y2_2, D2, w2_2 * D0);
+  const T D8 = fma(z2_1, D2, y2_1 * D3);
   const T D9 = -(D4 + D7);
-  const T D10 = -(T(5) * (T(3) * x * D4) + T(2) * (T(6) * D1)) * ir2 * cinv<T>(3);
-  const T D11 = -(T(5) * (T(2) * x * D5 + y * D4) + T(2) * (T(2) * D2)) * ir2 * cinv<T>(3);
-  const T D12 = -(T(5) * (T(2) * x * D6 + z * D4) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
-  const T D13 = -(T(5) * (x * D7 + T(2) * y * D5) + T(2) * (T(2) * D1)) * ir2 * cinv<T>(3);
-  const T D14 = -(T(5) * (x * D8 + y * D6 + z * D5)) * ir2 * cinv<T>(3);
+  const T w3_3 = crat<T>(-12, 3) * ir2;
+  const T x3_1 = crat<T>(-5, 3) * xr;
+  const T x3_3 = T(3) * x3_1;
+  const T D10 = fma(x3_3, D4, w3_3 * D1);
+  const T w3_2 = crat<T>(-4, 3) * ir2;
+  const T x3_2 = T(2) * x3_1;
+  const T y3_1 = crat<T>(-5, 3) * yr;
+  const T D11 = fma(y3_1, D4, fma(x3_2, D5, w3_2 * D2));
+  const T z3_1 = crat<T>(-5, 3) * zr;
+  const T D12 = fma(z3_1, D4, fma(x3_2, D6, w3_2 * D3));
+  const T y3_2 = T(2) * y3_1;
+  const T D13 = fma(y3_2, D5, fma(x3_1, D7, w3_2 * D1));
+  const T D14 = fma(z3_1, D5, fma(y3_1, D6, x3_1 * D8));
   const T D15 = -(D10 + D13);
-  const T D16 = -(T(5) * (T(3) * y * D7) + T(2) * (T(6) * D2)) * ir2 * cinv<T>(3);
-  const T D17 = -(T(5) * (T(2) * y * D8 + z * D7) + T(2) * (T(2) * D3)) * ir2 * cinv<T>(3);
+  const T y3_3 = T(3) * y3_1;
+  const T D16 = fma(y3_3, D7, w3_3 * D2);
+  const T D17 = fma(z3_1, D7, fma(y3_2, D8, w3_2 * D3));
   const T D18 = -(D11 + D16);
-  const T D19 = -(T(7) * (T(4) * x * D10) + T(3) * (T(12) * D4)) * ir2 * cinv<T>(4);
-  const T D20 = -(T(7) * (T(3) * x * D11 + y * D10) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D21 = -(T(7) * (T(3) * x * D12 + z * D10) + T(3) * (T(6) * D6)) * ir2 * cinv<T>(4);
-  const T D22 = -(T(7) * (T(2) * x * D13 + T(2) * y * D11) + T(3) * (T(2) * D7 + T(2) * D4)) * ir2 * cinv<T>(4);
-  const T D23 = -(T(7) * (T(2) * x * D14 + y * D12 + z * D11) + T(3) * (T(2) * D8)) * ir2 * cinv<T>(4);
+  const T w4_4 = crat<T>(-36, 4) * ir2;
+  const T x4_1 = crat<T>(-7, 4) * xr;
+  const T x4_4 = T(4) * x4_1;
+  const T D19 = fma(x4_4, D10, w4_4 * D4);
+  const T w4_3 = crat<T>(-18, 4) * ir2;
+  const T x4_3 = T(3) * x4_1;
+  const T y4_1 = crat<T>(-7, 4) * yr;
+  const T D20 = fma(y4_1, D10, fma(x4_3, D11, w4_3 * D5));
+  const T z4_1 = crat<T>(-7, 4) * zr;
+  const T D21 = fma(z4_1, D10, fma(x4_3, D12, w4_3 * D6));
+  const T w4_2 = crat<T>(-6, 4) * ir2;
+  const T x4_2 = T(2) * x4_1;
+  const T y4_2 = T(2) * y4_1;
+  const T D22 = fma(y4_2, D11, fma(x4_2, D13, fma(w4_2, D4, w4_2 * D7)));
+  const T D23 = fma(z4_1, D11, fma(y4_1, D12, fma(x4_2, D14, w4_2 * D8)));
   const T D24 = -(D19 + D22);
-  const T D25 = -(T(7) * (x * D16 + T(3) * y * D13) + T(3) * (T(6) * D5)) * ir2 * cinv<T>(4);
-  const T D26 = -(T(7) * (x * D17 + T(2) * y * D14 + z * D13) + T(3) * (T(2) * D6)) * ir2 * cinv<T>(4);
+  const T y4_3 = T(3) * y4_1;
+  const T D25 = fma(y4_3, D13, fma(x4_1, D16, w4_3 * D5));
+  const T D26 = fma(z4_1, D13, fma(y4_2, D14, fma(x4_1, D17, w4_2 * D6)));
   const T D27 = -(D20 + D25);
-  const T D28 = -(T(7) * (T(4) * y * D16) + T(3) * (T(12) * D7)) * ir2 * cinv<T>(4);
-  const T D29 = -(T(7) * (T(3) * y * D17 + z * D16) + T(3) * (T(6) * D8)) * ir2 * cinv<T>(4);
+  const T y4_4 = T(4) * y4_1;
+  const T D28 = fma(y4_4, D16, w4_4 * D7);
+  const T D29 = fma(z4_1, D16, fma(y4_3, D17, w4_3 * D8));
   const T D30 = -(D22 + D28);
-  const T D31 = -(T(9) * (T(5) * x * D19) + T(4) * (T(20) * D10)) * ir2 * cinv<T>(5);
-  const T D32 = -(T(9) * (T(4) * x * D20 + y * D19) + T(4) * (T(12) * D11)) * ir2 * cinv<T>(5);
-  const T D33 = -(T(9) * (T(4) * x * D21 + z * D19) + T(4) * (T(12) * D12)) * ir2 * cinv<T>(5);
-  const T D34 = -(T(9) * (T(3) * x * D22 + T(2) * y * D20) + T(4) * (T(6) * D13 + T(2) * D10)) * ir2 * cinv<T>(5);
-  const T D35 = -(T(9) * (T(3) * x * D23 + y * D21 + z * D20) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T w5_5 = crat<T>(-80, 5) * ir2;
+  const T x5_1 = crat<T>(-9, 5) * xr;
+  const T x5_5 = T(5) * x5_1;
+  const T D31 = fma(x5_5, D19, w5_5 * D10);
+  const T w5_4 = crat<T>(-48, 5) * ir2;
+  const T x5_4 = T(4) * x5_1;
+  const T y5_1 = crat<T>(-9, 5) * yr;
+  const T D32 = fma(y5_1, D19, fma(x5_4, D20, w5_4 * D11));
+  const T z5_1 = crat<T>(-9, 5) * zr;
+  const T D33 = fma(z5_1, D19, fma(x5_4, D21, w5_4 * D12));
+  const T w5_3 = crat<T>(-24, 5) * ir2;
+  const T w5_2 = crat<T>(-8, 5) * ir2;
+  const T x5_3 = T(3) * x5_1;
+  const T y5_2 = T(2) * y5_1;
+  const T D34 = fma(y5_2, D20, fma(x5_3, D22, fma(w5_2, D10, w5_3 * D13)));
+  const T D35 = fma(z5_1, D20, fma(y5_1, D21, fma(x5_3, D23, w5_3 * D14)));
   const T D36 = -(D31 + D34);
-  const T D37 = -(T(9) * (T(2) * x * D25 + T(3) * y * D22) + T(4) * (T(2) * D16 + T(6) * D11)) * ir2 * cinv<T>(5);
-  const T D38 = -(T(9) * (T(2) * x * D26 + T(2) * y * D23 + z * D22) + T(4) * (T(2) * D17 + T(2) * D12)) * ir2 * cinv<T>(5);
+  const T x5_2 = T(2) * x5_1;
+  const T y5_3 = T(3) * y5_1;
+  const T D37 = fma(y5_3, D22, fma(x5_2, D25, fma(w5_3, D11, w5_2 * D16)));
+  const T D38 = fma(z5_1, D22, fma(y5_2, D23, fma(x5_2, D26, fma(w5_2, D12, w5_2 * D17))));
   const T D39 = -(D32 + D37);
-  const T D40 = -(T(9) * (x * D28 + T(4) * y * D25) + T(4) * (T(12) * D13)) * ir2 * cinv<T>(5);
-  const T D41 = -(T(9) * (x * D29 + T(3) * y * D26 + z * D25) + T(4) * (T(6) * D14)) * ir2 * cinv<T>(5);
+  const T y5_4 = T(4) * y5_1;
+  const T D40 = fma(y5_4, D25, fma(x5_1, D28, w5_4 * D13));
+  const T D41 = fma(z5_1, D25, fma(y5_3, D26, fma(x5_1, D29, w5_3 * D14)));
   const T D42 = -(D34 + D40);
-  const T D43 = -(T(9) * (T(5) * y * D28) + T(4) * (T(20) * D16)) * ir2 * cinv<T>(5);
-  const T D44 = -(T(9) * (T(4) * y * D29 + z * D28) + T(4) * (T(12) * D17)) * ir2 * cinv<T>(5);
+  const T y5_5 = T(5) * y5_1;
+  const T D43 = fma(y5_5, D28, w5_5 * D16);
+  const T D44 = fma(z5_1, D28, fma(y5_4, D29, w5_4 * D17));
   const T D45 = -(D37 + D43);
-  const T D46 = -(T(11) * (T(6) * x * D31) + T(5) * (T(30) * D19)) * ir2 * cinv<T>(6);
-  const T D47 = -(T(11) * (T(5) * x * D32 + y * D31) + T(5) * (T(20) * D20)) * ir2 * cinv<T>(6);
-  const T D48 = -(T(11) * (T(5) * x * D33 + z * D31) + T(5) * (T(20) * D21)) * ir2 * cinv<T>(6);
-  const T D49 = -(T(11) * (T(4) * x * D34 + T(2) * y * D32) + T(5) * (T(12) * D22 + T(2) * D19)) * ir2 * cinv<T>(6);
-  const T D50 = -(T(11) * (T(4) * x * D35 + y * D33 + z * D32) + T(5) * (T(12) * D23)) * ir2 * cinv<T>(6);
+  const T w6_6 = crat<T>(-150, 6) * ir2;
+  const T x6_1 = crat<T>(-11, 6) * xr;
+  const T x6_6 = T(6) * x6_1;
+  const T D46 = fma(x6_6, D31, w6_6 * D19);
+  const T w6_5 = crat<T>(-100, 6) * ir2;
+  const T x6_5 = T(5) * x6_1;
+  const T y6_1 = crat<T>(-11, 6) * yr;
+  const T D47 = fma(y6_1, D31, fma(x6_5, D32, w6_5 * D20));
+  const T z6_1 = crat<T>(-11, 6) * zr;
+  const T D48 = fma(z6_1, D31, fma(x6_5, D33, w6_5 * D21));
+  const T w6_4 = crat<T>(-60, 6) * ir2;
+  const T w6_2 = crat<T>(-10, 6) * ir2;
+  const T x6_4 = T(4) * x6_1;
+  const T y6_2 = T(2) * y6_1;
+  const T D49 = fma(y6_2, D32, fma(x6_4, D34, fma(w6_2, D19, w6_4 * D22)));
+  const T D50 = fma(z6_1, D32, fma(y6_1, D33, fma(x6_4, D35, w6_4 * D23)));
   const T D51 = -(D46 + D49);
-  const T D52 = -(T(11) * (T(3) * x * D37 + T(3) * y * D34) + T(5) * (T(6) * D25 + T(6) * D20)) * ir2 * cinv<T>(6);
-  const T D53 = -(T(11) * (T(3) * x * D38 + T(2) * y * D35 + z * D34) + T(5) * (T(6) * D26 + T(2) * D21)) * ir2 * cinv<T>(6);
+  const T w6_3 = crat<T>(-30, 6) * ir2;
+  const T x6_3 = T(3) * x6_1;
+  const T y6_3 = T(3) * y6_1;
+  const T D52 = fma(y6_3, D34, fma(x6_3, D37, fma(w6_3, D20, w6_3 * D25)));
+  const T D53 = fma(z6_1, D34, fma(y6_2, D35, fma(x6_3, D38, fma(w6_2, D21, w6_3 * D26))));
   const T D54 = -(D47 + D52);
-  const T D55 = -(T(11) * (T(2) * x * D40 + T(4) * y * D37) + T(5) * (T(2) * D28 + T(12) * D22)) * ir2 * cinv<T>(6);
-  const T D56 = -(T(11) * (T(2) * x * D41 + T(3) * y * D38 + z * D37) + T(5) * (T(2) * D29 + T(6) * D23)) * ir2 * cinv<T>(6);
+  const T x6_2 = T(2) * x6_1;
+  const T y6_4 = T(4) * y6_1;
+  const T D55 = fma(y6_4, D37, fma(x6_2, D40, fma(w6_4, D22, w6_2 * D28)));
+  const T D56 = fma(z6_1, D37, fma(y6_3, D38, fma(x6_2, D41, fma(w6_3, D23, w6_2 * D29))));
   const T D57 = -(D49 + D55);
-  const T D58 = -(T(11) * (x * D43 + T(5) * y * D40) + T(5) * (T(20) * D25)) * ir2 * cinv<T>(6);
-  const T D59 = -(T(11) * (x * D44 + T(4) * y * D41 + z * D40) + T(5) * (T(12) * D26)) * ir2 * cinv<T>(6);
+  const T y6_5 = T(5) * y6_1;
+  const T D58 = fma(y6_5, D40, fma(x6_1, D43, w6_5 * D25));
+  const T D59 = fma(z6_1, D40, fma(y6_4, D41, fma(x6_1, D44, w6_4 * D26)));
   const T D60 = -(D52 + D58);
-  const T D61 = -(T(11) * (T(6) * y * D43) + T(5) * (T(30) * D28)) * ir2 * cinv<T>(6);
-  const T D62 = -(T(11) * (T(5) * y * D44 + z * D43) + T(5) * (T(20) * D29)) * ir2 * cinv<T>(6);
+  const T y6_6 = T(6) * y6_1;
+  const T D61 = fma(y6_6, D43, w6_6 * D28);
+  const T D62 = fma(z6_1, D43, fma(y6_5, D44, w6_5 * D29));
   const T D63 = -(D55 + D61);
   Dout[0] = D0;
   Dout[1] = D1;
