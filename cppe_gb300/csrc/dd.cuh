@@ -212,6 +212,42 @@ __device__ __forceinline__ dd2 dd2_exp_neg(dd2 v, const float* tab_h, const floa
 }
 
 // ---------------------------------------------------------------------------
+// Conversions by moving bits: the conversion instructions run at the FP64 rate.
+// ---------------------------------------------------------------------------
+// float -> double; zero becomes 2^-127
+__device__ __forceinline__ double f2d_bits(float x) {
+  const unsigned u = __float_as_uint(x);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)),
+                          (int)(u << 29));
+}
+// double -> float, truncated, by moving the bits: positive values in FP32's
+// range (d2f_bits), or any sign with small values taken as zero (d2f_bits0)
+__device__ __forceinline__ float d2f_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  return __uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ float d2f_bits0(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned m  = hi & 0x7fffffffu;
+  return m < 0x39000000u
+               ? 0.f
+               : __uint_as_float((hi & 0x80000000u) | ((m - 0x38000000u) << 3) | (lo >> 29));
+}
+// The 29 mantissa bits of a positive double that d2f_bits leaves out, as FP32.
+__device__ __forceinline__ float d2f_rest(double x) {
+  const unsigned ex = (unsigned)__double2hiint(x) >> 20;
+  return (float)((unsigned)__double2loint(x) & 0x1fffffffu) *
+         __uint_as_float((ex - (1023 - 127) - 52) << 23);
+}
+// 1/sqrt(r2) to FP32 accuracy as a double (0 for r2 = 0), the seed of FP64
+// corrections; below 2^-100, where FP32 would underflow, the FP64 function.
+__device__ __forceinline__ double rsqrt_seed(double r2) {
+  const int hi = __double2hiint(r2);
+  if (hi >= ((1023 - 100) << 20)) return f2d_bits(rsqrt_ftz(d2f_bits(r2)));
+  return (hi | __double2loint(r2)) == 0 ? 0.0 : rsqrt(r2);
+}
+
+// ---------------------------------------------------------------------------
 // A value type over dd for generic code (the generated M2L translations):
 // +, -, * with dd accuracy, division by a Newton-corrected quotient.
 // ---------------------------------------------------------------------------

@@ -41,8 +41,10 @@ This file is run by the build
 import os
 import sys
 
-# (source order m, expansion order p) pairs to emit
+# (source order m, expansion order p) pairs to emit: with shifts, and M2L only
+# (charges and quadrupoles of the static fields)
 ORDERS = [(1, 5), (1, 6)]
+M2L_ONLY = [(0, 5), (0, 6), (2, 5), (2, 6)]
 
 
 def nterms(p):
@@ -426,7 +428,7 @@ def emit_shifts(m, p):
 def main(out_path):
     parts = ["// Generated by gen_m2l.py -- do not edit.", "#pragma once", ""]
     red, shifts = [], []
-    for m, p in ORDERS:
+    for m, p in ORDERS + M2L_ONLY:
         code, *r = emit_reduced(m, p)
         parts += [code, ""]
         red.append((m, p, *r))
@@ -435,11 +437,10 @@ def main(out_path):
         parts += [code, ""]
         shifts.append((m, p, ls, ms))
     # (m, p, name suffix, tensor entries, reduced Lsize, reduced Msize, widths of the
-    # folding and unfolding rows, Lsize, Msize)
+    # folding and unfolding rows, Lsize)
     parts.append("#define CPPE_M2L_REDUCED(X) \\")
-    parts.append(" \\\n".join(f"  X({m}, {p}, {nm}, {nd}, {ls}, {ms}, {fw}, {uw}, {sl}, {sm})"
-                              for (m, p, nm, nd, ls, ms, fw, uw), (_, _, sl, sm)
-                              in zip(red, shifts)))
+    parts.append(" \\\n".join(f"  X({m}, {p}, {nm}, {nd}, {ls}, {ms}, {fw}, {uw}, {nterms(p - m)})"
+                              for m, p, nm, nd, ls, ms, fw, uw in red))
     parts.append("")
     # (m, p, Lsize, Msize) of the straight-line shifts
     parts.append("#define CPPE_SHIFTS_GENERATED(X) \\")

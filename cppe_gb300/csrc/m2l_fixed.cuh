@@ -35,7 +35,7 @@ constexpr int nred(int p) { return p < 0 ? 0 : (p + 1) * (p + 1); }
 
 // Derivative tensors of the distinct M2L vectors (Geometry::make_vectors),
 // thread per vector, in T or in double-float.
-#define CPPE_DEF_DTAB(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                           \
+#define CPPE_DEF_DTAB(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                                \
   template <typename T>                                                                     \
   __global__ void k_dtab_##NAME(int nvec, const double4_32a* __restrict__ vec,              \
                                 T* __restrict__ D) {                                        \
@@ -44,6 +44,7 @@ constexpr int nred(int p) { return p < 0 ? 0 : (p + 1) * (p + 1); }
     const double4_32a r = vec[v];                                                           \
     dtensor_##NAME<T>((T)r.x, (T)r.y, (T)r.z, D + (size_t)v * (NT));                        \
   }                                                                                         \
+  template <int DD>                                                                         \
   __global__ void k_dtab_##NAME##_dd(int nvec, const double4_32a* __restrict__ vec,         \
                                      float2* __restrict__ D) {                              \
     const int v = blockIdx.x * blockDim.x + threadIdx.x;                                    \
@@ -60,21 +61,23 @@ CPPE_M2L_REDUCED(CPPE_DEF_DTAB)
 // Builds the tensor table of g's M2L vectors for order p into w (T, or
 // double-float when dd) on first use; returns it, or null when g has no
 // vector table or no fixed-order kernel serves (m, p).
-template <typename T>
-const void* m2l_dtab(const Geometry& g, int m, int p, FieldWork<T>& w, bool dd, cudaStream_t s) {
+template <bool DD, typename T>
+const void* m2l_dtab(const Geometry& g, int m, int p, FieldWork<T>& w, cudaStream_t s) {
   const int nv = (int)g.h_vec.size();
   if (nv == 0) return nullptr;
   const void* out = nullptr;
-#define CPPE_BUILD_DTAB(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                          \
+#define CPPE_BUILD_DTAB(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                               \
   if (!out && m == MM && p == PP) {                                                          \
     const size_t cnt = (size_t)nv * (NT);                                                    \
-    if (dd) {                                                                                \
-      if (w.dtab_dd.n != cnt) {                                                              \
-        w.dtab_dd.alloc(cnt);                                                                \
-        k_dtab_##NAME##_dd<<<(nv + 63) / 64, 64, 0, s>>>(nv, g.vec.p, w.dtab_dd.p);          \
-        CG_LAUNCH();                                                                         \
+    if constexpr (DD) {                                                                      \
+      if constexpr (MM == 1) {                                                               \
+        if (w.dtab_dd.n != cnt) {                                                            \
+          w.dtab_dd.alloc(cnt);                                                              \
+          k_dtab_##NAME##_dd<1><<<(nv + 63) / 64, 64, 0, s>>>(nv, g.vec.p, w.dtab_dd.p);     \
+          CG_LAUNCH();                                                                       \
+        }                                                                                    \
+        out = w.dtab_dd.p;                                                                   \
       }                                                                                      \
-      out = w.dtab_dd.p;                                                                     \
     } else {                                                                                 \
       if (w.dtab.n != cnt) {                                                                 \
         w.dtab.alloc(cnt);                                                                   \
@@ -90,7 +93,7 @@ const void* m2l_dtab(const Geometry& g, int m, int p, FieldWork<T>& w, bool dd, 
 }
 
 // Reduced multipole rows Mr (stride m_stride(MS)) of every cell from the full
-// ones (stride m_stride(FMS)); thread per (cell, reduced row).  To double-float
+// ones (stride mstride); thread per (cell, reduced row).  To double-float
 // pairs for the double-float translation (sums in T).
 __device__ __forceinline__ void m2l_store(float& o, float v) { o = v; }
 __device__ __forceinline__ void m2l_store(double& o, double v) { o = v; }
@@ -119,9 +122,10 @@ struct FoldRow<float2> {
     return r < 2 * o + 1 ? k + r : -1;
   }
 };
-#define CPPE_DEF_FOLD(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                            \
+#define CPPE_DEF_FOLD(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                                 \
   template <typename T, typename O>                                                          \
-  __global__ void k_m2l_fold_##NAME(int ncells, const T* __restrict__ M, O* __restrict__ Mr, \
+  __global__ void k_m2l_fold_##NAME(int ncells, const T* __restrict__ M, int mstride,        \
+                                    O* __restrict__ Mr,                                      \
                                     const int* __restrict__ cell_seg,                        \
                                     const int* __restrict__ seg_done) {                      \
     constexpr int RS = FoldRow<O>::stride(MM, PP, MS);                                       \
@@ -132,7 +136,7 @@ struct FoldRow<float2> {
     T v = T(0);                                                                              \
     const int row = FoldRow<O>::coef(MM, PP, MS, pos);                                       \
     if (row >= 0) {                                                                          \
-      const T* m = M + (size_t)cell * m_stride(FMS);                                         \
+      const T* m = M + (size_t)cell * mstride;                                               \
       _Pragma("unroll") for (int i = 0; i < (FW); ++i) {                                     \
         const int f = m2l_fold_##NAME[row][i][1];                                            \
         if (f != 0) v = fma(T(f), m[m2l_fold_##NAME[row][i][0]], v);                         \
@@ -187,7 +191,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // whole warp with cp.async, the L1 wavefronts fell by two thirds and the time
 // rose from 0.61 to 0.71 ms at 300,000 sites, the copies' instructions costing
 // more than the scattered loads.)
-#define CPPE_DEF_M2L_KERNEL(M, P, NAME, NT, LS, MS, FW, UW, FLS, FMS)                      \
+#define CPPE_DEF_M2L_KERNEL(M, P, NAME, NT, LS, MS, FW, UW, FLS)                           \
   template <typename T, bool PRE>                                                          \
   __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : ((P) == 5 ? 2 : 1))          \
         k_m2l_##NAME(TreeView tv, const int4* __restrict__ chunks, int nchunks,            \
@@ -285,7 +289,7 @@ __device__ __forceinline__ void m2l_contract_dd(const float2* __restrict__ D,
 }
 
 // TAB: tensors read from the table; else (vectors off the grid) built per entry.
-#define CPPE_DEF_M2L_DD_KERNEL(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                  \
+#define CPPE_DEF_M2L_DD_KERNEL(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                       \
   template <bool TAB>                                                                       \
   __global__ void __launch_bounds__(64, TAB ? ((PP) == 5 ? 8 : 6) : 1)                      \
         k_m2l_##NAME##_dd(TreeView tv, const int4* __restrict__ chunks, int nchunks,        \
@@ -343,7 +347,7 @@ CPPE_M2L_REDUCED(CPPE_DEF_M2L_DD_KERNEL)
 
 // The full local expansion of every cell (FLS rows) from the reduced partial
 // expansions of its chunks (LS rows), summed in order; 0 without chunks.
-#define CPPE_DEF_LSUM(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                             \
+#define CPPE_DEF_LSUM(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                                  \
   template <typename T>                                                                       \
   __global__ void k_lsum_##NAME(int ncells, const int* __restrict__ cell_chunk_ptr,           \
                                 const T* __restrict__ Lpart, T* __restrict__ L,               \
@@ -374,12 +378,13 @@ CPPE_M2L_REDUCED(CPPE_DEF_LSUM)
 // (Mr as float2).  Returns false otherwise.
 template <bool DD, typename T, typename O>
 bool launch_m2l_fixed(const TreeView& tv, int m, int p, const int4* chunks, int nchunks,
-                      const int* cell_chunk_ptr, const T* M, DBuf<O>& Mr, DBuf<T>& Lpart, T* L,
-                      cudaStream_t s, const int* cell_seg, const int* seg_done,
+                      const int* cell_chunk_ptr, const T* M, int mstride, DBuf<O>& Mr,
+                      DBuf<T>& Lpart, T* L, cudaStream_t s, const int* cell_seg, const int* seg_done,
                       const void* dtab, const int* vid) {
   bool ok = false;
   auto grid = [](long work, int b) { return (unsigned)((work + b - 1) / b); };
-#define CPPE_LAUNCH_M2L(MM, PP, NAME, NT, LS, MS, FW, UW, FLS, FMS)                            \
+#define CPPE_LAUNCH_M2L(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                                 \
+  if constexpr ((MM) == 1 || (!DD && sizeof(T) == 8))                                          \
   if (!ok && m == MM && p == PP) {                                                             \
     ok = true;                                                                                 \
     constexpr int RS = FoldRow<O>::stride(MM, PP, MS);                                         \
@@ -387,7 +392,7 @@ bool launch_m2l_fixed(const TreeView& tv, int m, int p, const int4* chunks, int 
     Lpart.alloc((size_t)std::max(1, nchunks) * (LS));                                          \
     if (nchunks > 0) {                                                                         \
       k_m2l_fold_##NAME<T, O><<<grid((long)tv.ncells * RS, 256), 256, 0, s>>>(                 \
-            tv.ncells, M, Mr.p, cell_seg, seg_done);                                           \
+            tv.ncells, M, mstride, Mr.p, cell_seg, seg_done);                                  \
       CG_LAUNCH();                                                                             \
       if constexpr (DD) {                                                                      \
         const unsigned b = grid((long)nchunks * 32, 64);                                       \

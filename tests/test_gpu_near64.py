@@ -73,3 +73,25 @@ def test_distance_classes(gpu, port, spacing, damp):
     ref = port.bmatrix_apply(xyz, alpha6, ptr, idx, v, fmm=0, damping=DAMPING if damp else 0.0)
     close(s.apply(v), ref)
     s.close()
+
+
+@pytest.mark.parametrize("damp", [False, True])
+@pytest.mark.parametrize("fmm", [False, True])
+@pytest.mark.parametrize("waters", [1, 32, 33, 64, 700])
+def test_static_fields(gpu, port, waters, fmm, damp):
+    """Charges, dipoles and quadrupoles together; 192 sources a tile for the
+    quadrupoles (waters 32, 33, 64).  The static fields cancel to a tenth of
+    their terms: ten times the tolerance."""
+    from cppe_gb300 import synthetic
+    from oracle import oracle as O
+    b = synthetic.water_box(waters, seed=waters)
+    one = np.ones(b.n, np.int32)
+    sites = O.Sites(xyz=b.xyz, elements=b.elements, q=b.q, mu=b.mu, quad=b.quad, max_order=2,
+                    alpha6=b.alpha6, polarizable=one, excl_ptr=b.excl_ptr, excl_idx=b.excl_idx)
+    ref = port.multipole_fields(sites, fmm=fmm, order=6, damping=DAMPING if damp else 0.0)
+    got = cabi.multipole_fields(b.xyz, b.q, b.mu, b.quad, 2, one, b.alpha_iso, b.excl_ptr,
+                                b.excl_idx, fmm=fmm, order=6, damp=damp)
+    if waters == 1:
+        assert np.abs(got).max() < 1e-14  # every pair is excluded
+    else:
+        close(got, ref, 10 * TOL)
