@@ -809,8 +809,8 @@ int cppe_gpu_tree_info(int n, const double* xyz, int ncrit, double theta, int* n
     make_layout(t, n, L);
     if (ncells) *ncells = L.ncells;
     if (nleaves) *nleaves = L.nleaves;
-    if (nm2l) *nm2l = (long)t.m2l.size();
-    if (np2p) *np2p = (long)t.p2p.size();
+    if (nm2l) *nm2l = t.nm2l;
+    if (np2p) *np2p = t.np2p;
     if (p2p_pairs) *p2p_pairs = L.p2p_pairs;
     return CPPE_GPU_OK;
   });
@@ -839,8 +839,9 @@ int cppe_gpu_tree_lists(int n, const double* xyz, int ncrit, double theta, int* 
     RefTree t;
     std::string err;
     if (!build_ref_tree(n, xyz, ncrit, theta, t, err)) fail(CPPE_GPU_INVALID_ARG, err);
-    for (size_t i = 0; i < t.m2l.size(); ++i) m2l[2 * i] = t.m2l[i].first, m2l[2 * i + 1] = t.m2l[i].second;
-    for (size_t i = 0; i < t.p2p.size(); ++i) p2p[2 * i] = t.p2p[i].first, p2p[2 * i + 1] = t.p2p[i].second;
+    const RefTree::Pairs lm = t.m2l_by_source(), lp = t.p2p_flat();
+    for (size_t i = 0; i < lm.size(); ++i) m2l[2 * i] = lm[i].first, m2l[2 * i + 1] = lm[i].second;
+    for (size_t i = 0; i < lp.size(); ++i) p2p[2 * i] = lp[i].first, p2p[2 * i + 1] = lp[i].second;
     return CPPE_GPU_OK;
   });
 }

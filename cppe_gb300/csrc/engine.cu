@@ -22,7 +22,6 @@
 #include <cstring>
 #include <numeric>
 #include <type_traits>
-#include <unordered_map>
 
 #include "engine.h"
 #include "dd.cuh"
@@ -183,7 +182,9 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
   auto& p64 = h_pos64;
   auto& hi  = h_hi;
   auto& lo  = h_lo;
-  for (int k = 0; k < n; ++k) {
+  const int threads = host_threads(n, 4096);
+  host_parallel(threads, n, [&](int, long k0, long k1) {
+  for (long k = k0; k < k1; ++k) {
     const int i  = L.perm[k];
     const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
     const double sd = s_damp ? s_damp[i] : 0.0;
@@ -206,6 +207,7 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
     h_mid[k]       = make_float4(m[0], m[1], m[2], 0.f);
     h_low[k]       = make_float4(e[0], e[1], e[2], (float)(sd - (double)sh));
   }
+  });
 
   // Exclusion corrections: pairs the reference skips but the near-field pass
   // includes.  Direct: every listed exclusion; FMM: those whose source sits in
@@ -216,32 +218,34 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
   auto& cptr = h_cptr;
   auto& cidx = h_cidx;
   if (excl_ptr) {
-    std::vector<std::vector<int>> sorted_src;
-    if (fmm) {
-      sorted_src.resize(L.nleaves);
-      for (int a = 0; a < L.nleaves; ++a) {
-        sorted_src[a].assign(L.p2p_src.begin() + L.p2p_ptr[a], L.p2p_src.begin() + L.p2p_ptr[a + 1]);
-        std::sort(sorted_src[a].begin(), sorted_src[a].end());
-      }
-    }
-    for (int k = 0; k < n; ++k) {
-      const int i = L.perm[k];
+    // (an excluded site is in its target's own leaf most of the time, and every
+    // leaf lists itself; else the target's list is searched)
+    std::vector<std::vector<int>> part(threads);
+    host_parallel(threads, n, [&](int t, long k0, long k1) {
       std::vector<int> mine;
-      for (int e = excl_ptr[i]; e < excl_ptr[i + 1]; ++e) {
-        const int j = excl_idx[e];
-        if (j < 0 || j >= n || j == i) continue;
-        const int kj = L.inv_perm[j];
-        if (fmm) {
-          const auto& v = sorted_src[site_leaf_h[k]];
-          if (!std::binary_search(v.begin(), v.end(), site_leaf_h[kj])) continue;
+      for (long k = k0; k < k1; ++k) {
+        const int i  = L.perm[k];
+        const int la = site_leaf_h[k];
+        mine.clear();
+        for (int e = excl_ptr[i]; e < excl_ptr[i + 1]; ++e) {
+          const int j = excl_idx[e];
+          if (j < 0 || j >= n || j == i) continue;
+          const int kj = L.inv_perm[j], lb = site_leaf_h[kj];
+          if (fmm && lb != la) {
+            const auto p0 = L.p2p_src.begin() + L.p2p_ptr[la],
+                       p1 = L.p2p_src.begin() + L.p2p_ptr[la + 1];
+            if (std::find(p0, p1, lb) == p1) continue;
+          }
+          mine.push_back(kj);
         }
-        mine.push_back(kj);
+        std::sort(mine.begin(), mine.end());
+        mine.erase(std::unique(mine.begin(), mine.end()), mine.end());
+        part[t].insert(part[t].end(), mine.begin(), mine.end());
+        cptr[k + 1] = (int)mine.size();
       }
-      std::sort(mine.begin(), mine.end());
-      mine.erase(std::unique(mine.begin(), mine.end()), mine.end());
-      cidx.insert(cidx.end(), mine.begin(), mine.end());
-      cptr[k + 1] = (int)cidx.size();
-    }
+    });
+    for (const auto& v : part) cidx.insert(cidx.end(), v.begin(), v.end());
+    for (int k = 0; k < n; ++k) cptr[k + 1] += cptr[k];
   }
   // algorithmic pairs: the ordered pairs the reference evaluates in its
   // near-field / direct loops (self pairs and excluded pairs are skipped there)
@@ -260,33 +264,75 @@ bool m2l_vectors(const TreeLayout& L, std::vector<int>& vid, std::vector<double4
   if (!(rmin > 0.0)) return false;
   const double u = 0.5 * rmin;
   constexpr long long OFF = 1LL << 20;
-  std::unordered_map<long long, int> ids;
+  // each cell's centre in units of u from the first one
+  std::vector<int> grid(3 * (size_t)L.ncells);
+  for (int c = 0; c < L.ncells; ++c)
+    for (int i = 0; i < 3; ++i) {
+      const double d = (L.center[4 * (size_t)c + i] - L.center[i]) / u;
+      const double k = std::nearbyint(d);
+      if (std::fabs(d - k) > 5e-4 || std::fabs(k) >= (double)(OFF / 2)) return false;  // off the grid
+      grid[3 * (size_t)c + i] = (int)k;
+    }
   vid.resize(L.m2l_src.size());
-  for (int A = 0; A < L.ncells; ++A)
-    for (int q = L.m2l_ptr[A]; q < L.m2l_ptr[A + 1]; ++q) {
-      const int B = L.m2l_src[q];
-      long long k[3];
-      for (int c = 0; c < 3; ++c) {
-        const double d = (L.center[4 * (size_t)A + c] - L.center[4 * (size_t)B + c]) / u;
-        k[c]           = std::llround(d);
-        if (std::fabs(d - (double)k[c]) > 1e-3 || std::llabs(k[c]) >= OFF) {
-          vid.clear();  // off the grid
-          vec.clear();
-          return false;
+  // Keys per entry, then ids in the order of first appearance: threads take
+  // contiguous shares of the cells with an open-addressing table each, whose
+  // distinct keys are merged share after share.
+  struct Share {
+    std::vector<long long> slot_key;
+    std::vector<int> slot_id;
+    std::vector<long long> keys;  // in order of appearance
+    int find(long long key) {
+      size_t mask = slot_key.size() - 1;
+      size_t h    = (size_t)((unsigned long long)key * 0x9e3779b97f4a7c15ull >> 20) & mask;
+      while (slot_id[h] >= 0 && slot_key[h] != key) h = (h + 1) & mask;
+      if (slot_id[h] < 0) {
+        if (2 * (keys.size() + 1) > slot_key.size()) {
+          grow();
+          return find(key);
         }
+        slot_key[h] = key, slot_id[h] = (int)keys.size();
+        keys.push_back(key);
       }
-      const long long key = (k[0] + OFF) | ((k[1] + OFF) << 21) | ((k[2] + OFF) << 42);
-      const auto it       = ids.find(key);
-      if (it == ids.end()) {
-        ids.emplace(key, (int)vec.size());
-        vid[q] = (int)vec.size();
-        double4_32a v;
-        v.x = (double)k[0] * u, v.y = (double)k[1] * u, v.z = (double)k[2] * u, v.w = 0.0;
-        vec.push_back(v);
-      } else {
-        vid[q] = it->second;
+      return slot_id[h];
+    }
+    void grow() {
+      const size_t sz = slot_key.empty() ? 1 << 14 : 2 * slot_key.size();
+      slot_key.assign(sz, 0), slot_id.assign(sz, -1);
+      for (size_t k = 0; k < keys.size(); ++k) {
+        size_t h = (size_t)((unsigned long long)keys[k] * 0x9e3779b97f4a7c15ull >> 20) & (sz - 1);
+        while (slot_id[h] >= 0) h = (h + 1) & (sz - 1);
+        slot_key[h] = keys[k], slot_id[h] = (int)k;
       }
     }
+  };
+  const int threads = host_threads((long)L.m2l_src.size(), 1 << 14);
+  std::vector<Share> share(threads);
+  host_parallel(threads, L.ncells, [&](int t, long c0, long c1) {
+    Share& S = share[t];
+    S.grow();
+    for (long A = c0; A < c1; ++A)
+      for (int q = L.m2l_ptr[A]; q < L.m2l_ptr[A + 1]; ++q) {
+        const int *ga = &grid[3 * (size_t)A], *gb = &grid[3 * (size_t)L.m2l_src[q]];
+        const long long k[3] = {ga[0] - gb[0], ga[1] - gb[1], ga[2] - gb[2]};
+        vid[q] = S.find((k[0] + OFF) | ((k[1] + OFF) << 21) | ((k[2] + OFF) << 42));
+      }
+  });
+  Share all;
+  all.grow();
+  std::vector<std::vector<int>> global(threads);
+  for (int t = 0; t < threads; ++t)
+    for (long long key : share[t].keys) global[t].push_back(all.find(key));
+  for (long long key : all.keys) {
+    double4_32a v;
+    constexpr long long M = (1LL << 21) - 1;
+    v.x = (double)((key & M) - OFF) * u, v.y = (double)(((key >> 21) & M) - OFF) * u;
+    v.z = (double)((key >> 42) - OFF) * u, v.w = 0.0;
+    vec.push_back(v);
+  }
+  if (threads > 1)
+    host_parallel(threads, L.ncells, [&](int t, long c0, long c1) {
+      for (int q = L.m2l_ptr[c0]; q < L.m2l_ptr[c1]; ++q) vid[q] = global[t][vid[q]];
+    });
   return true;
 }
 
@@ -318,11 +364,15 @@ void Geometry::make_schedules() {
       has_l[c] = L.m2l_ptr[c + 1] > L.m2l_ptr[c];
       for (int q = L.m2l_ptr[c]; q < L.m2l_ptr[c + 1]; ++q) need_m[L.m2l_src[q]] = 1;
     }
-    std::vector<std::vector<int>> sub(L.ncells);  // subtree leaves of the cells needing M
-    std::vector<int> ref(L.ncells, -1);
+    // subtree leaves of the cells needing M, cell after cell
+    std::vector<int> sub_ptr(L.ncells + 1, 0), ref(L.ncells, -1);
+    for (int a = 0; a < L.nleaves; ++a)
+      for (int c = L.leaf_cell[a]; c >= 0; c = L.parent[c]) sub_ptr[c + 1] += need_m[c];
+    for (int c = 0; c < L.ncells; ++c) sub_ptr[c + 1] += sub_ptr[c];
+    std::vector<int> sub(sub_ptr[L.ncells]), fill(sub_ptr.begin(), sub_ptr.end() - 1);
     for (int a = 0; a < L.nleaves; ++a) {
       for (int c = L.leaf_cell[a]; c >= 0; c = L.parent[c]) {
-        if (need_m[c]) sub[c].push_back(a);
+        if (need_m[c]) sub[fill[c]++] = a;
         if (ref[c] < 0 && L.leaf_start[a + 1] > L.leaf_start[a]) ref[c] = L.leaf_start[a];
         if (has_l[c]) h_lanc_cell.push_back(c);
       }
@@ -337,10 +387,10 @@ void Geometry::make_schedules() {
       // non-leaf cells: tasks of <= M2M_TASK_LEAVES subtree leaves (leaf
       // multipoles are formed by k_p2m_leaf)
       if (!L.is_leaf[c]) {
-        for (size_t k0 = 0; k0 < sub[c].size(); k0 += M2M_TASK_LEAVES) {
-          const size_t k1 = std::min(sub[c].size(), k0 + M2M_TASK_LEAVES);
+        for (int k0 = sub_ptr[c]; k0 < sub_ptr[c + 1]; k0 += M2M_TASK_LEAVES) {
+          const int k1    = std::min(sub_ptr[c + 1], k0 + M2M_TASK_LEAVES);
           const int first = (int)h_task_leaf.size();
-          for (size_t k = k0; k < k1; ++k) h_task_leaf.push_back(sub[c][k]);
+          for (int k = k0; k < k1; ++k) h_task_leaf.push_back(sub[k]);
           h_p2m_tasks.push_back(make_int4(c, first, (int)h_task_leaf.size(), 0));
         }
       }
@@ -383,8 +433,10 @@ void Geometry::make_schedules() {
           smin[a] = std::min(smin[a], q.w > 0.0 ? q.w : 1e300);
         }
       }
+      host_parallel(host_threads((long)L.p2p_src.size(), 1 << 13), L.nleaves,
+                    [&](int, long l0, long l1) {
       std::vector<int> nearer, farther;
-      for (int a = 0; a < L.nleaves; ++a) {
+      for (long a = l0; a < l1; ++a) {
         const double* ba = &box[6 * (size_t)a];
         nearer.clear(), farther.clear();
         for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q) {
@@ -403,6 +455,7 @@ void Geometry::make_schedules() {
         h_leaf_split[a] = q;
         for (int b : farther) layout.p2p_src[q++] = b;
       }
+      });
     }
   }
   // ---- near-field work items
@@ -494,7 +547,6 @@ void Geometry::make_sym_schedule(long W) {
     int split;
   };
   std::vector<Item> its;
-  std::vector<int> item_of_entry(h_usrc.size(), -1);
   for (int a = 0; a < nl; ++a) {
     const long na = nsite(a);
     int q0        = uptr[a];
@@ -511,21 +563,27 @@ void Geometry::make_sym_schedule(long W) {
       its.push_back({0, make_int4(a, uptr[a], uptr[a], 0), uptr[a]});
   }
   // rows, leaf by leaf: first each leaf's own items, then its rows as a partner
-  std::vector<std::vector<std::pair<int, int>>> partner_rows(nl);  // (item, entry)
+  // (items are numbered leaf by leaf, entries item by item)
+  std::vector<int> pptr(nl + 1, 0), optr(nl + 1, 0);
+  for (size_t k = 0; k < its.size(); ++k) {
+    optr[its[k].v.x + 1]++;
+    for (int q = its[k].v.y; q < its[k].v.z; ++q)
+      if (h_usrc[q] != its[k].v.x) pptr[h_usrc[q] + 1]++;
+  }
+  for (int a = 0; a < nl; ++a) pptr[a + 1] += pptr[a], optr[a + 1] += optr[a];
+  std::vector<int> pent(pptr[nl]), pfill(pptr.begin(), pptr.end() - 1);
   for (size_t k = 0; k < its.size(); ++k)
     for (int q = its[k].v.y; q < its[k].v.z; ++q)
-      if (h_usrc[q] != its[k].v.x) partner_rows[h_usrc[q]].push_back({(int)k, q});
-  std::vector<std::vector<int>> own(nl);
-  for (size_t k = 0; k < its.size(); ++k) own[its[k].v.x].push_back((int)k);
+      if (h_usrc[q] != its[k].v.x) pent[pfill[h_usrc[q]]++] = q;
   h_sym_aoff.assign(its.size(), 0);
   h_usrc_off.assign(h_usrc.size(), -1);
   long long off = 0;
   for (int a = 0; a < nl; ++a) {
     h_sym_leaf_off[a] = off;
     const long row    = 3 * nsite(a);
-    for (int k : own[a]) h_sym_aoff[k] = off, off += row;
-    for (const auto& pr : partner_rows[a]) h_usrc_off[pr.second] = off, off += row;
-    h_sym_leaf_rows[a] = (int)(own[a].size() + partner_rows[a].size());
+    for (int k = optr[a]; k < optr[a + 1]; ++k) h_sym_aoff[k] = off, off += row;
+    for (int e = pptr[a]; e < pptr[a + 1]; ++e) h_usrc_off[pent[e]] = off, off += row;
+    h_sym_leaf_rows[a] = optr[a + 1] - optr[a] + pptr[a + 1] - pptr[a];
   }
   h_sym_leaf_off[nl] = off;
   sym_floats         = off;

@@ -7,11 +7,50 @@
 // every GPU pass reads contiguous ranges.
 #pragma once
 
+#include <algorithm>
+#include <exception>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
 namespace cg {
+
+// Threads for host work over `items` elements of which one thread should take
+// at least `grain`.
+inline int host_threads(long items, long grain) {
+  const long hw = std::max(1u, std::thread::hardware_concurrency());
+  return (int)std::max(1L, std::min({hw, 16L, items / std::max(1L, grain)}));
+}
+// f(t, begin, end) on contiguous shares of [0, n), share t on thread t; an
+// exception is passed on after every thread has ended.
+template <class F>
+void host_parallel(int threads, long n, F&& f) {
+  if (threads <= 1) {
+    f(0, 0L, n);
+    return;
+  }
+  std::vector<std::thread> pool;
+  std::vector<std::exception_ptr> err(threads);
+  auto run = [&](int t) {
+    try {
+      f(t, n * t / threads, n * (t + 1) / threads);
+    } catch (...) {
+      err[t] = std::current_exception();
+    }
+  };
+  int started = 1;
+  try {
+    for (; started < threads; ++started) pool.emplace_back(run, started);
+  } catch (const std::system_error&) {  // no more threads: the rest runs here
+  }
+  run(0);
+  for (int t = started; t < threads; ++t) run(t);
+  for (auto& p : pool) p.join();
+  for (auto& e : err)
+    if (e) std::rethrow_exception(e);
+}
 
 // Cells in the reference's creation order (tree.cc:134-237).
 struct RefTree {
@@ -21,9 +60,15 @@ struct RefTree {
   std::vector<int> parent, level, nleaf;
   std::vector<unsigned> nchild;          // occupancy bit mask, bit o = octant o
   std::vector<int> child;                // 8 per cell, valid where the bit is set
-  std::vector<std::vector<int>> leaf;    // particle indices (valid while nleaf < ncrit)
-  std::vector<std::pair<int, int>> m2l;  // (source, target), sorted by source
-  std::vector<std::pair<int, int>> p2p;  // (target, source)
+  std::vector<int> next, head, tail;     // a cell's particles as a list (-1 ends it)
+  // interaction lists in walk order, as the walk's parts in sequence
+  using Pairs = std::vector<std::pair<int, int>>;
+  std::vector<Pairs> m2l;  // (source, target)
+  std::vector<Pairs> p2p;  // (target, source)
+  long nm2l = 0, np2p = 0;
+  // both lists flat, the M2L list ordered by source (tree.cc:224-227)
+  Pairs m2l_by_source() const;
+  Pairs p2p_flat() const;
 };
 
 // Builds the tree and both lists.  Returns false (with a message) on input the
