@@ -493,6 +493,16 @@ int cppe_gpu_solve(cppe_gpu_system* sys, const double* rhs, const double* guess,
     System& S = sys->s;
     CG_CUDA(cudaSetDevice(S.device));
     const size_t n3 = 3 * (size_t)S.n;
+    if (S.small_solver()) {  // through pinned memory, which the kernel reads and writes
+      if (!S.h_io) CG_CUDA(cudaMallocHost(&S.h_io, 3 * n3 * sizeof(double)));
+      const bool g = guess && !make_guess;
+      std::copy(rhs, rhs + n3, S.h_io);
+      if (g) std::copy(guess, guess + n3, S.h_io + n3);
+      const int st = S.solve_device(S.h_io, g ? S.h_io + n3 : nullptr, make_guess,
+                                    S.h_io + 2 * n3, iters, rnorm_hist, hist_cap);
+      std::copy(S.h_io + 2 * n3, S.h_io + 3 * n3, mu);
+      return st;
+    }
     S.io_rhs.upload(rhs, n3, S.stream);
     if (guess && !make_guess) S.io_guess.upload(guess, n3, S.stream);
     S.io_mu.alloc(n3);

@@ -66,7 +66,8 @@ __global__ void k_cg_update(int n, const T* __restrict__ p, const T* __restrict_
                             const T* __restrict__ a6, T* __restrict__ x, T* __restrict__ r,
                             T* __restrict__ z, ReduceSlots rs, double* scal, int* flags,
                             double* hist, double thresh, int maxiter, T* __restrict__ r_old,
-                            float4* __restrict__ z4 = nullptr) {
+                            float4* __restrict__ z4 = nullptr,
+                            int* host_flags = nullptr) {
   __shared__ double sh[64];
   if (flags[0]) return;
   const double a = scal[S_RZ] / scal[S_PAP];
@@ -105,6 +106,8 @@ __global__ void k_cg_update(int n, const T* __restrict__ p, const T* __restrict_
       flags[0] = 1;
     else if (it + 1 >= maxiter)
       flags[0] = 2;
+    // (pinned memory: the host's poll needs no copy in the stream)
+    if (host_flags) host_flags[1] = flags[1], host_flags[0] = flags[0];
   }
 }
 
@@ -202,6 +205,8 @@ System::~System() {
   }
   if (h_flags) cudaFreeHost(h_flags);
   if (h_scal) cudaFreeHost(h_scal);
+  if (h_hist) cudaFreeHost(h_hist);
+  if (h_io) cudaFreeHost(h_io);
 }
 
 static void inv_sym3(const double* s, double* o6) {
@@ -540,6 +545,10 @@ ReduceSlots System::slots(int k) const { return ReduceSlots{partials.p, ticket.p
 
 void System::apply64(const double* in, double* out, bool with_dot, int near_mode) {
   ReduceSlots rs = slots(S_PAP);
+  if (near_mode == NEAR_FP64 && !with_dot && dense_operator()) {
+    dense_apply(in, out, false);
+    return;
+  }
   eval_field<double>(geo, ops.get(), w64, 1, in, opt.damp != 0, opt.damping_factor,
                      FINISH_APPLY, ainv64.p, out, nullptr, 1.0, with_dot ? &rs : nullptr,
                      stream, nullptr, near_mode, &side);
@@ -572,9 +581,11 @@ struct Poller {
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
   }
-  // Returns true once a finished state has been observed.
-  bool after_iteration() {
-    CG_CUDA(cudaMemcpyAsync(h_flags, d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  // Returns true once a finished state has been observed.  copy: false where the
+  // iteration's kernels write h_flags themselves.
+  bool after_iteration(bool copy = true) {
+    if (copy)
+      CG_CUDA(cudaMemcpyAsync(h_flags, d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaEventRecord(ev[k & 1], s));
     bool done = false;
     if (k > 0) {
@@ -588,6 +599,7 @@ struct Poller {
 }  // namespace
 
 int System::solve_fp64(bool zero_guess, double* hist_out, int hist_cap, int* iters) {
+  const bool dense = dense_operator() && !use_model;
   const int nb   = (n + VB - 1) / VB;
   const int n3   = 3 * n;
   const double t = opt.induced_thresh;
@@ -601,18 +613,24 @@ int System::solve_fp64(bool zero_guess, double* hist_out, int hist_cap, int* ite
   CG_LAUNCH();
   if (use_model) learned_precond<double>(z.p, r.p, p.p, true);
   if (zero_guess) CG_CUDA(cudaMemsetAsync(x.p, 0, sizeof(double) * n3, stream));
+  h_flags[0] = 0;  // (no kernel of an earlier solve is in flight: each ends synchronised)
   Poller poll(stream, flags.p, h_flags);
   for (int k = 0; k < opt.maxiter; ++k) {
-    apply64(p.p, Ap.p, true);
     last.fp64_applies++;
-    k_cg_update<double><<<nb, VB, 0, stream>>>(n, p.p, Ap.p, alpha64.p, x.p, r.p, z.p,
-                                               slots(S_RED), scal.p, flags.p, hist.p, t,
-                                               opt.maxiter, use_model ? lf_rold64.p : nullptr);
-    CG_LAUNCH();
-    const double* zd = use_model ? learned_precond<double>(z.p, r.p, p.p, false) : z.p;
-    k_cg_dir<double><<<(n3 + VB - 1) / VB, VB, 0, stream>>>(n3, zd, p.p, scal.p, flags.p);
-    CG_LAUNCH();
-    if (poll.after_iteration()) break;
+    if (dense) {
+      dense_iteration();
+    } else {
+      apply64(p.p, Ap.p, true);
+      k_cg_update<double><<<nb, VB, 0, stream>>>(n, p.p, Ap.p, alpha64.p, x.p, r.p, z.p,
+                                                 slots(S_RED), scal.p, flags.p, hist.p, t,
+                                                 opt.maxiter, use_model ? lf_rold64.p : nullptr,
+                                                 nullptr, h_flags);
+      CG_LAUNCH();
+      const double* zd = use_model ? learned_precond<double>(z.p, r.p, p.p, false) : z.p;
+      k_cg_dir<double><<<(n3 + VB - 1) / VB, VB, 0, stream>>>(n3, zd, p.p, scal.p, flags.p);
+      CG_LAUNCH();
+    }
+    if (poll.after_iteration(false)) break;
   }
   CG_CUDA(cudaMemcpyAsync(h_flags, flags.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
   CG_CUDA(cudaMemcpyAsync(h_scal, scal.p, S_NSCAL * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1019,6 +1037,9 @@ int System::solve_mixed(bool zero_guess, double* hist_out, int hist_cap, int* it
 int System::solve_device(const double* d_rhs, const double* d_guess, int make_guess,
                          double* d_mu, int* iters, double* hist_out, int hist_cap) {
   CG_CUDA(cudaSetDevice(device));
+  if (small_solver())
+    return solve_small(d_rhs, make_guess ? nullptr : d_guess, make_guess != 0, d_mu, iters,
+                       hist_out, hist_cap);
   const int n3 = 3 * n;
   permute_in(geo, d_rhs, F.p, 3, stream);
   bool zero = false;

@@ -34,6 +34,12 @@ struct SolveStats {
   int fp64_applies = 0, fp32_applies = 0, iterations = 0;
 };
 
+// Direct-summation FP64 systems up to DENSE_MAX sites keep the operator as a
+// dense matrix, up to SMALL_MAX sites the whole solve is one block with the
+// matrix in shared memory (dense.cu).
+constexpr int DENSE_MAX = 1024;
+constexpr int SMALL_MAX = 53;  // 8 (3n)(3n + 2) <= 227 KB
+
 struct System {
   int n = 0;
   cppe_gpu_options opt{};
@@ -68,6 +74,18 @@ struct System {
   DBuf<int> flags;  // [0] done, [1] iteration counter
   int* h_flags = nullptr;     // pinned mirror
   double* h_scal = nullptr;   // pinned mirror
+  double* h_hist = nullptr;   // pinned: the norms of a one-block solve
+  double* h_io   = nullptr;   // pinned: its right-hand side, guess and solution
+  DBuf<double> Tmat;          // the operator without alpha^-1 as a dense matrix (built on first use)
+  bool small_ready = false;
+  bool dense_operator() const;
+  void dense_build();
+  void dense_apply(const double* in, double* out, bool iteration);
+  void dense_iteration();
+  bool small_solver() const;
+  // (pointers the device can address; solve_device's arguments otherwise)
+  int solve_small(const double* rhs, const double* guess, int make_guess, double* mu, int* iters,
+                  double* hist_out, int hist_cap);
   SolveStats last;
   std::vector<int> excl_ptr_h, excl_idx_h;  // caller-order exclusions (dense matrix)
 

@@ -24,6 +24,26 @@ def close(a, ref, tol=TOL):
     assert np.linalg.norm(a - ref) < tol * np.linalg.norm(ref)
 
 
+def check_dipole_field(port, xyz, alpha, ptr, idx, v, damp):
+    from oracle import oracle as O
+    n = xyz.shape[0]
+    a6 = np.zeros((n, 6))
+    a6[:, [0, 3, 5]] = alpha[:, None]
+    mu, one = v.reshape(n, 3), np.ones(n, np.int32)
+    sites = O.Sites(xyz=xyz, elements=["O"] * n, q=np.zeros(n), mu=mu, quad=np.zeros((n, 6)),
+                    max_order=1, alpha6=a6, polarizable=one, excl_ptr=ptr, excl_idx=idx)
+    ref = port.multipole_fields(sites, fmm=False, order=5, damping=DAMPING if damp else 0.0)
+
+    def run(m):
+        return cabi.multipole_fields(xyz, np.zeros(n), m, np.zeros((n, 6)), 1, one, alpha, ptr, idx,
+                                     damp=damp)
+    got = run(mu)
+    # (no alpha^-1 term beside the field: measured against the dipoles' own size)
+    assert np.linalg.norm(got - ref) < TOL * (np.linalg.norm(ref) + 0.1 * np.linalg.norm(v))
+    for e in (-900, 900):
+        assert np.array_equal(run(mu * 2.0 ** e), got * 2.0 ** e)
+
+
 @pytest.mark.parametrize("damp", [False, True])
 @pytest.mark.parametrize("waters", [1, 10, 11, 22, 43, 101, 102, 333, 700])
 def test_direct_sizes(gpu, port, waters, damp):
@@ -38,6 +58,9 @@ def test_direct_sizes(gpu, port, waters, damp):
     for e in (-900, 900):
         assert np.array_equal(s.apply(v * 2.0 ** e), s.apply(v) * 2.0 ** e)
     s.close()
+    # the same pairs through the static field of dipoles (the pair kernel at
+    # every size; the operator itself is a dense matrix up to 1,024 sites)
+    check_dipole_field(port, b.xyz, b.alpha_iso, b.excl_ptr, b.excl_idx, v, damp)
 
 
 @pytest.mark.parametrize("ncrit", [16, 64, 300])
@@ -73,6 +96,8 @@ def test_distance_classes(gpu, port, spacing, damp):
     ref = port.bmatrix_apply(xyz, alpha6, ptr, idx, v, fmm=0, damping=DAMPING if damp else 0.0)
     close(s.apply(v), ref)
     s.close()
+    v = rng.normal(size=3 * n)
+    check_dipole_field(port, xyz, alpha6[:, 0], ptr, idx, v, damp)
 
 
 @pytest.mark.parametrize("damp", [False, True])
