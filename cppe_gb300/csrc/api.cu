@@ -1043,10 +1043,9 @@ int cppe_gpu_mlp_loss_grad(cppe_gpu_mlp* h, int rows, const float* feats, const 
     need(h && feats && targets && rows > 0, "null argument");
     Mlp& M = h->m;
     CG_CUDA(cudaSetDevice(M.device));
-    DBuf<float> f, t;
-    f.upload(feats, (size_t)rows * Mlp::IN, M.stream);
-    t.upload(targets, (size_t)rows * Mlp::TROW, M.stream);
-    const double l = M.loss_grad(rows, f.p, t.p, lam);
+    M.upload(M.in_feats, feats, (size_t)rows * Mlp::IN);
+    M.upload(M.in_targets, targets, (size_t)rows * Mlp::TROW);
+    const double l = M.loss_grad(rows, M.in_feats.p, M.in_targets.p, lam);
     if (loss) *loss = l;
     if (grads)
       CG_CUDA(cudaMemcpy(grads, M.grads.p, Mlp::NPARAM * sizeof(float), cudaMemcpyDeviceToHost));

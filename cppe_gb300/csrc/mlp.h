@@ -22,14 +22,17 @@ struct Mlp {
   int step = 0;
   // workspace for a batch of up to `cap` rows
   int cap = 0;
-  DBuf<float> X, Z1, H1, Z2, H2, Y, dY, dA, dB, part;
-  DBuf<double> loss_part, loss;
-  DBuf<unsigned> ticket;
+  static constexpr int MAX_PARTS = 128;  // parts of the gradients' sums over rows
+  DBuf<float> Z1, H1, Z2, H2, dZ1, dZ2, part;
+  DBuf<float> in_feats, in_targets;  // a host caller's batch (up to the largest so far)
+  DBuf<double> loss_part;
+  double* h_loss = nullptr;  // pinned
   DBuf<int> tc_err;  // error code of the tensor-core inference (0: none)
 
   ~Mlp();
   void init(int device, unsigned seed);
   void reserve(int rows);
+  void upload(DBuf<float>& d, const float* h, size_t count);
   float* W1() { return params.p; }
   float* b1() { return params.p + NW1; }
   float* W2() { return params.p + NW1 + NB1; }
@@ -38,6 +41,7 @@ struct Mlp {
   float* b3() { return params.p + NW1 + NB1 + NW2 + NB2 + NW3; }
   // Y (rows x 4) for raw descriptors (rows x 64, device); normalises first.
   // forward keeps the intermediate layers (training); infer is one fused pass.
+  void hidden(int rows, const float* raw, cudaStream_t s);
   void forward(int rows, const float* raw, float* Y_out, cudaStream_t s);
   void infer(int rows, const float* raw, float* Y_out, cudaStream_t s);
   // loss and parameter gradients (into grads) for one batch; returns loss.
@@ -49,10 +53,5 @@ struct Mlp {
 // operands, FP32 accumulation); *err receives 1 if a wait timed out.
 void mlp_infer_tc(int device, int rows, const float* raw, const float* params,
                   const float* mean, const float* inv_std, float* Y, int* err, cudaStream_t s);
-
-// C = op(A) op(B) (+ bias over columns), row-major, FP32; split over K into
-// `splits` partial products added in fixed order.
-void gemm(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-          float* C, int ldc, const float* bias, int splits, float* part, cudaStream_t s);
 
 }  // namespace cg
