@@ -648,24 +648,30 @@ static void exp_neg_pair(double v, double& hi, double& lo) {
   hi = sh, lo = sl;
 }
 
-void Geometry::upload(cudaStream_t s) {
-  {
-    std::vector<float2> tab(DD_EXP_TAB);
-    for (int k = 0; k < DD_EXP_TAB; ++k) {
-      const double e = std::exp(-0.0625 * k);
-      tab[k]         = make_float2((float)e, (float)(e - (double)(float)e));
-    }
-    dd_exp.upload(tab, s);
-    tab.resize(NEAR64_DDTAB);
-    std::vector<double> tab64(2 * NEAR64_ETAB);  // value and rest (a Taylor product below)
-    for (int k = 0; k < NEAR64_DDTAB; ++k) {
-      const double e = std::exp(-0.0625 * k);
-      tab[k]         = make_float2((float)e, (float)(e - (double)(float)e));
-      if (k < NEAR64_ETAB) exp_neg_pair(0.0625 * k, tab64[2 * k], tab64[2 * k + 1]);
-    }
-    near_exp.upload(tab, s);
-    near_exp64.upload(tab64, s);
+// Tables of e^-v at steps of 1/16, formed once per process.
+namespace {
+struct ExpTables {
+  std::vector<float2> dd, near;
+  std::vector<double> near64;  // value and rest
+  ExpTables() : dd(DD_EXP_TAB), near(NEAR64_DDTAB), near64(2 * NEAR64_ETAB) {
+    for (auto* t : {&dd, &near})
+      for (size_t k = 0; k < t->size(); ++k) {
+        const double e = std::exp(-0.0625 * k);
+        (*t)[k]        = make_float2((float)e, (float)(e - (double)(float)e));
+      }
+    for (int k = 0; k < NEAR64_ETAB; ++k) exp_neg_pair(0.0625 * k, near64[2 * k], near64[2 * k + 1]);
   }
+};
+const ExpTables& exp_tables() {
+  static const ExpTables t;
+  return t;
+}
+}  // namespace
+
+void Geometry::upload(cudaStream_t s) {
+  dd_exp.upload(exp_tables().dd, s);
+  near_exp.upload(exp_tables().near, s);
+  near_exp64.upload(exp_tables().near64, s);
   items.upload(h_items, s);
   item_split.upload(h_item_split, s);
   leaf_nslot.upload(h_leaf_nslot, s);
