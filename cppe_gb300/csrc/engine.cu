@@ -1714,31 +1714,117 @@ __device__ __forceinline__ void dd2_thole(const dd2& ai, const dd2& s, const dd2
   G2 = dd2_sel(sx, sy, G2n, G2);
 }
 
-struct DDSrc2 {
-  dd2 x, y, z, s, mx, my, mz;
+// Sums of many products, each entering with its rounding error: S starts at an
+// offset C that is larger than anything added to it, so that S and S' = fl(S + a b)
+// lie within a factor of two, S - S' is exact (Sterbenz) and fma(a, b, S - S') is
+// what the addition and the product rounded off.  Six operations a product, where
+// a product with its error and a two-sum take twelve; C is taken off at the end
+// (exactly).  The error is some 2^-48 of C for each product, as it is of the sum
+// in the other form.  The near field is bound by the FP32 pipe (FFMA2 with three
+// different operands reaches 2/3 of its rate, FADD2 all of it); with offset sums
+// for R^2, m.r and the field: 30,000 sites (126.6 M pairs) 0.99 -> 0.88 ms, 300,000
+// 4.20 -> 4.05 ms, eight right-hand sides (32 snapshots, 500 to 20,000 sites) 14.6
+// -> 11.5 ms; error of an apply against FP64, 30,000 sites 4.0e-13 -> 2.8e-13,
+// 100,002 sites 1.08e-12 -> 4.9e-13.
+struct OffsetSum {
+  float2 s, l;
 };
-template <bool DAMP, int MODE>
-__device__ __forceinline__ void dd2_pair_m1(const dd2& tx, const dd2& ty, const dd2& tz,
-                                            const dd2& ai, const DDSrc2& q, const float* eh,
-                                            const float* el, dd2 (&f)[3]) {
-  const dd2 x  = {psub(tx.h, q.x.h), psub(tx.l, q.x.l)};
-  const dd2 y  = {psub(ty.h, q.y.h), psub(ty.l, q.y.l)};
-  const dd2 z  = {psub(tz.h, q.z.h), psub(tz.l, q.z.l)};
-  const dd2 r2 = dd2_add(dd2_add_lazy(dd2_sqr_full(x), dd2_sqr_full(y)), dd2_sqr_full(z));
-  const bool okx = r2.h.x > 0.f, oky = r2.h.y > 0.f;  // false: a site paired with itself
-  const dd2 zero = {p2(0.f), p2(0.f)};
-  const dd2 ir   = dd2_sel(okx, oky, dd2_rsqrt(dd2_sel(okx, oky, r2, {p2(1.f), p2(0.f)})), zero);
-  const dd2 ir2  = dd2_sqr(ir);
-  const dd2 ir3  = dd2_mul(ir2, ir);
-  dd2 G1         = dd2_neg(ir3);
-  dd2 G2         = dd2_mul_f(dd2_mul(ir3, ir2), p2(3.f));
-  if (DAMP && MODE < 2) dd2_thole<MODE>(ai, q.s, r2, ir, eh, el, G1, G2);
-  const dd2 mr = dd2_add(dd2_add_lazy(dd2_mul(q.mx, x), dd2_mul(q.my, y)), dd2_mul(q.mz, z));
-  const dd2 sg = dd2_mul(mr, G2);
-  f[0] = dd2_add_lazy(f[0], dd2_neg(dd2_add_lazy(dd2_mul(q.mx, G1), dd2_mul(sg, x))));
-  f[1] = dd2_add_lazy(f[1], dd2_neg(dd2_add_lazy(dd2_mul(q.my, G1), dd2_mul(sg, y))));
-  f[2] = dd2_add_lazy(f[2], dd2_neg(dd2_add_lazy(dd2_mul(q.mz, G1), dd2_mul(sg, z))));
+__device__ __forceinline__ void offset_fma(OffsetSum& S, const dd2& a, const dd2& b) {
+  const float2 t = pfma(a.h, b.h, S.s);
+  const float2 e = pfma(a.h, b.h, psub(S.s, t));
+  S.l            = padd(S.l, pfma(a.l, b.h, pfma(a.h, b.l, e)));
+  S.s            = t;
 }
+
+struct DDSrc2 {
+  dd2 x, y, z, s;
+};
+// Of a packed pair: the separation, R in FP32, G1 = f_E R^-3 and G2 = -3 f_T R^-5.
+template <bool DAMP, int MODE>
+__device__ __forceinline__ void dd2_pair_tensor(const dd2& tx, const dd2& ty, const dd2& tz,
+                                                const dd2& ai, const DDSrc2& q, const float* eh,
+                                                const float* el, dd2& x, dd2& y, dd2& z,
+                                                float2& R, dd2& G1, dd2& G2) {
+  x = {psub(tx.h, q.x.h), psub(tx.l, q.x.l)};
+  y = {psub(ty.h, q.y.h), psub(ty.l, q.y.l)};
+  z = {psub(tz.h, q.z.h), psub(tz.l, q.z.l)};
+  // R^2: the squares of the high parts as an offset sum (C = twice their FP32
+  // sum), (2 h + l) l of the low parts
+  const float2 C = pmul(p2(2.f), pfma(z.h, z.h, pfma(y.h, y.h, pmul(x.h, x.h))));
+  OffsetSum S    = {C, p2(0.f)};
+  auto square    = [&](const dd2& v) {
+    const float2 t = pfma(v.h, v.h, S.s);
+    S.l            = pfma(pfma(p2(2.f), v.h, v.l), v.l, padd(S.l, pfma(v.h, v.h, psub(S.s, t))));
+    S.s            = t;
+  };
+  square(x), square(y), square(z);
+  const dd2 r2   = dd2_fast_two_sum(psub(S.s, C), S.l);
+  const bool okx = r2.h.x > 0.f, oky = r2.h.y > 0.f;  // false: a site paired with itself
+  // y = 1/R in FP32 and h = R^2 y^2 - 1 (|h| < 2^-21), y^2 split by an FMA
+  const float2 w  = make_float2(okx ? rsqrt_ftz(r2.h.x) : 0.f, oky ? rsqrt_ftz(r2.h.y) : 0.f);
+  const float2 w2 = pmul(w, w);
+  const float2 we = pfma(w, w, pneg(w2));
+  const float2 h  = pfma(r2.h, we, pfma(r2.l, w2, pfma(r2.h, w2, p2(-1.f))));
+  R               = pmul(r2.h, w);
+  // R^-3 = y^3 (1 - 3 h / 2 + 15 h^2 / 8), -3 R^-2 = -3 y^2 (1 - h + h^2)
+  const float2 w3 = pmul(w, w2);
+  G1 = {w3, pfma(w3, pmul(h, pfma(p2(1.875f), h, p2(-1.5f))),
+                 pfma(w, we, pfma(w, w2, pneg(w3))))};
+  const float2 t3 = pmul(p2(-3.f), w2);
+  G2 = dd2_mul(G1, {t3, pfma(t3, pfma(h, h, pneg(h)),
+                             pfma(p2(-3.f), we, pfma(p2(-3.f), w2, pneg(t3))))});
+  G2 = dd2_fast_two_sum(G2.h, G2.l);
+  if (DAMP && MODE < 2) {
+    const dd2 ir = {w, pmul(pmul(w, h), pfma(p2(0.375f), h, p2(-0.5f)))};
+    dd2_thole<MODE>(ai, q.s, r2, ir, eh, el, G1, G2);
+  }
+}
+// m.r of a packed pair, |m.r| <= C / 2.
+__device__ __forceinline__ dd2 dd2_dot(const dd2& mx, const dd2& my, const dd2& mz, const dd2& x,
+                                       const dd2& y, const dd2& z, float2 C) {
+  OffsetSum S = {C, p2(0.f)};
+  offset_fma(S, mx, x), offset_fma(S, my, y), offset_fma(S, mz, z);
+  // (renormalised: the low parts of the separations are up to 2^-16 of it)
+  return dd2_fast_two_sum(psub(S.s, C), S.l);
+}
+// A bound of a packed pair's f_E R^-3 in FP32 (0 for R = 0), from the high parts of
+// the separation unless they are as small as the low ones (R^2 < lim).  Damped:
+// f_T <= f_E <= v^3 / 6, so R^-3 f_E <= (a 6^(-1/3))^3; ac = 0.551 damping s_i.
+template <bool DAMP>
+__device__ __forceinline__ float2 dd2_cube_bound(const dd2& tx, const dd2& ty, const dd2& tz,
+                                                 float ac, float4 A0, float4 B0, float lim,
+                                                 const float4* C0, const float4* D0) {
+  float2 x = psub(tx.h, make_float2(A0.x, A0.y)), y = psub(ty.h, make_float2(A0.z, A0.w)),
+         z = psub(tz.h, make_float2(B0.x, B0.y));
+  float2 r2 = pfma(x, x, pfma(y, y, pmul(z, z)));
+  float2 w;
+  if (r2.x < lim || r2.y < lim) {
+    const float4 c = *C0, d = *D0;
+    x  = padd(x, psub(tx.l, make_float2(c.x, c.y)));
+    y  = padd(y, psub(ty.l, make_float2(c.z, c.w)));
+    z  = padd(z, psub(tz.l, make_float2(d.x, d.y)));
+    r2 = pfma(x, x, pfma(y, y, pmul(z, z)));
+    w  = make_float2(r2.x > 0.f ? rsqrt_ftz(r2.x) : 0.f, r2.y > 0.f ? rsqrt_ftz(r2.y) : 0.f);
+  } else {
+    w = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+  }
+  if (DAMP) {  // (s = 0: undamped)
+    const float2 a = pmul(p2(ac), make_float2(B0.z, B0.w));
+    w = make_float2(a.x > 0.f ? fminf(w.x, a.x) : w.x, a.y > 0.f ? fminf(w.y, a.y) : w.y);
+  }
+  return pmul(pmul(w, w), w);
+}
+// Twice a bound of |m|: sqrt(x^2 + y^2 + z^2) <= max + (sqrt(2) - 1) (the others).
+__device__ __forceinline__ float dd_moment_bound(float mx, float my, float mz) {
+  const float a = fabsf(mx), b = fabsf(my), c = fabsf(mz), m = fmaxf(a, fmaxf(b, c));
+  return 2.002f * fmaf(0.41422f, (a + b + c) - m, m);
+}
+// The offset over the sum of R^-3 times that bound: pairs move S by no more than
+// 2 |m| R^-3 each and a product is at most 3 |m| R^-3, so 3.5 keeps every S and S'
+// within a factor of two.  Runs of DD_RUN source pairs: the offset follows the
+// distance, and few low parts are added up before they are renormalised.
+constexpr float DD_OFFSET = 4.1f;
+constexpr int DD_RUN      = 16;
 
 // One target per thread (its packed accumulators are already 4 x 3 floats),
 // sources staged in pairs: positions (high and low parts), s and the
@@ -1749,9 +1835,11 @@ __global__ void __launch_bounds__(P2P_BLOCK)
       k_p2p_dd2(int n, const int* __restrict__ leaf_start, const int4* __restrict__ items,
                 const int* __restrict__ item_split, const int* __restrict__ p2p_src,
                 PosArgs<float> pa, const float2* __restrict__ src,
-                const float2* __restrict__ etab, double damping, double* __restrict__ Fnear) {
+                const float2* __restrict__ etab, double damping, float lim,
+                double* __restrict__ Fnear) {
   constexpr int TILE = 2 * P2P_DD_PAIRS;
   __shared__ float4 s_q[7][P2P_DD_PAIRS];
+  __shared__ float2 s_mn[P2P_DD_PAIRS];
   __shared__ float s_eh[DD_EXP_TAB], s_el[DD_EXP_TAB];
   __shared__ TilePlan s_plan;
   __shared__ double s_red[P2P_BLOCK * 3];
@@ -1775,8 +1863,8 @@ __global__ void __launch_bounds__(P2P_BLOCK)
     const dd2 tx = {p2(me.x), p2(me.lx)}, ty = {p2(me.y), p2(me.ly)}, tz = {p2(me.z), p2(me.lz)};
     const dd ai1 = dd_mul(dmp, dd{me.s, me.ls});
     const dd2 ai = {p2(ai1.h), p2(ai1.l)};
-    const dd2 zero = {p2(0.f), p2(0.f)};
-    dd2 f[3] = {zero, zero, zero};
+    const float ac = 0.551f * ai1.h;
+    dd f[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};  // over the tiles
     // phase 0: sources [b0, sp); phase 1: [sp, b1), every pair with v >= 27
     for (int ph = 0; ph < 2; ++ph) {
       const int pend = ph == 0 ? sp : b1;
@@ -1810,13 +1898,23 @@ __global__ void __launch_bounds__(P2P_BLOCK)
           s_q[4][q] = make_float4(m0x.x, m1x.x, m0y.x, m1y.x);
           s_q[5][q] = make_float4(m0z.x, m1z.x, m0x.y, m1x.y);
           s_q[6][q] = make_float4(m0y.y, m1y.y, m0z.y, m1z.y);
+          s_mn[q]   = make_float2(dd_moment_bound(m0x.x, m0y.x, m0z.x),
+                                  dd_moment_bound(m1x.x, m1y.x, m1z.x));
         }
         __syncthreads();
         if (active) {
-          auto sweep = [&](auto mode) {
+          auto sweep = [&](auto mode, int j0, int j1) {
             constexpr int MD = decltype(mode)::value;
+            float2 C = p2(0.f);
+#pragma unroll 4
+            for (int jj = j0; jj < j1; jj += S)
+              C = pfma(dd2_cube_bound<DAMP>(tx, ty, tz, ac, s_q[0][jj], s_q[1][jj], lim,
+                                            &s_q[2][jj], &s_q[3][jj]),
+                       s_mn[jj], C);
+            C = pmul(C, p2(DD_OFFSET));
+            OffsetSum F[3] = {{C, p2(0.f)}, {C, p2(0.f)}, {C, p2(0.f)}};
 #pragma unroll 1
-            for (int jj = g; jj < npairs; jj += S) {
+            for (int jj = j0; jj < j1; jj += S) {
               const float4 A0 = s_q[0][jj], B0 = s_q[1][jj], C0 = s_q[2][jj], D0 = s_q[3][jj];
               const float4 E0 = s_q[4][jj], F0 = s_q[5][jj], G0 = s_q[6][jj];
               DDSrc2 q;
@@ -1824,16 +1922,30 @@ __global__ void __launch_bounds__(P2P_BLOCK)
               q.y  = {make_float2(A0.z, A0.w), make_float2(C0.z, C0.w)};
               q.z  = {make_float2(B0.x, B0.y), make_float2(D0.x, D0.y)};
               q.s  = {make_float2(B0.z, B0.w), make_float2(D0.z, D0.w)};
-              q.mx = {make_float2(E0.x, E0.y), make_float2(F0.z, F0.w)};
-              q.my = {make_float2(E0.z, E0.w), make_float2(G0.x, G0.y)};
-              q.mz = {make_float2(F0.x, F0.y), make_float2(G0.z, G0.w)};
-              dd2_pair_m1<DAMP, MD>(tx, ty, tz, ai, q, s_eh, s_el, f);
+              const dd2 mx = {make_float2(E0.x, E0.y), make_float2(F0.z, F0.w)};
+              const dd2 my = {make_float2(E0.z, E0.w), make_float2(G0.x, G0.y)};
+              const dd2 mz = {make_float2(F0.x, F0.y), make_float2(G0.z, G0.w)};
+              dd2 x, y, z, G1, G2;
+              float2 R;
+              dd2_pair_tensor<DAMP, MD>(tx, ty, tz, ai, q, s_eh, s_el, x, y, z, R, G1, G2);
+              const dd2 sg = dd2_mul(dd2_dot(mx, my, mz, x, y, z, pmul(s_mn[jj], R)), G2);
+              offset_fma(F[0], mx, G1), offset_fma(F[0], sg, x);
+              offset_fma(F[1], my, G1), offset_fma(F[1], sg, y);
+              offset_fma(F[2], mz, G1), offset_fma(F[2], sg, z);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const float2 h = psub(F[c].s, C);
+              f[c] = dd_add(f[c], dd_add(dd{h.x, F[c].l.x}, dd{h.y, F[c].l.y}));
             }
           };
-          if (!DAMP || ph == 0)
-            sweep(std::integral_constant<int, 0>{});
-          else
-            sweep(std::integral_constant<int, 1>{});
+          for (int j0 = g; j0 < npairs; j0 += DD_RUN * S) {
+            const int j1 = min(npairs, j0 + DD_RUN * S);
+            if (!DAMP || ph == 0)
+              sweep(std::integral_constant<int, 0>{}, j0, j1);
+            else
+              sweep(std::integral_constant<int, 1>{}, j0, j1);
+          }
         }
         __syncthreads();
       }
@@ -1841,11 +1953,7 @@ __global__ void __launch_bounds__(P2P_BLOCK)
     if (active) {
       double* r = &s_red[(g * nT + t) * 3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        // the two halves' sums, added in double-float, then widened
-        const dd h0 = {f[c].h.x, f[c].l.x}, h1 = {f[c].h.y, f[c].l.y};
-        r[c] = dd_to(dd_add(h0, h1));
-      }
+      for (int c = 0; c < 3; ++c) r[c] = dd_to(f[c]);
     }
     __syncthreads();
     if (threadIdx.x < nT) {
@@ -1868,42 +1976,29 @@ namespace cg {
 // Double-float near field over a batch's right-hand sides together (the
 // residual counterpart of k_p2p32_m1_multi): the pair tensor G1 I + G2 r r^T
 // in double-float (separation, 1/R powers, Thole factors) once per pair,
-// applied to the source moments of every copy.  Same arithmetic per term as
-// dd2_pair_m1; one target per thread with R packed accumulators; the
+// applied to the source moments of every copy.  Same arithmetic per term;
+// one target per thread with R packed accumulators; the
 // per-copy sums are reduced and written one copy at a time.
 // ---------------------------------------------------------------------------
-template <bool DAMP, int MODE>
-__device__ __forceinline__ void dd2_pair_tensor(const dd2& tx, const dd2& ty, const dd2& tz,
-                                                const dd2& ai, const dd2& qx, const dd2& qy,
-                                                const dd2& qz, const dd2& qs, const float* eh,
-                                                const float* el, dd2& x, dd2& y, dd2& z,
-                                                dd2& G1, dd2& G2) {
-  x = {psub(tx.h, qx.h), psub(tx.l, qx.l)};
-  y = {psub(ty.h, qy.h), psub(ty.l, qy.l)};
-  z = {psub(tz.h, qz.h), psub(tz.l, qz.l)};
-  const dd2 r2 = dd2_add(dd2_add_lazy(dd2_sqr_full(x), dd2_sqr_full(y)), dd2_sqr_full(z));
-  const bool okx = r2.h.x > 0.f, oky = r2.h.y > 0.f;  // false: a site paired with itself
-  const dd2 zero = {p2(0.f), p2(0.f)};
-  const dd2 ir   = dd2_sel(okx, oky, dd2_rsqrt(dd2_sel(okx, oky, r2, {p2(1.f), p2(0.f)})), zero);
-  const dd2 ir2  = dd2_sqr(ir);
-  const dd2 ir3  = dd2_mul(ir2, ir);
-  G1 = dd2_neg(ir3);
-  G2 = dd2_mul_f(dd2_mul(ir3, ir2), p2(3.f));
-  if (DAMP && MODE < 2) dd2_thole<MODE>(ai, qs, r2, ir, eh, el, G1, G2);
-}
-
 constexpr int P2PM_DD_PAIRS = 80;  // staged source pairs per tile (160 sources)
+constexpr int P2PM_DD_SMEM  = P2PM_MAXR * (P2PM_DD_PAIRS * (3 * 16 + 8) + 4 * P2P_BLOCK * 8);
 template <bool DAMP>
 __global__ void __launch_bounds__(P2P_BLOCK)
       k_p2p_dd2_multi(int n, const int* __restrict__ leaf_start, const int4* __restrict__ items,
                       const int* __restrict__ item_split, const int2* __restrict__ item_stride,
                       int c0, int nr, const int* __restrict__ p2p_src, PosArgs<float> pa,
                       const float2* __restrict__ src, const float2* __restrict__ etab,
-                      double damping, double* __restrict__ Fnear) {
+                      double damping, float lim, double* __restrict__ Fnear) {
   constexpr int TILE = 2 * P2PM_DD_PAIRS;
   constexpr int R    = P2PM_MAXR;
   __shared__ float4 s_g[4][P2PM_DD_PAIRS];       // positions (high, low) and s
-  __shared__ float4 s_m[3][P2PM_DD_PAIRS * R];   // per copy: the moments' pairs
+  extern __shared__ float4 s_dyn[];
+  float4(*s_m)[P2PM_DD_PAIRS * R] =               // per copy: the moments' pairs,
+        reinterpret_cast<float4(*)[P2PM_DD_PAIRS * R]>(s_dyn);
+  float2(*s_f)[P2P_BLOCK] =                       // each thread's sums (double-float)
+        reinterpret_cast<float2(*)[P2P_BLOCK]>(s_dyn + 3 * P2PM_DD_PAIRS * R);
+  float2(*s_c)[P2P_BLOCK] = s_f + 3 * R;          // and offsets,
+  float2* s_mn = &s_c[R][0];                      // the moments' bounds
   __shared__ int s_site[TILE];
   __shared__ float s_eh[DD_EXP_TAB], s_el[DD_EXP_TAB];
   __shared__ TilePlan s_plan;
@@ -1929,10 +2024,9 @@ __global__ void __launch_bounds__(P2P_BLOCK)
     const dd2 tx = {p2(me.x), p2(me.lx)}, ty = {p2(me.y), p2(me.ly)}, tz = {p2(me.z), p2(me.lz)};
     const dd ai1 = dd_mul(dmp, dd{me.s, me.ls});
     const dd2 ai = {p2(ai1.h), p2(ai1.l)};
-    const dd2 zero = {p2(0.f), p2(0.f)};
-    dd2 f[R][3];
+    const float ac = 0.551f * ai1.h;
 #pragma unroll
-    for (int r = 0; r < R; ++r) f[r][0] = f[r][1] = f[r][2] = zero;
+    for (int r = 0; r < 3 * R; ++r) s_f[r][threadIdx.x] = p2(0.f);
     for (int ph = 0; ph < 2; ++ph) {
       const int pend = ph == 0 ? sp : b1;
       if (threadIdx.x == 0) s_plan.cur = ph == 0 ? b0 : sp, s_plan.coff = 0;
@@ -1972,51 +2066,88 @@ __global__ void __launch_bounds__(P2P_BLOCK)
           s_m[0][q * R + r] = make_float4(m0x.x, m1x.x, m0y.x, m1y.x);
           s_m[1][q * R + r] = make_float4(m0z.x, m1z.x, m0x.y, m1x.y);
           s_m[2][q * R + r] = make_float4(m0y.y, m1y.y, m0z.y, m1z.y);
+          s_mn[q * R + r]   = make_float2(dd_moment_bound(m0x.x, m0y.x, m0z.x),
+                                          dd_moment_bound(m1x.x, m1y.x, m1z.x));
         }
         __syncthreads();
         if (active) {
-          // all R copies in this pass: their updates run unguarded
-          auto sweep = [&](auto mode, auto all) {
-            constexpr int MD  = decltype(mode)::value;
-            constexpr bool AL = decltype(all)::value;
+          for (int j0 = g; j0 < npairs; j0 += DD_RUN * S) {
+            const int j1 = min(npairs, j0 + DD_RUN * S);
+            OffsetSum F[R][3];
+            {
+              float2 C[R];
+#pragma unroll
+              for (int r = 0; r < R; ++r) C[r] = p2(0.f);
 #pragma unroll 1
-            for (int jj = g; jj < npairs; jj += S) {
-              const float4 A0 = s_g[0][jj], B0 = s_g[1][jj], C0 = s_g[2][jj], D0 = s_g[3][jj];
-              const dd2 qx = {make_float2(A0.x, A0.y), make_float2(C0.x, C0.y)};
-              const dd2 qy = {make_float2(A0.z, A0.w), make_float2(C0.z, C0.w)};
-              const dd2 qz = {make_float2(B0.x, B0.y), make_float2(D0.x, D0.y)};
-              const dd2 qs = {make_float2(B0.z, B0.w), make_float2(D0.z, D0.w)};
-              dd2 x, y, z, G1, G2;
-              dd2_pair_tensor<DAMP, MD>(tx, ty, tz, ai, qx, qy, qz, qs, s_eh, s_el, x, y, z, G1,
-                                        G2);
+              for (int jj = j0; jj < j1; jj += S) {
+                const float2 w = dd2_cube_bound<DAMP>(tx, ty, tz, ac, s_g[0][jj], s_g[1][jj], lim,
+                                                &s_g[2][jj], &s_g[3][jj]);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                  if (r < nr) C[r] = pfma(w, s_mn[jj * R + r], C[r]);
+              }
 #pragma unroll
               for (int r = 0; r < R; ++r) {
-                if (AL || r < nr) {
-                  const float4 E0 = s_m[0][jj * R + r], F0 = s_m[1][jj * R + r],
-                               G0 = s_m[2][jj * R + r];
-                  const dd2 mx = {make_float2(E0.x, E0.y), make_float2(F0.z, F0.w)};
-                  const dd2 my = {make_float2(E0.z, E0.w), make_float2(G0.x, G0.y)};
-                  const dd2 mz = {make_float2(F0.x, F0.y), make_float2(G0.z, G0.w)};
-                  const dd2 mr =
-                        dd2_add(dd2_add_lazy(dd2_mul(mx, x), dd2_mul(my, y)), dd2_mul(mz, z));
-                  const dd2 sg = dd2_mul(mr, G2);
-                  f[r][0] = dd2_add_lazy(f[r][0], dd2_neg(dd2_add_lazy(dd2_mul(mx, G1), dd2_mul(sg, x))));
-                  f[r][1] = dd2_add_lazy(f[r][1], dd2_neg(dd2_add_lazy(dd2_mul(my, G1), dd2_mul(sg, y))));
-                  f[r][2] = dd2_add_lazy(f[r][2], dd2_neg(dd2_add_lazy(dd2_mul(mz, G1), dd2_mul(sg, z))));
-                }
+                C[r]               = pmul(C[r], p2(DD_OFFSET));
+                s_c[r][threadIdx.x] = C[r];
+                F[r][0] = F[r][1] = F[r][2] = {C[r], p2(0.f)};
               }
             }
-          };
-          if (nr == R) {
-            if (!DAMP || ph == 0)
-              sweep(std::integral_constant<int, 0>{}, std::true_type{});
-            else
-              sweep(std::integral_constant<int, 1>{}, std::true_type{});
-          } else {
-            if (!DAMP || ph == 0)
-              sweep(std::integral_constant<int, 0>{}, std::false_type{});
-            else
-              sweep(std::integral_constant<int, 1>{}, std::false_type{});
+            // all R copies in this pass: their updates run unguarded
+            auto sweep = [&](auto mode, auto all) {
+              constexpr int MD  = decltype(mode)::value;
+              constexpr bool AL = decltype(all)::value;
+#pragma unroll 1
+              for (int jj = j0; jj < j1; jj += S) {
+                const float4 A0 = s_g[0][jj], B0 = s_g[1][jj], C0 = s_g[2][jj], D0 = s_g[3][jj];
+                DDSrc2 q;
+                q.x = {make_float2(A0.x, A0.y), make_float2(C0.x, C0.y)};
+                q.y = {make_float2(A0.z, A0.w), make_float2(C0.z, C0.w)};
+                q.z = {make_float2(B0.x, B0.y), make_float2(D0.x, D0.y)};
+                q.s = {make_float2(B0.z, B0.w), make_float2(D0.z, D0.w)};
+                dd2 x, y, z, G1, G2;
+                float2 R1;
+                dd2_pair_tensor<DAMP, MD>(tx, ty, tz, ai, q, s_eh, s_el, x, y, z, R1, G1, G2);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  if (AL || r < nr) {
+                    const float4 E0 = s_m[0][jj * R + r], F0 = s_m[1][jj * R + r],
+                                 G0 = s_m[2][jj * R + r];
+                    const dd2 mx = {make_float2(E0.x, E0.y), make_float2(F0.z, F0.w)};
+                    const dd2 my = {make_float2(E0.z, E0.w), make_float2(G0.x, G0.y)};
+                    const dd2 mz = {make_float2(F0.x, F0.y), make_float2(G0.z, G0.w)};
+                    const dd2 sg = dd2_mul(
+                          dd2_dot(mx, my, mz, x, y, z, pmul(s_mn[jj * R + r], R1)), G2);
+                    offset_fma(F[r][0], mx, G1), offset_fma(F[r][0], sg, x);
+                    offset_fma(F[r][1], my, G1), offset_fma(F[r][1], sg, y);
+                    offset_fma(F[r][2], mz, G1), offset_fma(F[r][2], sg, z);
+                  }
+                }
+              }
+            };
+            if (nr == R) {
+              if (!DAMP || ph == 0)
+                sweep(std::integral_constant<int, 0>{}, std::true_type{});
+              else
+                sweep(std::integral_constant<int, 1>{}, std::true_type{});
+            } else {
+              if (!DAMP || ph == 0)
+                sweep(std::integral_constant<int, 0>{}, std::false_type{});
+              else
+                sweep(std::integral_constant<int, 1>{}, std::false_type{});
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              if (r >= nr) break;
+              const float2 C = s_c[r][threadIdx.x];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) {
+                const float2 h = psub(F[r][c].s, C), o = s_f[3 * r + c][threadIdx.x];
+                const dd v     = dd_add(dd{o.x, o.y}, dd_add(dd{h.x, F[r][c].l.x},
+                                                             dd{h.y, F[r][c].l.y}));
+                s_f[3 * r + c][threadIdx.x] = make_float2(v.h, v.l);
+              }
+            }
           }
         }
         __syncthreads();
@@ -2030,8 +2161,8 @@ __global__ void __launch_bounds__(P2P_BLOCK)
         double* rr = &s_red[(g * nT + t) * 3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const dd h0 = {f[r][c].h.x, f[r][c].l.x}, h1 = {f[r][c].h.y, f[r][c].l.y};
-          rr[c] = dd_to(dd_add(h0, h1));
+          const float2 v = s_f[3 * r + c][threadIdx.x];
+          rr[c]          = dd_to(dd{v.x, v.y});
         }
       }
       __syncthreads();
@@ -2710,23 +2841,21 @@ __global__ void k_split_dd(long n, const double* __restrict__ in, float2* __rest
 
 static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, double damping,
                           FieldWork<double>& w, cudaStream_t s) {
-  const long n3 = 3L * g.n;
+  const long n3   = 3L * g.n;
+  const float lim = (float)(4096.0 * g.grid * g.grid);  // R^2 of 64 grid steps
   w.dd_src.alloc(std::max(1L, n3));
   k_split_dd<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(n3, src, w.dd_src.p);
   CG_LAUNCH();
   if (!g.h_mitems.empty() && g.ncopies > 1) {
     // a batch's right-hand sides together, up to P2PM_MAXR per launch
     const int mg = (int)g.h_mitems.size();
+    auto kern = damp ? k_p2p_dd2_multi<true> : k_p2p_dd2_multi<false>;
+    CG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P2PM_DD_SMEM));
     for (int c0 = 0; c0 < g.ncopies; c0 += P2PM_MAXR) {
       const int nr = std::min(P2PM_MAXR, g.ncopies - c0);
-      if (damp)
-        k_p2p_dd2_multi<true><<<mg, P2P_BLOCK, 0, s>>>(
-              g.n, g.leaf_start.p, g.mitems.p, g.mitem_split.p, g.mitem_stride.p, c0, nr,
-              g.p2p_src.p, pos_args<float>(g), w.dd_src.p, g.dd_exp.p, damping, w.Fnear.p);
-      else
-        k_p2p_dd2_multi<false><<<mg, P2P_BLOCK, 0, s>>>(
-              g.n, g.leaf_start.p, g.mitems.p, g.mitem_split.p, g.mitem_stride.p, c0, nr,
-              g.p2p_src.p, pos_args<float>(g), w.dd_src.p, g.dd_exp.p, damping, w.Fnear.p);
+      kern<<<mg, P2P_BLOCK, P2PM_DD_SMEM, s>>>(
+            g.n, g.leaf_start.p, g.mitems.p, g.mitem_split.p, g.mitem_stride.p, c0, nr,
+            g.p2p_src.p, pos_args<float>(g), w.dd_src.p, g.dd_exp.p, damping, lim, w.Fnear.p);
       CG_LAUNCH();
     }
     return;
@@ -2735,11 +2864,11 @@ static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, doubl
   if (damp)
     k_p2p_dd2<true><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
                                                g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                               g.dd_exp.p, damping, w.Fnear.p);
+                                               g.dd_exp.p, damping, lim, w.Fnear.p);
   else
     k_p2p_dd2<false><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
                                                 g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                                g.dd_exp.p, damping, w.Fnear.p);
+                                                g.dd_exp.p, damping, lim, w.Fnear.p);
   CG_LAUNCH();
 }
 
