@@ -2420,10 +2420,12 @@ __global__ void __launch_bounds__(SHIFT_THREADS)
 #pragma unroll
   for (int r = 0; r < MS; ++r) s_part[threadIdx.x * (MS + 1) + r] = acc[r];
   __syncthreads();
+  // (a leaf of 9 to 64 sites: only the threads that have one are added up)
+  const int nt = min(SHIFT_THREADS, a1 - a0);
   for (int r = threadIdx.x; r < MST; r += SHIFT_THREADS) {
     T v = T(0);
     if (r < MS)
-      for (int t = 0; t < SHIFT_THREADS; ++t) v += s_part[t * (MS + 1) + r];
+      for (int t = 0; t < nt; ++t) v += s_part[t * (MS + 1) + r];
     M[(size_t)cell * MST + r] = v;
   }
 }
