@@ -251,6 +251,12 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
   // near-field / direct loops (self pairs and excluded pairs are skipped there)
   alg_pairs = near_pairs - n - (long)cidx.size();
   make_schedules();
+  // four sources a lane: faster with long partner lists and enough items (120,000
+  // sites, 4,090 pairs a site: 0.479 against 0.497 ms; 600,000, 2,800: 1.90 against
+  // 1.97; 1M, 4,750: 4.23 against 4.51), slower with short ones (300,000 sites,
+  // 1,680: 0.884 against 0.870; 60,000, 1,980: 0.193 against 0.184) or few items
+  // (30,000 sites, 4,230: 0.154 against 0.147)
+  sym_pack = near_pairs >= 2500L * n && near_pairs >= 400000000L ? 2 : 1;
   make_vectors();
 }
 
@@ -503,7 +509,10 @@ void Geometry::make_schedules() {
   // the symmetric schedule of single systems (a batch keeps per-leaf items:
   // its passes skip finished segments and serve several right-hand sides)
   if (sym_enabled && h_leaf_seg.empty() && ncopies == 1)
-    make_sym_schedule(W);
+    // half the evaluations a pair: twice the pairs an item, unless there are few items
+    // (30,000 sites 0.172 -> 0.147 ms, 120,000 0.512 -> 0.497; 12,000 and 300,000 the
+    // same), and never below 8,192 (4,200 sites: 31 us, with smaller items 35)
+    make_sym_schedule(item_pairs > 0 ? W : W <= 8192 ? 8192 : 2 * W);
   else
     h_usrc.clear(), h_sym_items.clear();
   // a batch's copy-0 items, for the near-field pass over all its copies
@@ -2960,6 +2969,9 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
         k_m2m_tasks<T><<<ntask, TB, 0, fs>>>(tv, ov, g.p2m_tasks.p, g.task_leaf.p,
                                             cell_pos<T>(g), w.M.p, w.Mpart.p);
       CG_LAUNCH();
+    }
+    // (the fixed-order M2L adds the partials as it folds the multipoles)
+    if (ntask > 0 && !fixed_m2l) {
       const long work = (long)tv.ncells * mst;
       k_msum<T><<<(unsigned)((work + 255) / 256), 256, 0, fs>>>(
             tv.ncells, mst, g.cell_task_ptr.p, w.Mpart.p, w.M.p, cseg, seg_done);
@@ -2971,12 +2983,14 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
     // and double-float, where the recurrence is the expensive part; the FP32
     // translation builds its tensor in registers faster than it loads one
     const int nchunks = (int)g.h_m2l_chunks.size();
+    const int* task_ptr = ntask > 0 ? g.cell_task_ptr.p : nullptr;
     if constexpr (std::is_same<T, double>::value) {
       if (fixedP && near_mode == NEAR_DD) {
         const void* dt = m2l_dtab<true, T>(g, ov.m, ov.p, w, fs);
         m2l_done = launch_m2l_fixed<true>(tv, ov.m, ov.p, g.m2l_chunks.p, nchunks,
                                           g.cell_chunk_ptr.p, w.M.p, mst, w.Mdd, w.Lpart, w.L.p, fs,
-                                          nullptr, nullptr, dt, dt ? g.m2l_vid.p : nullptr);
+                                          nullptr, nullptr, dt, dt ? g.m2l_vid.p : nullptr, task_ptr,
+                                          w.Mpart.p);
       }
     }
     if (fixed_m2l && !m2l_done) {
@@ -2984,7 +2998,7 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
       if constexpr (std::is_same<T, double>::value) dt = m2l_dtab<false, T>(g, ov.m, ov.p, w, fs);
       m2l_done = launch_m2l_fixed<false>(tv, ov.m, ov.p, g.m2l_chunks.p, nchunks,
                                          g.cell_chunk_ptr.p, w.M.p, mst, w.Mr, w.Lpart, w.L.p, fs, cseg,
-                                         seg_done, dt, dt ? g.m2l_vid.p : nullptr);
+                                         seg_done, dt, dt ? g.m2l_vid.p : nullptr, task_ptr, w.Mpart.p);
     }
     if (!m2l_done) {
       size_t smem = (size_t)(ov.nm2l_terms + 9 * ov.nt) * sizeof(int);
