@@ -2304,7 +2304,8 @@ __global__ void __launch_bounds__(128)
 // Upward pass above the leaves, one block per task {cell, leaves}: thread
 // `row` adds the M2M shifts of the task's leaf multipoles straight to the
 // cell centre (the shift is exact, so going through the intermediate levels
-// changes nothing).  Partial expansions per task; k_msum adds a cell's tasks.
+// changes nothing).  Partial expansions per task; k_msum (or the
+// fixed-order M2L's fold) adds a cell's tasks.
 template <typename T>
 __global__ void __launch_bounds__(128)
       k_m2m_tasks(TreeView tv, OpsView ov, const int4* __restrict__ tasks,
