@@ -2910,6 +2910,9 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
                 double* out64, double sign, const ReduceSlots* dot, cudaStream_t s,
                 const PhaseEvents* pe, int near_mode, const SideStream* side,
                 const int* seg_done) {
+  // (a factor that is not positive damps nothing, as in radial(): the undamped
+  // kernels, since the damped ones take the squares or exponentials of v as they come)
+  damp = damp && damping > 0.0;
   const TreeView tv = g.view();
   OpsView ov{};
   int fixedP  = 0;  // order of the straight-line expansion operators in use (0: tables)
@@ -3044,9 +3047,9 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
     if (near_mode == NEAR_DD && m == 1) {
       launch_p2p_dd(g, damp, src, damping, w, s);
       done = true;
-    } else if (m > 0 && g.grid <= NEAR64_GRID) {
+    } else if (m > 0 && g.grid <= NEAR64_GRID && (!damp || damping >= NEAR64_DAMPING)) {
       // (k_p2p keeps systems of more than 2^18 bohr, whose coordinate grid is too
-      // coarse for the distance classes)
+      // coarse for the distance classes, and factors below NEAR64_DAMPING)
       launch_p2p64(g, m, damp, src, damping, w.Fnear.p, s, seg_done);
       nskip.hi = g.hi32.p, nskip.damping = (float)damping;
       done = true;

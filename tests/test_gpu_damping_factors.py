@@ -78,3 +78,46 @@ def test_batch(gpu):
     mu = [cabi.Batch(boxes, 2, thresh=1e-9, **kw).solve(rhs)[0]
           for kw in (dict(damp=True, damping=0.0), dict(damp=False))]
     np.testing.assert_allclose(mu[0], mu[1], rtol=0, atol=1e-8)
+
+
+@pytest.mark.parametrize("factor", [0.0, -2.1304, -1e-3, float("nan")])
+@pytest.mark.parametrize("waters,fmm", [(11, False), (343, False), (901, True)])
+def test_factors_that_damp_nothing(gpu, port, waters, fmm, factor):
+    """A factor that is not positive: the undamped operator in every arithmetic, and
+    the undamped fields."""
+    from cppe_gb300 import synthetic
+    b = synthetic.water_box(waters, seed=waters)
+    v = np.random.default_rng(1).normal(size=3 * b.n)
+    opts = dict(order=5, summation=cabi.FMM if fmm else cabi.DIRECT)
+    s = cabi.System(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, damp=True, damping=factor, **opts)
+    u = cabi.System(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, damp=False, **opts)
+    ref = port.bmatrix_apply(b.xyz, b.alpha6, b.excl_ptr, b.excl_idx, v, fmm=int(fmm), order=5)
+    assert np.linalg.norm(s.apply(v) - ref) < TOL * np.linalg.norm(ref)
+    for kw in (dict(fp32=True), dict(dd=True)):
+        assert np.array_equal(s.apply(v, **kw), u.apply(v, **kw))
+    one = np.ones(b.n, np.int32)
+    args = (b.xyz, b.q, b.mu, b.quad, 2, one, b.alpha_iso, b.excl_ptr, b.excl_idx)
+    got = cabi.multipole_fields(*args, fmm=fmm, damp=True, damping=factor)
+    want = cabi.multipole_fields(*args, fmm=fmm)
+    assert np.linalg.norm(got - want) <= 10 * TOL * np.linalg.norm(want)
+    s.close(), u.close()
+
+
+@pytest.mark.parametrize("factor", [1e-6, 1e-15])
+def test_sites_without_a_damping_partner(gpu, port, factor):
+    """Half of the sites take no part in the damping: their pairs stay undamped
+    whatever the factor."""
+    from cppe_gb300 import synthetic
+    from oracle import oracle as O
+    b = free(synthetic.water_box(343, seed=3))
+    pol = (np.arange(b.n) % 2).astype(np.int32)
+    a6 = b.alpha6 * pol[:, None]
+    for order in (1, 2):
+        site = O.Sites(xyz=b.xyz, elements=b.elements, q=b.q, mu=b.mu, quad=b.quad,
+                       max_order=order, alpha6=a6, polarizable=pol, excl_ptr=b.excl_ptr,
+                       excl_idx=b.excl_idx)
+        und = port.multipole_fields(site, fmm=False, order=5, damping=0.0)
+        ref = port.multipole_fields(site, fmm=False, order=5, damping=factor)
+        got = cabi.multipole_fields(b.xyz, b.q, b.mu, b.quad, order, pol, b.alpha_iso, b.excl_ptr,
+                                    b.excl_idx, damp=True, damping=factor)
+        assert np.linalg.norm(got - ref) < 10 * TOL * np.linalg.norm(und)
