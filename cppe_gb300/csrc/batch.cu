@@ -44,7 +44,10 @@ void Geometry::combine(const std::vector<const Geometry*>& parts, int copies, Ge
   out.damping   = parts[0]->damping;
   out.theta     = parts[0]->theta;
   out.ncopies   = copies;
-  for (auto* p : parts) out.grid = std::max(out.grid, p->grid);
+  for (auto* p : parts) {
+    out.grid = std::max(out.grid, p->grid);
+    for (int m = 0; m < 2; ++m) out.far_share[m] = std::max(out.far_share[m], p->far_share[m]);
+  }
   // cells: by (level, segment, cell)
   std::vector<std::vector<int>> cmap(nseg);
   for (int s = 0; s < nseg; ++s) cmap[s].assign(parts[part_of(s)]->layout.ncells, -1);

@@ -250,6 +250,7 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
   // algorithmic pairs: the ordered pairs the reference evaluates in its
   // near-field / direct loops (self pairs and excluded pairs are skipped there)
   alg_pairs = near_pairs - n - (long)cidx.size();
+  make_far_share();
   make_schedules();
   // four sources a lane: faster with long partner lists and enough items (120,000
   // sites, 4,090 pairs a site: 0.479 against 0.497 ms; 600,000, 2,800: 1.90 against
@@ -1981,6 +1982,30 @@ __global__ void __launch_bounds__(P2P_BLOCK)
 #include "near64.cuh"
 namespace cg {
 
+// far_share from some 16,000 pairs of evenly spaced sites (40 us).
+void Geometry::make_far_share() {
+  const TreeLayout& L = layout;
+  const long per = std::max(1L, near_pairs / std::max(1, n));
+  const int take = (int)std::min<long>(n, std::min(64L, std::max(4L, 16384 / per)));
+  double near[2] = {0.0, 0.0}, far[2] = {0.0, 0.0};
+  for (int t = 0; t < take; ++t) {
+    const int i          = (int)((2L * t + 1) * n / (2L * take));
+    const double4_32a pi = h_pos64[i];
+    const int a          = h_site_leaf[i];
+    for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q)
+      for (int k = L.leaf_start[L.p2p_src[q]]; k < L.leaf_start[L.p2p_src[q] + 1]; ++k) {
+        const double4_32a pk = h_pos64[k];
+        const double x = pi.x - pk.x, y = pi.y - pk.y, z = pi.z - pk.z;
+        const double r2 = x * x + y * y + z * z;
+        if (!(r2 > 0.0)) continue;
+        const double w = 1.0 / r2, w3 = w * w * w;
+        (r2 < Near64<1>::r2 ? near : far)[0] += w3;
+        (r2 < Near64<2>::r2 ? near : far)[1] += w3 * w;
+      }
+  }
+  for (int m = 0; m < 2; ++m) far_share[m] = far[m] > 0.0 ? std::sqrt(far[m] / near[m]) : 0.0;
+}
+
 // ---------------------------------------------------------------------------
 // Double-float near field over a batch's right-hand sides together (the
 // residual counterpart of k_p2p32_m1_multi): the pair tensor G1 I + G2 r r^T
@@ -3047,9 +3072,11 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
     if (near_mode == NEAR_DD && m == 1) {
       launch_p2p_dd(g, damp, src, damping, w, s);
       done = true;
-    } else if (m > 0 && g.grid <= NEAR64_GRID && (!damp || damping >= NEAR64_DAMPING)) {
+    } else if (m > 0 && g.grid <= NEAR64_GRID && g.far_share[m - 1] <= NEAR64_SHARE &&
+               (!damp || damping >= NEAR64_DAMPING)) {
       // (k_p2p keeps systems of more than 2^18 bohr, whose coordinate grid is too
-      // coarse for the distance classes, and factors below NEAR64_DAMPING)
+      // coarse for the distance classes, sparse systems, in whose fields the far pairs'
+      // rounding would show, and factors below NEAR64_DAMPING)
       launch_p2p64(g, m, damp, src, damping, w.Fnear.p, s, seg_done);
       nskip.hi = g.hi32.p, nskip.damping = (float)damping;
       done = true;

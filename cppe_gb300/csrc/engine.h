@@ -107,6 +107,9 @@ struct Geometry {
   DBuf<float2> near_exp;
   DBuf<double> near_exp64;
   double grid = 0.0;    // spacing of hi32's grid (bohr)
+  // sums of R^-6 (dipoles) and R^-8 (quadrupoles) over the near-field pairs beyond
+  // the FP64 operator's double-float limits, relative to those within them
+  double far_share[2] = {0.0, 0.0};
   DBuf<float2> dd_exp;  // e^-(k/16), k = 0..320, as double-float pairs
   // pairs the reference skips (exclusions) that the near-field pass computed
   DBuf<int> corr_ptr, corr_idx;
@@ -157,6 +160,7 @@ struct Geometry {
   DBuf<int> m2l_vid;
   DBuf<double4_32a> vec;
   void make_vectors();
+  void make_far_share();
 
   // Batches whose snapshots repeat once per right-hand side (ncopies):
   // the copy of each leaf's segment, the sites and leaves between copies,

@@ -1,0 +1,109 @@
+"""FP64 static fields and applies over sparse, wide and mixed systems: where the far
+pairs are most of the field they have to be as accurate as near ones.
+
+The sums in extended precision are numpy longdoubles (64 or 113 bits of mantissa).
+Tolerance: a term takes about ten FP64 roundings, of 3e-16 together at random, and
+the fields here have few terms of their size: 1.5e-15 of the field's norm is four
+times that.  Double-float far pairs carry 2e-14.
+"""
+import numpy as np
+import pytest
+
+import cabi
+
+pytestmark = pytest.mark.gpu
+DAMPING = 2.1304
+L = np.longdouble
+
+
+def lattice(k, spacing, seed=7, jitter=0.1):
+    rng = np.random.default_rng(seed)
+    g = np.stack(np.meshgrid(*[np.arange(float(k))] * 3, indexing="ij"), -1).reshape(-1, 3)
+    return spacing * (g + rng.uniform(-jitter, jitter, g.shape)), rng
+
+
+def field(xyz, mom, order, alpha, damp):
+    """The static field of dipoles or quadrupoles at every site."""
+    n, X = len(xyz), xyz.astype(L)
+    out = np.zeros((n, 3), L)
+    s = alpha.astype(L) ** (L(-1) / 6)
+    for i in range(n):
+        ok = np.arange(n) != i
+        d, m = (X[i] - X)[ok], mom[ok].astype(L)
+        r = np.sqrt((d * d).sum(1))
+        fE = fT = fD = L(1)
+        if damp:
+            v = L(DAMPING) * s[i] * s[ok] * r
+            e = np.exp(-v)
+            fE = 1 - (1 + v + v * v / 2) * e
+            fT = fE - v ** 3 / 6 * e
+            fD = fT - v ** 4 / 30 * e
+        if order == 1:
+            f = d * ((d * m).sum(1) * 3 * fT / r ** 5)[:, None] - m * (fE / r ** 3)[:, None]
+        else:
+            T = m[:, [0, 1, 2, 1, 3, 4, 2, 4, 5]].reshape(-1, 3, 3)
+            Td = (T * d[:, None, :]).sum(2)
+            f = d * (7.5 * fD / r ** 7 * (d * Td).sum(1) -
+                     1.5 * fT / r ** 5 * (m[:, 0] + m[:, 3] + m[:, 5]))[:, None] - \
+                Td * (3 * fT / r ** 5)[:, None]
+        out[i] = f.sum(0)
+    return out
+
+
+def static(xyz, mom, order, alpha, damp, ptr=None, idx=None):
+    n = len(xyz)
+    zero3, zero6 = np.zeros((n, 3)), np.zeros((n, 6))
+    ptr = np.zeros(n + 1, np.int32) if ptr is None else ptr
+    idx = np.zeros(1, np.int32) if idx is None else idx
+    return cabi.multipole_fields(xyz, np.zeros(n), mom if order == 1 else zero3,
+                                 mom if order == 2 else zero6, order, np.ones(n, np.int32), alpha,
+                                 ptr, idx, damp=damp).reshape(n, 3)
+
+
+def norm(a):
+    return float(np.sqrt((a * a).sum()))
+
+
+@pytest.mark.parametrize("damp", [False, True])
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("spacing", [3.0, 12.0, 40.0, 1.0e3, 3.0e4])
+def test_sparse_fields(gpu, spacing, order, damp):
+    xyz, rng = lattice(6, spacing)
+    mom = rng.normal(size=(len(xyz), 3 * order))
+    alpha = rng.uniform(1, 12, len(xyz))
+    ref = field(xyz, mom, order, alpha, damp)
+    got = static(xyz, mom, order, alpha, damp)
+    # (a dipole's field is returned with the sign of the others)
+    assert min(norm(got - ref), norm(got + ref)) < 1.5e-15 * norm(ref)
+
+
+@pytest.mark.parametrize("damp", [False, True])
+def test_dense_lattice_with_far_exclusions(gpu, port, damp):
+    """Near and far pairs and exclusions of both kinds beside each other (a dense
+    lattice, 33 bohr across), against the oracle with the tolerances of
+    test_gpu_near64.py."""
+    from oracle import oracle as O
+    xyz, rng = lattice(11, 3.0)
+    n = len(xyz)
+    alpha = rng.uniform(0.5, 1.5, n)
+    a6 = np.zeros((n, 6))
+    a6[:, [0, 3, 5]] = alpha[:, None]
+    excl = [sorted(rng.choice(n, rng.integers(0, 9), replace=False)) for _ in range(n)]
+    ptr = np.concatenate([[0], np.cumsum([len(e) for e in excl])]).astype(np.int32)
+    idx = np.array([j for e in excl for j in e], np.int32)
+    f = DAMPING if damp else 0.0
+    v = rng.normal(size=3 * n)
+    s = cabi.System(xyz, a6, ptr, idx, damp=damp)
+    ref = port.bmatrix_apply(xyz, a6, ptr, idx, v, fmm=0, damping=f)
+    assert np.linalg.norm(s.apply(v) - ref) < 4e-15 * np.linalg.norm(ref)
+    s.close()
+    for order in (1, 2):
+        mom = rng.normal(size=(n, 3 * order))
+        zero = np.zeros((n, 6))
+        sites = O.Sites(xyz=xyz, elements=["O"] * n, q=np.zeros(n),
+                        mu=mom if order == 1 else zero[:, :3], quad=mom if order == 2 else zero,
+                        max_order=order, alpha6=a6, polarizable=np.ones(n, np.int32), excl_ptr=ptr,
+                        excl_idx=idx)
+        want = port.multipole_fields(sites, fmm=False, order=5, damping=f)
+        got = static(xyz, mom, order, alpha, damp, ptr, idx).ravel()
+        assert np.linalg.norm(got - want) < 4e-14 * np.linalg.norm(want)
