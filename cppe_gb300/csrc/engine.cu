@@ -3072,10 +3072,10 @@ void eval_field(const Geometry& g, const DeviceOps* ops, FieldWork<T>& w, int m,
     if (near_mode == NEAR_DD && m == 1) {
       launch_p2p_dd(g, damp, src, damping, w, s);
       done = true;
-    } else if (m > 0 && g.grid <= NEAR64_GRID && g.far_share[m - 1] <= NEAR64_SHARE &&
+    } else if (m > 0 && g.grid <= near64_grid(m) && g.far_share[m - 1] <= NEAR64_SHARE &&
                (!damp || damping >= NEAR64_DAMPING)) {
-      // (k_p2p keeps systems of more than 2^18 bohr, whose coordinate grid is too
-      // coarse for the distance classes, sparse systems, in whose fields the far pairs'
+      // (k_p2p keeps systems of more than 2^19 bohr, whose coordinate grid is too
+      // coarse for the distance classes, for quadrupoles 2^13 bohr, sparse systems, in whose fields the far pairs'
       // rounding would show, and factors below NEAR64_DAMPING)
       launch_p2p64(g, m, damp, src, damping, w.Fnear.p, s, seg_done);
       nskip.hi = g.hi32.p, nskip.damping = (float)damping;

@@ -107,3 +107,24 @@ def test_dense_lattice_with_far_exclusions(gpu, port, damp):
         want = port.multipole_fields(sites, fmm=False, order=5, damping=f)
         got = static(xyz, mom, order, alpha, damp, ptr, idx).ravel()
         assert np.linalg.norm(got - want) < 4e-14 * np.linalg.norm(want)
+
+
+def cluster_and_outlier(distance):
+    """A dense cluster (every sum over its sites is one of near pairs) and a site far
+    from it, whose field is one of far pairs only."""
+    xyz, rng = lattice(6, 3.0)
+    return np.concatenate([xyz, [[distance, 0.3 * distance, 0.2 * distance]]]), rng
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("distance", [1.0e3, 7.0e3, 1.0e4, 3.0e4, 1.0e5, 1.0e6])
+def test_far_site(gpu, distance, order):
+    """The far pairs' accuracy does not fall with the distance: 2e-14 a pair and the
+    terms' cancellation, 2e-13 of the outlier's own field."""
+    xyz, rng = cluster_and_outlier(distance)
+    mom = rng.normal(size=(len(xyz), 3 * order))
+    mom[-1] = 0
+    alpha = rng.uniform(1, 12, len(xyz))
+    ref = field(xyz, mom, order, alpha, False)[-1]
+    got = static(xyz, mom, order, alpha, False)[-1]
+    assert min(norm(got - ref), norm(got + ref)) < 2e-13 * norm(ref)
