@@ -109,6 +109,43 @@ def test_dense_lattice_with_far_exclusions(gpu, port, damp):
         assert np.linalg.norm(got - want) < 4e-14 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("damp", [False, True])
+def test_wide_system(gpu, port, damp):
+    """Half extent 3.5e5 bohr: the coordinate grid (1/8 bohr) is too coarse for the
+    distance classes and the all-FP64 kernel serves dipoles and quadrupoles, with every
+    exclusion subtracted afterwards.  Eight dense clusters with exclusions inside and
+    between them, against the oracle with the tolerances of test_gpu_near64.py."""
+    from oracle import oracle as O
+    one, rng = lattice(6, 3.0)
+    corners = 7.0e5 * np.stack(np.meshgrid(*[[0.0, 1.0]] * 3, indexing="ij"), -1).reshape(-1, 3)
+    xyz = np.concatenate([one + c for c in corners])
+    n = len(xyz)
+    alpha = rng.uniform(0.5, 1.5, n)
+    a6 = np.zeros((n, 6))
+    a6[:, [0, 3, 5]] = alpha[:, None]
+    excl = [sorted({int(j) for j in rng.choice(n, rng.integers(0, 5))} |
+                   {int(j) for j in 216 * (i // 216) + rng.choice(216, rng.integers(0, 5))})
+            for i in range(n)]
+    ptr = np.concatenate([[0], np.cumsum([len(e) for e in excl])]).astype(np.int32)
+    idx = np.array([j for e in excl for j in e], np.int32)
+    f = DAMPING if damp else 0.0
+    v = rng.normal(size=3 * n)
+    s = cabi.System(xyz, a6, ptr, idx, damp=damp)
+    ref = port.bmatrix_apply(xyz, a6, ptr, idx, v, fmm=0, damping=f)
+    assert np.linalg.norm(s.apply(v) - ref) < 4e-15 * np.linalg.norm(ref)
+    s.close()
+    for order in (1, 2):
+        mom = rng.normal(size=(n, 3 * order))
+        zero = np.zeros((n, 6))
+        sites = O.Sites(xyz=xyz, elements=["O"] * n, q=np.zeros(n),
+                        mu=mom if order == 1 else zero[:, :3], quad=mom if order == 2 else zero,
+                        max_order=order, alpha6=a6, polarizable=np.ones(n, np.int32), excl_ptr=ptr,
+                        excl_idx=idx)
+        want = port.multipole_fields(sites, fmm=False, order=5, damping=f)
+        got = static(xyz, mom, order, alpha, damp, ptr, idx).ravel()
+        assert np.linalg.norm(got - want) < 4e-14 * np.linalg.norm(want)
+
+
 def cluster_and_outlier(distance):
     """A dense cluster (every sum over its sites is one of near pairs) and a site far
     from it, whose field is one of far pairs only."""
