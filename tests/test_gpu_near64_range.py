@@ -165,3 +165,28 @@ def test_far_site(gpu, distance, order):
     ref = field(xyz, mom, order, alpha, False)[-1]
     got = static(xyz, mom, order, alpha, False)[-1]
     assert min(norm(got - ref), norm(got + ref)) < 2e-13 * norm(ref)
+
+
+@pytest.mark.parametrize("damp", [False, True])
+@pytest.mark.parametrize("order", [1, 2])
+def test_no_source_no_field(gpu, order, damp):
+    """One site; a molecule whose pairs are all excluded: exactly zero."""
+    from cppe_gb300 import synthetic
+    rng = np.random.default_rng(3)
+    assert not static(np.zeros((1, 3)), rng.normal(size=(1, 3 * order)), order, np.ones(1),
+                      damp).any()
+    b = synthetic.water_box(1, seed=1)
+    assert not static(b.xyz, rng.normal(size=(3, 3 * order)), order, b.alpha_iso, damp, b.excl_ptr,
+                      b.excl_idx).any()
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_a_moment_that_is_not_a_number(gpu, order):
+    """reaches the field of every other molecule, near and far."""
+    from cppe_gb300 import synthetic
+    b = synthetic.water_box(700, seed=2)
+    mom = np.random.default_rng(3).normal(size=(b.n, 3 * order))
+    mom[999] = np.nan
+    got = static(b.xyz, mom, order, b.alpha_iso, False, b.excl_ptr, b.excl_idx)
+    others = np.arange(b.n) // 3 != 333
+    assert np.isnan(got[others]).all()
