@@ -245,10 +245,12 @@ __device__ __forceinline__ float d2f_rest(double x) {
          __uint_as_float((ex - (1023 - 127) - 52) << 23);
 }
 // 1/sqrt(r2) to FP32 accuracy as a double (0 for r2 = 0), the seed of FP64
-// corrections; below 2^-100, where FP32 would underflow, the FP64 function.
+// corrections; outside 2^-100 .. 2^100, where FP32 would not hold r2 (or not its
+// inverse's powers), the FP64 function.
 __device__ __forceinline__ double rsqrt_seed(double r2) {
   const int hi = __double2hiint(r2);
-  if (hi >= ((1023 - 100) << 20)) return f2d_bits(rsqrt_ftz(d2f_bits(r2)));
+  if ((unsigned)(hi - ((1023 - 100) << 20)) < (200u << 20))
+    return f2d_bits(rsqrt_ftz(d2f_bits(r2)));
   return (hi | __double2loint(r2)) == 0 ? 0.0 : rsqrt(r2);
 }
 

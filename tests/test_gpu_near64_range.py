@@ -190,3 +190,14 @@ def test_a_moment_that_is_not_a_number(gpu, order):
     got = static(b.xyz, mom, order, b.alpha_iso, False, b.excl_ptr, b.excl_idx)
     others = np.arange(b.n) // 3 != 333
     assert np.isnan(got[others]).all()
+
+
+@pytest.mark.parametrize("distance", [1e-60, 1e-20, 1e-3, 1e10, 3e19, 1e25, 1e100])
+def test_two_charges(gpu, distance):
+    """q / R^2 over the range in which R^2 and R^-2 are FP64 numbers."""
+    xyz = np.array([[0.0, 0, 0], [distance, 0, 0]])
+    got = cabi.multipole_fields(xyz, np.array([2.0, 3.0]), np.zeros((2, 3)), np.zeros((2, 6)), 0,
+                                np.ones(2, np.int32), np.ones(2), np.zeros(3, np.int32),
+                                np.zeros(1, np.int32)).reshape(2, 3)
+    want = np.array([[-3.0, 0, 0], [2.0, 0, 0]]) / distance ** 2
+    np.testing.assert_allclose(got, want, rtol=1e-15, atol=0)
