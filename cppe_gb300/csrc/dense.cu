@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "system.h"
@@ -310,22 +311,47 @@ __global__ void __launch_bounds__(SMALL_THREADS)
 
 static size_t small_smem(int n) { return sizeof(double) * (3 * (size_t)n) * (3 * (size_t)n + 2); }
 
+// Bytes of all systems' matrices in this process.
+static std::atomic<size_t> s_dense_bytes{0};
+
 bool System::dense_operator() const {
-  return !geo.fmm && opt.precision == CPPE_GPU_FP64 && n <= DENSE_MAX;
+  return !geo.fmm && opt.precision == CPPE_GPU_FP64 && n <= DENSE_MAX && dense != DENSE_NONE;
 }
 
-void System::dense_build() {
-  if (Tmat.p) return;
-  const size_t N3 = 3 * (size_t)n;
-  Tmat.alloc(N3 * N3);
+// Builds the matrix on first use; false (for good) where the matrices of other
+// systems leave no room for it or the device has none: the pair kernels then serve
+// this system, as they serve larger ones.
+bool System::dense_build() {
+  if (dense != DENSE_UNTRIED) return dense == DENSE_BUILT;
+  const size_t N3 = 3 * (size_t)n, bytes = N3 * N3 * sizeof(double);
+  dense = DENSE_NONE;
+  if (s_dense_bytes.fetch_add(bytes) + bytes > DENSE_POOL) {
+    s_dense_bytes -= bytes;
+    return false;
+  }
+  dense_bytes = bytes;
+  try {
+    Tmat.alloc(N3 * N3);
+  } catch (const Failure&) {
+    cudaGetLastError();  // (out of memory is not sticky)
+    dense_release();
+    return false;
+  }
   const long pairs = (long)n * (n + 1) / 2;
   k_dense_build<<<(unsigned)((pairs + 127) / 128), 128, 0, stream>>>(
         n, geo.pos64.p, geo.corr_ptr.p, geo.corr_idx.p, opt.damp != 0, opt.damping_factor, Tmat.p);
   CG_LAUNCH();
+  dense = DENSE_BUILT;
+  return true;
+}
+
+void System::dense_release() {
+  Tmat.release();
+  s_dense_bytes -= dense_bytes;
+  dense_bytes = 0;
 }
 
 void System::dense_apply(const double* in, double* out, bool iteration) {
-  dense_build();
   k_dense_apply<<<n, DENSE_BLOCK, 0, stream>>>(n, Tmat.p, ainv64.p, in, out,
                                                iteration ? partials.p : nullptr,
                                                iteration ? flags.p : nullptr);
@@ -341,14 +367,14 @@ void System::dense_iteration() {
   CG_LAUNCH();
 }
 
-bool System::small_solver() const {
+bool System::small_solver() {
   // (its stopping rule compares squares)
-  return dense_operator() && n <= SMALL_MAX && !model && opt.induced_thresh > 1e-140;
+  return dense_operator() && n <= SMALL_MAX && !model && opt.induced_thresh > 1e-140 &&
+         dense_build();
 }
 
 int System::solve_small(const double* rhs, const double* guess, int make_guess, double* mu,
                         int* iters, double* hist_out, int hist_cap) {
-  dense_build();
   if (!h_hist) CG_CUDA(cudaMallocHost(&h_hist, sizeof(double) * (std::max(1, opt.maxiter) + 64)));
   if (!small_ready) {
     CG_CUDA(cudaFuncSetAttribute(k_solve_small<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -207,6 +207,7 @@ System::~System() {
   if (h_scal) cudaFreeHost(h_scal);
   if (h_hist) cudaFreeHost(h_hist);
   if (h_io) cudaFreeHost(h_io);
+  dense_release();
 }
 
 static void inv_sym3(const double* s, double* o6) {
@@ -545,7 +546,7 @@ ReduceSlots System::slots(int k) const { return ReduceSlots{partials.p, ticket.p
 
 void System::apply64(const double* in, double* out, bool with_dot, int near_mode) {
   ReduceSlots rs = slots(S_PAP);
-  if (near_mode == NEAR_FP64 && !with_dot && dense_operator()) {
+  if (near_mode == NEAR_FP64 && !with_dot && dense_operator() && dense_build()) {
     dense_apply(in, out, false);
     return;
   }
@@ -599,7 +600,7 @@ struct Poller {
 }  // namespace
 
 int System::solve_fp64(bool zero_guess, double* hist_out, int hist_cap, int* iters) {
-  const bool dense = dense_operator() && !use_model;
+  const bool dense_op = dense_operator() && !use_model && dense_build();
   const int nb   = (n + VB - 1) / VB;
   const int n3   = 3 * n;
   const double t = opt.induced_thresh;
@@ -617,7 +618,7 @@ int System::solve_fp64(bool zero_guess, double* hist_out, int hist_cap, int* ite
   Poller poll(stream, flags.p, h_flags);
   for (int k = 0; k < opt.maxiter; ++k) {
     last.fp64_applies++;
-    if (dense) {
+    if (dense_op) {
       dense_iteration();
     } else {
       apply64(p.p, Ap.p, true);

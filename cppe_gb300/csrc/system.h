@@ -39,6 +39,9 @@ struct SolveStats {
 // matrix in shared memory (dense.cu).
 constexpr int DENSE_MAX = 1024;
 constexpr int SMALL_MAX = 53;  // 8 (3n)(3n + 2) <= 227 KB
+// Matrices of all live systems together (227 systems of DENSE_MAX sites): a program
+// that holds more systems than that keeps its memory, and the pair kernels.
+constexpr size_t DENSE_POOL = size_t(16) << 30;
 
 struct System {
   int n = 0;
@@ -77,12 +80,15 @@ struct System {
   double* h_hist = nullptr;   // pinned: the norms of a one-block solve
   double* h_io   = nullptr;   // pinned: its right-hand side, guess and solution
   DBuf<double> Tmat;          // the operator without alpha^-1 as a dense matrix (built on first use)
+  enum { DENSE_UNTRIED, DENSE_BUILT, DENSE_NONE } dense = DENSE_UNTRIED;
+  size_t dense_bytes = 0;     // Tmat's share of DENSE_POOL
   bool small_ready = false;
   bool dense_operator() const;
-  void dense_build();
+  bool dense_build();
+  void dense_release();
   void dense_apply(const double* in, double* out, bool iteration);
   void dense_iteration();
-  bool small_solver() const;
+  bool small_solver();
   // (pointers the device can address; solve_device's arguments otherwise)
   int solve_small(const double* rhs, const double* guess, int make_guess, double* mu, int* iters,
                   double* hist_out, int hist_cap);
