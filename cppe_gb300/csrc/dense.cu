@@ -368,9 +368,10 @@ void System::dense_iteration() {
 }
 
 bool System::small_solver() {
-  // (its stopping rule compares squares)
-  return dense_operator() && n <= SMALL_MAX && !model && opt.induced_thresh > 1e-140 &&
-         dense_build();
+  // (its stopping rule compares squares; with a limit of more iterations than it
+  // could take in some milliseconds, the loop of launches, which the host can leave)
+  return dense_operator() && n <= SMALL_MAX && opt.maxiter <= SMALL_MAXITER && !model &&
+         opt.induced_thresh > 1e-140 && dense_build();
 }
 
 int System::solve_small(const double* rhs, const double* guess, int make_guess, double* mu,

@@ -39,6 +39,7 @@ struct SolveStats {
 // matrix in shared memory (dense.cu).
 constexpr int DENSE_MAX = 1024;
 constexpr int SMALL_MAX = 53;  // 8 (3n)(3n + 2) <= 227 KB
+constexpr int SMALL_MAXITER = 1024;
 // Matrices of all live systems together (227 systems of DENSE_MAX sites): a program
 // that holds more systems than that keeps its memory, and the pair kernels.
 constexpr size_t DENSE_POOL = size_t(16) << 30;
