@@ -167,31 +167,16 @@ __device__ __forceinline__ dd2 dd2_sqr(dd2 a) {
   e              = pfma(padd(a.h, a.h), a.l, e);
   return {p, e};
 }
-__device__ __forceinline__ dd2 dd2_sqr_full(dd2 a) {
-  const float2 p = pmul(a.h, a.h);
-  float2 e       = pfma(a.h, a.h, pneg(p));
-  e              = pfma(padd(a.h, a.h), a.l, e);
-  e              = pfma(a.l, a.l, e);
-  return {p, e};
-}
 __device__ __forceinline__ dd2 dd2_mul_f(dd2 a, float2 b) {
   const float2 p = pmul(a.h, b);
   return {p, pfma(a.l, b, pfma(a.h, b, pneg(p)))};
 }
-// 1/sqrt(a) for a > 0 (as dd_rsqrt); the estimate is one MUFU operation per
-// half (`rsqrt.approx.ftz`: the inputs are squared distances, never subnormal)
+// 1/sqrt(x) to FP32 accuracy, one MUFU operation (`rsqrt.approx.ftz`: the inputs are
+// squared distances, never subnormal)
 __device__ __forceinline__ float rsqrt_ftz(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-__device__ __forceinline__ dd2 dd2_rsqrt(dd2 a) {
-  const float2 y  = make_float2(rsqrt_ftz(a.h.x), rsqrt_ftz(a.h.y));
-  const float2 q  = pmul(y, y);
-  const float2 qe = pfma(y, y, pneg(q));
-  float2 h        = pfma(a.h, q, p2(-1.f));
-  h               = pfma(a.h, qe, pfma(a.l, q, h));
-  return {y, pmul(pmul(y, h), pfma(p2(0.375f), h, p2(-0.5f)))};
 }
 // e^-v as dd_exp_neg, each half with its own table entry; v.h < 20 (callers
 // clamp the halves they do not use)
