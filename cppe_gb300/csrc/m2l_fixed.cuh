@@ -111,17 +111,30 @@ constexpr int m2l_dd_off(int m, int o) {
 template <typename O>
 struct FoldRow {  // plain rows: stride and reduced coefficient of a position
   static constexpr int stride(int, int, int ms) { return m_stride(ms); }
-  __device__ static int coef(int, int, int ms, int r) { return r < ms ? r : -1; }
+  __host__ __device__ static constexpr int coef(int, int, int ms, int r) { return r < ms ? r : -1; }
 };
 template <>
 struct FoldRow<float2> {
   static constexpr int stride(int m, int p, int) { return m2l_dd_off(m, p + 1); }
-  __device__ static int coef(int m, int, int, int r) {
+  __host__ __device__ static constexpr int coef(int m, int, int, int r) {
     int o = m, k = 0;
     while (r >= 2 * o + 2) r -= 2 * o + 2, k += 2 * o + 1, ++o;
     return r < 2 * o + 1 ? k + r : -1;
   }
 };
+// What the translation relies on: coefficient k of order o at m2l_dd_off(m, o) + k,
+// an even position each, and nothing else in the row.
+constexpr bool m2l_dd_rows_hold(int m, int p) {
+  int used = 0;
+  for (int o = m; o <= p; ++o) {
+    const int n = nred(o) - nred(o - 1), at = m2l_dd_off(m, o);
+    if (at & 1) return false;
+    for (int k = 0; k < n; ++k, ++used)
+      if (FoldRow<float2>::coef(m, p, 0, at + k) != nred(o - 1) - nred(m - 1) + k) return false;
+  }
+  for (int r = 0; r < m2l_dd_off(m, p + 1); ++r) used -= FoldRow<float2>::coef(m, p, 0, r) >= 0;
+  return used == 0;
+}
 // Folded rows of the cells, FOLD_LANES threads a cell.  A cell with upward tasks
 // is the sum of its task partials in order: added up here, not in a launch of its
 // own (one of seven in the far-field chain, which is the longer path of small
@@ -266,6 +279,14 @@ constexpr int m2l_wbase(int m, int p, int ko) {
   for (int o = m; o < ko; ++o) b += (nred(o) - nred(o - 1)) * nred(p - o);
   return b;
 }
+#define CPPE_CHECK_ROWS(MM, PP, NAME, NT, LS, MS, FW, UW, FLS)                               \
+  static_assert((NT) % 2 == 0, "FP64 tensors are read in 16-byte loads");                   \
+  static_assert(m2l_dd_rows_hold(MM, PP), "double-float rows");                             \
+  static_assert(m2l_wbase(MM, PP, (PP) + 1) == sizeof(m2l_w_##NAME), "one entry per term"); \
+  static_assert((LS) == nred((PP) - (MM)) && (MS) == nred(PP) - nred((MM) - 1), "reduced rows");
+CPPE_M2L_REDUCED(CPPE_CHECK_ROWS)
+#undef CPPE_CHECK_ROWS
+
 // The multipole coefficients of order KO of a lane's source, all loads in
 // flight at once.
 template <int M, int KO>
