@@ -205,11 +205,6 @@ __device__ __forceinline__ double f2d_bits(float x) {
   return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)),
                           (int)(u << 29));
 }
-// the same for sums that may be zero, subnormal, infinite or NaN
-__device__ __forceinline__ double f2d_any(float x) {
-  const unsigned e = (__float_as_uint(x) >> 23) & 0xffu;
-  return e - 1u < 254u ? f2d_bits(x) : (double)x;
-}
 // double -> float, truncated, by moving the bits: positive values in FP32's
 // range (d2f_bits), or any sign with small values taken as zero (d2f_bits0)
 __device__ __forceinline__ float d2f_bits(double x) {

@@ -1982,26 +1982,32 @@ __global__ void __launch_bounds__(P2P_BLOCK)
 #include "near64.cuh"
 namespace cg {
 
-// far_share from some 16,000 pairs of evenly spaced sites (40 us).
+// far_share from some 5,000 pairs of evenly spaced sites: each with its own leaf,
+// where the bonded partners are, and every so many of the others in its list.
 void Geometry::make_far_share() {
   const TreeLayout& L = layout;
-  const long per = std::max(1L, near_pairs / std::max(1, n));
-  const int take = (int)std::min<long>(n, std::min(64L, std::max(4L, 16384 / per)));
+  constexpr int SITES = 8, PAIRS = 512;
+  const int take   = std::min(n, SITES);
+  const int stride = (int)std::max(1L, near_pairs / std::max(1, n) / PAIRS);
   double near[2] = {0.0, 0.0}, far[2] = {0.0, 0.0};
   for (int t = 0; t < take; ++t) {
     const int i          = (int)((2L * t + 1) * n / (2L * take));
     const double4_32a pi = h_pos64[i];
     const int a          = h_site_leaf[i];
-    for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q)
-      for (int k = L.leaf_start[L.p2p_src[q]]; k < L.leaf_start[L.p2p_src[q] + 1]; ++k) {
+    auto add = [&](int b, double weight) {
+      for (int k = L.leaf_start[b]; k < L.leaf_start[b + 1]; ++k) {
         const double4_32a pk = h_pos64[k];
         const double x = pi.x - pk.x, y = pi.y - pk.y, z = pi.z - pk.z;
-        const double r2 = x * x + y * y + z * z;
-        if (!(r2 > 0.0)) continue;
-        const double w = 1.0 / r2, w3 = w * w * w;
-        (r2 < Near64<1>::r2 ? near : far)[0] += w3;
-        (r2 < Near64<2>::r2 ? near : far)[1] += w3 * w;
+        const double r2 = x * x + y * y + z * z, w = r2 > 0.0 ? 1.0 / r2 : 0.0;
+        const double w3 = weight * w * w * w, w4 = w3 * w;
+        const bool n1 = r2 < Near64<1>::r2, n2 = r2 < Near64<2>::r2;
+        near[0] += n1 ? w3 : 0.0, far[0] += n1 ? 0.0 : w3;
+        near[1] += n2 ? w4 : 0.0, far[1] += n2 ? 0.0 : w4;
       }
+    };
+    add(a, 1.0);
+    for (int q = L.p2p_ptr[a] + t % stride; q < L.p2p_ptr[a + 1]; q += stride)
+      if (L.p2p_src[q] != a) add(L.p2p_src[q], stride);
   }
   for (int m = 0; m < 2; ++m) far_share[m] = far[m] > 0.0 ? std::sqrt(far[m] / near[m]) : 0.0;
 }
