@@ -10,7 +10,6 @@
 #include <algorithm>
 #include <exception>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -33,6 +32,7 @@ void host_parallel(int threads, long n, F&& f) {
   }
   std::vector<std::thread> pool;
   std::vector<std::exception_ptr> err(threads);
+  pool.reserve(threads - 1);
   auto run = [&](int t) {
     try {
       f(t, n * t / threads, n * (t + 1) / threads);
@@ -43,7 +43,7 @@ void host_parallel(int threads, long n, F&& f) {
   int started = 1;
   try {
     for (; started < threads; ++started) pool.emplace_back(run, started);
-  } catch (const std::system_error&) {  // no more threads: the rest runs here
+  } catch (...) {  // no more threads (or memory for one): the rest runs here
   }
   run(0);
   for (int t = started; t < threads; ++t) run(t);
