@@ -177,6 +177,18 @@ def static_rhs_gpu(b, summation, order):
     return (b.external_field() + Fm).ravel()
 
 
+def fp64_pairs(b, alg_pairs, samples=256):
+    """Near-field pairs that the FP64 dipole operator evaluates in FP64 (within 24 bohr or
+    a Thole argument of 24; the others run in double-float), from evenly spaced sites."""
+    s = b.alpha_iso ** (-1.0 / 6.0)
+    near = 0
+    sites = np.linspace(0, b.n - 1, min(b.n, samples)).astype(int)
+    for i in sites:
+        r = np.sqrt(((b.xyz - b.xyz[i]) ** 2).sum(axis=1))
+        near += int(((r < 24.0) | (2.1304 * s[i] * s * r < 24.0)).sum()) - 1
+    return int(min(alg_pairs, b.n * near / len(sites)))
+
+
 def peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -700,7 +712,8 @@ def run_ours(args):
     fp32_peak = capi.fma_peak_tflops(False, dev)
     fp64_peak = capi.fma_peak_tflops(True, dev)
     achieved = alg_pairs * FLOP_PER_PAIR / (tim32["near"] * 1e-3) / 1e12
-    achieved64 = alg_pairs * FLOP_PER_PAIR / (tim64["near"] * 1e-3) / 1e12
+    pairs64 = fp64_pairs(b, alg_pairs)
+    achieved64 = pairs64 * FLOP_PER_PAIR / (tim64["near"] * 1e-3) / 1e12
     pairs_per_s = {"fp32": alg_pairs / (tim32["near"] * 1e-3),
                    "double_float": alg_pairs / (timdd["near"] * 1e-3),
                    "fp64": alg_pairs / (tim64["near"] * 1e-3)}
@@ -786,7 +799,9 @@ def run_ours(args):
                                   "figure in MEASURED_PEAKS.json",
                      "algorithmic": f"{alg_pairs} pairs x {FLOP_PER_PAIR} FLOP per launch"},
         "roofline_fp64": {"bound": "fp64", "achieved": achieved64, "peak": fp64_peak,
-                          "unit": "TFLOP/s", "frac": achieved64 / fp64_peak},
+                          "unit": "TFLOP/s", "frac": achieved64 / fp64_peak,
+                          "algorithmic": f"{pairs64} of {alg_pairs} pairs (those evaluated in "
+                                         f"FP64) x {FLOP_PER_PAIR} FLOP per launch"},
         "phases_ms": {"fp32": tim32, "double_float_residual": timdd, "fp64": tim64},
         "m2l_translations_per_apply": m2l_pairs,
         "near_pairs_per_s": pairs_per_s,

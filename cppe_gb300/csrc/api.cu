@@ -559,6 +559,8 @@ int cppe_gpu_multipole_fields(int n, const double* xyz, const double* q, const d
         if (polarizable && polarizable[i] && alpha_iso && alpha_iso[i] > 0.0)
           sd[i] = std::pow(alpha_iso[i], -1.0 / 6.0);
     Geometry g;
+    // (read by FP32 passes only; its seven uploads are 30 of 530 us at 18 sites)
+    g.sym_enabled = false;
     g.build(n, xyz, sd.data(), excl_ptr, excl_idx, fmm, ncrit, theta, s);
     const size_t n3 = 3 * (size_t)n;
     DBuf<double> out, tmp, srcp;

@@ -6,9 +6,11 @@
 // lane-operations per clock and SM) against 88 us of k_p2p64 and k_finish; 60
 // sites 6 us against 51.  The matrix is built once per system, each pair once
 // (66 us at 999 sites).  DENSE_MAX: up to there build and apply together cost
-// what one pair-kernel apply does, so that a first call is no slower, and the
-// matrix (75 MB) stays in L2; at 1,998 sites they take 243 + 80 us against 144,
-// at 2,997 536 + 162 us against 206.
+// what one pair-kernel apply does, so that a first call of one apply is no slower,
+// the matrix (75 MB) stays in L2 and one cluster takes the iteration's vector part;
+// at 1,998 sites they take 243 + 80 us against 144 (a solve of 14 applies would still
+// gain), at 2,997 536 + 162 us against 206.  The matrices of all systems share
+// DENSE_POOL bytes.
 #include <cooperative_groups.h>
 
 #include <algorithm>

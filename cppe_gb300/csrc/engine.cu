@@ -97,8 +97,13 @@ TreeView Geometry::view() const {
 void Geometry::build(int n_, const double* xyz, const double* s_damp, const int* excl_ptr,
                      const int* excl_idx, bool fmm_, int ncrit_, double theta_,
                      cudaStream_t s) {
-  // small direct systems in chunks of 32 (999 sites: 1,024 work items instead of
-  // 256, evenly over the SMs)
+  // Small direct systems in chunks of 32: four times the work items.  FP32 near field
+  // with chunks of 64 / 32: 510 sites 14.2 / 11.5 us, 999 14.2 / 12.0, 2,049 24.3 / 16.3,
+  // 4,095 63.3 / 36.7; a mixed solve of 999 sites 549 / 531 us, of 4,095 1,477 / 1,074.
+  // k_p2p64 gains below (510 sites 72 / 52 us) and loses above (1,500 84 / 98 us, 2,049
+  // and 4,095 269 / 276).  From 4,096 on FP32 gains up to 6,000 sites (122 / 69 us, 8,805
+  // 76.6 / 80.0), FP64 loses 2 to 24 % (4,200 277 / 317 us, 8,805 779 / 1,027): the line
+  // leaves these to the default precision.
   direct_chunk = n_ < 4096 ? 32 : 64;
   prepare(n_, xyz, s_damp, excl_ptr, excl_idx, fmm_, ncrit_, theta_);
   upload(s);
@@ -184,29 +189,29 @@ void Geometry::prepare(int n_, const double* xyz, const double* s_damp, const in
   auto& lo  = h_lo;
   const int threads = host_threads(n, 4096);
   host_parallel(threads, n, [&](int, long k0, long k1) {
-  for (long k = k0; k < k1; ++k) {
-    const int i  = L.perm[k];
-    const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
-    const double sd = s_damp ? s_damp[i] : 0.0;
-    p64[k]         = make_double4_32a(x, y, z, sd);
-    double r[3]    = {x - ctr[0], y - ctr[1], z - ctr[2]};
-    float h[3], l[3], m[3], e[3];
-    const double in[3] = {x, y, z};
-    for (int c = 0; c < 3; ++c) {
-      h[c] = (float)(std::nearbyint(r[c] / quantum) * quantum);
-      l[c] = (float)(r[c] - (double)h[c]);
-      // three parts: the rounding of x - ctr (a two-sum) goes to the last one
-      const double rem = r[c] - (double)h[c], b = r[c] - in[c];
-      const double rerr = (in[c] - (r[c] - b)) + (-ctr[c] - b);
-      m[c] = (float)(std::nearbyint(rem / fine) * fine);
-      e[c] = (float)((rem - (double)m[c]) + rerr);
+    for (long k = k0; k < k1; ++k) {
+      const int i  = L.perm[k];
+      const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+      const double sd = s_damp ? s_damp[i] : 0.0;
+      p64[k]         = make_double4_32a(x, y, z, sd);
+      double r[3]    = {x - ctr[0], y - ctr[1], z - ctr[2]};
+      float h[3], l[3], m[3], e[3];
+      const double in[3] = {x, y, z};
+      for (int c = 0; c < 3; ++c) {
+        h[c] = (float)(std::nearbyint(r[c] / quantum) * quantum);
+        l[c] = (float)(r[c] - (double)h[c]);
+        // three parts: the rounding of x - ctr (a two-sum) goes to the last one
+        const double rem = r[c] - (double)h[c], b = r[c] - in[c];
+        const double rerr = (in[c] - (r[c] - b)) + (-ctr[c] - b);
+        m[c] = (float)(std::nearbyint(rem / fine) * fine);
+        e[c] = (float)((rem - (double)m[c]) + rerr);
+      }
+      const float sh = (float)sd;
+      hi[k]          = make_float4(h[0], h[1], h[2], sh);
+      lo[k]          = make_float4(l[0], l[1], l[2], (float)(sd - (double)sh));
+      h_mid[k]       = make_float4(m[0], m[1], m[2], 0.f);
+      h_low[k]       = make_float4(e[0], e[1], e[2], (float)(sd - (double)sh));
     }
-    const float sh = (float)sd;
-    hi[k]          = make_float4(h[0], h[1], h[2], sh);
-    lo[k]          = make_float4(l[0], l[1], l[2], (float)(sd - (double)sh));
-    h_mid[k]       = make_float4(m[0], m[1], m[2], 0.f);
-    h_low[k]       = make_float4(e[0], e[1], e[2], (float)(sd - (double)sh));
-  }
   });
 
   // Exclusion corrections: pairs the reference skips but the near-field pass
@@ -442,26 +447,26 @@ void Geometry::make_schedules() {
       }
       host_parallel(host_threads((long)L.p2p_src.size(), 1 << 13), L.nleaves,
                     [&](int, long l0, long l1) {
-      std::vector<int> nearer, farther;
-      for (long a = l0; a < l1; ++a) {
-        const double* ba = &box[6 * (size_t)a];
-        nearer.clear(), farther.clear();
-        for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q) {
-          const int b      = L.p2p_src[q];
-          const double* bb = &box[6 * (size_t)b];
-          double r2 = 0.0;
-          for (int c = 0; c < 3; ++c) {
-            const double d = std::max(0.0, std::max(ba[c] - bb[c + 3], bb[c] - ba[c + 3]));
-            r2 += d * d;
+        std::vector<int> nearer, farther;
+        for (long a = l0; a < l1; ++a) {
+          const double* ba = &box[6 * (size_t)a];
+          nearer.clear(), farther.clear();
+          for (int q = L.p2p_ptr[a]; q < L.p2p_ptr[a + 1]; ++q) {
+            const int b      = L.p2p_src[q];
+            const double* bb = &box[6 * (size_t)b];
+            double r2 = 0.0;
+            for (int c = 0; c < 3; ++c) {
+              const double d = std::max(0.0, std::max(ba[c] - bb[c + 3], bb[c] - ba[c + 3]));
+              r2 += d * d;
+            }
+            const double v = 0.999 * damping * smin[a] * smin[b] * std::sqrt(r2);
+            (v >= P2P_UNDAMPED_V ? farther : nearer).push_back(b);
           }
-          const double v = 0.999 * damping * smin[a] * smin[b] * std::sqrt(r2);
-          (v >= P2P_UNDAMPED_V ? farther : nearer).push_back(b);
+          int q = L.p2p_ptr[a];
+          for (int b : nearer) layout.p2p_src[q++] = b;
+          h_leaf_split[a] = q;
+          for (int b : farther) layout.p2p_src[q++] = b;
         }
-        int q = L.p2p_ptr[a];
-        for (int b : nearer) layout.p2p_src[q++] = b;
-        h_leaf_split[a] = q;
-        for (int b : farther) layout.p2p_src[q++] = b;
-      }
       });
     }
   }
@@ -658,30 +663,29 @@ static void exp_neg_pair(double v, double& hi, double& lo) {
   hi = sh, lo = sl;
 }
 
-// Tables of e^-v at steps of 1/16, formed once per process.
-namespace {
-struct ExpTables {
-  std::vector<float2> dd, near;
-  std::vector<double> near64;  // value and rest
-  ExpTables() : dd(DD_EXP_TAB), near(NEAR64_DDTAB), near64(2 * NEAR64_ETAB) {
-    for (auto* t : {&dd, &near})
-      for (size_t k = 0; k < t->size(); ++k) {
-        const double e = std::exp(-0.0625 * k);
-        (*t)[k]        = make_float2((float)e, (float)(e - (double)(float)e));
-      }
-    for (int k = 0; k < NEAR64_ETAB; ++k) exp_neg_pair(0.0625 * k, near64[2 * k], near64[2 * k + 1]);
-  }
-};
-const ExpTables& exp_tables() {
-  static const ExpTables t;
-  return t;
+// Tables of e^-v at steps of 1/16, formed once per process: NEAR64_ETAB values and
+// rests in FP64, then NEAR64_DDTAB double-float pairs (the double-float near field
+// reads the first DD_EXP_TAB), in one buffer.
+static_assert(NEAR64_DDTAB >= DD_EXP_TAB, "one table of pairs");
+static const std::vector<double>& exp_tables() {
+  static const std::vector<double> tab = [] {
+    std::vector<double> t(2 * NEAR64_ETAB + NEAR64_DDTAB);
+    for (int k = 0; k < NEAR64_ETAB; ++k) exp_neg_pair(0.0625 * k, t[2 * k], t[2 * k + 1]);
+    for (int k = 0; k < NEAR64_DDTAB; ++k) {
+      const double e = std::exp(-0.0625 * k);
+      const float2 v = make_float2((float)e, (float)(e - (double)(float)e));
+      std::memcpy(&t[2 * NEAR64_ETAB + k], &v, sizeof v);
+    }
+    return t;
+  }();
+  return tab;
 }
-}  // namespace
+const float2* Geometry::exp_dd() const {
+  return reinterpret_cast<const float2*>(exp_tab.p + 2 * NEAR64_ETAB);
+}
 
 void Geometry::upload(cudaStream_t s) {
-  dd_exp.upload(exp_tables().dd, s);
-  near_exp.upload(exp_tables().near, s);
-  near_exp64.upload(exp_tables().near64, s);
+  exp_tab.upload(exp_tables(), s);
   items.upload(h_items, s);
   item_split.upload(h_item_split, s);
   leaf_nslot.upload(h_leaf_nslot, s);
@@ -732,8 +736,11 @@ void Geometry::upload(cudaStream_t s) {
   pos64.upload(h_pos64, s);
   hi32.upload(h_hi, s);
   lo32.upload(h_lo, s);
-  mid32.upload(h_mid, s);
-  low32.upload(h_low, s);
+  fine32.alloc(2 * (size_t)n);
+  if (n) {
+    CG_CUDA(cudaMemcpyAsync(fine32.p, h_mid.data(), n * sizeof(float4), cudaMemcpyHostToDevice, s));
+    CG_CUDA(cudaMemcpyAsync(fine32.p + n, h_low.data(), n * sizeof(float4), cudaMemcpyHostToDevice, s));
+  }
   corr_ptr.upload(h_cptr, s);
   corr_idx.upload(h_cidx.empty() ? std::vector<int>{0} : h_cidx, s);
   CG_CUDA(cudaStreamSynchronize(s));
@@ -1768,6 +1775,8 @@ __device__ __forceinline__ void dd2_pair_tensor(const dd2& tx, const dd2& ty, co
     S.s            = t;
   };
   square(x), square(y), square(z);
+  // (within a step or two of the coordinate grid the low parts may be the larger ones:
+  // R^2 then has FP32's bits, as the separations do)
   const dd2 r2   = dd2_fast_two_sum(psub(S.s, C), S.l);
   const bool okx = r2.h.x > 0.f, oky = r2.h.y > 0.f;  // false: a site paired with itself
   // y = 1/R in FP32 and h = R^2 y^2 - 1 (|h| < 2^-21), y^2 split by an FMA
@@ -2898,7 +2907,7 @@ static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, doubl
       const int nr = std::min(P2PM_MAXR, g.ncopies - c0);
       kern<<<mg, P2P_BLOCK, P2PM_DD_SMEM, s>>>(
             g.n, g.leaf_start.p, g.mitems.p, g.mitem_split.p, g.mitem_stride.p, c0, nr,
-            g.p2p_src.p, pos_args<float>(g), w.dd_src.p, g.dd_exp.p, damping, lim, w.Fnear.p);
+            g.p2p_src.p, pos_args<float>(g), w.dd_src.p, g.exp_dd(), damping, lim, w.Fnear.p);
       CG_LAUNCH();
     }
     return;
@@ -2907,11 +2916,11 @@ static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, doubl
   if (damp)
     k_p2p_dd2<true><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
                                                g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                               g.dd_exp.p, damping, lim, w.Fnear.p);
+                                               g.exp_dd(), damping, lim, w.Fnear.p);
   else
     k_p2p_dd2<false><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
                                                 g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                                g.dd_exp.p, damping, lim, w.Fnear.p);
+                                                g.exp_dd(), damping, lim, w.Fnear.p);
   CG_LAUNCH();
 }
 
@@ -2920,11 +2929,11 @@ static void launch_p2p64(const Geometry& g, int m, bool damp, const double* src,
   const int grid  = (int)g.h_items.size();
   const int* lseg = seg_done ? g.leaf_seg.p : nullptr;
   if (seg_done && !lseg) fail(CPPE_GPU_INVALID_ARG, "segment mask without segments");
-  const Pos3 ps{g.hi32.p, g.mid32.p, g.low32.p};
+  const Pos3 ps{g.hi32.p, g.fine32.p, g.fine32.p + g.n};
   auto run = [&](auto order, auto d) {
     k_p2p64<decltype(order)::value, decltype(d)::value><<<grid, P2P_BLOCK, 0, s>>>(
-          g.n, g.leaf_start.p, g.items.p, g.p2p_src.p, ps, g.pos64.p, src, g.near_exp.p,
-          g.near_exp64.p, damping, g.corr_ptr.p, g.corr_idx.p, Fnear, lseg, seg_done);
+          g.n, g.leaf_start.p, g.items.p, g.p2p_src.p, ps, g.pos64.p, src, g.exp_dd(),
+          g.exp_tab.p, damping, g.corr_ptr.p, g.corr_idx.p, Fnear, lseg, seg_done);
   };
   const std::integral_constant<int, 1> dip{};
   const std::integral_constant<int, 2> quad{};

@@ -100,17 +100,16 @@ struct Geometry {
   DBuf<double4_32a> pos64;
   DBuf<float4> hi32, lo32;
   // the FP64 operator's three-part coordinates: hi32 plus the remainder on a
-  // finer grid (mid32) plus what is left (low32; w: s - float(s)), and the
-  // tables of e^-(k/16) of its Thole factors (near64.cuh)
+  // finer grid (fine32) plus what is left (the n entries after; w: s - float(s))
   std::vector<float4> h_mid, h_low;
-  DBuf<float4> mid32, low32;
-  DBuf<float2> near_exp;
-  DBuf<double> near_exp64;
+  DBuf<float4> fine32;
+  // tables of e^-(k/16): in FP64, value and rest, then as double-float pairs (exp_dd)
+  DBuf<double> exp_tab;
+  const float2* exp_dd() const;
   double grid = 0.0;    // spacing of hi32's grid (bohr)
   // sums of R^-6 (dipoles) and R^-8 (quadrupoles) over the near-field pairs beyond
   // the FP64 operator's double-float limits, relative to those within them
   double far_share[2] = {0.0, 0.0};
-  DBuf<float2> dd_exp;  // e^-(k/16), k = 0..320, as double-float pairs
   // pairs the reference skips (exclusions) that the near-field pass computed
   DBuf<int> corr_ptr, corr_idx;
   long near_pairs = 0;  // ordered pairs evaluated by the near-field pass
