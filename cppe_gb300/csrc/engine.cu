@@ -2891,6 +2891,7 @@ __global__ void k_split_dd(long n, const double* __restrict__ in, float2* __rest
   out[i]         = make_float2(h, (float)(v - (double)h));
 }
 
+constexpr int P2P_DD_SHARE = 32 * 1024;  // unused shared memory of k_p2p_dd2 (see its launch)
 static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, double damping,
                           FieldWork<double>& w, cudaStream_t s) {
   const long n3   = 3L * g.n;
@@ -2913,14 +2914,19 @@ static void launch_p2p_dd(const Geometry& g, bool damp, const double* src, doubl
     return;
   }
   const int grid = (int)g.h_items.size();
-  if (damp)
-    k_p2p_dd2<true><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
-                                               g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                               g.exp_dd(), damping, lim, w.Fnear.p);
-  else
-    k_p2p_dd2<false><<<grid, P2P_BLOCK, 0, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p,
-                                                g.p2p_src.p, pos_args<float>(g), w.dd_src.p,
-                                                g.exp_dd(), damping, lim, w.Fnear.p);
+  auto kern      = damp ? k_p2p_dd2<true> : k_p2p_dd2<false>;
+  // Four blocks an SM take all of its registers, and with a few items an SM they all
+  // start at once: the far field beside them, the longer path of small systems, waited
+  // for them kernel by kernel.  Up to 16 items an SM, shared memory for three: 1,440
+  // sites order 5 116 -> 104 us an apply (108 with a sixth of the items, before small
+  // systems had smaller ones), 2,100 129 -> 109, 3,900 192 -> 168, 6,000 197 -> 186;
+  // two blocks lose a little of that again.
+  const int smem = g.fmm && grid <= 16 * 152 ? P2P_DD_SHARE : 0;
+  if (smem)
+    CG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<grid, P2P_BLOCK, smem, s>>>(g.n, g.leaf_start.p, g.items.p, g.item_split.p, g.p2p_src.p,
+                                     pos_args<float>(g), w.dd_src.p, g.exp_dd(), damping, lim,
+                                     w.Fnear.p);
   CG_LAUNCH();
 }
 
