@@ -75,7 +75,8 @@ typedef struct {
   int tree_expansion_order;  /* PeOptions::tree_expansion_order  (default 5)   */
   double theta;              /* PeOptions::theta                 (default 0.5) */
   int damp;                  /* PeOptions::damp_induced          (default 0)   */
-  double damping_factor;     /* PeOptions::damping_factor_induced (2.1304)     */
+  double damping_factor;     /* PeOptions::damping_factor_induced (2.1304);
+                                not positive: no damping                       */
   double induced_thresh;     /* PeOptions::induced_thresh        (1e-8)        */
   int maxiter;               /* PeOptions::maxiter               (50)          */
   int precision;             /* CPPE_GPU_FP64 or CPPE_GPU_MIXED                */
